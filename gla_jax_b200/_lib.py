@@ -56,6 +56,9 @@ SIGNATURES = {
                                 c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t]),
     "gla_recurrent_fwd": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int]),
+    "gla_recurrent_fwd_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64, c_int64, c_int]),
+    "gla_recurrent_fwd_ws": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p,
+                                     c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_size_t]),
     "gla_decode_step": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_int]),
     "gla_layer_gate_fwd": (c_int, [c_void_p, c_int64, c_int, c_void_p, ctypes.c_float, c_void_p]),

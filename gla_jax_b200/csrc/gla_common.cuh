@@ -106,6 +106,15 @@ int simt_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, 
 int simt_chunk_dstate_only(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int bf,
                            const float* g, const void* q, const void* dout, float* dS_local, void* ws);
 
+// float32-precision chunk path on the tensor cores (head sizes 32, 64, 128; any number of tokens), gla_split.cu.
+bool px_supported(int64_t D);
+size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D);
+int px_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
+           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int reverse, const char* label = "px_fwd_kernel");
+int px_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
+           const void* v, const void* k, const void* q, const void* dhidden_final, const void* dout, int do_bf,
+           void* dhidden_init, float* dg, void* dv, void* dk, void* dq, void* states, int have_states, void* ws, int reverse);
+
 // tcgen05 tensor-core chunk path (bf16, D = 128 or 256, chunk a multiple of 128).
 bool tc_supported(int64_t D, int64_t C, int dtype);
 bool tc_supported_local_state(int64_t D, int64_t C, int dtype);
@@ -150,9 +159,10 @@ int launch_sp_combine(cudaStream_t st, int64_t R, int64_t rank, int64_t BH, int6
 int launch_sp_combine2(cudaStream_t st, int64_t R, int64_t rank, int64_t BH, int64_t D, const float* all_G, int64_t gstride,
                        const float* all_S, int64_t sstride, const void* init, int init_bf16, float* entering, void* total,
                        int total_bf16, int reverse);
+size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D);
 int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, void* hidden_final, void* out,
-                  int out_bf, int reverse);
+                  int out_bf, int reverse, void* ws = nullptr, size_t ws_bytes = 0);
 size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D);
 int recurrent_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, const void* dhidden_final,

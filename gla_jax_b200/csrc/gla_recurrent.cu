@@ -25,6 +25,7 @@
 // during the current block's arithmetic.  dlog_fgate follows gla.py:263:
 //   dg = cumsum over the remaining tokens of (q dq - k dk) + sum_v(dS_T * S_T).
 #include "gla_common.cuh"
+#include <initializer_list>
 
 namespace gla {
 
@@ -446,9 +447,23 @@ static int launch_rec_bwd(cudaStream_t st, const RecParams& p) {
 static int launch_rec_fwd_d(cudaStream_t st, int D, const RecParams& p) { REC_DISPATCH_D(launch_rec_fwd, st, D, p) }
 static int launch_rec_bwd_d(cudaStream_t st, int D, const RecParams& p) { REC_DISPATCH_D(launch_rec_bwd, st, D, p) }
 
+// The chunked form (gla_split.cu) serves sequences of more than a chunk or so; below that the walk over the tokens here
+// is one launch instead of three.  Its vector accesses need aligned arrays; the walk's need less.
+constexpr int64_t REC_CHUNKED_MIN_T = 48;
+static bool rec_chunked(int64_t T, int64_t D) { return px_supported(D) && T >= REC_CHUNKED_MIN_T; }
+static bool rec_aligned(std::initializer_list<const void*> ps) {
+  for (const void* p : ps) if (!aligned16(p)) return false;
+  return true;
+}
+size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
+  return rec_chunked(T, D) ? px_state_bytes(B, T, H, D) : 0;
+}
+
 int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, void* hidden_final, void* out,
-                  int out_bf, int reverse) {
+                  int out_bf, int reverse, void* ws, size_t ws_bytes) {
+  if (ws != nullptr && rec_chunked(T, D) && ws_bytes >= px_state_bytes(B, T, H, D) && rec_aligned({hidden_init, g, v, k, q, hidden_final, out, ws}))
+    return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, out_bf, ws, reverse);
   RecParams p{};
   p.B = B; p.T = T; p.H = H; p.bf = bf; p.out_bf = out_bf;
   p.hidden_init = hidden_init; p.g = g; p.v = v; p.k = k; p.q = q;
@@ -457,14 +472,19 @@ int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, i
 }
 
 size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
-  return 2 * align_up((size_t)B * T * H * D * 4, 256) + align_up((size_t)B * H * D * 4, 256) +
-         align_up(cumsum_scratch_bytes(B, T, H * D), 256);
+  const size_t n = 2 * align_up((size_t)B * T * H * D * 4, 256) + align_up((size_t)B * H * D * 4, 256) +
+                   align_up(cumsum_scratch_bytes(B, T, H * D), 256);
+  const size_t px = rec_chunked(T, D) ? 2 * px_state_bytes(B, T, H, D) : 0;      // states and gradient states
+  return px > n ? px : n;
 }
 
 int recurrent_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, const void* dhidden_final,
                   const void* dout, int do_bf, void* dhidden_init, float* dg, void* dv, void* dk, void* dq,
                   int reverse, void* ws) {
+  if (rec_chunked(T, D) && rec_aligned({hidden_init, g, v, k, q, dhidden_final, dout, dhidden_init, dg, dv, dk, dq, ws}))
+    return px_bwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, dhidden_final, dout, do_bf, dhidden_init, dg, dv, dk, dq, ws, 0,
+                  (char*)ws + px_state_bytes(B, T, H, D), reverse);
   RecParams p{};
   p.B = B; p.T = T; p.H = H; p.bf = bf; p.do_bf = do_bf;
   p.hidden_init = hidden_init; p.g = g; p.v = v; p.k = k; p.q = q;

@@ -1,0 +1,962 @@
+// Chunked GLA in float32 precision on the tensor cores: forward and backward for float32 callers, for head sizes
+// that the 128-wide kernels do not serve, and for recurrent_gla over any number of tokens.
+//
+// Reference algorithm: gla.py:483-625 (chunk forward / backward), gla.py:26-47 and 172-269 (the recurrence, which the
+// chunked form equals for any chunk length).
+//
+// Why split operands.  These paths used to run on float32 FMAs (one SGEMM launch per product, or one FMA chain per
+// token), which the CUDA cores bound.  A float32 number is the sum of three bf16 numbers (8 + 8 + 8 significant
+// bits), so a float32 product is six bf16 products (the terms below 2^-24 dropped), three when the other side is
+// bf16 data already, one when both are; the accumulation is float32 throughout.  That is the precision of the FMA
+// form at 1/6 to 1/1 of the tensor rate, several times the FMA rate.  The instruction is the register-operand
+// mma.sync: chunks of 64 rows with every operand three planes deep leave room for two blocks per SM at head size 64
+// (tcgen05's 128-row tiles of three planes leave it for one, with nothing to run beside its serial phases), and the
+// planes need no canonical layout, so that rows, columns and lengths come in any multiple of 16.
+//
+// One anchor per chunk.  lam = running sum of the log gates inside the chunk, G = its total.  With m = G / 2 per
+// feature, q~ = q exp(lam - m) and k~ = k exp(m - lam) give every product of the chunk:
+//   P = tril(q~ k~^T)                      O  = P V + q~ (e^m S)
+//   dq = exp(lam - m) (dP k~ + dO (e^m S)^T)   dk = exp(m - lam) (dP^T q~ + V (e^m dS)^T)
+//   dV = P^T dO + k~ (e^m dS)              dP = tril(dO V^T)
+// (S: the state entering the chunk, dS: the gradient of the state leaving it; the factor e^m rides on the rows of
+// the state while they are split.)  The weights stay within exp(+-LIMIT / 2) as long as sum |g| <= LIMIT over the
+// chunk and no single |g| exceeds ONE_GATE (the weights are running products of exp(g), which must not vanish); chunks beyond that ("sharp") take
+// the weights anchored at the chunk's ends for the state products and form the scores and their gradients pair by
+// pair with the exponent lam_i - lam_j, in float32.
+//
+// Three launches forward, three backward: per-chunk state products (k^^T V, resp. q^^T dO), a scan over the chunks
+// in place, and the chunk kernel.  States are float32, N + 1 of them per head (slot n enters chunk n; slot N is the
+// final state; gradient states: slot n + 1 leaves chunk n, slot 0 is the gradient of the initial state), so that
+//   dG_n[d] = <S_{n+1}[d,:], dS_n[d,:]>
+// is a dot product of two stored rows and dlam = q dq - k dk needs no other inter-chunk term.
+#include "gla_common.cuh"
+#include "tc_ptx.cuh"
+#include "tma_maps.cuh"
+
+namespace gla {
+
+using namespace tc;
+
+namespace {
+
+constexpr float PX_LIMIT = 140.f;
+constexpr float PX_ONE_GATE = 60.f;
+constexpr float PX_GATE_FLOOR = -1000.f;      // exp() is zero far above this; a gate of -inf must not make inf - inf
+
+// D features, chunks of L rows.  Element-wise stages: a thread owns a column pair and RPT consecutive rows.  Products:
+// warps in WR row groups of 16 x WC column groups.
+template <int D_, int L_>
+struct Px {
+  static constexpr int D = D_, L = L_;
+  static constexpr int NT = D >= 128 && L == 64 ? 512 : D >= 64 ? 256 : 128;
+  static constexpr int CP = D / 2, RG = NT / CP, RPT = L / RG;
+  static constexpr int WR = L / 16, WC = (NT / 32) / WR, CW = D / WC;
+  static constexpr int NB = (WR + WC - 1) / WC;  // 16 x 16 score blocks per warp, at most
+  static constexpr int LD = 2 * D + 16;          // row pitch in bytes: the 16-byte pad spreads ldmatrix rows over the banks
+  static constexpr int PLANE = L * LD;
+  static constexpr int PW = D < 64 ? D : 64, NP = D / PW, PC = PW / WC;   // state pieces of PW value columns, PC per warp
+  static constexpr int LDS = 2 * PW + 16, SPLANE = D * LDS;
+  static constexpr int LDT = 2 * L + 16, TPLANE = L * LDT;                // score tile
+  static constexpr int SREG = D * PW / 4 / NT;   // float4 loads per thread and state piece
+  static constexpr int AP = D + 8;               // row pitch (floats) of the float32 tiles of the closing pass
+  static_assert(PC % 16 == 0 && CW % 16 == 0, "a warp's columns come in pairs of 8-wide tiles");
+};
+
+struct PxParams {
+  int64_t B, T, H, N;
+  int trev;                     // tokens in reverse order (recurrent_gla(reverse=True))
+  int out_bf, in_bf;
+  const float* g;
+  const void *v, *k, *q, *dout;
+  float *S, *dS;                // (B H, N + 1, D, D)
+  float* eG;                    // (B H, N, D): exp of every chunk's total log decay
+  void *out, *dq, *dk, *dv;
+  float* dg;
+  const char* label;            // name of the forward chunk kernel in launch profiles
+};
+
+// ---- operands --------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void hmma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// x = hi + mid + lo, eight significant bits each (two values side by side)
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&s)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    s[i] = pack_bf16x2(x, y);
+    if (i < 2) {
+      x -= __uint_as_float(s[i] << 16);
+      y -= __uint_as_float(s[i] & 0xffff0000u);
+    }
+  }
+}
+__device__ __forceinline__ void st_split3(uint8_t* p, uint32_t plane, float x, float y) {
+  uint32_t s[3];
+  split3(x, y, s);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(p + i * plane) = s[i];
+}
+__device__ __forceinline__ void st_split3(uint8_t* p, uint32_t plane, float4 v) {
+  uint32_t a[3], b[3];
+  split3(v.x, v.y, a);
+  split3(v.z, v.w, b);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(p + i * plane) = make_uint2(a[i], b[i]);
+}
+// A operand (16 rows x 16 of K) of NS planes, stored row-major [m][k] ...
+template <int NS>
+__device__ __forceinline__ void ld_a(uint32_t (&a)[NS][4], uint32_t base, uint32_t plane, uint32_t ld, int m0, int k0, int lane) {
+  const uint32_t addr = base + (uint32_t)(m0 + (lane & 15)) * ld + (uint32_t)(k0 + (lane >> 4) * 8) * 2;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) ldsm4(a[s], addr + s * plane);
+}
+// ... or [k][m]
+template <int NS>
+__device__ __forceinline__ void ld_a_t(uint32_t (&a)[NS][4], uint32_t base, uint32_t plane, uint32_t ld, int m0, int k0, int lane) {
+  const uint32_t addr = base + (uint32_t)(k0 + (lane & 7) + ((lane >> 4) & 1) * 8) * ld + (uint32_t)(m0 + ((lane >> 3) & 1) * 8) * 2;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) ldsm4t(a[s], addr + s * plane);
+}
+// c[2 NQ tiles of 8 columns] += A B over 16 of K.  B is stored [n][k] (BT = false) or [k][n] (BT = true).  Products of
+// planes sa and sb with sa + sb > 2 lie below 2^-24 of the result and are left out; the small ones come first.
+template <int NSA, int NSB, int NQ, bool BT>
+__device__ __forceinline__ void mma_step(float (*c)[4], const uint32_t (&a)[NSA][4], uint32_t base, uint32_t plane,
+                                         uint32_t ld, int n0, int k0, int lane) {
+  const int r8 = lane & 7, h3 = (lane >> 3) & 1, h4 = (lane >> 4) & 1;
+#pragma unroll
+  for (int j = 0; j < NQ; ++j) {
+    const int n = n0 + 16 * j;
+    const uint32_t addr = BT ? base + (uint32_t)(k0 + r8 + 8 * h3) * ld + (uint32_t)(n + 8 * h4) * 2
+                             : base + (uint32_t)(n + r8 + 8 * h4) * ld + (uint32_t)(k0 + 8 * h3) * 2;
+    uint32_t b[NSB][4];
+#pragma unroll
+    for (int s = 0; s < NSB; ++s) {
+      if (BT) ldsm4t(b[s], addr + s * plane); else ldsm4(b[s], addr + s * plane);
+    }
+#pragma unroll
+    for (int t = 2; t >= 0; --t)
+#pragma unroll
+      for (int sa = 0; sa < NSA; ++sa) {
+        const int sb = t - sa;
+        if (sb >= 0 && sb < NSB) {
+          hmma(c[2 * j], a[sa], b[sb][0], b[sb][1]);
+          hmma(c[2 * j + 1], a[sa], b[sb][2], b[sb][3]);
+        }
+      }
+  }
+}
+template <typename TI> struct Pair;
+template <> struct Pair<bf16> {
+  uint32_t u;
+  __device__ __forceinline__ void load(const void* p, int64_t e) { u = __ldg(reinterpret_cast<const unsigned int*>((const bf16*)p + e)); }
+  __device__ __forceinline__ void zero() { u = 0u; }
+  __device__ __forceinline__ float2 get() const { return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+};
+template <> struct Pair<float> {
+  float2 u;
+  __device__ __forceinline__ void load(const void* p, int64_t e) { u = __ldg(reinterpret_cast<const float2*>((const float*)p + e)); }
+  __device__ __forceinline__ void zero() { u = make_float2(0.f, 0.f); }
+  __device__ __forceinline__ float2 get() const { return u; }
+};
+template <typename TI> constexpr int planes_of() { return sizeof(TI) == 2 ? 1 : 3; }
+
+// Where a chunk's rows lie.
+template <class C>
+struct ChunkAt {
+  int64_t n, bh, row0;
+  int step, nv;                 // elements from row to row (negative in reverse), rows inside the sequence
+  __device__ __forceinline__ ChunkAt(const PxParams& p, int64_t blk) {
+    n = blk % p.N; bh = blk / p.N;
+    const int64_t b = bh / p.H, h = bh % p.H;
+    const int64_t t0 = n * C::L, left = p.T - t0;
+    step = (int)(p.H * C::D);
+    row0 = ((b * p.T + (p.trev ? p.T - 1 - t0 : t0)) * p.H + h) * C::D;
+    if (p.trev) step = -step;
+    nv = left < C::L ? (int)left : C::L;
+  }
+  __device__ __forceinline__ int64_t row(int r) const { return row0 + (int64_t)r * step; }
+};
+__device__ __forceinline__ float clamp_gate(float g) { return g < PX_GATE_FLOOR ? PX_GATE_FLOOR : g; }      // NaN stays
+template <class C>
+__device__ __forceinline__ void load_gates(float2 (&g)[C::RPT], const float* gp, const ChunkAt<C>& at, int r0, int cp) {
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i)
+    g[i] = r0 + i < at.nv ? __ldg(reinterpret_cast<const float2*>(gp + at.row(r0 + i) + 2 * cp)) : make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i) g[i] = make_float2(clamp_gate(g[i].x), clamp_gate(g[i].y));
+}
+template <class C, typename TI>
+__device__ __forceinline__ void load_pairs(Pair<TI> (&x)[C::RPT], const void* xp, const ChunkAt<C>& at, int r0, int cp) {
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i)
+    if (r0 + i < at.nv) x[i].load(xp, at.row(r0 + i) + 2 * cp); else x[i].zero();
+}
+// A chunk of v or dO into planes (row-major, pitch LD)
+template <class C, typename TI>
+__device__ __forceinline__ void copy_rows(uint8_t* dst, const void* src, const ChunkAt<C>& at) {
+  if constexpr (sizeof(TI) == 2) {
+#pragma unroll
+    for (int j = 0; j < C::L * C::D / 8 / C::NT; ++j) {
+      const int id = threadIdx.x + C::NT * j, r = id / (C::D / 8), c = id % (C::D / 8);
+      uint4 u = make_uint4(0u, 0u, 0u, 0u);
+      if (r < at.nv) u = __ldg(reinterpret_cast<const uint4*>((const bf16*)src + at.row(r) + c * 8));
+      *reinterpret_cast<uint4*>(dst + r * C::LD + c * 16) = u;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < C::L * C::D / 4 / C::NT; ++j) {
+      const int id = threadIdx.x + C::NT * j, r = id / (C::D / 4), c = id % (C::D / 4);
+      float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < at.nv) u = __ldg(reinterpret_cast<const float4*>((const float*)src + at.row(r) + c * 4));
+      st_split3(dst + r * C::LD + c * 8, C::PLANE, u);
+    }
+  }
+}
+// Gate sums of the thread's rows, exchanged between the row groups: sums before the thread's rows, of the whole chunk,
+// and whether the chunk needs the pairwise form.  seg: [RG][D], sab: [RG][D] floats.
+template <class C>
+__device__ __forceinline__ bool gate_sums(const float2 (&g)[C::RPT], float* seg, float* sab, int rg, int cp,
+                                          float2& before, float2& own, float2& total) {
+  float2 s = make_float2(0.f, 0.f), a = s;
+  bool big = false;
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i) {
+    s.x += g[i].x; s.y += g[i].y;
+    a.x += fabsf(g[i].x); a.y += fabsf(g[i].y);
+    big = big || !(fabsf(g[i].x) <= PX_ONE_GATE) || !(fabsf(g[i].y) <= PX_ONE_GATE);
+  }
+  *reinterpret_cast<float2*>(seg + rg * C::D + 2 * cp) = s;
+  *reinterpret_cast<float2*>(sab + rg * C::D + 2 * cp) = a;
+  __syncthreads();
+  own = s; before = total = make_float2(0.f, 0.f); a = before;
+#pragma unroll
+  for (int r = 0; r < C::RG; ++r) {
+    const float2 t = *reinterpret_cast<const float2*>(seg + r * C::D + 2 * cp);
+    const float2 u = *reinterpret_cast<const float2*>(sab + r * C::D + 2 * cp);
+    if (r < rg) { before.x += t.x; before.y += t.y; }
+    total.x += t.x; total.y += t.y;
+    a.x += u.x; a.y += u.y;
+  }
+  return __syncthreads_or(big || !(a.x <= PX_LIMIT) || !(a.y <= PX_LIMIT)) != 0;
+}
+
+// ---- per-chunk state products ----------------------------------------------------------------------------------------
+// MODE 0: S slot n + 1 = k^^T V, k^ = k exp(G - lam);  MODE 1: dS slot n = q^^T dO, q^ = q exp(lam).  The weights are
+// anchored at the chunk's ends here and never exceed one for log gates <= 0.  Also leaves exp(G).
+template <class C, typename TI, typename TY, int MODE>
+__global__ void __launch_bounds__(C::NT) px_product_kernel(PxParams p) {
+  constexpr int NSY = planes_of<TY>();
+  extern __shared__ __align__(16) uint8_t sm[];
+  uint8_t* sX = sm;
+  uint8_t* sY = sm + 3 * C::PLANE;
+  float* seg = reinterpret_cast<float*>(sY + NSY * C::PLANE);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
+  const ChunkAt<C> at(p, blockIdx.x);
+  float2 g[C::RPT];
+  Pair<TI> x[C::RPT];
+  load_gates<C>(g, p.g, at, r0, cp);
+  load_pairs<C, TI>(x, MODE == 0 ? p.k : p.q, at, r0, cp);
+  copy_rows<C, TY>(sY, MODE == 0 ? p.v : p.dout, at);
+  float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i) { s.x += g[i].x; s.y += g[i].y; }
+  *reinterpret_cast<float2*>(seg + rg * C::D + 2 * cp) = s;
+  __syncthreads();
+  float2 side = make_float2(0.f, 0.f), total = side;        // gates after (MODE 0) or before (MODE 1) the thread's rows
+#pragma unroll
+  for (int r = 0; r < C::RG; ++r) {
+    const float2 t = *reinterpret_cast<const float2*>(seg + r * C::D + 2 * cp);
+    if (MODE == 0 ? r > rg : r < rg) { side.x += t.x; side.y += t.y; }
+    total.x += t.x; total.y += t.y;
+  }
+  float2 run = make_float2(expf(side.x), expf(side.y));
+  if (rg == 0) *reinterpret_cast<float2*>(p.eG + (at.bh * p.N + at.n) * C::D + 2 * cp) = make_float2(expf(total.x), expf(total.y));
+  if (MODE == 0) {
+#pragma unroll
+    for (int i = C::RPT - 1; i >= 0; --i) {
+      const float2 v = x[i].get();
+      st_split3(sX + (r0 + i) * C::LD + cp * 4, C::PLANE, v.x * run.x, v.y * run.y);
+      run.x *= expf(g[i].x); run.y *= expf(g[i].y);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < C::RPT; ++i) {
+      const float2 v = x[i].get();
+      run.x *= expf(g[i].x); run.y *= expf(g[i].y);
+      st_split3(sX + (r0 + i) * C::LD + cp * 4, C::PLANE, v.x * run.x, v.y * run.y);
+    }
+  }
+  __syncthreads();
+  constexpr int WM = C::D / 16, WN = (C::NT / 32) / WM, NW = C::D / WN;       // warps over key rows, value columns per warp
+  static_assert(WM * WN == C::NT / 32, "warps must tile the state");
+  const int m0 = 16 * (warp % WM), c0 = NW * (warp / WM);
+  float acc[NW / 8][4];
+#pragma unroll
+  for (int j = 0; j < NW / 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+  const uint32_t aX = smem_u32(sX), aY = smem_u32(sY);
+#pragma unroll 2
+  for (int ks = 0; ks < C::L / 16; ++ks) {
+    uint32_t a[3][4];
+    ld_a_t<3>(a, aX, C::PLANE, C::LD, m0, 16 * ks, lane);
+    mma_step<3, NSY, NW / 16, true>(acc, a, aY, C::PLANE, C::LD, c0, 16 * ks, lane);
+  }
+  float* o = (MODE == 0 ? p.S : p.dS) + (at.bh * (p.N + 1) + at.n + (MODE == 0 ? 1 : 0)) * C::D * C::D;
+#pragma unroll
+  for (int j = 0; j < NW / 8; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      *reinterpret_cast<float2*>(o + (m0 + (lane >> 2) + 8 * h) * C::D + c0 + 8 * j + 2 * (lane & 3)) =
+          make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
+}
+
+// ---- scan over the chunks, in place --------------------------------------------------------------------------------------
+// mode 0: slot 0 = init, slot n + 1 = eG_n slot n + slot n + 1;  mode 1: slot N = init, slot n = eG_n slot n + 1 + slot n.
+// One thread per four value columns; eight chunks' loads in flight (the chain itself is one FMA per chunk).
+template <typename TS>
+__global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, int64_t N, const float* __restrict__ eG,
+                                                      const TS* __restrict__ init, float* S, TS* __restrict__ fin, int mode) {
+  constexpr int AHEAD = 8;
+  const int64_t e4 = (int64_t)blockIdx.x * 128 + threadIdx.x, DD = D * D;
+  if (e4 * 4 >= total) return;
+  const int64_t bh = e4 * 4 / DD, e = e4 * 4 % DD, dk = e / D;
+  float* sp = S + bh * (N + 1) * DD + e;
+  const float* gp = eG + bh * N * D + dk;
+  float4 s;
+  s.x = ld_f(init, bh * DD + e); s.y = ld_f(init, bh * DD + e + 1); s.z = ld_f(init, bh * DD + e + 2); s.w = ld_f(init, bh * DD + e + 3);
+  *reinterpret_cast<float4*>(sp + (mode ? N : 0) * DD) = s;
+  float4 x[AHEAD];
+  float f[AHEAD];
+  auto fetch = [&](int64_t i, int u) {
+    const int64_t n = mode ? N - 1 - i : i;
+    x[u] = *reinterpret_cast<const float4*>(sp + (mode ? n : n + 1) * DD);
+    f[u] = __ldg(gp + n * D);
+  };
+#pragma unroll
+  for (int u = 0; u < AHEAD; ++u) if (u < N) fetch(u, u);
+  for (int64_t i0 = 0; i0 < N; i0 += AHEAD) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int64_t i = i0 + u;
+      if (i < N) {
+        const int64_t n = mode ? N - 1 - i : i;
+        s = make_float4(fmaf(f[u], s.x, x[u].x), fmaf(f[u], s.y, x[u].y), fmaf(f[u], s.z, x[u].z), fmaf(f[u], s.w, x[u].w));
+        *reinterpret_cast<float4*>(sp + (mode ? n : n + 1) * DD) = s;
+        if (i + AHEAD < N) fetch(i + AHEAD, u);
+      }
+    }
+  }
+  if (fin != nullptr) {
+    st_f(fin, bh * DD + e, s.x); st_f(fin, bh * DD + e + 1, s.y); st_f(fin, bh * DD + e + 2, s.z); st_f(fin, bh * DD + e + 3, s.w);
+  }
+}
+
+// ---- pieces of the chunk kernels -------------------------------------------------------------------------------------------
+// q~ and k~ (mild chunk), or q^ = q exp(lam) and k^ = k exp(G - lam) (sharp chunk) as split planes; em[d] = the factor
+// that the rows of the states take.
+template <class C, typename TI>
+__device__ __forceinline__ void build_qk(uint8_t* sQ, uint8_t* sK, float* em, float2 (&g)[C::RPT], const Pair<TI> (&q)[C::RPT],
+                                         const Pair<TI> (&k)[C::RPT], bool sharp, float2 before, float2 own, float2 total,
+                                         int rg, int cp) {
+  const int r0 = rg * C::RPT;
+  const float2 half = sharp ? make_float2(0.f, 0.f) : make_float2(0.5f * total.x, 0.5f * total.y);
+  if (rg == 0) *reinterpret_cast<float2*>(em + 2 * cp) = make_float2(expf(half.x), expf(half.y));
+  float2 run = make_float2(expf(before.x - half.x), expf(before.y - half.y));
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i) {
+    g[i] = make_float2(expf(g[i].x), expf(g[i].y));
+    run.x *= g[i].x; run.y *= g[i].y;
+    const float2 x = q[i].get();
+    st_split3(sQ + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
+  }
+  if (sharp) run = make_float2(expf(total.x - before.x - own.x), expf(total.y - before.y - own.y));
+  else run = make_float2(1.f / run.x, 1.f / run.y);
+#pragma unroll
+  for (int i = C::RPT - 1; i >= 0; --i) {
+    const float2 x = k[i].get();
+    st_split3(sK + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
+    run.x *= g[i].x; run.y *= g[i].y;
+  }
+}
+// Value columns [PW pc, PW pc + PW) of a state (float32, D x D), rows scaled by em, as split planes.
+template <class C>
+__device__ __forceinline__ void fetch_piece(float4 (&x)[C::SREG], const float* st, int pc) {
+#pragma unroll
+  for (int j = 0; j < C::SREG; ++j) {
+    const int id = threadIdx.x + C::NT * j, r = id / (C::PW / 4), c = id % (C::PW / 4);
+    x[j] = *reinterpret_cast<const float4*>(st + r * C::D + pc * C::PW + c * 4);
+  }
+}
+template <class C>
+__device__ __forceinline__ void store_piece(uint8_t* dst, const float4 (&x)[C::SREG], const float* em) {
+#pragma unroll
+  for (int j = 0; j < C::SREG; ++j) {
+    const int id = threadIdx.x + C::NT * j, r = id / (C::PW / 4), c = id % (C::PW / 4);
+    const float w = em[r];
+    st_split3(dst + r * C::LDS + c * 8, C::SPLANE, make_float4(x[j].x * w, x[j].y * w, x[j].z * w, x[j].w * w));
+  }
+}
+// lam of the chunk, float32, [L][D]
+template <class C>
+__device__ __forceinline__ void store_lam(float* lam, const float* gp, const ChunkAt<C>& at, float2 before, int rg, int cp) {
+  float2 run = before;
+#pragma unroll 1
+  for (int i = 0; i < C::RPT; ++i) {
+    const int r = rg * C::RPT + i;
+    float2 x = make_float2(0.f, 0.f);
+    if (r < at.nv) x = __ldg(reinterpret_cast<const float2*>(gp + at.row(r) + 2 * cp));
+    run.x += clamp_gate(x.x); run.y += clamp_gate(x.y);
+    *reinterpret_cast<float2*>(lam + r * C::D + 2 * cp) = run;
+  }
+}
+// A 16 x 16 block of P = tril(q~ k~^T) of a sharp chunk, pair by pair: rows m0 + lane / 4 (+ 8), columns c0 + 8 j +
+// 2 (lane % 4) (+ 1), the accumulator layout.
+template <class C, typename TI>
+__device__ __noinline__ void block_by_pair(float (*acc)[4], const float* lam, const void* q, const void* k,
+                                           const ChunkAt<C>& at, int m0, int c0, int lane) {
+  const int ra = m0 + (lane >> 2), rb = ra + 8;
+#pragma unroll 1
+  for (int d = 0; d < C::D; ++d) {
+    const float qa = ra < at.nv ? ld_f((const TI*)q, at.row(ra) + d) : 0.f, qb = rb < at.nv ? ld_f((const TI*)q, at.row(rb) + d) : 0.f;
+    const float la = lam[ra * C::D + d], lb = lam[rb * C::D + d];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 8 * j + 2 * (lane & 3) + e;
+        const float y = c < at.nv ? ld_f((const TI*)k, at.row(c) + d) : 0.f, lc = lam[c * C::D + d];
+        if (c <= ra) acc[j][e] = fmaf(qa * y, expf(la - lc), acc[j][e]);
+        if (c <= rb) acc[j][2 + e] = fmaf(qb * y, expf(lb - lc), acc[j][2 + e]);
+      }
+  }
+}
+// The warp's score blocks (row block wr, column blocks wc, wc + WC, ... up to the diagonal): A B^T over D.
+template <class C, int NSA, int NSB>
+__device__ __forceinline__ void score_blocks(float (&x)[C::NB][2][4], uint32_t aA, uint32_t aB, int wr, int wc, int lane) {
+#pragma unroll
+  for (int i = 0; i < C::NB; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][j][e] = 0.f;
+  if (wc <= wr) {
+#pragma unroll 2
+    for (int ks = 0; ks < C::D / 16; ++ks) {
+      uint32_t a[NSA][4];
+      ld_a<NSA>(a, aA, C::PLANE, C::LD, 16 * wr, 16 * ks, lane);
+#pragma unroll
+      for (int i = 0; i < C::NB; ++i)
+        if (wc + C::WC * i <= wr) mma_step<NSA, NSB, 1, false>(x[i], a, aB, C::PLANE, C::LD, 16 * (wc + C::WC * i), 16 * ks, lane);
+    }
+  }
+}
+template <class C, typename TI>
+__device__ __forceinline__ void score_blocks_by_pair(float (&x)[C::NB][2][4], const float* lam, const PxParams& p,
+                                                     const ChunkAt<C>& at, int wr, int wc, int lane) {
+#pragma unroll
+  for (int i = 0; i < C::NB; ++i) {
+    float y[2][4] = {};                                    // (its address is taken; x stays in registers)
+    if (wc + C::WC * i <= wr) block_by_pair<C, TI>(y, lam, p.q, p.k, at, 16 * wr, 16 * (wc + C::WC * i), lane);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][j][e] = y[j][e];
+  }
+}
+// ... as split planes of the score tile [i][j], entries above the diagonal zero
+template <class C>
+__device__ __forceinline__ void store_scores(uint8_t* t, const float (&x)[C::NB][2][4], int wr, int wc, int lane) {
+#pragma unroll
+  for (int i = 0; i < C::NB; ++i) {
+    const int cb = wc + C::WC * i;
+    if (cb <= wr) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 16 * wr + (lane >> 2) + 8 * h, c = 16 * cb + 8 * j + 2 * (lane & 3);
+          st_split3(t + r * C::LDT + c * 2, C::TPLANE, c <= r ? x[i][j][2 * h] : 0.f, c + 1 <= r ? x[i][j][2 * h + 1] : 0.f);
+        }
+    }
+  }
+}
+template <typename TI>
+__device__ __forceinline__ void st_pair(void* p, int64_t e, float x, float y) {
+  if constexpr (sizeof(TI) == 2) *reinterpret_cast<uint32_t*>((bf16*)p + e) = pack_bf16x2(x, y);
+  else *reinterpret_cast<float2*>((float*)p + e) = make_float2(x, y);
+}
+template <int N>
+__device__ __forceinline__ void zero_acc(float (&c)[N][4]) {
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
+}
+
+// ---- forward chunk kernel ---------------------------------------------------------------------------------------------
+template <class C, typename TI>
+struct FwdLay {
+  static constexpr int NSV = planes_of<TI>();
+  static constexpr uint32_t most(uint32_t a, uint32_t b) { return a > b ? a : b; }
+  // two pieces of the state: the second takes the region of k~ once the scores are formed; one piece: the scores do
+  static constexpr uint32_t KREG = C::NP > 1 ? most(3 * C::SPLANE, 3 * C::PLANE) : most(3 * C::TPLANE, 3 * C::PLANE);
+  static constexpr uint32_t Q = 0, K = Q + 3 * C::PLANE, V = K + KREG, S = V + NSV * C::PLANE;
+  static constexpr uint32_t T = C::NP > 1 ? S + 3 * C::SPLANE : K, SEG = C::NP > 1 ? T + 3 * C::TPLANE : S + 3 * C::SPLANE;
+  static constexpr uint32_t EM = SEG + 2 * C::RG * C::D * 4, END = EM + C::D * 4;
+  static_assert(C::L * C::D * 4 <= 3 * C::PLANE, "the pairwise form keeps lam where k~ would be");
+};
+template <class C, typename TI>
+__global__ void __launch_bounds__(C::NT) px_fwd_kernel(PxParams p) {
+  using Lay = FwdLay<C, TI>;
+  extern __shared__ __align__(16) uint8_t sm[];
+  float* seg = reinterpret_cast<float*>(sm + Lay::SEG);
+  float* em = reinterpret_cast<float*>(sm + Lay::EM);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
+  const ChunkAt<C> at(p, blockIdx.x);
+  const float* Sn = p.S + (at.bh * (p.N + 1) + at.n) * C::D * C::D;
+  float4 sx[C::SREG];
+  bool sharp;
+  {
+    float2 g[C::RPT];
+    Pair<TI> q[C::RPT], k[C::RPT];
+    load_gates<C>(g, p.g, at, r0, cp);
+    load_pairs<C, TI>(q, p.q, at, r0, cp);
+    load_pairs<C, TI>(k, p.k, at, r0, cp);
+    copy_rows<C, TI>(sm + Lay::V, p.v, at);
+    fetch_piece<C>(sx, Sn, 0);
+    float2 before, own, total;
+    sharp = gate_sums<C>(g, seg, seg + C::RG * C::D, rg, cp, before, own, total);
+    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, sharp, before, own, total, rg, cp);
+    __syncthreads();
+    if (sharp) store_lam<C>(reinterpret_cast<float*>(sm + Lay::K), p.g, at, before, rg, cp);
+  }
+  store_piece<C>(sm + Lay::S, sx, em);
+  if (C::NP > 1) fetch_piece<C>(sx, Sn, 1);
+  if (sharp) __syncthreads();
+  const int wr = warp % C::WR, wc = warp / C::WR, m0 = 16 * wr;
+  const uint32_t aQ = smem_u32(sm + Lay::Q), aK = smem_u32(sm + Lay::K), aV = smem_u32(sm + Lay::V), aS = smem_u32(sm + Lay::S);
+  const uint32_t aT = smem_u32(sm + Lay::T);
+  {
+    float x[C::NB][2][4];
+    if (!sharp) score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);
+    else score_blocks_by_pair<C, TI>(x, reinterpret_cast<const float*>(sm + Lay::K), p, at, wr, wc, lane);
+    __syncthreads();                      // the scores are formed: the region of k~ is free
+    store_scores<C>(sm + Lay::T, x, wr, wc, lane);
+  }
+  if (C::NP > 1) store_piece<C>(sm + Lay::K, sx, em);
+  __syncthreads();
+  float o[C::NP][C::PC / 8][4];
+#pragma unroll
+  for (int pc = 0; pc < C::NP; ++pc) zero_acc(o[pc]);
+#pragma unroll 1
+  for (int kk = 0; kk <= wr; ++kk) {
+    uint32_t a[3][4];
+    ld_a<3>(a, aT, C::TPLANE, C::LDT, m0, 16 * kk, lane);
+#pragma unroll
+    for (int pc = 0; pc < C::NP; ++pc)
+      mma_step<3, Lay::NSV, C::PC / 16, true>(o[pc], a, aV, C::PLANE, C::LD, pc * C::PW + wc * C::PC, 16 * kk, lane);
+  }
+#pragma unroll 2
+  for (int ks = 0; ks < C::D / 16; ++ks) {
+    uint32_t a[3][4];
+    ld_a<3>(a, aQ, C::PLANE, C::LD, m0, 16 * ks, lane);
+#pragma unroll
+    for (int pc = 0; pc < C::NP; ++pc)
+      mma_step<3, 3, C::PC / 16, true>(o[pc], a, pc == 0 ? aS : aK, C::SPLANE, C::LDS, wc * C::PC, 16 * ks, lane);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = m0 + (lane >> 2) + 8 * h;
+    if (r < at.nv) {
+      const int64_t e = at.row(r) + wc * C::PC + 2 * (lane & 3);
+#pragma unroll
+      for (int pc = 0; pc < C::NP; ++pc)
+#pragma unroll
+        for (int j = 0; j < C::PC / 8; ++j) {
+          const int64_t c = e + pc * C::PW + 8 * j;
+          if (p.out_bf) st_pair<bf16>(p.out, c, o[pc][j][2 * h], o[pc][j][2 * h + 1]);
+          else st_pair<float>(p.out, c, o[pc][j][2 * h], o[pc][j][2 * h + 1]);
+        }
+    }
+  }
+}
+
+// ---- backward chunk kernel --------------------------------------------------------------------------------------------
+// A warp's 16 rows serve twice: as rows i for dq = dP k~ + dO S^T, and as rows j for dk = dP^T q~ + V dS^T and
+// dV = P^T dO + k~ dS.  dP and then P pass through one score tile (read transposed for the second role), which shares
+// its place with the states' pieces of 64 value columns.
+template <class C, typename TI, typename TY>
+struct BwdLay {
+  static constexpr int NSV = planes_of<TI>(), NSD = planes_of<TY>();
+  static constexpr uint32_t most(uint32_t a, uint32_t b) { return a > b ? a : b; }
+  // score tile, state pieces; the pairwise form also keeps lam there for a while
+  static constexpr uint32_t SREGION = most(3 * C::SPLANE, most(3 * C::TPLANE, C::L * C::D * 4));
+  static constexpr uint32_t Q = 0, K = Q + 3 * C::PLANE, V = K + 3 * C::PLANE, DO = V + NSV * C::PLANE, S = DO + NSD * C::PLANE;
+  static constexpr uint32_t SEG = S + SREGION, EM = SEG + 2 * C::RG * C::D * 4, DG = EM + C::D * 4, END = DG + C::D * 4;
+  static_assert(C::L * C::AP * 4 <= 3 * C::PLANE, "dq and dk are staged in float32 over q~ and k~");
+  static_assert(C::L * C::D * 4 <= (NSV + NSD) * C::PLANE, "pairwise form: lam over V and dO at the end");
+};
+// dG[d] += <S_{n+1}[d, piece], dS_n[d, piece]>: PW / 4 consecutive threads hold a row of the piece
+template <class C>
+__device__ __forceinline__ void dot_piece(float* dG, const float4 (&x)[C::SREG], const float* Snext, int pc) {
+  float4 y[C::SREG];
+  fetch_piece<C>(y, Snext, pc);
+#pragma unroll
+  for (int j = 0; j < C::SREG; ++j) {
+    float s = x[j].x * y[j].x + x[j].y * y[j].y + x[j].z * y[j].z + x[j].w * y[j].w;
+#pragma unroll
+    for (int o = C::PW / 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const int id = threadIdx.x + C::NT * j, r = id / (C::PW / 4);
+    if (id % (C::PW / 4) == 0) dG[r] = pc == 0 ? s : dG[r] + s;
+  }
+}
+// Sharp chunk: the accumulators of dq and dk hold the inter-chunk terms only; applies their weights exp(lam) and
+// exp(G - lam) and adds the pairs inside the chunk, dP (three planes) times exp(lam_i - lam_j).
+template <class C, typename TI>
+__device__ __noinline__ void close_by_pair(float* tq, float* tk, const uint8_t* dP, const float* lam, const PxParams& p,
+                                           const ChunkAt<C>& at, float2 total, int r0, int cp) {
+  auto dp_at = [&](int i, int j) {
+    const bf16* t = reinterpret_cast<const bf16*>(dP + i * C::LDT + j * 2);
+    return (__bfloat162float(t[C::TPLANE]) + __bfloat162float(t[C::TPLANE / 2])) + __bfloat162float(t[0]);
+  };
+  auto at2 = [&](const float* t, int r, int pitch) { return *reinterpret_cast<const float2*>(t + r * pitch + 2 * cp); };
+#pragma unroll 1
+  for (int r = r0; r < r0 + C::RPT; ++r) {
+    const float2 lr = at2(lam, r, C::D);
+    float2 x = at2(tq, r, C::AP), y = at2(tk, r, C::AP);
+    x.x *= expf(lr.x); x.y *= expf(lr.y);
+    y.x *= expf(total.x - lr.x); y.y *= expf(total.y - lr.y);
+#pragma unroll 1
+    for (int j = 0; j <= r && j < at.nv; ++j) {
+      Pair<TI> kj;
+      kj.load(p.k, at.row(j) + 2 * cp);
+      const float2 kf = kj.get(), lj = at2(lam, j, C::D);
+      const float w = dp_at(r, j);
+      x.x = fmaf(w * kf.x, expf(lr.x - lj.x), x.x);
+      x.y = fmaf(w * kf.y, expf(lr.y - lj.y), x.y);
+    }
+#pragma unroll 1
+    for (int i = r; i < at.nv; ++i) {
+      Pair<TI> qi;
+      qi.load(p.q, at.row(i) + 2 * cp);
+      const float2 qf = qi.get(), li = at2(lam, i, C::D);
+      const float w = dp_at(i, r);
+      y.x = fmaf(w * qf.x, expf(li.x - lr.x), y.x);
+      y.y = fmaf(w * qf.y, expf(li.y - lr.y), y.y);
+    }
+    *reinterpret_cast<float2*>(tq + r * C::AP + 2 * cp) = x;
+    *reinterpret_cast<float2*>(tk + r * C::AP + 2 * cp) = y;
+  }
+}
+template <class C, typename TI, typename TY>
+__global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
+  using Lay = BwdLay<C, TI, TY>;
+  constexpr int NSV = Lay::NSV, NSD = Lay::NSD, L = C::L, D = C::D;
+  extern __shared__ __align__(16) uint8_t sm[];
+  float* seg = reinterpret_cast<float*>(sm + Lay::SEG);
+  float* em = reinterpret_cast<float*>(sm + Lay::EM);
+  float* dG = reinterpret_cast<float*>(sm + Lay::DG);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
+  const ChunkAt<C> at(p, blockIdx.x);
+  const float* Sn = p.S + (at.bh * (p.N + 1) + at.n) * D * D;
+  const float* dSn = p.dS + (at.bh * (p.N + 1) + at.n + 1) * D * D;
+  float4 sx[C::SREG];
+  float2 before, own, total;
+  bool sharp;
+  {
+    float2 g[C::RPT];
+    Pair<TI> q[C::RPT], k[C::RPT];
+    load_gates<C>(g, p.g, at, r0, cp);
+    load_pairs<C, TI>(q, p.q, at, r0, cp);
+    load_pairs<C, TI>(k, p.k, at, r0, cp);
+    copy_rows<C, TI>(sm + Lay::V, p.v, at);
+    copy_rows<C, TY>(sm + Lay::DO, p.dout, at);
+    sharp = gate_sums<C>(g, seg, seg + C::RG * D, rg, cp, before, own, total);
+    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, sharp, before, own, total, rg, cp);
+  }
+  fetch_piece<C>(sx, Sn, 0);
+  __syncthreads();
+
+  const int wr = warp % C::WR, wc = warp / C::WR, m0 = 16 * wr;
+  const uint32_t aQ = smem_u32(sm + Lay::Q), aK = smem_u32(sm + Lay::K), aV = smem_u32(sm + Lay::V);
+  const uint32_t aD = smem_u32(sm + Lay::DO), aS = smem_u32(sm + Lay::S);
+  const float* Snext = p.S + (at.bh * (p.N + 1) + at.n + 1) * D * D;
+  float dq[C::CW / 8][4], dk[C::CW / 8][4], dv[C::NP][C::PC / 8][4];
+  zero_acc(dq);
+  zero_acc(dk);
+#pragma unroll
+  for (int pc = 0; pc < C::NP; ++pc) zero_acc(dv[pc]);
+  float x[C::NB][2][4];
+  if (!sharp) {
+    score_blocks<C, NSD, NSV>(x, aD, aV, wr, wc, lane);               // dP = tril(dO V^T)
+    store_scores<C>(sm + Lay::S, x, wr, wc, lane);
+    __syncthreads();
+#pragma unroll 1
+    for (int kk = 0; kk <= wr; ++kk) {                                // dq += dP k~
+      uint32_t a[3][4];
+      ld_a<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
+      mma_step<3, 3, C::CW / 16, true>(dq, a, aK, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
+    }
+#pragma unroll 1
+    for (int kk = wr; kk < L / 16; ++kk) {                            // dk += dP^T q~
+      uint32_t a[3][4];
+      ld_a_t<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
+      mma_step<3, 3, C::CW / 16, true>(dk, a, aQ, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
+    }
+    score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);                   // P = tril(q~ k~^T)
+  } else {
+    float* lam = reinterpret_cast<float*>(sm + Lay::S);
+    store_lam<C>(lam, p.g, at, before, rg, cp);
+    __syncthreads();
+    score_blocks_by_pair<C, TI>(x, lam, p, at, wr, wc, lane);
+  }
+  __syncthreads();
+  store_scores<C>(sm + Lay::S, x, wr, wc, lane);
+  __syncthreads();
+#pragma unroll 1
+  for (int kk = wr; kk < L / 16; ++kk) {                              // dV = P^T dO
+    uint32_t a[3][4];
+    ld_a_t<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
+#pragma unroll
+    for (int pc = 0; pc < C::NP; ++pc)
+      mma_step<3, NSD, C::PC / 16, true>(dv[pc], a, aD, C::PLANE, C::LD, pc * C::PW + wc * C::PC, 16 * kk, lane);
+  }
+#pragma unroll
+  for (int i = 0; i < 2 * C::NP; ++i) {       // the pieces of S_n (dq += dO S^T), then those of dS_n (dk += V dS^T, dV += k~ dS)
+    const int pc = i % C::NP;
+    __syncthreads();                          // what the buffer held is consumed
+    if (i >= C::NP) dot_piece<C>(dG, sx, Snext, pc);
+    store_piece<C>(sm + Lay::S, sx, em);
+    if (i + 1 < 2 * C::NP) fetch_piece<C>(sx, i + 1 < C::NP ? Sn : dSn, (i + 1) % C::NP);
+    __syncthreads();
+    if (i < C::NP) {
+#pragma unroll 1
+      for (int ks = 0; ks < C::PW / 16; ++ks) {
+        uint32_t a[NSD][4];
+        ld_a<NSD>(a, aD, C::PLANE, C::LD, m0, pc * C::PW + 16 * ks, lane);
+        mma_step<NSD, 3, C::CW / 16, false>(dq, a, aS, C::SPLANE, C::LDS, wc * C::CW, 16 * ks, lane);
+      }
+    } else {
+#pragma unroll 1
+      for (int ks = 0; ks < C::PW / 16; ++ks) {
+        uint32_t a[NSV][4];
+        ld_a<NSV>(a, aV, C::PLANE, C::LD, m0, pc * C::PW + 16 * ks, lane);
+        mma_step<NSV, 3, C::CW / 16, false>(dk, a, aS, C::SPLANE, C::LDS, wc * C::CW, 16 * ks, lane);
+      }
+#pragma unroll 1
+      for (int ks = 0; ks < D / 16; ++ks) {
+        uint32_t a[3][4];
+        ld_a<3>(a, aK, C::PLANE, C::LD, m0, 16 * ks, lane);
+        mma_step<3, 3, C::PC / 16, true>(dv[pc], a, aS, C::SPLANE, C::LDS, wc * C::PC, 16 * ks, lane);
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = m0 + (lane >> 2) + 8 * h;
+    if (r < at.nv) {
+      const int64_t e = at.row(r) + wc * C::PC + 2 * (lane & 3);
+#pragma unroll
+      for (int pc = 0; pc < C::NP; ++pc)
+#pragma unroll
+        for (int j = 0; j < C::PC / 8; ++j) st_pair<TI>(p.dv, e + pc * C::PW + 8 * j, dv[pc][j][2 * h], dv[pc][j][2 * h + 1]);
+    }
+  }
+  __syncthreads();                                        // every operand but V and dO is dead
+  float* tq = reinterpret_cast<float*>(sm + Lay::Q);
+  float* tk = reinterpret_cast<float*>(sm + Lay::K);
+#pragma unroll
+  for (int j = 0; j < C::CW / 8; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = (m0 + (lane >> 2) + 8 * h) * C::AP + wc * C::CW + 8 * j + 2 * (lane & 3);
+      *reinterpret_cast<float2*>(tq + e) = make_float2(dq[j][2 * h], dq[j][2 * h + 1]);
+      *reinterpret_cast<float2*>(tk + e) = make_float2(dk[j][2 * h], dk[j][2 * h + 1]);
+    }
+  if (sharp) {
+    score_blocks<C, NSD, NSV>(x, aD, aV, wr, wc, lane);
+    store_scores<C>(sm + Lay::S, x, wr, wc, lane);
+    __syncthreads();
+    float* lam = reinterpret_cast<float*>(sm + Lay::V);
+    store_lam<C>(lam, p.g, at, before, rg, cp);
+    __syncthreads();
+    close_by_pair<C, TI>(tq, tk, sm + Lay::S, lam, p, at, total, r0, cp);     // a thread's own entries of tq and tk
+  }
+  __syncthreads();
+
+  // ---- closing pass: a thread finishes RPT rows of two features ------------------------------------------------------
+  float2 g[C::RPT];
+  Pair<TI> q[C::RPT], k[C::RPT];
+  load_gates<C>(g, p.g, at, r0, cp);
+  load_pairs<C, TI>(q, p.q, at, r0, cp);
+  load_pairs<C, TI>(k, p.k, at, r0, cp);
+  float2 run = sharp ? make_float2(1.f, 1.f) : make_float2(expf(before.x - 0.5f * total.x), expf(before.y - 0.5f * total.y));
+  float2 dl[C::RPT];
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i) {
+    const int r = r0 + i;
+    g[i] = sharp ? make_float2(1.f, 1.f) : make_float2(expf(g[i].x), expf(g[i].y));
+    run.x *= g[i].x; run.y *= g[i].y;
+    float2 y = *reinterpret_cast<const float2*>(tq + r * C::AP + 2 * cp);
+    y.x *= run.x; y.y *= run.y;
+    const float2 qf = q[i].get();
+    dl[i] = make_float2(qf.x * y.x, qf.y * y.y);
+    if (r < at.nv) st_pair<TI>(p.dq, at.row(r) + 2 * cp, y.x, y.y);
+  }
+  run = make_float2(1.f / run.x, 1.f / run.y);
+#pragma unroll
+  for (int i = C::RPT - 1; i >= 0; --i) {
+    const int r = r0 + i;
+    float2 y = *reinterpret_cast<const float2*>(tk + r * C::AP + 2 * cp);
+    y.x *= run.x; y.y *= run.y;
+    run.x *= g[i].x; run.y *= g[i].y;
+    const float2 kf = k[i].get();
+    dl[i].x -= kf.x * y.x; dl[i].y -= kf.y * y.y;
+    if (r < at.nv) st_pair<TI>(p.dk, at.row(r) + 2 * cp, y.x, y.y);
+  }
+#pragma unroll
+  for (int i = C::RPT - 2; i >= 0; --i) { dl[i].x += dl[i + 1].x; dl[i].y += dl[i + 1].y; }
+  *reinterpret_cast<float2*>(seg + rg * D + 2 * cp) = dl[0];
+  __syncthreads();
+  float2 off = *reinterpret_cast<const float2*>(dG + 2 * cp);
+#pragma unroll
+  for (int r = C::RG - 1; r > 0; --r)
+    if (r > rg) {
+      const float2 t = *reinterpret_cast<const float2*>(seg + r * D + 2 * cp);
+      off.x += t.x; off.y += t.y;
+    }
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i)
+    if (r0 + i < at.nv) *reinterpret_cast<float2*>(p.dg + at.row(r0 + i) + 2 * cp) = make_float2(dl[i].x + off.x, dl[i].y + off.y);
+}
+
+// ---- host side ----------------------------------------------------------------------------------------------------------
+template <class C, typename TI, typename TY, int MODE>
+int launch_product(cudaStream_t st, const PxParams& p, int64_t chunks) {
+  constexpr size_t smem = (3 + planes_of<TY>()) * C::PLANE + C::RG * C::D * 4;
+  static SmemAttrOnce attr;
+  GLA_TRY(attr.ensure(px_product_kernel<C, TI, TY, MODE>, smem));
+  ProfScope ps(MODE == 0 ? "px_state_product" : "px_dstate_product", st);
+  px_product_kernel<C, TI, TY, MODE><<<(unsigned)chunks, C::NT, smem, st>>>(p);
+  GLA_CHECK_LAUNCH();
+  return GLA_OK;
+}
+template <typename TS>
+int launch_scan(cudaStream_t st, int64_t BH, int64_t D, int64_t N, const float* eG, const void* init, float* S, void* fin, int mode) {
+  const int64_t total = BH * D * D;
+  ProfScope ps("px_scan_kernel", st);
+  px_scan_kernel<TS><<<(unsigned)((total / 4 + 127) / 128), 128, 0, st>>>(total, D, N, eG, (const TS*)init, S, (TS*)fin, mode);
+  GLA_CHECK_LAUNCH();
+  return GLA_OK;
+}
+template <class C, typename TI>
+int run_fwd(cudaStream_t st, const PxParams& p, const void* init, void* fin) {
+  const int64_t BH = p.B * p.H, chunks = BH * p.N;
+  GLA_TRY((launch_product<C, TI, TI, 0>(st, p, chunks)));
+  GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.eG, init, p.S, fin, 0));
+  static SmemAttrOnce attr;
+  GLA_TRY(attr.ensure(px_fwd_kernel<C, TI>, FwdLay<C, TI>::END));
+  ProfScope ps(p.label, st);
+  px_fwd_kernel<C, TI><<<(unsigned)chunks, C::NT, FwdLay<C, TI>::END, st>>>(p);
+  GLA_CHECK_LAUNCH();
+  return GLA_OK;
+}
+// states != 0: the states are in p.S and p.eG already (a forward's residuals); otherwise they are formed here first
+template <class C, typename TI, typename TY>
+int run_bwd(cudaStream_t st, const PxParams& p, int states, const void* init, const void* dfin, void* dinit) {
+  const int64_t BH = p.B * p.H, chunks = BH * p.N;
+  if (!states) {
+    GLA_TRY((launch_product<C, TI, TI, 0>(st, p, chunks)));
+    GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.eG, init, p.S, nullptr, 0));
+  }
+  GLA_TRY((launch_product<C, TI, TY, 1>(st, p, chunks)));
+  GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.eG, dfin, p.dS, dinit, 1));
+  static SmemAttrOnce attr;
+  GLA_TRY(attr.ensure(px_bwd_kernel<C, TI, TY>, BwdLay<C, TI, TY>::END));
+  ProfScope ps("px_bwd_kernel", st);
+  px_bwd_kernel<C, TI, TY><<<(unsigned)chunks, C::NT, BwdLay<C, TI, TY>::END, st>>>(p);
+  GLA_CHECK_LAUNCH();
+  return GLA_OK;
+}
+template <int D, int L>
+int dispatch_fwd(cudaStream_t st, const PxParams& p, const void* init, void* fin) {
+  return p.in_bf ? run_fwd<Px<D, L>, bf16>(st, p, init, fin) : run_fwd<Px<D, (D >= 128 ? 32 : L)>, float>(st, p, init, fin);
+}
+size_t f32b(int64_t n) { return align_up((size_t)n * 4, 256); }
+
+}  // namespace
+
+// Rows of a chunk: 64, or 32 where three planes of every operand at head size 128 leave no room for more.
+static int64_t px_rows(int64_t D, int narrow) { return D >= 128 && narrow ? 32 : 64; }
+bool px_supported(int64_t D) { return D == 32 || D == 64 || D == 128; }
+// states: (B H, N + 1, D, D) float32 | exp(G): (B H, N, D) float32
+size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
+  const int64_t N = (T + 31) / 32;                      // the shorter chunk bounds both
+  const int64_t n = D >= 128 ? N : (T + 63) / 64;
+  return f32b(B * H * (n + 1) * D * D) + f32b(B * H * n * D);
+}
+int px_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
+           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int reverse, const char* label) {
+  const int64_t N = (T + px_rows(D, !bf) - 1) / px_rows(D, !bf);
+  if (B * H * N > 2147483647LL || B * H * D * D / 512 > 2147483647LL) return GLA_ERR_TOO_LARGE;
+  PxParams p{};
+  p.B = B; p.T = T; p.H = H; p.N = N; p.trev = reverse; p.in_bf = bf; p.out_bf = out_bf;
+  p.g = g; p.v = v; p.k = k; p.q = q; p.out = out; p.label = label;
+  p.S = (float*)states;
+  p.eG = (float*)((char*)states + f32b(B * H * (N + 1) * D * D));
+  switch (D) {
+    case 32: return dispatch_fwd<32, 64>(st, p, hidden_init, hidden_final);
+    case 64: return dispatch_fwd<64, 64>(st, p, hidden_init, hidden_final);
+    case 128: return dispatch_fwd<128, 64>(st, p, hidden_init, hidden_final);
+    default: return GLA_ERR_UNSUPPORTED;
+  }
+}
+template <int D>
+static int dispatch_bwd(cudaStream_t st, const PxParams& p, int do_bf, int states, const void* init, const void* dfin, void* dinit) {
+  constexpr int LN = D >= 128 ? 32 : 64;
+  if (p.in_bf && do_bf) return run_bwd<Px<D, 64>, bf16, bf16>(st, p, states, init, dfin, dinit);
+  if (p.in_bf) return run_bwd<Px<D, LN>, bf16, float>(st, p, states, init, dfin, dinit);
+  return do_bf ? run_bwd<Px<D, LN>, float, bf16>(st, p, states, init, dfin, dinit)
+               : run_bwd<Px<D, LN>, float, float>(st, p, states, init, dfin, dinit);
+}
+// states: a forward's (px_fwd) when have_states, else scratch of px_state_bytes; ws: px_state_bytes more
+int px_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
+           const void* v, const void* k, const void* q, const void* dhidden_final, const void* dout, int do_bf,
+           void* dhidden_init, float* dg, void* dv, void* dk, void* dq, void* states, int have_states, void* ws, int reverse) {
+  const int64_t L = px_rows(D, !(bf && do_bf)), N = (T + L - 1) / L;
+  if (have_states && L != px_rows(D, !bf)) return GLA_ERR_UNSUPPORTED;
+  if (B * H * N > 2147483647LL || B * H * D * D / 512 > 2147483647LL) return GLA_ERR_TOO_LARGE;
+  PxParams p{};
+  p.B = B; p.T = T; p.H = H; p.N = N; p.trev = reverse; p.in_bf = bf;
+  p.g = g; p.v = v; p.k = k; p.q = q; p.dout = dout;
+  p.dq = dq; p.dk = dk; p.dv = dv; p.dg = dg;
+  p.S = (float*)states;
+  p.eG = (float*)((char*)states + f32b(B * H * (N + 1) * D * D));
+  p.dS = (float*)ws;
+  if (have_states == 0) {
+    switch (D) {
+      case 32: return dispatch_bwd<32>(st, p, do_bf, 0, hidden_init, dhidden_final, dhidden_init);
+      case 64: return dispatch_bwd<64>(st, p, do_bf, 0, hidden_init, dhidden_final, dhidden_init);
+      case 128: return dispatch_bwd<128>(st, p, do_bf, 0, hidden_init, dhidden_final, dhidden_init);
+      default: return GLA_ERR_UNSUPPORTED;
+    }
+  }
+  switch (D) {
+    case 32: return dispatch_bwd<32>(st, p, do_bf, 1, hidden_init, dhidden_final, dhidden_init);
+    case 64: return dispatch_bwd<64>(st, p, do_bf, 1, hidden_init, dhidden_final, dhidden_init);
+    case 128: return dispatch_bwd<128>(st, p, do_bf, 1, hidden_init, dhidden_final, dhidden_init);
+    default: return GLA_ERR_UNSUPPORTED;
+  }
+}
+
+}  // namespace gla

@@ -155,9 +155,11 @@ class _RecurrentGLA(torch.autograd.Function):
         g32 = g if g.dtype == torch.float32 else g.float()
         hf = torch.empty_like(hidden)
         out = torch.empty(v.shape, dtype=torch.float32 if out_fp32 else v.dtype, device=dev)
-        st = lib.gla_recurrent_fwd(_stream(dev), B, T, H, D, dt, _ptr(hidden), _ptr(g32), _ptr(v), _ptr(k), _ptr(q),
-                                   _ptr(hf), _ptr(out), _DT[out.dtype], int(reverse))
-        _lib.check(st, "gla_recurrent_fwd")
+        ws_n = lib.gla_recurrent_fwd_workspace_bytes(B, T, H, D, dt)
+        ws = torch.empty(ws_n, dtype=torch.uint8, device=dev) if ws_n else None
+        st = lib.gla_recurrent_fwd_ws(_stream(dev), B, T, H, D, dt, _ptr(hidden), _ptr(g32), _ptr(v), _ptr(k), _ptr(q),
+                                      _ptr(hf), _ptr(out), _DT[out.dtype], int(reverse), _ptr(ws), ws_n)
+        _lib.check(st, "gla_recurrent_fwd_ws")
         ctx.save_for_backward(hidden, g32, v, k, q)
         ctx.reverse, ctx.g_dtype = bool(reverse), g.dtype
         return hf, out

@@ -258,6 +258,14 @@ GLA_API int gla_recurrent_fwd(void* stream, int64_t B, int64_t T, int64_t H, int
                       const void* value, const void* key, const void* query,
                       void* hidden_final, void* out, int out_dtype, int reverse);
 
+/* The same with a workspace of gla_recurrent_fwd_workspace_bytes (0 bytes: none is of use for these sizes): chunks of
+ * the sequence then run side by side, from states kept in the workspace for the duration of the call.  Without one (or
+ * with arrays that are not 16-byte aligned) this is gla_recurrent_fwd, which walks the tokens in order. */
+GLA_API size_t gla_recurrent_fwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int dtype);
+GLA_API int gla_recurrent_fwd_ws(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int dtype,
+                      const void* hidden_init, const float* log_fgate, const void* value, const void* key,
+                      const void* query, void* hidden_final, void* out, int out_dtype, int reverse,
+                      void* workspace, size_t workspace_bytes);
 /* Bytes of workspace gla_recurrent_bwd needs for these sizes. */
 GLA_API size_t gla_recurrent_bwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int dtype);
 

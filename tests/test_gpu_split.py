@@ -1,0 +1,95 @@
+"""GPU parity tests (pytest -m gpu) of the float32-precision chunk kernels: chunk edges, every head size they serve, element
+types, directions, and chunks on both sides of the gate limits, against the float64 oracle.
+
+Tolerances (relative L2).  bfloat16: 1e-2 outputs, 2e-2 gradients.  float32: operand splits keep 24 bits, so what is left is
+float32 rounding: a state or a row is a sum of up to T (here <= 300) terms with a running product of up to 64 gates in
+front of each, about (sqrt(300) + 64) 2^-24 = 5e-6; the gate gradient is a running sum of terms that cancel, twice that.
+With gates around log f = shift < 0 every token's own contribution (the same in q dq and k dk, where it cancels) is
+exp(-shift) times what is left of the gate gradient, and so is the rounding error that it leaves there.
+"""
+import math
+
+import pytest
+import torch
+
+from oracle import gla_oracle as O
+from test_gpu_ops import NAMES, _case, _oracle, _run_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(ref, got, dtype, what, shift=5.0):
+    tol_f, tol_g = (1e-2, 2e-2) if dtype == torch.bfloat16 else (5e-6, 1e-5)
+    errs = {"hidden_final": O.rel_l2(ref[0], got[0]), "out": O.rel_l2(ref[1], got[1])}
+    errs.update({n: O.rel_l2(a, b) for n, a, b in zip(NAMES, ref[2], got[2])})
+    tol = {n: tol_f if n in ("hidden_final", "out") else tol_g for n in errs}
+    tol["dlog_fgate"] *= math.exp(max(0.0, -shift))
+    bad = {n: e for n, e in errs.items() if not e < tol[n]}
+    assert not bad, f"{what}: {bad} (all: {errs})"
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,T,H,D,shift,reverse", [
+    (1, 48, 1, 64, 5.0, False),       # the shortest sequence that takes the chunked form, one partial chunk
+    (2, 64, 2, 32, 5.0, False),       # exactly one chunk
+    (1, 65, 3, 64, 5.0, True),        # one row in the second chunk, reversed
+    (1, 129, 2, 128, 2.0, False),
+    (1, 300, 1, 128, 0.0, True),      # sharp gates, reversed, short last chunk
+    (2, 97, 1, 32, 0.0, True),
+    (1, 127, 2, 64, -4.0, False),     # past the limit: every chunk pair by pair
+    (1, 100, 1, 128, -4.0, False),
+    (1, 70, 1, 32, -4.0, True),
+])
+def test_recurrent_gla_in_chunks_vs_oracle(cuda_device, B, T, H, D, shift, reverse, dtype):
+    from gla_jax_b200 import recurrent_gla
+    case = _case(B, T, H, D, dtype, 7, shift)
+    ref = _oracle(*case, reverse=reverse)
+    got = _run_gpu(recurrent_gla, cuda_device, *case, reverse=reverse)
+    _check(ref, got, dtype, f"recurrent {B, T, H, D, shift, reverse, dtype}", shift)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_chunks_on_both_sides_of_the_gate_limits(cuda_device, D):
+    """Three chunks: mild, one feature past the sum limit, one single gate whose exponential vanishes (and an infinite one)."""
+    from gla_jax_b200 import chunk_gla, recurrent_gla
+    h, g, v, k, q, dhf, do = _case(1, 192, 2, D, torch.float32, 9, 5.0)
+    g[0, 64:128, 1, 3] = -3.0
+    g[0, 140, 0, 5] = -95.0
+    for fn, kw in ((chunk_gla, dict(chunk_size=64)), (recurrent_gla, {})):
+        ref = _oracle(h, g, v, k, q, dhf, do)
+        _check(ref, _run_gpu(fn, cuda_device, h, g, v, k, q, dhf, do, **kw), torch.float32, f"limits {D} {fn.__name__}")
+    g[0, 150, 1, 7] = -float("inf")       # forget everything: the state row restarts
+    hf, out = recurrent_gla(*[x.to(cuda_device) for x in (h, g, v, k, q)])
+    hf0, out0 = O.recurrent_gla_naive(*[x[0].double() for x in (h, g, v, k, q)])
+    assert O.rel_l2(hf0, hf[0].cpu()) < 5e-6 and O.rel_l2(out0, out[0].cpu()) < 5e-6
+
+
+def test_naive_with_bf16_inputs_and_float32_cotangent(cuda_device):
+    """bf16 operands with a float32 output and output gradient (recurrent_gla_naive), head size 128: shorter chunks."""
+    from gla_jax_b200 import recurrent_gla_naive
+    h, g, v, k, q, dhf, do = _case(1, 150, 2, 128, torch.bfloat16, 11, 5.0)
+    do = do.float() + 1e-3 * torch.randn(do.shape, generator=torch.Generator().manual_seed(1))
+    leaves = [x.to(cuda_device).requires_grad_(True) for x in (h, g, v, k, q)]
+    hf, out = recurrent_gla_naive(*leaves)
+    assert out.dtype == torch.float32
+    grads = torch.autograd.grad([hf, out], leaves, [dhf.to(cuda_device), do.to(cuda_device)])
+    ref = _oracle(h, g, v, k, q, dhf, do)
+    assert O.rel_l2(ref[1], out.detach().cpu()) < 5e-6
+    _check((ref[0], ref[0], ref[2]), (hf.detach().cpu(), hf.detach().cpu(), [x.cpu() for x in grads]), torch.bfloat16, "naive")
+
+
+def test_wait_for_workspace_is_not_needed(cuda_device):
+    """The entry point without a workspace walks the tokens; with one it runs chunks: same results to float32 rounding."""
+    from gla_jax_b200 import _lib
+    lib = _lib.load()
+    h, g, v, k, q, _, _ = [x.to(cuda_device) for x in _case(1, 200, 2, 64, torch.float32, 13, 5.0)]
+    st = _lib.stream_of(v.device)
+    res = []
+    for ws_n in (0, lib.gla_recurrent_fwd_workspace_bytes(1, 200, 2, 64, _lib.GLA_F32)):
+        ws = torch.empty(max(ws_n, 1), dtype=torch.uint8, device=cuda_device)
+        hf, out = torch.empty_like(h), torch.empty_like(v)
+        _lib.check(lib.gla_recurrent_fwd_ws(st, 1, 200, 2, 64, _lib.GLA_F32, h.data_ptr(), g.data_ptr(), v.data_ptr(), k.data_ptr(),
+                                            q.data_ptr(), hf.data_ptr(), out.data_ptr(), _lib.GLA_F32, 0,
+                                            ws.data_ptr() if ws_n else None, ws_n), "gla_recurrent_fwd_ws")
+        res.append((hf.cpu(), out.cpu()))
+    assert O.rel_l2(res[0][0], res[1][0]) < 5e-6 and O.rel_l2(res[0][1], res[1][1]) < 5e-6
