@@ -131,6 +131,26 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_native = None
+
+
+def native():
+    """The native host path of the torch operators (csrc/gla_host.cc), linked against the same libgla_b200.so; raises
+    if it is not built."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        load()
+        try:
+            from . import gla_b200_host
+        except ImportError as e:
+            raise RuntimeError("gla_b200_host.so is missing or does not load: the host library is not built "
+                               "(run `python -m gla_jax_b200.build`). This package has no Python fallback.") from e
+        gla_b200_host.set_error_class(GlaError)
+        _native = gla_b200_host
+    return _native
+
+
 def lib_path() -> Path:
     return _LIB_PATH
 

@@ -1,4 +1,4 @@
-"""Builds libgla_b200.so in-tree with nvcc for sm_100a.
+"""Builds libgla_b200.so in-tree with nvcc for sm_100a, and gla_b200_host.so (the torch operators' host path) beside it.
 
     python -m gla_jax_b200.build [--force] [--verbose]
 
@@ -34,8 +34,9 @@ def _stale() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every translation unit to an object file and link the shared library."""
+    """Compile every translation unit to an object file, link the shared library, and build the host path beside it."""
     if not force and not _stale():
+        build_host()
         return LIB
     objdir = PKG / "build"
     objdir.mkdir(exist_ok=True)
@@ -64,7 +65,32 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
         raise RuntimeError("link failed")
+    build_host(force)
     return LIB
+
+
+HOST_LIB = PKG / "gla_b200_host.so"
+
+
+def build_host(force: bool = False) -> Path:
+    """Compile csrc/gla_host.cc against the installed torch and link it with libgla_b200.so."""
+    src, hdr = CSRC / "gla_host.cc", PKG.parent / "include" / "gla_b200.h"
+    if not force and HOST_LIB.exists() and HOST_LIB.stat().st_mtime >= max(p.stat().st_mtime for p in (src, hdr)):
+        return HOST_LIB
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    inc = [a for d in [*cpp_extension.include_paths(), str(Path(NVCC).parent.parent / "include"), sysconfig.get_paths()["include"]]
+           for a in ("-isystem", d)]
+    libdir = str(Path(torch.__file__).parent / "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=gla_b200_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, str(src), "-o", str(HOST_LIB), "-L", libdir,
+           "-L", str(PKG), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda", "-lgla_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout)
+        raise RuntimeError("building the host path failed")
+    return HOST_LIB
 
 
 def build_xla_ffi() -> Path:

@@ -1,0 +1,249 @@
+// Host path of the torch operators: argument checks, allocation, the library calls and the autograd nodes in native code.
+//
+// The small calls (a decode step, a short prompt, a correctness run) take less time on the GPU than a Python autograd
+// function and a foreign-function call with twenty arguments take on the host, so the whole path from the Python
+// signature to the launches is here.  Every operator returns None for arguments that are not of its plain form; the
+// Python wrapper then repeats the checks one by one and raises the error that says which one failed.
+// No kernel and no arithmetic lives here: everything goes through the C ABI of include/gla_b200.h.
+#include <torch/extension.h>
+#include <torch/csrc/Exceptions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include "../../include/gla_b200.h"
+
+namespace {
+
+using torch::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+PyObject* g_error = nullptr;      // gla_jax_b200._lib.GlaError
+
+[[noreturn]] void raise(const std::string& msg) {
+  py::gil_scoped_acquire gil;
+  PyErr_SetString(g_error ? g_error : PyExc_RuntimeError, msg.c_str());
+  python_error e;
+  e.persist();
+  throw e;
+}
+void check(int status, const char* what) {
+  if (status == 0) return;
+  std::string m = std::string(what) + ": " + gla_status_string(status);
+  if (status == GLA_ERR_LAUNCH) m += " (cudaError " + std::to_string(gla_last_cuda_error()) + ")";
+  raise(m);
+}
+int dt_of(const Tensor& t) {
+  return t.scalar_type() == torch::kFloat32 ? GLA_F32 : t.scalar_type() == torch::kBFloat16 ? GLA_BF16 : -1;
+}
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+void* stream_of(const Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+bool here(const Tensor& t) { return t.is_cuda() && t.device().index() == c10::cuda::current_device(); }
+Tensor bytes(const Tensor& like, size_t n) {
+  return n ? torch::empty({(int64_t)n}, like.options().dtype(torch::kUInt8)) : Tensor();
+}
+Tensor f32(const Tensor& g) { return (g.scalar_type() == torch::kFloat32 ? g : g.to(torch::kFloat32)).contiguous(); }
+bool wants_grad(std::initializer_list<const Tensor*> ts) {
+  if (!torch::GradMode::is_enabled()) return false;
+  for (const Tensor* t : ts) if (t->requires_grad()) return true;
+  return false;
+}
+// a gradient that may be absent, in the dtype and layout the library takes
+Tensor grad_or_zeros(const Tensor& g, const Tensor& like) {
+  return g.defined() ? g.to(like.scalar_type()).contiguous() : torch::zeros(like.sizes(), like.options().requires_grad(false));
+}
+
+struct Dims { int64_t B, T, H, D; int dt; };
+// (T,H,D) or (B,T,H,D) arrays of one dtype with a matching state; false: let the wrapper say what is wrong
+bool dims_of(const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q, Dims& d) {
+  if (!v.defined() || !here(v) || (v.dim() != 3 && v.dim() != 4)) return false;
+  for (const Tensor* t : {&h, &g, &k, &q}) if (!t->defined() || t->device() != v.device()) return false;
+  if (g.sizes() != v.sizes() || k.sizes() != v.sizes() || q.sizes() != v.sizes() || !g.is_floating_point()) return false;
+  d.dt = dt_of(v);
+  if (d.dt < 0 || k.scalar_type() != v.scalar_type() || q.scalar_type() != v.scalar_type() || h.scalar_type() != v.scalar_type()) return false;
+  const int b = v.dim() == 4;
+  d.B = b ? v.size(0) : 1; d.T = v.size(b); d.H = v.size(b + 1); d.D = v.size(b + 2);
+  if (h.dim() != 3 + b || (b && h.size(0) != d.B)) return false;
+  return h.size(b) == d.H && h.size(b + 1) == d.D && h.size(b + 2) == d.D;
+}
+std::string shape_text(const Dims& d, int64_t chunk, const Tensor& v) {
+  return "T=" + std::to_string(d.T) + " H=" + std::to_string(d.H) + " D=" + std::to_string(d.D) + " chunk=" + std::to_string(chunk) +
+         " dtype=" + (d.dt == GLA_F32 ? "torch.float32" : "torch.bfloat16");
+}
+
+// ---- chunk_gla ---------------------------------------------------------------------------------------------------
+variable_list chunk_forward(const Dims& d, const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
+                            int64_t chunk, int64_t impl, bool residuals) {
+  const size_t n = gla_chunk_fwd_workspace_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl);
+  if (n == 0) raise("chunk_gla: unsupported configuration " + shape_text(d, chunk, v));
+  Tensor saved = residuals ? bytes(v, gla_chunk_saved_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl)) : Tensor();
+  Tensor ws = bytes(v, n), hf = torch::empty_like(h), out = torch::empty_like(v);
+  check(gla_chunk_fwd(stream_of(v), d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl, ptr(h), (const float*)ptr(g), ptr(v), ptr(k), ptr(q),
+                      ptr(hf), ptr(out), ptr(saved), ptr(ws), n), "gla_chunk_fwd");
+  return {hf, out, saved};
+}
+struct ChunkFn : torch::autograd::Function<ChunkFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& h0, const Tensor& g0, const Tensor& v0, const Tensor& k0,
+                               const Tensor& q0, int64_t B, int64_t T, int64_t H, int64_t D, int64_t dt, int64_t chunk, int64_t impl) {
+    const Dims d{B, T, H, D, (int)dt};
+    Tensor h = h0.contiguous(), g = f32(g0), v = v0.contiguous(), k = k0.contiguous(), q = q0.contiguous();
+    variable_list r = chunk_forward(d, h, g, v, k, q, chunk, impl, true);
+    ctx->save_for_backward({g, v, k, q, r[2]});
+    ctx->set_materialize_grads(false);
+    ctx->saved_data["d"] = std::vector<int64_t>{B, T, H, D, dt, chunk, impl, (int64_t)g0.scalar_type()};
+    return {r[0], r[1]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto a = ctx->saved_data["d"].toIntVector();
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &g = s[0], &v = s[1], &k = s[2], &q = s[3];
+    const int dt = (int)a[4], impl = (int)a[6];
+    std::vector<int64_t> hs(v.sizes().begin(), v.sizes().end());        // (B,) H, D, D
+    hs[hs.size() - 3] = a[2]; hs[hs.size() - 2] = a[3];
+    Tensor dh = torch::empty(hs, v.options());
+    Tensor dhf = grad_or_zeros(grads[0], dh), dout = grad_or_zeros(grads[1], v);
+    Tensor dg = torch::empty_like(g), dv = torch::empty_like(v), dk = torch::empty_like(k), dq = torch::empty_like(q);
+    const size_t n = gla_chunk_bwd_workspace_bytes(a[0], a[1], a[2], a[3], a[5], dt, impl);
+    Tensor ws = bytes(v, n);
+    check(gla_chunk_bwd(stream_of(v), a[0], a[1], a[2], a[3], a[5], dt, impl, (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(s[4]),
+                        ptr(dhf), ptr(dout), ptr(dh), (float*)ptr(dg), ptr(dv), ptr(dk), ptr(dq), ptr(ws), n), "gla_chunk_bwd");
+    const auto gt = (torch::ScalarType)a[7];
+    variable_list r{dh, gt == torch::kFloat32 ? dg : dg.to(gt), dv, dk, dq};
+    r.resize(12);
+    return r;
+  }
+};
+std::optional<std::tuple<Tensor, Tensor>> chunk_gla(const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
+                                                    int64_t chunk, int64_t impl) {
+  Dims d;
+  if (!dims_of(h, g, v, k, q, d) || chunk <= 0 || (chunk & (chunk - 1)) || d.T % chunk) return std::nullopt;
+  if (wants_grad({&h, &g, &v, &k, &q})) {
+    variable_list r = ChunkFn::apply(h, g, v, k, q, d.B, d.T, d.H, d.D, d.dt, chunk, impl);
+    return std::make_tuple(r[0], r[1]);
+  }
+  variable_list r = chunk_forward(d, h.contiguous(), f32(g), v.contiguous(), k.contiguous(), q.contiguous(), chunk, impl, false);
+  return std::make_tuple(r[0], r[1]);
+}
+
+// ---- recurrent_gla -------------------------------------------------------------------------------------------------
+variable_list recurrent_forward(const Dims& d, const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
+                                bool reverse, bool out_f32) {
+  Tensor hf = torch::empty_like(h), out = torch::empty(v.sizes(), v.options().dtype(out_f32 ? torch::kFloat32 : v.scalar_type()));
+  const size_t n = gla_recurrent_fwd_workspace_bytes(d.B, d.T, d.H, d.D, d.dt);
+  Tensor ws = bytes(v, n);
+  check(gla_recurrent_fwd_ws(stream_of(v), d.B, d.T, d.H, d.D, d.dt, ptr(h), (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(hf),
+                             ptr(out), dt_of(out), reverse, ptr(ws), n), "gla_recurrent_fwd_ws");
+  return {hf, out};
+}
+struct RecurrentFn : torch::autograd::Function<RecurrentFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& h0, const Tensor& g0, const Tensor& v0, const Tensor& k0,
+                               const Tensor& q0, int64_t B, int64_t T, int64_t H, int64_t D, int64_t dt, bool reverse, bool out_f32) {
+    const Dims d{B, T, H, D, (int)dt};
+    Tensor h = h0.contiguous(), g = f32(g0), v = v0.contiguous(), k = k0.contiguous(), q = q0.contiguous();
+    variable_list r = recurrent_forward(d, h, g, v, k, q, reverse, out_f32);
+    ctx->save_for_backward({h, g, v, k, q});
+    ctx->set_materialize_grads(false);
+    ctx->saved_data["d"] = std::vector<int64_t>{B, T, H, D, dt, reverse, (int64_t)g0.scalar_type(), (int64_t)r[1].scalar_type()};
+    return r;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto a = ctx->saved_data["d"].toIntVector();
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &h = s[0], &g = s[1], &v = s[2], &k = s[3], &q = s[4];
+    Tensor dhf = grad_or_zeros(grads[0], h);
+    Tensor dout = grads[1].defined() ? grads[1].contiguous() : torch::zeros(v.sizes(), v.options().dtype((torch::ScalarType)a[7]));
+    if (dt_of(dout) < 0) dout = dout.to(torch::kFloat32);
+    Tensor dh = torch::empty_like(h), dg = torch::empty_like(g), dv = torch::empty_like(v), dk = torch::empty_like(k), dq = torch::empty_like(q);
+    const size_t n = gla_recurrent_bwd_workspace_bytes(a[0], a[1], a[2], a[3], (int)a[4]);
+    Tensor ws = bytes(v, n);
+    check(gla_recurrent_bwd(stream_of(v), a[0], a[1], a[2], a[3], (int)a[4], ptr(h), (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(dhf),
+                            ptr(dout), dt_of(dout), ptr(dh), (float*)ptr(dg), ptr(dv), ptr(dk), ptr(dq), (int)a[5], ptr(ws), n),
+          "gla_recurrent_bwd");
+    const auto gt = (torch::ScalarType)a[6];
+    variable_list r{dh, gt == torch::kFloat32 ? dg : dg.to(gt), dv, dk, dq};
+    r.resize(12);
+    return r;
+  }
+};
+std::optional<std::tuple<Tensor, Tensor>> recurrent_gla(const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k,
+                                                        const Tensor& q, bool reverse, bool out_f32) {
+  Dims d;
+  if (!dims_of(h, g, v, k, q, d)) return std::nullopt;
+  variable_list r = wants_grad({&h, &g, &v, &k, &q})
+                        ? RecurrentFn::apply(h, g, v, k, q, d.B, d.T, d.H, d.D, d.dt, reverse, out_f32)
+                        : recurrent_forward(d, h.contiguous(), f32(g), v.contiguous(), k.contiguous(), q.contiguous(), reverse, out_f32);
+  return std::make_tuple(r[0], r[1]);
+}
+
+// ---- decode step ---------------------------------------------------------------------------------------------------
+std::optional<Tensor> decode_step(Tensor state, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
+                                  std::optional<torch::ScalarType> out_dtype) {
+  if (!state.defined() || !here(state) || state.dim() != 4 || state.scalar_type() != torch::kFloat32 || !state.is_contiguous()) return std::nullopt;
+  const int64_t B = state.size(0), H = state.size(1), D = state.size(2);
+  if (state.size(3) != D || v.dim() != 3 || v.size(0) != B || v.size(1) != H || v.size(2) != D) return std::nullopt;
+  for (const Tensor* t : {&g, &k, &q}) if (t->sizes() != v.sizes()) return std::nullopt;
+  for (const Tensor* t : {&g, &v, &k, &q}) if (t->device() != state.device()) return std::nullopt;
+  if (dt_of(v) < 0 || k.scalar_type() != v.scalar_type() || q.scalar_type() != v.scalar_type()) return std::nullopt;
+  const auto od = out_dtype.value_or(v.scalar_type());
+  if (od != torch::kFloat32 && od != torch::kBFloat16) return std::nullopt;
+  torch::NoGradGuard no_grad;
+  Tensor g32 = f32(g), vc = v.contiguous(), kc = k.contiguous(), qc = q.contiguous(), out = torch::empty({B, H, D}, v.options().dtype(od));
+  check(gla_decode_step(stream_of(v), B, H, D, dt_of(v), (float*)ptr(state), (const float*)ptr(g32), ptr(vc), ptr(kc), ptr(qc), ptr(out),
+                        dt_of(out)), "gla_decode_step");
+  return out;
+}
+
+// ---- scans ---------------------------------------------------------------------------------------------------------
+std::optional<Tensor> scan(int64_t op, const Tensor& src, int64_t axis, const std::optional<Tensor>& init, bool reverse,
+                           std::optional<torch::ScalarType> out_dtype) {
+  const int64_t nd = src.dim();
+  if (axis < 0) axis += nd;
+  if (!here(src) || dt_of(src) < 0 || axis < 0 || axis >= nd) return std::nullopt;
+  const auto od = out_dtype.value_or(src.scalar_type());
+  if (od != torch::kFloat32 && od != torch::kBFloat16) return std::nullopt;
+  int64_t N = 1, D = 1;
+  for (int64_t i = 0; i < axis; ++i) N *= src.size(i);
+  for (int64_t i = axis + 1; i < nd; ++i) D *= src.size(i);
+  torch::NoGradGuard no_grad;
+  Tensor i0;
+  if (init.has_value()) {
+    if (init->dim() != nd - 1 || init->device() != src.device()) return std::nullopt;
+    for (int64_t i = 0; i < nd - 1; ++i) if (init->size(i) != src.size(i < axis ? i : i + 1)) return std::nullopt;
+    i0 = init->to(src.scalar_type()).contiguous();
+  }
+  Tensor x = src.contiguous(), dst = torch::empty(src.sizes(), src.options().dtype(od));
+  check(gla_scan(stream_of(src), (int)op, N, src.size(axis), D, ptr(x), ptr(i0), ptr(dst), reverse, dt_of(src), dt_of(dst)), "gla_scan");
+  return dst;
+}
+std::optional<std::tuple<Tensor, Tensor>> rnn(const Tensor& g, const Tensor& kv, const std::optional<Tensor>& ig,
+                                              const std::optional<Tensor>& ikv, bool reverse, bool last_only) {
+  if (!here(kv) || (kv.dim() != 3 && kv.dim() != 4) || dt_of(kv) < 0 || ig.has_value() != ikv.has_value()) return std::nullopt;
+  const int b = kv.dim() == 4;
+  const int64_t N = b ? kv.size(0) : 1, T = kv.size(b), K = kv.size(b + 1), V = kv.size(b + 2);
+  if (g.dim() != 2 + b || (b && g.size(0) != N) || g.size(b) != T || g.size(b + 1) != K || g.device() != kv.device()) return std::nullopt;
+  torch::NoGradGuard no_grad;
+  Tensor g32 = f32(g), x = kv.contiguous(), ig32, ikvc;
+  if (ig.has_value()) {
+    if (ig->device() != kv.device() || ikv->device() != kv.device() || ig->numel() != N * K || ikv->numel() != N * K * V) return std::nullopt;
+    ig32 = f32(*ig);
+    ikvc = ikv->to(kv.scalar_type()).contiguous();
+  }
+  // every row is written, except with last_only, where the rows in between are documented as undefined but were zero
+  Tensor out_log = last_only ? torch::zeros_like(g32) : torch::empty_like(g32), out_state = last_only ? torch::zeros_like(x) : torch::empty_like(x);
+  const size_t n = last_only ? 0 : gla_rnn_scan_workspace_bytes(N, T, K, V);
+  Tensor ws = bytes(kv, n);
+  check(gla_rnn_scan_ws(stream_of(kv), N, T, K, V, (const float*)ptr(g32), ptr(x), (const float*)ptr(ig32), ptr(ikvc), (float*)ptr(out_log),
+                        ptr(out_state), reverse, last_only, dt_of(kv), ptr(ws), n), "gla_rnn_scan_ws");
+  return std::make_tuple(g.scalar_type() == torch::kFloat32 ? out_log : out_log.to(g.scalar_type()), out_state);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(gla_b200_host, m) {
+  using release = py::call_guard<py::gil_scoped_release>;
+  m.def("set_error_class", [](py::object c) { g_error = c.release().ptr(); });
+  m.def("chunk_gla", &chunk_gla, release());
+  m.def("recurrent_gla", &recurrent_gla, release());
+  m.def("decode_step", &decode_step, release());
+  m.def("scan", &scan, release());
+  m.def("rnn", &rnn, release());
+}

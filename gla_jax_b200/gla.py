@@ -10,9 +10,9 @@ All return ``(hidden_final, out)``.  Shapes are the reference's per-sequence sha
 adds a batch axis with ``jax.vmap`` (gla.py:1335), pass arrays with a leading batch axis
 instead (``(B, T, H, D)`` and ``(B, H, D, D)``) — the kernels take the batch natively.
 
-This adapter holds device memory in torch CUDA tensors and differentiates through
-``torch.autograd.Function`` objects that mirror the reference's ``jax.custom_vjp`` pairs
-(gla.py:362/441 and gla.py:628/655).  The JAX adapter (XLA FFI handlers plus
+This adapter holds device memory in torch CUDA tensors and differentiates through autograd
+nodes that mirror the reference's ``jax.custom_vjp`` pairs (gla.py:362/441 and gla.py:628/655);
+the nodes and the host path to the library calls are native (csrc/gla_host.cc).  The JAX adapter (XLA FFI handlers plus
 ``jax.custom_vjp``) is ``jax_ffi.py`` / ``csrc/gla_xla_ffi.cc``; both call the same C ABI.
 There is no CPU path: CPU tensors raise.
 """
@@ -34,9 +34,9 @@ def _ptr(t):
 _stream = _lib.stream_of
 
 
-def _prepare(hidden, log_fgate, value, key, query):
-    """Validate like the reference's trace-time asserts (gla.py:118-127, 498-500) and return
-    contiguous batched tensors plus whether a batch axis has to be stripped again."""
+def _refused(what, hidden, log_fgate, value, key, query):
+    """The native host path did not take these arguments: raise the error that says why (the reference's trace-time
+    asserts, gla.py:118-127, 498-500)."""
     if not value.is_cuda:
         raise RuntimeError("gla_jax_b200 operators need CUDA tensors; there is no CPU fallback")
     if value.dim() not in (3, 4):
@@ -45,18 +45,15 @@ def _prepare(hidden, log_fgate, value, key, query):
     if not (log_fgate.shape == value.shape == key.shape == query.shape):
         raise ValueError("log_fgate, value, key, query must have the same shape "
                          f"({tuple(log_fgate.shape)}, {tuple(value.shape)}, {tuple(key.shape)}, {tuple(query.shape)})")
-    if not batched:
-        hidden, log_fgate, value, key, query = (x.unsqueeze(0) for x in (hidden, log_fgate, value, key, query))
-    B, T, H, D = value.shape
-    if tuple(hidden.shape) != (B, H, D, D):
-        raise ValueError(f"hidden must be {'(B,' if batched else '('}H,D,D) = {(B, H, D, D)}, got {tuple(hidden.shape)}")
-    dt = value.dtype
-    if dt not in _DT:
-        raise TypeError(f"unsupported dtype {dt}: float32 and bfloat16 are implemented")
-    if not (key.dtype == query.dtype == hidden.dtype == dt):
+    want = (*value.shape[:-3], value.shape[-2], value.shape[-1], value.shape[-1])
+    if tuple(hidden.shape) != want:
+        raise ValueError(f"hidden must be {'(B,' if batched else '('}H,D,D) = {want}, got {tuple(hidden.shape)}")
+    if value.dtype not in _DT:
+        raise TypeError(f"unsupported dtype {value.dtype}: float32 and bfloat16 are implemented")
+    if not (key.dtype == query.dtype == hidden.dtype == value.dtype):
         raise TypeError("value, key, query and hidden must share one dtype")
-    return (hidden.contiguous(), log_fgate.contiguous(), value.contiguous(), key.contiguous(), query.contiguous(),
-            batched)
+    _stream(value.device)
+    raise ValueError(f"{what}: log_fgate must be a floating-point tensor and all arrays must be on {value.device}")
 
 
 def _chunk_fwd_raw(hidden, g32, v, k, q, chunk, impl, need_grad):
@@ -99,28 +96,6 @@ def _chunk_bwd_raw(g32, v, k, q, residuals, dhf, dout, chunk, impl):
     return dh, dg, dv, dk, dq
 
 
-class _ChunkGLA(torch.autograd.Function):
-    """custom-VJP pair of chunk_gla (gla.py:628-655)."""
-
-    @staticmethod
-    def forward(ctx, hidden, g, v, k, q, chunk, impl):
-        g32 = g if g.dtype == torch.float32 else g.float()
-        need_grad = any(ctx.needs_input_grad[:5])
-        hf, out, res = _chunk_fwd_raw(hidden, g32, v, k, q, chunk, impl, need_grad)
-        ctx.save_for_backward(g32, v, k, q, *res)
-        ctx.chunk, ctx.impl, ctx.g_dtype = chunk, impl, g.dtype
-        return hf, out
-
-    @staticmethod
-    def backward(ctx, dhf, dout):
-        g32, v, k, q, *res = ctx.saved_tensors
-        B, T, H, D = v.shape
-        dhf = torch.zeros(B, H, D, D, dtype=v.dtype, device=v.device) if dhf is None else dhf.to(v.dtype).contiguous()
-        dout = torch.zeros_like(v) if dout is None else dout.to(v.dtype).contiguous()
-        dh, dg, dv, dk, dq = _chunk_bwd_raw(g32, v, k, q, tuple(res), dhf, dout, ctx.chunk, ctx.impl)
-        return dh, dg.to(ctx.g_dtype), dv, dk, dq, None, None
-
-
 def chunk_gla(hidden_init, log_fgate, value, key, query, chunk_size: int,
               block_size_t: int = 64, block_size_d: int = 64, interpret: bool = False,
               num_warps: int = 4, num_stages: int = 2, impl: str = "auto") -> Tuple[torch.Tensor, torch.Tensor]:
@@ -132,59 +107,16 @@ def chunk_gla(hidden_init, log_fgate, value, key, query, chunk_size: int,
     ``"auto"`` (tensor cores when the shape has a kernel), ``"tcgen05"`` or ``"fp32"``.
     """
     del block_size_t, block_size_d, interpret, num_warps, num_stages
-    chunk_size = int(chunk_size)
+    chunk_size, impl = int(chunk_size), _lib.IMPL_BY_NAME[impl]
+    r = _lib.native().chunk_gla(hidden_init, log_fgate, value, key, query, chunk_size, impl)
+    if r is not None:
+        return r
     T = value.shape[-3]
     if chunk_size <= 0 or chunk_size & (chunk_size - 1):
         raise ValueError(f"Chunk length must be power of 2, but got {chunk_size}")   # gla.py:500
     if T % chunk_size:
         raise ValueError(f"sequence length {T} is not a multiple of chunk_size {chunk_size}")  # gla.py:674
-    h, g, v, k, q, batched = _prepare(hidden_init, log_fgate, value, key, query)
-    hf, out = _ChunkGLA.apply(h, g, v, k, q, chunk_size, _lib.IMPL_BY_NAME[impl])
-    return (hf, out) if batched else (hf[0], out[0])
-
-
-class _RecurrentGLA(torch.autograd.Function):
-    """custom-VJP pair of recurrent_gla (gla.py:362-388, 441)."""
-
-    @staticmethod
-    def forward(ctx, hidden, g, v, k, q, reverse, out_fp32):
-        lib = _lib.load()
-        B, T, H, D = v.shape
-        dt = _DT[v.dtype]
-        dev = v.device
-        g32 = g if g.dtype == torch.float32 else g.float()
-        hf = torch.empty_like(hidden)
-        out = torch.empty(v.shape, dtype=torch.float32 if out_fp32 else v.dtype, device=dev)
-        ws_n = lib.gla_recurrent_fwd_workspace_bytes(B, T, H, D, dt)
-        ws = torch.empty(ws_n, dtype=torch.uint8, device=dev) if ws_n else None
-        st = lib.gla_recurrent_fwd_ws(_stream(dev), B, T, H, D, dt, _ptr(hidden), _ptr(g32), _ptr(v), _ptr(k), _ptr(q),
-                                      _ptr(hf), _ptr(out), _DT[out.dtype], int(reverse), _ptr(ws), ws_n)
-        _lib.check(st, "gla_recurrent_fwd_ws")
-        ctx.save_for_backward(hidden, g32, v, k, q)
-        ctx.reverse, ctx.g_dtype = bool(reverse), g.dtype
-        return hf, out
-
-    @staticmethod
-    def backward(ctx, dhf, dout):
-        lib = _lib.load()
-        hidden, g32, v, k, q = ctx.saved_tensors
-        B, T, H, D = v.shape
-        dt = _DT[v.dtype]
-        dev = v.device
-        dhf = torch.zeros_like(hidden) if dhf is None else dhf.to(v.dtype).contiguous()
-        dout = torch.zeros_like(v) if dout is None else dout.contiguous()
-        if dout.dtype not in _DT:
-            dout = dout.float()
-        ws_n = lib.gla_recurrent_bwd_workspace_bytes(B, T, H, D, dt)
-        ws = torch.empty(ws_n, dtype=torch.uint8, device=dev)
-        dh = torch.empty_like(hidden)
-        dg = torch.empty_like(g32)
-        dv, dk, dq = torch.empty_like(v), torch.empty_like(k), torch.empty_like(q)
-        st = lib.gla_recurrent_bwd(_stream(dev), B, T, H, D, dt, _ptr(hidden), _ptr(g32), _ptr(v), _ptr(k), _ptr(q),
-                                   _ptr(dhf), _ptr(dout), _DT[dout.dtype], _ptr(dh), _ptr(dg), _ptr(dv), _ptr(dk),
-                                   _ptr(dq), int(ctx.reverse), _ptr(ws), ws_n)
-        _lib.check(st, "gla_recurrent_bwd")
-        return dh, dg.to(ctx.g_dtype), dv, dk, dq, None, None
+    return _refused("chunk_gla", hidden_init, log_fgate, value, key, query)
 
 
 def recurrent_gla(hidden_init, log_fgate, value, key, query, reverse: bool = False,
@@ -193,20 +125,20 @@ def recurrent_gla(hidden_init, log_fgate, value, key, query, reverse: bool = Fal
     """Exact recurrence that never writes hidden states to memory (reference: gla.py:405-439).
     ``max_block_size``, ``num_warps``, ``num_stages``, ``interpret`` are accepted and ignored."""
     del max_block_size, num_warps, num_stages, interpret
+    r = _lib.native().recurrent_gla(hidden_init, log_fgate, value, key, query, bool(reverse), False)
+    if r is not None:
+        return r
     if value.shape[-2] != key.shape[-2]:
         raise ValueError("value and key must have the same number of heads")   # gla.py:417
-    h, g, v, k, q, batched = _prepare(hidden_init, log_fgate, value, key, query)
-    hf, out = _RecurrentGLA.apply(h, g, v, k, q, bool(reverse), False)
-    return (hf, out) if batched else (hf[0], out[0])
+    return _refused("recurrent_gla", hidden_init, log_fgate, value, key, query)
 
 
 def recurrent_gla_naive(hidden, log_fgate, value, key, query, reverse: bool = False):
     """The definitional recurrence (reference: gla.py:26-47).  On this backend it runs the same
     on-chip recurrence kernel as ``recurrent_gla``; as in the reference ``out`` is float32
     and ``hidden_final`` keeps ``hidden``'s dtype (gla.py:43-46)."""
-    h, g, v, k, q, batched = _prepare(hidden, log_fgate, value, key, query)
-    hf, out = _RecurrentGLA.apply(h, g, v, k, q, bool(reverse), True)
-    return (hf, out) if batched else (hf[0], out[0])
+    r = _lib.native().recurrent_gla(hidden, log_fgate, value, key, query, bool(reverse), True)
+    return r if r is not None else _refused("recurrent_gla_naive", hidden, log_fgate, value, key, query)
 
 
 class _ChunkGLAPacked(torch.autograd.Function):
@@ -312,22 +244,19 @@ def decode_step(state, log_fgate, value, key, query, out_dtype=None):
     ``out = query @ S`` of shape (B, H, D) in ``out_dtype`` (default: value's dtype).  ``log_fgate``,
     ``value``, ``key``, ``query`` are (B, H, D).  T calls equal one ``recurrent_gla`` over T tokens
     (``hidden_init`` -> ``hidden_final`` chaining, gla.py:720-723).  Not differentiable (serving path)."""
-    lib = _lib.load()
+    out = _lib.native().decode_step(state, log_fgate, value, key, query, out_dtype)
+    if out is not None:
+        return out
     if state.dtype != torch.float32 or not state.is_contiguous() or state.dim() != 4:
         raise TypeError("decode_step: state must be a contiguous float32 (B, H, D, D) tensor")
     B, H, D, D2 = state.shape
     if D != D2 or tuple(value.shape) != (B, H, D) or key.shape != value.shape or query.shape != value.shape \
             or log_fgate.shape != value.shape:
         raise ValueError("decode_step: expected state (B, H, D, D) and log_fgate, value, key, query (B, H, D)")
-    if key.dtype != value.dtype or query.dtype != value.dtype:
-        raise TypeError("decode_step: value, key, query must share a dtype")
-    g32 = log_fgate.float().contiguous()
-    v, k, q = value.contiguous(), key.contiguous(), query.contiguous()
-    out = torch.empty(B, H, D, dtype=out_dtype or v.dtype, device=v.device)
-    st = lib.gla_decode_step(_stream(v.device), B, H, D, _DT[v.dtype], _ptr(state), _ptr(g32), _ptr(v), _ptr(k), _ptr(q),
-                             _ptr(out), _DT[out.dtype])
-    _lib.check(st, "gla_decode_step")
-    return out
+    if key.dtype != value.dtype or query.dtype != value.dtype or value.dtype not in _DT or (out_dtype or value.dtype) not in _DT:
+        raise TypeError("decode_step: value, key, query must share a dtype, float32 or bfloat16")
+    _stream(value.device)
+    raise RuntimeError("decode_step needs CUDA tensors on one device; there is no CPU fallback")
 
 
 def auto_block_size(value_dim: int, key_dim: int, num_heads: int, max_block_size: int):

@@ -35,32 +35,20 @@ def scan(op: str, src, axis: int, init: Optional[torch.Tensor] = None, reverse: 
     """Inclusive associative scan of one array along ``axis`` under a named combine rule (``SCAN_OPS``), float32
     math, with ``init`` (shape = src.shape without ``axis``) combined in front of every prefix: the generic scan of
     the reference (ops.py:82-104) for the rules a precompiled library can offer."""
-    _need_cuda(src)
     if op not in SCAN_OPS:
+        _need_cuda(src)
         raise NotImplementedError(f"scan: unknown combine rule {op!r}; available: {sorted(SCAN_OPS)}")
-    lib = _lib.load()
-    nd = src.dim()
-    axis = axis if axis >= 0 else axis + nd
-    pre, T, post = src.shape[:axis], src.shape[axis], src.shape[axis + 1:]
-    N = 1
-    for s in pre:
-        N *= s
-    D = 1
-    for s in post:
-        D *= s
-    if src.dtype not in _DT:
-        raise TypeError(f"unsupported dtype {src.dtype}")
-    out_dtype = out_dtype or src.dtype
-    x = src.contiguous()
-    if init is not None:
-        if tuple(init.shape) != tuple(pre) + tuple(post):
-            raise ValueError(f"init must have shape {tuple(pre) + tuple(post)}, got {tuple(init.shape)}")  # ops.py:184
-        init = init.to(src.dtype).contiguous()
-    dst = torch.empty(src.shape, dtype=out_dtype, device=src.device)
-    st = lib.gla_scan(_stream(src.device), SCAN_OPS[op], N, T, D, x.data_ptr(), None if init is None else init.data_ptr(),
-                      dst.data_ptr(), int(reverse), _DT[src.dtype], _DT[out_dtype])
-    _lib.check(st, "gla_scan")
-    return dst
+    dst = _lib.native().scan(SCAN_OPS[op], src, axis, init, reverse, out_dtype)
+    if dst is not None:
+        return dst
+    _need_cuda(src)
+    _stream(src.device)
+    axis = axis if axis >= 0 else axis + src.dim()
+    if src.dtype not in _DT or (out_dtype or src.dtype) not in _DT:
+        raise TypeError(f"unsupported dtype {src.dtype if src.dtype not in _DT else out_dtype}")
+    want = tuple(src.shape[:axis]) + tuple(src.shape[axis + 1:])
+    raise ValueError(f"init must have shape {want} and lie on {src.device}, got "
+                     f"{None if init is None else tuple(init.shape)}")  # ops.py:184
 
 
 def cumsum_pallas(src, axis: int, init: Optional[torch.Tensor] = None, reverse: bool = False,
@@ -92,36 +80,18 @@ def rnn_pallas(log_fgate, kv, init_log_fgate: Optional[torch.Tensor] = None,
     (reference: ops.py:338-394, kernel ops.py:299-334).  With ``last_only`` only the final row
     (first row when reversed) is defined, as in the reference's masked store.  A leading
     batch axis on all arguments is accepted (the reference vmaps, ops.py:432,447)."""
+    r = _lib.native().rnn(log_fgate, kv, init_log_fgate, init_kv, reverse, last_only)
+    if r is not None:
+        return r
     _need_cuda(kv)
-    lib = _lib.load()
+    _stream(kv.device)
     if (init_log_fgate is None) != (init_kv is None):
         raise ValueError("init_log_fgate and init_kv must be given together")   # ops.py:351
-    batched = kv.dim() == 4
-    if not batched:
-        log_fgate, kv = log_fgate.unsqueeze(0), kv.unsqueeze(0)
-        if init_kv is not None:
-            init_log_fgate, init_kv = init_log_fgate.unsqueeze(0), init_kv.unsqueeze(0)
-    Bn, T, K, V = kv.shape
-    if tuple(log_fgate.shape) != (Bn, T, K):
-        raise ValueError(f"log_fgate must be {(T, K)}, got {tuple(log_fgate.shape[1:])}")   # ops.py:348
+    if kv.dim() not in (3, 4) or tuple(log_fgate.shape) != tuple(kv.shape[:-1]):
+        raise ValueError(f"log_fgate must be {tuple(kv.shape[-3:-1])}, got {tuple(log_fgate.shape)}")   # ops.py:348
     if kv.dtype not in _DT:
         raise TypeError(f"unsupported dtype {kv.dtype}")
-    g = log_fgate.float().contiguous()
-    x = kv.contiguous()
-    ig = None if init_log_fgate is None else init_log_fgate.float().contiguous()
-    ikv = None if init_kv is None else init_kv.to(kv.dtype).contiguous()
-    out_log = torch.zeros(Bn, T, K, dtype=torch.float32, device=kv.device)
-    out_state = torch.zeros_like(x)
-    # scratch for long axes with few rows (0 bytes when the plain scan serves)
-    nws = 0 if last_only else lib.gla_rnn_scan_workspace_bytes(Bn, T, K, V)
-    ws = torch.empty(nws, dtype=torch.uint8, device=kv.device) if nws else None
-    st = lib.gla_rnn_scan_ws(_stream(kv.device), Bn, T, K, V, g.data_ptr(), x.data_ptr(),
-                             None if ig is None else ig.data_ptr(), None if ikv is None else ikv.data_ptr(),
-                             out_log.data_ptr(), out_state.data_ptr(), int(reverse), int(last_only), _DT[kv.dtype],
-                             None if ws is None else ws.data_ptr(), nws)
-    _lib.check(st, "gla_rnn_scan_ws")
-    out_log = out_log.to(log_fgate.dtype)
-    return (out_log, out_state) if batched else (out_log[0], out_state[0])
+    raise ValueError("rnn_pallas: the initial pair must have the shapes of one row and all arrays must be on one device")
 
 
 def rnn_recursive(log_fgate, kv, init_log_fgate: Optional[torch.Tensor] = None,
