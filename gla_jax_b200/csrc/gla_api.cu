@@ -136,7 +136,7 @@ int gla_scan(void* stream, int op, int64_t N, int64_t T, int64_t D, const void* 
   GLA_TRY(check_dtype(in_dtype));
   GLA_TRY(check_dtype(out_dtype));
   return launch_cumsum((cudaStream_t)stream, N, T, D, src, init, dst, reverse, in_dtype == GLA_BF16,
-                       out_dtype == GLA_BF16, nullptr, nullptr, op);
+                       out_dtype == GLA_BF16, nullptr, op);
 }
 
 int gla_rnn_scan(void* stream, int64_t batch, int64_t T, int64_t K, int64_t V, const float* log_fgate,

@@ -472,8 +472,7 @@ int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, i
 }
 
 size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
-  const size_t n = 2 * align_up((size_t)B * T * H * D * 4, 256) + align_up((size_t)B * H * D * 4, 256) +
-                   align_up(cumsum_scratch_bytes(B, T, H * D), 256);
+  const size_t n = 2 * align_up((size_t)B * T * H * D * 4, 256) + align_up((size_t)B * H * D * 4, 256);
   const size_t px = rec_chunked(T, D) ? 2 * px_state_bytes(B, T, H, D) : 0;      // states and gradient states
   return px > n ? px : n;
 }
@@ -494,11 +493,10 @@ int recurrent_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, i
   p.E = (float*)ws;
   p.F = (float*)((char*)ws + plane);
   p.boundary = (float*)((char*)ws + 2 * plane);
-  float* seg_sums = (float*)((char*)ws + 2 * plane + align_up((size_t)B * H * D * 4, 256));
   p.time_reversed = reverse;
   GLA_TRY(launch_rec_bwd_d(st, (int)D, p));
   // dg[t] = sum over the tokens processed at or after t of (E - F), plus the boundary term
-  return launch_cumsum(st, B, T, H * D, p.E, p.boundary, dg, reverse ? 0 : 1, 0, 0, p.F, seg_sums);
+  return launch_cumsum(st, B, T, H * D, p.E, p.boundary, dg, reverse ? 0 : 1, 0, 0, p.F);
 }
 
 }  // namespace gla

@@ -9,16 +9,13 @@
 #include "gla_common.cuh"
 #include "tc_ptx.cuh"
 #include "tma_maps.cuh"
+#include <cmath>
 
 namespace gla {
 
 // ---------------------------------------------------------------------------------------
 // cumsum: src (N, T, D) -> dst (N, T, D), inclusive along T, + init (N, D).
-// Block = 32 column lanes x 8 row lanes; a tile is 64 rows; each thread scans 8
-// consecutive rows of one column in registers, row lanes are combined through shared memory.
 // ---------------------------------------------------------------------------------------
-constexpr int CS_RPT = 8;    // rows per thread
-constexpr int CS_RL = 8;     // row lanes
 
 // The combine rules of the scan library (gla_scan_op): each is associative with an identity element, which is what
 // the tiled scan needs (padding, carries, segment totals).  ops.py:82-104 scans with an arbitrary traced function;
@@ -39,82 +36,156 @@ struct OpLogAddExp {      // log(exp(a) + exp(b)), evaluated around the larger a
   }
 };
 
-// The scan axis may be cut into `nseg` segments of `seg_len` positions (in scan order) that run
-// as separate blocks: a first launch with TOTALS = true leaves every segment's column sums in
-// `totals` (N, nseg, D); the second adds the sums of the segments before its own to its carry.
-// nseg = 1 with totals = nullptr is the plain one-pass scan.
-template <typename TI, typename TO, bool TOTALS, typename OP>
-__global__ void __launch_bounds__(256) cumsum_kernel(const TI* __restrict__ src, const TI* __restrict__ sub,
-                                                     const TI* __restrict__ init, TO* __restrict__ dst, int64_t T,
-                                                     int64_t D, int reverse, int nseg, int64_t seg_len,
-                                                     float* __restrict__ totals) {
-  __shared__ float tot[CS_RL][33];
-  const int64_t n = blockIdx.x / nseg;
-  const int seg = (int)(blockIdx.x % nseg);
-  const int tx = threadIdx.x, rl = threadIdx.y;
-  const int64_t c = (int64_t)blockIdx.y * 32 + tx;
-  const bool cvalid = c < D;
-  float carry = (!TOTALS && init != nullptr && cvalid) ? ld_f(init, n * D + c) : OP::id();
-  if (!TOTALS && totals != nullptr && cvalid)
-    for (int s2 = 0; s2 < seg; ++s2) carry = OP::f(carry, totals[(n * nseg + s2) * D + c]);
-  const TI* s = src + n * T * D;
-  const TI* s2 = sub ? sub + n * T * D : nullptr;   // optional second source, subtracted element-wise
-  TO* o = dst + n * T * D;
-  const int64_t tbeg = (int64_t)seg * seg_len;
-  const int64_t tend = tbeg + seg_len < T ? tbeg + seg_len : T;
-  // The loads of the NEXT tile are issued before the current one is combined: a block walks its rows in order, so
-  // without this every tile would wait out a full memory latency with nothing in flight.
-  auto fetch = [&](int64_t t0, float (&y)[CS_RPT]) {
+// One scan kernel for every layout.  What bounds it is HBM, so what counts is how many bytes are in flight and that
+// every byte moves once, also when the array has few rows and a long axis: a block of 32 column lanes x 8 row lanes
+// holds 8 RPT rows of 32 VEC columns in registers, and up to sixteen blocks of a thread-block cluster take consecutive
+// pieces of the axis and exchange their totals through distributed shared memory, so that the axis is cut over
+// blocks without a second pass over the data.  A row segment is one coalesced access per warp (128 to 512 bytes) at
+// any width and alignment.  A thread holds 32 values, so that four blocks fit an SM and 128 KB of loads are in flight
+// there; other blocks' loads cover a block's combine phase (prefetching the next tile in registers instead halves
+// the blocks: measured slower).  Longer axes are walked in steps of a cluster's rows with the carry in registers.
+// Measured, float32 (N, T, D) unless marked, us before (a ring of TMA tiles, one block per 128 columns) -> now, and the
+// time of the bytes at the copy rate: (24, 4096, 136) 70 -> 27, 16; (96, 4096, 128) 72 -> 72, 62; (512, 128, 768)
+// 75 -> 63, 62; (1, 16384, 96) 385 -> 12, 2; (2, 16384, 1024) 263 -> 64, 41; bf16 (9, 1342, 808) 37 -> 17, 6.
+constexpr int SK_RL = 8;      // row lanes
+constexpr int SK_MAXCL = 16;  // blocks of a cluster, at most (above 8: opt-in)
+template <typename T, int VEC> __device__ __forceinline__ void sk_load(const T* p, float (&y)[VEC]) {
+  if constexpr (VEC == 1) y[0] = ld_f(p, 0);
+  else if constexpr (sizeof(T) == 4 && VEC == 2) { const float2 u = __ldg(reinterpret_cast<const float2*>(p)); y[0] = u.x; y[1] = u.y; }
+  else if constexpr (sizeof(T) == 4) { const float4 u = __ldg(reinterpret_cast<const float4*>(p)); y[0] = u.x; y[1] = u.y; y[2] = u.z; y[3] = u.w; }
+  else {
 #pragma unroll
-    for (int r = 0; r < CS_RPT; ++r) {
-      int64_t tt = t0 + rl * CS_RPT + r;
-      int64_t tp = reverse ? (T - 1 - tt) : tt;
-      y[r] = (cvalid && tt < tend) ? ld_f(s, tp * D + c) : OP::id();
-      if (s2 && cvalid && tt < tend) y[r] -= ld_f(s2, tp * D + c);
+    for (int i = 0; i < VEC; i += 2) {
+      const uint32_t u = __ldg(reinterpret_cast<const unsigned int*>(p) + i / 2);
+      y[i] = __uint_as_float(u << 16); y[i + 1] = __uint_as_float(u & 0xffff0000u);
     }
-  };
-  float xn[CS_RPT];
-  fetch(tbeg, xn);
-  for (int64_t t0 = tbeg; t0 < tend; t0 += CS_RPT * CS_RL) {
-    float x[CS_RPT];
-#pragma unroll
-    for (int r = 0; r < CS_RPT; ++r) x[r] = xn[r];
-    if (t0 + CS_RPT * CS_RL < tend) fetch(t0 + CS_RPT * CS_RL, xn);
-#pragma unroll
-    for (int r = 1; r < CS_RPT; ++r) x[r] = OP::f(x[r - 1], x[r]);
-    if (TOTALS) {
-      // the row lanes hold consecutive pieces of the tile: combined in order after the loop (each lane keeps the
-      // running combination of ITS pieces, which is only order-safe for commutative rules; all rules here are)
-      carry = OP::f(carry, x[CS_RPT - 1]);
-      continue;
-    }
-    tot[rl][tx] = x[CS_RPT - 1];
-    __syncthreads();
-    float off = carry, total = OP::id();
-#pragma unroll
-    for (int r2 = 0; r2 < CS_RL; ++r2) {
-      float v = tot[r2][tx];
-      if (r2 < rl) off = OP::f(off, v);
-      total = OP::f(total, v);
-    }
-#pragma unroll
-    for (int r = 0; r < CS_RPT; ++r) {
-      int64_t tt = t0 + rl * CS_RPT + r;
-      int64_t tp = reverse ? (T - 1 - tt) : tt;
-      if (cvalid && tt < tend) st_f(o, tp * D + c, OP::f(off, x[r]));
-    }
-    carry = OP::f(carry, total);
-    __syncthreads();
   }
-  if (TOTALS) {
-    tot[rl][tx] = carry;
-    __syncthreads();
-    if (rl == 0 && cvalid) {
-      float total = OP::id();
+}
+template <typename T, int VEC> __device__ __forceinline__ void sk_store(T* p, const float (&y)[VEC]) {
+  if constexpr (VEC == 1) st_f(p, 0, y[0]);
+  else if constexpr (sizeof(T) == 4 && VEC == 2) *reinterpret_cast<float2*>(p) = make_float2(y[0], y[1]);
+  else if constexpr (sizeof(T) == 4) *reinterpret_cast<float4*>(p) = make_float4(y[0], y[1], y[2], y[3]);
+  else {
 #pragma unroll
-      for (int r2 = 0; r2 < CS_RL; ++r2) total = OP::f(total, tot[r2][tx]);
-      totals[(n * nseg + seg) * D + c] = total;
+    for (int i = 0; i < VEC; i += 2) *(reinterpret_cast<uint32_t*>(p) + i / 2) = tc::pack_bf16x2(y[i], y[i + 1]);
+  }
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <typename TI, typename TO, typename OP, int VEC, int RPT>
+__global__ void __launch_bounds__(32 * SK_RL, 4) scan_kernel(const TI* __restrict__ src, const TI* __restrict__ sub,
+                                                          const TI* __restrict__ init, TO* __restrict__ dst, int64_t T,
+                                                          int64_t D, int gy, int cl, int reverse) {
+  __shared__ float tot[2][SK_RL][32 * VEC];        // totals of the row lanes, double-buffered by tile parity
+  __shared__ float peer[2][SK_MAXCL][32 * VEC];         // totals of the cluster's blocks; every block writes its own into all
+  const int tx = threadIdx.x, rl = threadIdx.y;
+  const int rank = (int)(blockIdx.x % cl);
+  const int64_t item = blockIdx.x / cl, n = item / gy;
+  const int64_t c = (item % gy) * (32 * VEC) + tx * VEC;
+  const bool cvalid = c < D;                        // VEC divides D
+  constexpr int ROWS = SK_RL * RPT;
+  float carry[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) carry[v] = OP::id();
+  if (init != nullptr && cvalid) sk_load<TI, VEC>(init + n * D + c, carry);
+  // scan position p lies at row p (forward) or T - 1 - p (reversed); a thread's rows are `rs` elements apart
+  const int64_t rs = reverse ? -D : D, p0 = (int64_t)rank * ROWS + rl * RPT;
+  const int64_t off0 = n * T * D + c + (reverse ? T - 1 - p0 : p0) * D, step = (int64_t)cl * ROWS;
+  const TI* ps = src + off0;
+  const TI* ps2 = sub ? sub + off0 : nullptr;
+  TO* po = dst + off0;
+  auto rows_in = [&](int64_t t0) -> int {           // this thread's rows inside the axis for the step at t0
+    const int64_t left = T - (t0 + p0);
+    return !cvalid || left <= 0 ? 0 : left < RPT ? (int)left : RPT;
+  };
+  auto fetch = [&](int nr, float (&y)[RPT][VEC]) {
+    if (nr == RPT) {                                // whole tiles: nothing between the loads
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) sk_load<TI, VEC>(ps + r * rs, y[r]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) y[r][v] = OP::id();
+        if (r < nr) sk_load<TI, VEC>(ps + r * rs, y[r]);
+      }
     }
+    if (ps2) {
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+        if (r < nr) {
+          float z[VEC];
+          sk_load<TI, VEC>(ps2 + r * rs, z);
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) y[r][v] -= z[v];
+        }
+      ps2 += step * rs;
+    }
+    ps += step * rs;
+  };
+  if (cl > 1) cluster_barrier();                    // every block of the cluster runs before one writes to another
+  int par = 0;
+  for (int64_t t0 = 0; t0 < T; t0 += step, par ^= 1) {
+    float x[RPT][VEC];
+    const int nr = rows_in(t0);
+    fetch(nr, x);
+#pragma unroll
+    for (int r = 1; r < RPT; ++r)
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) x[r][v] = OP::f(x[r - 1][v], x[r][v]);
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) tot[par][rl][v * 32 + tx] = x[RPT - 1][v];
+    __syncthreads();
+    float off[VEC], all[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) {
+      float lower = OP::id(), sum = OP::id();
+#pragma unroll
+      for (int r = 0; r < SK_RL; ++r) {
+        const float y = tot[par][r][v * 32 + tx];
+        if (r < rl) lower = OP::f(lower, y);
+        sum = OP::f(sum, y);
+      }
+      off[v] = lower;
+      all[v] = sum;
+    }
+    if (cl > 1) {
+      for (int to = rl; to < cl; to += SK_RL) {     // row lane r hands the block's totals to blocks r, r + 8 of the cluster
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+          uint32_t a = tc::smem_u32(&peer[par][rank][v * 32 + tx]);
+          asm volatile("{\n\t.reg .u32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.f32 [ra], %2;\n\t}"
+                       :: "r"(a), "r"(to), "f"(all[v]) : "memory");
+        }
+      }
+      // a buffer is rewritten two steps later, past a barrier that every reader of it has arrived at
+      cluster_barrier();
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        float before = carry[v];
+        for (int k = 0; k < cl; ++k) {
+          if (k == rank) off[v] = OP::f(before, off[v]);
+          before = OP::f(before, peer[par][k][v * 32 + tx]);
+        }
+        carry[v] = before;
+      }
+    } else {
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        off[v] = OP::f(carry[v], off[v]);
+        carry[v] = OP::f(carry[v], all[v]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RPT; ++r)
+      if (r < nr) {
+        float y[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) y[v] = OP::f(off[v], x[r][v]);
+        sk_store<TO, VEC>(po + r * rs, y);
+      }
+    po += step * rs;
   }
 }
 
@@ -133,107 +204,13 @@ __device__ __forceinline__ void st4_f(bf16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-
-// The same scan with FOUR consecutive columns per thread (16-byte accesses: a warp reads 512 contiguous bytes of a
-// row) and 16 row lanes: a block covers 128 columns and walks the axis in tiles of 128 rows, 64 KB of float32 per
-// tile with the next tile's loads already in flight.  Rows this wide keep the memory system busy from few blocks,
-// which is what a long scan axis with few rows offers.  Serves D % 4 == 0 with suitably aligned pointers.
-constexpr int C4_RL = 16;    // row lanes
 template <typename OP> __device__ __forceinline__ float4 op4(float4 a, float4 b) {
   return make_float4(OP::f(a.x, b.x), OP::f(a.y, b.y), OP::f(a.z, b.z), OP::f(a.w, b.w));
 }
-template <typename TI, typename TO, bool TOTALS, typename OP>
-__global__ void __launch_bounds__(32 * C4_RL) cumsum_v4_kernel(const TI* __restrict__ src, const TI* __restrict__ sub,
-                                                               const TI* __restrict__ init, TO* __restrict__ dst,
-                                                               int64_t T, int64_t D, int reverse, int nseg,
-                                                               int64_t seg_len, float* __restrict__ totals) {
-  // both arrays are double-buffered by tile parity, which is what lets a tile get by with ONE block barrier: a
-  // buffer is rewritten two tiles later, after a barrier that every reader of it has passed
-  __shared__ float4 tot[2][C4_RL][32];
-  __shared__ float4 car[2][32];
-  const int64_t n = blockIdx.x / nseg;
-  const int seg = (int)(blockIdx.x % nseg);
-  const int tx = threadIdx.x, rl = threadIdx.y;
-  const int64_t c = ((int64_t)blockIdx.y * 32 + tx) * 4;
-  const bool cvalid = c < D;
-  const float4 ident = make_float4(OP::id(), OP::id(), OP::id(), OP::id());
-  float4 carry = (!TOTALS && init != nullptr && cvalid) ? ld4_f(init + n * D + c) : ident;
-  if (!TOTALS && totals != nullptr && cvalid)
-    for (int s2 = 0; s2 < seg; ++s2)
-      carry = op4<OP>(carry, *reinterpret_cast<const float4*>(totals + (n * nseg + s2) * D + c));
-  const int64_t tbeg = (int64_t)seg * seg_len;
-  const int64_t tend = tbeg + seg_len < T ? tbeg + seg_len : T;
-  // a thread's rows of a tile are `rs` elements apart (backwards in memory for a reversed scan) and its first row
-  // moves by a whole tile per iteration: no multiplication and no 64-bit compare inside the loop
-  const int64_t rs = reverse ? -D : D;
-  const int64_t row0 = tbeg + rl * CS_RPT;
-  const int64_t off0 = n * T * D + c + (reverse ? (T - 1 - row0) : row0) * D;
-  const TI* ps = src + off0;
-  const TI* ps2 = sub ? sub + off0 : nullptr;
-  TO* po = dst + off0;
-  const int64_t step = (int64_t)CS_RPT * C4_RL * rs;
-  // rows of this thread that lie inside the segment, for the tile being fetched / stored (<= 0: none)
-  auto rows_in = [&](int64_t t0) -> int {
-    const int64_t left = tend - (t0 + rl * CS_RPT);
-    return !cvalid ? 0 : left >= CS_RPT ? CS_RPT : left < 0 ? 0 : (int)left;
-  };
-  auto fetch = [&](int nr, float4 (&y)[CS_RPT]) {
-#pragma unroll
-    for (int r = 0; r < CS_RPT; ++r) {
-      y[r] = r < nr ? ld4_f(ps + r * rs) : ident;
-      if (ps2 && r < nr) {
-        const float4 z = ld4_f(ps2 + r * rs);
-        y[r].x -= z.x; y[r].y -= z.y; y[r].z -= z.z; y[r].w -= z.w;
-      }
-    }
-    ps += step;
-    if (ps2) ps2 += step;
-  };
-  float4 xn[CS_RPT];
-  fetch(rows_in(tbeg), xn);
-  if (!TOTALS) {
-    if (rl == C4_RL - 1) car[0][tx] = carry;
-  }
-  int par = 0;
-  for (int64_t t0 = tbeg; t0 < tend; t0 += CS_RPT * C4_RL, par ^= 1) {
-    float4 x[CS_RPT];
-#pragma unroll
-    for (int r = 0; r < CS_RPT; ++r) x[r] = xn[r];
-    const int nr = rows_in(t0);
-    if (t0 + CS_RPT * C4_RL < tend) fetch(rows_in(t0 + CS_RPT * C4_RL), xn);
-#pragma unroll
-    for (int r = 1; r < CS_RPT; ++r) x[r] = op4<OP>(x[r - 1], x[r]);
-    if (TOTALS) {
-      carry = op4<OP>(carry, x[CS_RPT - 1]);    // commutative rules only, as in the scalar form
-      continue;
-    }
-    tot[par][rl][tx] = x[CS_RPT - 1];
-    __syncthreads();
-    // the carry into this tile (left by the last row lane at the end of the tile before) combined with the row
-    // lanes before this one: the trip count is the same for the whole warp
-    float4 off = car[par][tx];
-    for (int r2 = 0; r2 < rl; ++r2) off = op4<OP>(off, tot[par][r2][tx]);
-    if (rl == C4_RL - 1) car[par ^ 1][tx] = op4<OP>(off, x[CS_RPT - 1]);
-#pragma unroll
-    for (int r = 0; r < CS_RPT; ++r)
-      if (r < nr) st4_f(po + r * rs, op4<OP>(off, x[r]));
-    po += step;
-  }
-  if (TOTALS) {
-    tot[0][rl][tx] = carry;
-    __syncthreads();
-    if (rl == 0 && cvalid) {
-      float4 total = ident;
-#pragma unroll
-      for (int r2 = 0; r2 < C4_RL; ++r2) total = op4<OP>(total, tot[0][r2][tx]);
-      *reinterpret_cast<float4*>(totals + (n * nseg + seg) * D + c) = total;
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------------------
-// The float32 scan of wide rows as a TMA pipeline.  What limits the kernels above on a long axis is how many bytes
-// a thread block can keep in flight with ordinary loads; here a 64-row x 128-column tile travels as ONE tensor copy
+// The float32 scan of wide rows as a TMA pipeline.  Serves the shapes whose column blocks
+// nearly fill the device once but not evenly with smaller blocks (see scan_ring_us).  A 64-row x 128-column tile travels
+// as ONE tensor copy
 // (cp.async.bulk.tensor over a 3-d map (column, row, n): rows past the end of the axis and columns past D are
 // zero-filled on the way in and skipped on the way out) into a ring of NST shared-memory stages, the threads scan
 // a landed tile out of shared memory, write the result into one of two staging tiles, and a tensor store takes it
@@ -241,7 +218,7 @@ __global__ void __launch_bounds__(32 * C4_RL) cumsum_v4_kernel(const TI* __restr
 // measured first: 128 copy instructions per tile made the kernel twice as slow as the load/store one.)
 //   thread 0       issues the copy of tile i + NST once tile i has been read
 //   thread 32      issues the store of tile i and waits for the store of tile i - 2 to have read its stage
-//   all 8 warps    thread = four columns x eight consecutive scan positions; row lanes combine as in the kernel above
+//   all 8 warps    thread = four columns x eight consecutive scan positions; row lanes combine through shared memory
 // A reversed scan walks the tiles from the end of the axis; its tiles are laid out so that every one but the FIRST
 // in scan order starts on a multiple of 64 rows from the end (no store ever starts at a negative row), and a
 // thread's scan position p sits in stage row nr - 1 - p.
@@ -251,8 +228,9 @@ __global__ void __launch_bounds__(32 * C4_RL) cumsum_v4_kernel(const TI* __restr
 namespace {
 using namespace tc;
 __device__ unsigned int g_scan_wait_timeouts = 0;
+constexpr int BK_RPT = 8;                      // rows per thread
 constexpr int BK_RL = 8;                       // row lanes
-constexpr int BK_ROWS = CS_RPT * BK_RL;        // rows of a tile (64)
+constexpr int BK_ROWS = BK_RPT * BK_RL;        // rows of a tile (64)
 constexpr int BK_NST = 4;                      // input stages
 constexpr int BK_TILE = BK_ROWS * 128 * 4;     // bytes of a tile (32 KB)
 constexpr int BK_SMEM = (BK_NST + 2) * BK_TILE + 1024;
@@ -333,16 +311,16 @@ __global__ void __launch_bounds__(32 * BK_RL, 1) cumsum_tma_kernel(const __grid_
     const bool cvalid = (int64_t)c0 + tx * 4 < D;
     ok = mbar_wait(full0 + 8 * st, phase);       // on expiry the tile is garbage: voted on below
     const int nrt = rows_of(i);
-    const int nr = nrt - rl * CS_RPT;                 // this thread's scan positions inside the tile (<= 0: none)
+    const int nr = nrt - rl * BK_RPT;                 // this thread's scan positions inside the tile (<= 0: none)
     // scan position p = 8 rl + r of the tile sits in stage row p (forward) or nrt - 1 - p (reversed)
-    const int row0 = reverse ? nrt - 1 - rl * CS_RPT : rl * CS_RPT, rstep = reverse ? -32 : 32;
+    const int row0 = reverse ? nrt - 1 - rl * BK_RPT : rl * BK_RPT, rstep = reverse ? -32 : 32;
     const float4* in = reinterpret_cast<const float4*>(sm + st * BK_TILE) + row0 * 32 + tx;
-    float4 x[CS_RPT];
+    float4 x[BK_RPT];
 #pragma unroll
-    for (int r = 0; r < CS_RPT; ++r) x[r] = (cvalid && r < nr) ? in[r * rstep] : ident;
+    for (int r = 0; r < BK_RPT; ++r) x[r] = (cvalid && r < nr) ? in[r * rstep] : ident;
 #pragma unroll
-    for (int r = 1; r < CS_RPT; ++r) x[r] = op4<OP>(x[r - 1], x[r]);
-    tot[par][rl][tx] = x[CS_RPT - 1];
+    for (int r = 1; r < BK_RPT; ++r) x[r] = op4<OP>(x[r - 1], x[r]);
+    tot[par][rl][tx] = x[BK_RPT - 1];
     // the staging tile that this tile is about to write was last read by the store of two tiles ago: all but the
     // newest store group must have read their stage
     if (tid == 32) bulk_wait_read<1>();
@@ -357,10 +335,10 @@ __global__ void __launch_bounds__(32 * BK_RL, 1) cumsum_tma_kernel(const __grid_
     if (last_tile) { const int64_t nx = item + gridDim.x; n2 = (int)(nx / gy); c2 = (int)(nx % gy) * 128; }
     // the carry into the next tile: this item's running value, or the next item's initial value
     if (rl == BK_RL - 1)
-      car[par ^ 1][tx] = !last_tile ? op4<OP>(off, x[CS_RPT - 1]) : item + gridDim.x < items ? init_of(n2, c2) : ident;
+      car[par ^ 1][tx] = !last_tile ? op4<OP>(off, x[BK_RPT - 1]) : item + gridDim.x < items ? init_of(n2, c2) : ident;
     float4* o = reinterpret_cast<float4*>(sm + (BK_NST + par) * BK_TILE) + row0 * 32 + tx;
 #pragma unroll
-    for (int r = 0; r < CS_RPT; ++r)
+    for (int r = 0; r < BK_RPT; ++r)
       if (r < nr) o[r * rstep] = op4<OP>(off, x[r]);
     fence_async_smem();                                // the staging tile is read by the async proxy
     __syncthreads();
@@ -390,6 +368,7 @@ unsigned int scan_read_wait_timeouts() {
 template <typename OP>
 static int launch_cumsum_tma_op(cudaStream_t st, int64_t N, int64_t T, int64_t D, const float* src, const float* init, float* dst,
                                 int reverse) {
+  ProfScope ps("cumsum_kernel", st);
   static SmemAttrOnce attr[2];
   GLA_TRY(attr[0].ensure(cumsum_tma_kernel<OP, false>, BK_SMEM));
   GLA_TRY(attr[1].ensure(cumsum_tma_kernel<OP, true>, BK_SMEM));
@@ -403,107 +382,107 @@ static int launch_cumsum_tma_op(cudaStream_t st, int64_t N, int64_t T, int64_t D
   dim3 block(32, BK_RL);
   if (items <= sms) cumsum_tma_kernel<OP, false><<<dim3((unsigned)items), block, BK_SMEM, st>>>(maps, init, N, T, D, reverse);
   else              cumsum_tma_kernel<OP, true><<<dim3((unsigned)sms), block, BK_SMEM, st>>>(maps, init, N, T, D, reverse);
+  GLA_CHECK_LAUNCH();
   return GLA_OK;
 }
 
-// Column width of a block: the four-columns-per-thread kernel serves rows of at least 128 columns that are a
-// multiple of four (and, checked at launch, 16-byte aligned pointers); the scalar kernel everything else.
-static bool cumsum_wide(int64_t D) { return D >= 128 && D % 4 == 0; }
-
-// Segments for a scan of N rows of length T: enough blocks to fill the device when N alone
-// gives too few, but never segments shorter than 256 positions.
-static int cumsum_segments(int64_t N, int64_t T, int64_t D) {
-  const int64_t blocks = cumsum_wide(D) ? N * ((D + 127) / 128) : N * ((D + 31) / 32);
-  const int64_t target = cumsum_wide(D) ? 2 * 148 : 4 * 148;
-  const int64_t want = (target + blocks - 1) / blocks;
-  int64_t nseg = want < 1 ? 1 : want;
-  if (nseg > T / 256) nseg = T / 256;
-  if (nseg < 1) nseg = 1;
-  if (nseg > 64) nseg = 64;
-  return (int)nseg;
-}
-
-size_t cumsum_scratch_bytes(int64_t N, int64_t T, int64_t D) {
-  return (size_t)N * cumsum_segments(N, T, D) * D * sizeof(float);
-}
-
-template <typename TI, typename TO, typename OP>
-static void cumsum_dispatch_op(cudaStream_t st, dim3 grid, dim3 block, const void* src, const void* sub,
-                               const void* init, void* dst, int64_t T, int64_t D, int reverse, int nseg,
-                               int64_t seg_len, float* totals) {
-  if (block.y == C4_RL) {
-    if (nseg > 1)
-      cumsum_v4_kernel<TI, TO, true, OP><<<grid, block, 0, st>>>((const TI*)src, (const TI*)sub, (const TI*)init, (TO*)dst, T,
-                                                                  D, reverse, nseg, seg_len, totals);
-    cumsum_v4_kernel<TI, TO, false, OP><<<grid, block, 0, st>>>((const TI*)src, (const TI*)sub, (const TI*)init, (TO*)dst, T,
-                                                                 D, reverse, nseg, seg_len, nseg > 1 ? totals : nullptr);
-    return;
+// Blocks per cluster: the time of a grid is its waves over the SMs (four blocks each) times a block's steps; a step costs
+// the larger of its latency (about 2.5 us, 2 us more with the exchange) and of its SM's share of HBM.  The count that
+// minimises that by a clear margin is taken: 1 where rows and columns alone fill the device, up to 16 for a few rows with a long axis.
+static int scan_cluster(int64_t items, int64_t T, int rows, double tile_bytes, double* us = nullptr) {
+  constexpr int SMS = 148, PER_SM = 4;
+  int best = 1;
+  double best_t = 0;
+  for (int cl = 1; cl <= SK_MAXCL; cl *= 2) {
+    if (cl > 1 && (int64_t)(cl / 2) * rows >= T) break;
+    const double total = (double)items * cl, full = floor(total / (SMS * PER_SM)), rest = total - full * SMS * PER_SM;
+    const double lat = cl > 1 ? 4.5 : 2.5, share = tile_bytes / 44e3;       // us; 44 KB/us per SM
+    const double steps = (double)((T + (int64_t)cl * rows - 1) / ((int64_t)cl * rows));
+    const double t = steps * (full * fmax(lat, PER_SM * share) + (rest > 0 ? fmax(lat, ceil(rest / SMS) * share) : 0.0));
+    if (cl == 1 || t < 0.85 * best_t) { best = cl; best_t = t; }
   }
-  if (nseg > 1)
-    cumsum_kernel<TI, TO, true, OP><<<grid, block, 0, st>>>((const TI*)src, (const TI*)sub, (const TI*)init, (TO*)dst, T, D,
-                                                             reverse, nseg, seg_len, totals);
-  cumsum_kernel<TI, TO, false, OP><<<grid, block, 0, st>>>((const TI*)src, (const TI*)sub, (const TI*)init, (TO*)dst, T, D,
-                                                            reverse, nseg, seg_len, nseg > 1 ? totals : nullptr);
+  if (us != nullptr) *us = best_t;
+  return best;
+}
+// The ring's time (us): a block streams its item's rows at about 58 GB/s, read and write, one block per SM, all of them
+// at 5.9 TB/s at most (measured at N = 96, D = 128 and N = 90, D = 132, T = 4096: 72 and 144 us).
+static double scan_ring_us(int64_t N, int64_t T, int64_t D) {
+  const double items = (double)N * ((D + 127) / 128), bytes = (double)T * 128 * 8;
+  return fmax(ceil(items / 148) * bytes / 58e3, items * bytes / 5.9e6);
+}
+template <typename TI, typename TO, typename OP, int VEC, int RPT>
+static int launch_scan_rows(cudaStream_t st, int64_t N, int64_t T, int64_t D, const void* src, const void* sub, const void* init,
+                            void* dst, int reverse) {
+  const int64_t gy = (D + 32 * VEC - 1) / (32 * VEC), items = N * gy;
+  const int cl = scan_cluster(items, T, SK_RL * RPT, (double)SK_RL * RPT * 32 * VEC * (sizeof(TI) + sizeof(TO)));
+  if (items * cl > 2147483647LL || gy > 2147483647LL) return GLA_ERR_TOO_LARGE;
+  static SmemAttrOnce attr16;
+  if (cl > 8) GLA_TRY(attr16.allow_large_clusters(scan_kernel<TI, TO, OP, VEC, RPT>));
+  ProfScope ps("cumsum_kernel", st);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(items * cl));
+  cfg.blockDim = dim3(32, SK_RL);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cl > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, scan_kernel<TI, TO, OP, VEC, RPT>, (const TI*)src, (const TI*)sub, (const TI*)init,
+                                           (TO*)dst, T, D, (int)gy, cl, reverse);
+  if (e != cudaSuccess) return record_cuda_error(e);
+  GLA_CHECK_LAUNCH();
+  return GLA_OK;
+}
+// Columns per lane and rows per lane (32 values together): a block's 8 row lanes should not outrun a short axis, and on
+// a long one narrow blocks give more of them.  bf16 keeps two columns per lane, which fill a 128-byte line of a row.
+template <typename TI, typename TO, typename OP>
+static int launch_scan_op(cudaStream_t st, int64_t N, int64_t T, int64_t D, const void* src, const void* sub, const void* init,
+                          void* dst, int reverse) {
+  auto vec = [&](int v) {
+    auto on = [](const void* p, size_t a) { return ((uintptr_t)p % a) == 0; };
+    return D % v == 0 && on(src, v * sizeof(TI)) && on(sub, v * sizeof(TI)) && on(init, v * sizeof(TI)) && on(dst, v * sizeof(TO));
+  };
+  auto fits = [&](int v) { return vec(v) && (D + 32 * v - 1) / (32 * v) * (32 * v) * 4 <= D * 5; };      // idle columns
+  if (sizeof(TI) == 4 && T <= 8 * SK_RL && fits(4)) return launch_scan_rows<TI, TO, OP, 4, 8>(st, N, T, D, src, sub, init, dst, reverse);
+  if (T <= 16 * SK_RL && fits(2)) return launch_scan_rows<TI, TO, OP, 2, 16>(st, N, T, D, src, sub, init, dst, reverse);
+  if (sizeof(TI) == 2 && vec(2)) return launch_scan_rows<TI, TO, OP, 2, 16>(st, N, T, D, src, sub, init, dst, reverse);
+  if constexpr (sizeof(TI) == 4 && sizeof(TO) == 4) {
+    // (12 %: what the model of the register kernel leaves out where two or three blocks share an SM, 83 us at N = 50,
+    // T = 4096, D = 256 against 72 with the ring)
+    if (sub == nullptr && T >= 1024 && vec(4) && (D + 127) / 128 <= 65535 && N <= 2147483647LL && T <= 2147483647LL) {
+      double us;
+      scan_cluster(N * ((D + 31) / 32), T, SK_RL * 32, SK_RL * 32 * 32 * 8.0, &us);
+      if (scan_ring_us(N, T, D) < 1.12 * us) return launch_cumsum_tma_op<OP>(st, N, T, D, (const float*)src, (const float*)init, (float*)dst, reverse);
+    }
+  }
+  return T <= 8 * SK_RL ? launch_scan_rows<TI, TO, OP, 1, 8>(st, N, T, D, src, sub, init, dst, reverse)
+                        : launch_scan_rows<TI, TO, OP, 1, 32>(st, N, T, D, src, sub, init, dst, reverse);
 }
 template <typename TI, typename TO>
-static void cumsum_dispatch(cudaStream_t st, dim3 grid, dim3 block, const void* src, const void* sub,
-                            const void* init, void* dst, int64_t T, int64_t D, int reverse, int nseg,
-                            int64_t seg_len, float* totals, int op = GLA_SCAN_ADD) {
+static int launch_scan_types(cudaStream_t st, int64_t N, int64_t T, int64_t D, const void* src, const void* sub, const void* init,
+                             void* dst, int reverse, int op) {
   switch (op) {
-    case GLA_SCAN_MUL: cumsum_dispatch_op<TI, TO, OpMul>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, totals); break;
-    case GLA_SCAN_MAX: cumsum_dispatch_op<TI, TO, OpMax>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, totals); break;
-    case GLA_SCAN_MIN: cumsum_dispatch_op<TI, TO, OpMin>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, totals); break;
-    case GLA_SCAN_LOGADDEXP: cumsum_dispatch_op<TI, TO, OpLogAddExp>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, totals); break;
-    default: cumsum_dispatch_op<TI, TO, OpAdd>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, totals); break;
+    case GLA_SCAN_MUL: return launch_scan_op<TI, TO, OpMul>(st, N, T, D, src, sub, init, dst, reverse);
+    case GLA_SCAN_MAX: return launch_scan_op<TI, TO, OpMax>(st, N, T, D, src, sub, init, dst, reverse);
+    case GLA_SCAN_MIN: return launch_scan_op<TI, TO, OpMin>(st, N, T, D, src, sub, init, dst, reverse);
+    case GLA_SCAN_LOGADDEXP: return launch_scan_op<TI, TO, OpLogAddExp>(st, N, T, D, src, sub, init, dst, reverse);
+    default: return launch_scan_op<TI, TO, OpAdd>(st, N, T, D, src, sub, init, dst, reverse);
   }
 }
 
 int launch_cumsum(cudaStream_t st, int64_t N, int64_t T, int64_t D, const void* src, const void* init,
-                  void* dst, int reverse, int in_bf16, int out_bf16, const void* sub, float* scratch, int op) {
+                  void* dst, int reverse, int in_bf16, int out_bf16, const void* sub, int op) {
   if (N <= 0 || T <= 0 || D <= 0) return GLA_ERR_BAD_DIMS;
   if (op < GLA_SCAN_ADD || op > GLA_SCAN_LOGADDEXP || (sub != nullptr && op != GLA_SCAN_ADD)) return GLA_ERR_UNSUPPORTED;
-  // 16-byte accesses need every row start on that boundary in each array: D % 4 == 0 makes the row pitch a
-  // multiple of 16 bytes (8 for bf16), so the base pointers decide
-  auto aligned = [](const void* p, int is_bf16) { return p == nullptr || ((uintptr_t)p % (is_bf16 ? 8 : 16)) == 0; };
-  const bool wide = cumsum_wide(D) && aligned(src, in_bf16) && aligned(sub, in_bf16) && aligned(init, in_bf16) &&
-                    aligned(dst, out_bf16) && aligned(scratch, 0);
-  // float32 in and out, no second source, one pass: the bulk-copy pipeline
-  if (wide && !in_bf16 && !out_bf16 && sub == nullptr && scratch == nullptr && T >= 2 * BK_ROWS) {
-    if ((D + 127) / 128 > 65535 || N > 2147483647LL) return GLA_ERR_TOO_LARGE;
-    ProfScope ps("cumsum_kernel", st);
-    int rc;
-    switch (op) {
-      case GLA_SCAN_MUL: rc = launch_cumsum_tma_op<OpMul>(st, N, T, D, (const float*)src, (const float*)init, (float*)dst, reverse); break;
-      case GLA_SCAN_MAX: rc = launch_cumsum_tma_op<OpMax>(st, N, T, D, (const float*)src, (const float*)init, (float*)dst, reverse); break;
-      case GLA_SCAN_MIN: rc = launch_cumsum_tma_op<OpMin>(st, N, T, D, (const float*)src, (const float*)init, (float*)dst, reverse); break;
-      case GLA_SCAN_LOGADDEXP: rc = launch_cumsum_tma_op<OpLogAddExp>(st, N, T, D, (const float*)src, (const float*)init, (float*)dst, reverse); break;
-      default: rc = launch_cumsum_tma_op<OpAdd>(st, N, T, D, (const float*)src, (const float*)init, (float*)dst, reverse); break;
-    }
-    if (rc != GLA_OK) return rc;
-    GLA_CHECK_LAUNCH();
-    return GLA_OK;
-  }
-  const int64_t gy = wide ? (D + 127) / 128 : (D + 31) / 32;
-  // without scratch for the segment sums the scan runs in one pass, one block per row and column group
-  const int nseg = scratch ? cumsum_segments(N, T, D) : 1;
-  const int64_t tile = CS_RPT * C4_RL;      // rows of the wide kernel's tile, a multiple of the scalar kernel's
-  static_assert((CS_RPT * C4_RL) % (CS_RPT * CS_RL) == 0, "segment lengths must be whole tiles of both kernels");
-  int64_t seg_len = (T + nseg - 1) / nseg;
-  seg_len = (seg_len + tile - 1) / tile * tile;
-  if (gy > 65535 || N * nseg > 2147483647LL) return GLA_ERR_TOO_LARGE;
-  dim3 grid((unsigned)(N * nseg), (unsigned)gy), block(32, wide ? C4_RL : CS_RL);
-  ProfScope ps("cumsum_kernel", st);
-  if (!in_bf16 && !out_bf16)
-    cumsum_dispatch<float, float>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, scratch, op);
-  else if (!in_bf16 && out_bf16)
-    cumsum_dispatch<float, bf16>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, scratch, op);
-  else if (in_bf16 && !out_bf16)
-    cumsum_dispatch<bf16, float>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, scratch, op);
-  else
-    cumsum_dispatch<bf16, bf16>(st, grid, block, src, sub, init, dst, T, D, reverse, nseg, seg_len, scratch, op);
-  GLA_CHECK_LAUNCH();
-  return GLA_OK;
+  if (in_bf16) return out_bf16 ? launch_scan_types<bf16, bf16>(st, N, T, D, src, sub, init, dst, reverse, op)
+                               : launch_scan_types<bf16, float>(st, N, T, D, src, sub, init, dst, reverse, op);
+  return out_bf16 ? launch_scan_types<float, bf16>(st, N, T, D, src, sub, init, dst, reverse, op)
+                  : launch_scan_types<float, float>(st, N, T, D, src, sub, init, dst, reverse, op);
 }
+
+
+
 
 // ---------------------------------------------------------------------------------------
 // rnn_scan: sequential over T, parallel over the elements of the state.  A thread owns FOUR consecutive value

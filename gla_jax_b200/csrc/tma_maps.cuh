@@ -103,7 +103,7 @@ inline int make_map_ntd_f32(CUtensorMap* m, const void* ptr, int64_t N, int64_t 
   return GLA_OK;
 }
 
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device) instead of on every call.
+// cudaFuncSetAttribute once per (kernel, device) instead of on every call.
 struct SmemAttrOnce {
   unsigned long long done = 0;       // bit per device; a lost update only repeats an idempotent call
   template <typename K>
@@ -112,6 +112,17 @@ struct SmemAttrOnce {
     if (cudaGetDevice(&dev) != cudaSuccess) return GLA_ERR_NO_DEVICE;
     if (dev >= 0 && dev < 64 && ((done >> dev) & 1ull)) return GLA_OK;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return record_cuda_error(e);
+    if (dev >= 0 && dev < 64) done |= 1ull << dev;
+    return GLA_OK;
+  }
+  // the same for clusters of more than eight blocks
+  template <typename K>
+  int allow_large_clusters(K kern) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return GLA_ERR_NO_DEVICE;
+    if (dev >= 0 && dev < 64 && ((done >> dev) & 1ull)) return GLA_OK;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev >= 0 && dev < 64) done |= 1ull << dev;
     return GLA_OK;
