@@ -83,6 +83,13 @@ SIGNATURES = {
     "gla_chunk_bwd_packed": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_int64, c_void_p, c_void_p,
                                      c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_void_p, c_void_p, c_void_p, c_void_p, c_size_t]),
+    "gla_chunk_ragged_saved_bytes": (c_size_t, [c_int64, c_int64, c_int, c_int64, c_void_p]),
+    "gla_chunk_ragged_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int, c_int64, c_void_p, c_int]),
+    "gla_chunk_fwd_ragged": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int, c_int64, c_void_p, c_void_p, c_void_p,
+                                     c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t]),
+    "gla_chunk_bwd_ragged": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int, c_int64, c_void_p, c_void_p, c_void_p,
+                                     c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                     c_void_p, c_void_p, c_void_p, c_size_t]),
     "gla_chunk_fwd_static_max_bytes": (c_size_t, []),
     "gla_chunk_fwd_static": (c_int, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int, c_void_p,
                                      c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),

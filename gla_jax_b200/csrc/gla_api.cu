@@ -377,6 +377,72 @@ int gla_chunk_bwd_packed(void* stream, int64_t T, int64_t H, int64_t D, int64_t 
                       dhidden_init, dlog_fgate, dvalue, dkey, dquery, workspace, 0, nseq, cu_seqlens);
 }
 
+// Offsets of a ragged batch: rising strictly from 0, to T where T is known (T >= 0).
+static bool ragged_ok(int64_t H, int64_t D, int dtype, int64_t nseq, const int32_t* cu, int64_t T) {
+  if (!cu || nseq <= 0 || nseq > (1 << 30) || H <= 0 || !tc_supported_local_state(D, 128, dtype) || cu[0] != 0) return false;
+  for (int64_t s = 0; s < nseq; ++s)
+    if (cu[s + 1] <= cu[s]) return false;
+  return T < 0 || cu[nseq] == T;
+}
+static bool ragged_aligned(int64_t nseq, const int32_t* cu) {
+  for (int64_t s = 1; s <= nseq; ++s)
+    if (cu[s] % 128 != 0) return false;
+  return true;
+}
+size_t gla_chunk_ragged_saved_bytes(int64_t H, int64_t D, int dtype, int64_t nseq, const int32_t* cu) {
+  return ragged_ok(H, D, dtype, nseq, cu, -1) ? tc_saved_bytes(1, 128 * ragged_chunks(nseq, cu), H, D, 128) : 0;
+}
+size_t gla_chunk_ragged_workspace_bytes(int64_t H, int64_t D, int dtype, int64_t nseq, const int32_t* cu, int backward) {
+  if (!ragged_ok(H, D, dtype, nseq, cu, -1)) return 0;
+  const int64_t n = ragged_chunks(nseq, cu), T = 128 * n;
+  return align_up(backward ? tc_bwd_ws_bytes(1, T, H, D, 128) : tc_fwd_ws_bytes(1, T, H, D, 128), 256) + ragged_table_bytes(nseq, n);
+}
+int gla_chunk_fwd_ragged(void* stream, int64_t T, int64_t H, int64_t D, int dtype, int64_t nseq, const int32_t* cu,
+                         const void* hidden_init, const float* log_fgate, const void* value, const void* key,
+                         const void* query, void* hidden_final, void* out, void* saved, void* workspace,
+                         size_t workspace_bytes) {
+  if (!cu || !hidden_init || !log_fgate || !value || !key || !query || !hidden_final || !out) return GLA_ERR_NULL_POINTER;
+  if (T <= 0 || H <= 0 || D <= 0 || nseq <= 0) return GLA_ERR_BAD_DIMS;
+  GLA_TRY(check_dtype(dtype));
+  if (!tc_supported_local_state(D, 128, dtype)) return GLA_ERR_UNSUPPORTED;
+  if (!ragged_ok(H, D, dtype, nseq, cu, T)) return GLA_ERR_BAD_DIMS;
+  if (!workspace || workspace_bytes < gla_chunk_ragged_workspace_bytes(H, D, dtype, nseq, cu, 0)) return GLA_ERR_WORKSPACE;
+  const void* ptrs[] = {hidden_init, log_fgate, value, key, query, hidden_final, out, saved, workspace};
+  for (const void* p : ptrs)
+    if (p && !aligned16(p)) return GLA_ERR_ALIGNMENT;
+  if (!aligned32(out)) return GLA_ERR_ALIGNMENT;
+  const int64_t n = ragged_chunks(nseq, cu);
+  Ragged r;
+  GLA_TRY(ragged_tables((cudaStream_t)stream, nseq, cu, (char*)workspace + align_up(tc_fwd_ws_bytes(1, 128 * n, H, D, 128), 256), &r));
+  const bool whole = ragged_aligned(nseq, cu);
+  return tc_chunk_fwd((cudaStream_t)stream, 1, T, H, D, 128, hidden_init, log_fgate, value, key, query, hidden_final, out, saved,
+                      workspace, 0, nullptr, nullptr, 0, nseq, r.cu, 0, nullptr, whole ? nullptr : &r);
+}
+int gla_chunk_bwd_ragged(void* stream, int64_t T, int64_t H, int64_t D, int dtype, int64_t nseq, const int32_t* cu,
+                         const float* log_fgate, const void* value, const void* key, const void* query, const void* saved,
+                         const void* dhidden_final, const void* dout, void* dhidden_init, float* dlog_fgate, void* dvalue,
+                         void* dkey, void* dquery, void* workspace, size_t workspace_bytes) {
+  if (!cu || !log_fgate || !value || !key || !query || !saved || !dhidden_final || !dout || !dhidden_init || !dlog_fgate ||
+      !dvalue || !dkey || !dquery)
+    return GLA_ERR_NULL_POINTER;
+  if (T <= 0 || H <= 0 || D <= 0 || nseq <= 0) return GLA_ERR_BAD_DIMS;
+  GLA_TRY(check_dtype(dtype));
+  if (!tc_supported_local_state(D, 128, dtype)) return GLA_ERR_UNSUPPORTED;
+  if (!ragged_ok(H, D, dtype, nseq, cu, T)) return GLA_ERR_BAD_DIMS;
+  if (!workspace || workspace_bytes < gla_chunk_ragged_workspace_bytes(H, D, dtype, nseq, cu, 1)) return GLA_ERR_WORKSPACE;
+  const void* ptrs[] = {log_fgate, value, key, query, saved, dhidden_final, dout, dhidden_init, dlog_fgate, dvalue, dkey,
+                        dquery, workspace};
+  for (const void* p : ptrs)
+    if (!aligned16(p)) return GLA_ERR_ALIGNMENT;
+  if (!aligned32(dvalue)) return GLA_ERR_ALIGNMENT;
+  const int64_t n = ragged_chunks(nseq, cu);
+  Ragged r;
+  GLA_TRY(ragged_tables((cudaStream_t)stream, nseq, cu, (char*)workspace + align_up(tc_bwd_ws_bytes(1, 128 * n, H, D, 128), 256), &r));
+  const bool whole = ragged_aligned(nseq, cu);
+  return tc_chunk_bwd((cudaStream_t)stream, 1, T, H, D, 128, log_fgate, value, key, query, saved, dhidden_final, dout, dhidden_init,
+                      dlog_fgate, dvalue, dkey, dquery, workspace, 0, nseq, r.cu, 0, nullptr, nullptr, whole ? nullptr : &r);
+}
+
 int gla_chunk_local_state(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype,
                           int impl, const float* log_fgate, const void* value, const void* key, float* G_total,
                           float* S_local, void* workspace, size_t workspace_bytes) {

@@ -352,8 +352,19 @@ __device__ __noinline__ bool fwd_load_state_late(const unsigned int* state_done,
   return done;
 }
 
+// Rows [nv, 128) of an operand tile of two SW128 halves become zero: the tail of a sequence's last chunk, where the
+// tensor copy brought the next sequence's rows.
+__device__ __forceinline__ void zero_tail_rows(uint8_t* tile, int nv) {
+  for (int id = threadIdx.x; id < (TC - nv) * 16; id += TTHREADS) {
+    const int r = nv + (id >> 4), ch = id & 15;
+    *reinterpret_cast<uint4*>(tile + (ch >> 3) * TILE_BYTES + r * 128 + (ch & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+// RAG: sequences of any length on one time axis; `tab` gives every chunk its first token and its rows.  A kernel of its
+// own so that the dense one carries nothing extra.
+template <bool RAG>
 __global__ void __launch_bounds__(TTHREADS, 1)
-tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, int R, int64_t N, bf16* __restrict__ out,
+tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, int R, int64_t N, const int2* __restrict__ tab, bf16* __restrict__ out,
                     bf16* __restrict__ P_saved, const unsigned int* __restrict__ state_done, unsigned int state_target,
                     int all_scales, int pf_dist) {
   extern __shared__ uint8_t smem_raw[];
@@ -378,7 +389,9 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
   const int64_t n = N - 1 - (int64_t)blockIdx.x / BHn, bh = (int64_t)blockIdx.x % BHn, b = bh / H, h_ = bh % H;
   const int64_t hk_ = (h_ / (R * R)) * R + (h_ % (R * R)) / R, hv_ = (h_ / (R * R)) * R + h_ % R;
   const int64_t HD = H * TD;
-  const int64_t row0 = ((b * T + n * TC) * H + h_) * TD;
+  const int2 span = RAG ? tab[n] : make_int2((int)(b * T + n * TC), TC);        // first token and rows of the chunk
+  const int nv = RAG ? span.y : TC;
+  const int64_t row0 = ((RAG ? (int64_t)span.x : b * T + n * TC) * H + h_) * TD;
   const int64_t chunk_id = bh * N + n;
 
   if (tid == 0) {
@@ -391,7 +404,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
     // ---- all global inputs of the chunk through TMA: 192 KB in flight.  g, q, k (needed at once) come first on
     // their own barrier; v and S_prev are only needed by the output product and land while the levels run.
     const uint32_t lb = smem_u32(bars + 3), lb2 = smem_u32(bars + 4);
-    const int z = (int)(b * T + n * TC), y = (int)hk_, yv = (int)hv_;
+    const int z = span.x, y = (int)hk_, yv = (int)hv_;
     mbar_arrive_expect_tx(lb, 4 * 2 * TILE_BYTES);
     mbar_arrive_expect_tx(lb2, 2 * 2 * TILE_BYTES);
     tma_load_3d(smem_u32(sm + FwdSmem::Q), &maps.g, 0, y, z, lb);                       // 128 x 128 float, row pitch 512 B
@@ -416,7 +429,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
     // ahead), requested into L2 only: seven instructions of this one thread, so that the next block's load phase
     // is served from L2.
     const int64_t nb = (int64_t)blockIdx.x + pf_dist;
-    if (pf_dist > 0 && nb < (int64_t)gridDim.x) {
+    if (!RAG && pf_dist > 0 && nb < (int64_t)gridDim.x) {
       const int64_t n2 = N - 1 - nb / BHn, bh2 = nb % BHn, h2 = bh2 % H;
       const int y2 = (int)((h2 / (R * R)) * R + (h2 % (R * R)) / R), yv2 = (int)((h2 / (R * R)) * R + h2 % R);
       const int z2 = (int)((bh2 / H) * T + n2 * TC);
@@ -451,9 +464,10 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int r = rg * 16 + i;
-      const float2 gg = *reinterpret_cast<const float2*>(gq + r * 512 + cp * 8);
+      float2 gg = *reinterpret_cast<const float2*>(gq + r * 512 + cp * 8);
       qv[i] = *reinterpret_cast<const uint32_t*>(qt + sw128_off(r, col));
       kv[i] = *reinterpret_cast<const uint32_t*>(kt + sw128_off(r, col));
+      if (RAG && r >= nv) { gg = make_float2(0.f, 0.f); qv[i] = kv[i] = 0u; }
       f[i] = make_float2(__expf(gg.x), __expf(gg.y));
       prod.x *= f[i].x; prod.y *= f[i].y;
       gsum.x += fabsf(gg.x); gsum.y += fabsf(gg.y);
@@ -720,9 +734,9 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
-  if (balanced) {
-    // the q_hat operand carries exp(-m_d): row d of the state tile takes exp(m_d) before the product.  Every thread
-    // waits for the tile itself here (a block that started beside the state kernel requests it first).
+  if (balanced || (RAG && nv < TC)) {
+    // the q_hat operand carries exp(-m_d): row d of the state tile takes exp(m_d) before the product (and a short
+    // chunk's value rows past its end are cleared).  Every thread waits for the tiles itself here (a block that started beside the state kernel requests it first).
     if (tid == 32 && *s_pending_sm != 0u) {
       if (!fwd_load_state_late(state_done, state_target, &maps.s, smem_u32(sm + FwdSmem::S), (int)(chunk_id * TD), smem_u32(bars + 4)))
         atomicAdd(&g_tc_wait_timeouts, 1u);
@@ -730,6 +744,8 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
     }
     __syncwarp();
     ok = mbar_wait(smem_u32(bars + 4), 0) && ok;
+    if (RAG && nv < TC) zero_tail_rows(sm + FwdSmem::V, nv);
+    if (balanced)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int id = tid + TTHREADS * j, row = id >> 4, ch = id & 15;
@@ -789,7 +805,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
       uint32_t u[8];
 #pragma unroll
       for (int m = 0; m < 8; ++m) u[m] = pack_bf16x2(__uint_as_float(r[16 * c8 + 2 * m]), __uint_as_float(r[16 * c8 + 2 * m + 1]));
-      st_global_v8(o + 16 * c8, u);
+      if (!RAG || q4 * 32 + lane < nv) st_global_v8(o + 16 * c8, u);
     }
   } else if (tid == 0) {
     atomicAdd(&g_tc_wait_timeouts, 1u);
@@ -944,8 +960,9 @@ __device__ __noinline__ void bwd_rescale_ds(uint8_t* ds, uint32_t bar, float w, 
   }
 }
 
+template <bool RAG>
 __global__ void __launch_bounds__(TTHREADS, 1)
-tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, int R, int64_t N, int pf_dist, const float* __restrict__ g, const bf16* __restrict__ v,
+tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, int R, int64_t N, const int2* __restrict__ tab, int pf_dist, const float* __restrict__ g, const bf16* __restrict__ v,
                     const bf16* __restrict__ k, const bf16* __restrict__ q, const bf16* __restrict__ dO,
                     const bf16* __restrict__ S_prev, const bf16* __restrict__ dS_next, const bf16* __restrict__ P_saved,
                     bf16* __restrict__ dq_out, bf16* __restrict__ dk_out, bf16* __restrict__ dv_out,
@@ -977,7 +994,9 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
   const int64_t n = (int64_t)blockIdx.x / BHn, bh = (int64_t)blockIdx.x % BHn, b = bh / H, h_ = bh % H;
   const int64_t hk_ = (h_ / (R * R)) * R + (h_ % (R * R)) / R, hv_ = (h_ / (R * R)) * R + h_ % R;
   const int64_t HD = H * TD;                                          // output row pitch (virtual heads)
-  const int64_t row0 = ((b * T + n * TC) * H + h_) * TD;              // outputs
+  const int2 span = RAG ? tab[n] : make_int2((int)(b * T + n * TC), TC);        // first token and rows of the chunk
+  const int nv = RAG ? span.y : TC;
+  const int64_t row0 = ((RAG ? (int64_t)span.x : b * T + n * TC) * H + h_) * TD;   // outputs
   const int64_t chunk_id = bh * N + n;
 
   if (warp == 0) {
@@ -993,7 +1012,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     // regions whose operand tiles are not needed until the products: g over the S_prev and dS_next regions, q over
     // the P region, k into the region that k_hat will occupy.  Every thread copies its 32 rows of one feature from
     // there into registers; after the barrier that follows, the three late tiles are requested.
-    const int z = (int)(b * T + n * TC), yv = (int)hv_, yk = (int)hk_;
+    const int z = span.x, yv = (int)hv_, yk = (int)hk_;
     {
       const uint32_t kb = smem_u32(bars + 6);
       mbar_arrive_expect_tx(kb, 8 * TILE_BYTES);
@@ -1034,6 +1053,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     for (int i = 0; i < 32; ++i) {
       f32r[i] = lok ? gs[i * TD] : 0.f;
       kraw[i] = lok ? ((uint32_t)ks[i * TD] | ((uint32_t)qs[i * TD] << 16)) : 0u;
+      if (RAG && 32 * wq_ + i >= nv) { f32r[i] = 0.f; kraw[i] = 0u; }
     }
     float p0 = 1.f, p1 = 1.f, ga = 0.f;
 #pragma unroll
@@ -1108,6 +1128,14 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     __syncthreads();
   }
 
+  if (RAG && nv < TC) {
+    ok = mbar_wait(smem_u32(bars + 5), 0) && ok;
+    zero_tail_rows(sm + BwdSmem::DO, nv);
+    zero_tail_rows(sm + BwdSmem::V, nv);
+    fence_async_smem();
+    __syncthreads();
+  }
+
   // ---- phase 1: the four dense products --------------------------------------------------------------
   // Issued by four threads of four warps on different schedulers (8 to 16 MMAs each instead of 40 from one): the
   // issuing thread's instruction stream is serial, so this shortens the wait of everybody else.  The two halves of
@@ -1153,7 +1181,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
   // box, where per-line prefetches cost every thread three instructions and measured 1 us slower).
   {
     const int64_t nb = (int64_t)blockIdx.x + pf_dist;
-    if (pf_dist > 0 && nb < (int64_t)gridDim.x && tid == 0) {
+    if (!RAG && pf_dist > 0 && nb < (int64_t)gridDim.x && tid == 0) {
       const int64_t n2 = nb / BHn, bh2 = nb % BHn, h2 = bh2 % H;
       const int y2 = (int)((h2 / (R * R)) * R + (h2 % (R * R)) / R), yv2 = (int)((h2 / (R * R)) * R + h2 % R);
       const int z2 = (int)((bh2 / H) * T + n2 * TC);
@@ -1178,7 +1206,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
   tc_fence_after();
   // dO, v and P have been consumed by the products: their regions take g, q, k of rows 64..127 and k of rows
   // 0..63 by TMA while phase 1.5 runs, so that the W64 build and the first pass read them from shared memory.
-  const int zrow = (int)(b * T + n * TC), yh = (int)hk_;
+  const int zrow = span.x, yh = (int)hk_;
   if (one_scale) {
     // every thread parks the raw k and q of its 32 rows in the regions the products have released; it alone reads
     // them back (for the q~ operand and in the closing pass), so no barrier is involved
@@ -1207,7 +1235,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     tmem_ld32(lane_base + TM_DV + 32 * wq_, r);       // row j = d here (row layout)
     tmem_ld32(lane_base + TM_DKH + 32 * wq_, r2);     // feature d, rows 32 wq_ + m (column layout)
     tmem_ld_wait();
-    if (ok) {
+    if (ok && (!RAG || d < nv)) {
       bf16* o = dv_out + row0 + (int64_t)d * HD + 32 * wq_;
       // a thread owns 64 contiguous bytes of one row; the rows of a warp are far apart, so what counts is the
       // number of store requests: two 32-byte stores instead of four 16-byte ones
@@ -1409,6 +1437,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
       for (int j = 0; j < 4; ++j) {
         const int id = tid + TTHREADS * j, row = id >> 4, ch = id & 15;
         const int64_t e = row0 + (int64_t)row * HD + ch * 8;
+        if (RAG && row >= nv) continue;
         *reinterpret_cast<uint4*>(dq_out + e) = *reinterpret_cast<const uint4*>(dqt + row * TD + ch * 8);
         *reinterpret_cast<uint4*>(dk_out + e) = *reinterpret_cast<const uint4*>(dkt + row * TD + ch * 8);
       }
@@ -1417,6 +1446,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int id = tid + TTHREADS * j, row = id >> 5, d0 = 4 * (id & 31), w = row >> 5;
+        if (RAG && row >= nv) continue;
         float4 x = *reinterpret_cast<const float4*>(dlb + row * TD + d0);
         float4 o = *reinterpret_cast<const float4*>(gab + d0);
 #pragma unroll
@@ -1440,7 +1470,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
                                (32 * (wq_ & 1)) * TD + d;
     uint32_t xraw[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) xraw[i] = xp[i * TD];
+    for (int i = 0; i < 32; ++i) xraw[i] = RAG && 32 * wq_ + i >= nv ? 0u : xp[i * TD];
     uint32_t pk[16];
     if (wq_ < 2) {
       float run = (wq_ == 0) ? tot[2 * TD + d] * tot[3 * TD + d] : 1.f;
@@ -1489,6 +1519,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
       for (int i = 0; i < 16; ++i) {
         f[i] = gs_[i * TD];
         qk[i] = (uint32_t)qs_[i * TD] | ((uint32_t)ks_[i * TD] << 16);
+        if (RAG && rbase + i >= nv) { f[i] = 0.f; qk[i] = 0u; }
       }
 #pragma unroll
       for (int i = 0; i < 16; ++i) f[i] = __expf(f[i]);
@@ -1683,7 +1714,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     for (int i = 0; i < 16; ++i) {
       const int64_t e = row0 + (int64_t)(rbase + i) * HD + d;
       dl[i] = bf16_lo(qk[i]) * dq[i] - bf16_hi(qk[i]) * dk[i];
-      if (ok) {
+      if (ok && (!RAG || rbase + i < nv)) {
         dq_out[e] = __float2bfloat16_rn(dq[i]);
         dk_out[e] = __float2bfloat16_rn(dk[i]);
       }
@@ -1697,7 +1728,8 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     for (int g2 = gi + 1; g2 < 4 * p + 4; ++g2) off += grp[g2 * TD + d];
     if (ok) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) dg_out[row0 + (int64_t)(rbase + i) * HD + d] = dl[i] + off;
+      for (int i = 0; i < 16; ++i)
+        if (!RAG || rbase + i < nv) dg_out[row0 + (int64_t)(rbase + i) * HD + d] = dl[i] + off;
     }
     if (p == 1) {
       later = 0.f;
@@ -1997,14 +2029,15 @@ constexpr size_t FWD_SMEM = 1024 + FwdSmem::END;
 int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, const void* hidden_init,
                  const float* g, const void* v, const void* k, const void* q, void* hidden_final, void* out,
                  void* saved, void* ws, int state_only, float* G_total, float* S_local, int opts, int64_t nseq,
-                 const int* cu, int sp_phase, const float* H_in) {
+                 const int* cu, int sp_phase, const float* H_in, const Ragged* rag) {
   (void)C;
   const int R = (int)(D / TD);
-  const int64_t N = T / TC, HV = H * R * R, HK = H * R, BHV = B * HV;
+  const int64_t N = rag ? rag->chunks : T / TC, HV = H * R * R, HK = H * R, BHV = B * HV;
   if (state_only && R != 1) return GLA_ERR_UNSUPPORTED;
   // sequence-parallel phases (sp_phase 1: states from a zero state, kept in `saved`; 2: correct them with H_in, then
   // the chunk kernel) exist for the plain head size and need the residual buffer to carry the states between them
   if (sp_phase != 0 && (R != 1 || saved == nullptr || cu != nullptr || state_only)) return GLA_ERR_UNSUPPORTED;
+  if (rag) cu = rag->cu;
   if (cu != nullptr && (B != 1 || R != 1 || state_only || nseq <= 0)) return GLA_ERR_UNSUPPORTED;   // packed sequences
   char* w = (char*)ws;
   float* kv = (float*)w; w += (R == 1 ? f32b(BHV * N * TD * TD) : 0);
@@ -2070,7 +2103,8 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
     GLA_TRY(launch_seg_scan(st, BHV, nsegs, fx, nullptr, fin_v, nullptr, 0));
     GLA_TRY(launch_fix_states(st, BHV, N, nsegs, 0, fx, fx.Cin, S_prev));
   } else if (fused_states) {
-    GLA_TRY(tc_state_fused(st, 0, B, T, HV, R, g, k, v, init_v, S_prev, fin_v, Gc, nseq, cu, early_flag, &early_target));
+    GLA_TRY(tc_state_fused(st, 0, B, T, HV, R, g, k, v, init_v, S_prev, fin_v, Gc, nseq, cu, early_flag, &early_target, nullptr, 1,
+                           rag ? rag->cub : nullptr, N));
   } else {
     GLA_TRY((launch_tc_kv<0>(st, B, T, H, g, k, v, kv, Gc)));
   }
@@ -2082,8 +2116,10 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
     return GLA_OK;
   }
   if (!fused_states && sp_phase == 0) GLA_TRY(launch_state_scan(st, BHV, N, TD, Gc, kv, 0, hidden_init, 1, S_prev, 1, hidden_final, 1, 0));
-  static SmemAttrOnce fwd_attr;
-  GLA_TRY(fwd_attr.ensure(tc_chunk_fwd_kernel, FWD_SMEM));
+  static SmemAttrOnce fwd_attr[2];
+  auto fwd_kernel = rag ? tc_chunk_fwd_kernel<true> : tc_chunk_fwd_kernel<false>;
+  const int2* tab = rag ? rag->tab : nullptr;
+  GLA_TRY(fwd_attr[rag != nullptr].ensure(fwd_kernel, FWD_SMEM));
   cudaError_t e;
   const int all_scales = (opts & GLA_OPT_ALL_SCALES) ? 1 : 0;
   FwdMaps maps;
@@ -2108,11 +2144,11 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
       attr[0].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, tc_chunk_fwd_kernel, maps, T, HV, R, N, out_p, P, (const unsigned int*)early_flag,
+      e = cudaLaunchKernelEx(&cfg, fwd_kernel, maps, T, HV, R, N, tab, out_p, P, (const unsigned int*)early_flag,
                              early_target, all_scales, pf_dist);
       if (e != cudaSuccess) return record_cuda_error(e);
     } else {
-      tc_chunk_fwd_kernel<<<(unsigned)(BHV * N), TTHREADS, FWD_SMEM, st>>>(maps, T, HV, R, N, out_p, P, nullptr, 0u, all_scales, pf_dist);
+      fwd_kernel<<<(unsigned)(BHV * N), TTHREADS, FWD_SMEM, st>>>(maps, T, HV, R, N, tab, out_p, P, nullptr, 0u, all_scales, pf_dist);
     }
   }
   GLA_CHECK_LAUNCH();
@@ -2141,10 +2177,11 @@ int tc_local_dstate(cudaStream_t st, int64_t B, int64_t T, int64_t H, const floa
 int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, const float* g,
                  const void* v, const void* k, const void* q, const void* saved, const void* dhidden_final,
                  const void* dout, void* dhidden_init, float* dg, void* dv, void* dk, void* dq, void* ws, int opts,
-                 int64_t nseq, const int* cu, int sp_phase, float* A_local, const float* dH_out) {
+                 int64_t nseq, const int* cu, int sp_phase, float* A_local, const float* dH_out, const Ragged* rag) {
   (void)C;
   const int R = (int)(D / TD);
-  const int64_t N = T / TC, HV = H * R * R, HK = H * R, BHV = B * HV;
+  const int64_t N = rag ? rag->chunks : T / TC, HV = H * R * R, HK = H * R, BHV = B * HV;
+  if (rag) cu = rag->cu;
   if (cu != nullptr && (B != 1 || R != 1 || nseq <= 0)) return GLA_ERR_UNSUPPORTED;   // packed sequences
   // sequence-parallel phases: 1 = gradient states from a zero final gradient (kept in the workspace) and the
   // gradient reaching the slice's initial state; 2 = correct them with dH_out, then the chunk kernel
@@ -2201,13 +2238,15 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
     GLA_TRY(launch_seg_scan(st, BHV, nsegs, fx, nullptr, dinit_v, nullptr, 1));
     GLA_TRY(launch_fix_states(st, BHV, N, nsegs, nsegs - 1, fx, fx.Cin, dS_next));
   } else if (fused_states) {
-    GLA_TRY(tc_state_fused(st, 1, B, T, HV, R, g, q, dout, dfin_v, dS_next, dinit_v, nullptr, nseq, cu));
+    GLA_TRY(tc_state_fused(st, 1, B, T, HV, R, g, q, dout, dfin_v, dS_next, dinit_v, nullptr, nseq, cu, nullptr, nullptr, nullptr, 1,
+                           rag ? rag->cub : nullptr, N));
   } else {
     GLA_TRY((launch_tc_kv<1>(st, B, T, H, g, q, dout, dstate, nullptr)));
     GLA_TRY(launch_state_scan(st, BHV, N, TD, Gc, dstate, 0, dhidden_final, 1, dS_next, 1, dhidden_init, 1, 1));
   }
-  static SmemAttrOnce bwd_attr;
-  GLA_TRY(bwd_attr.ensure(tc_chunk_bwd_kernel, BWD_SMEM));
+  static SmemAttrOnce bwd_attr[2];
+  auto bwd_kernel = rag ? tc_chunk_bwd_kernel<true> : tc_chunk_bwd_kernel<false>;
+  GLA_TRY(bwd_attr[rag != nullptr].ensure(bwd_kernel, BWD_SMEM));
   BwdMaps bmaps;
   GLA_TRY(make_map_bthd(&bmaps.g, g, 1, B, T, HK, 128, 0, 64));
   GLA_TRY(make_map_bthd(&bmaps.q, q, 0, B, T, HK, 128, 0, 64));
@@ -2219,8 +2258,8 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   GLA_TRY(make_map_rows(&bmaps.p, P, BHV * N * TC, 64, 128));
   {
     ProfScope ps("tc_chunk_bwd_kernel", st);
-    tc_chunk_bwd_kernel<<<(unsigned)(BHV * N), TTHREADS, BWD_SMEM, st>>>(
-        bmaps, T, HV, R, N, (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : prefetch_distance(1), g, (const bf16*)v, (const bf16*)k,
+    bwd_kernel<<<(unsigned)(BHV * N), TTHREADS, BWD_SMEM, st>>>(
+        bmaps, T, HV, R, N, rag ? rag->tab : nullptr, (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : prefetch_distance(1), g, (const bf16*)v, (const bf16*)k,
         (const bf16*)q, (const bf16*)dout, S_prev, dS_next, P, dq_v, dk_v, dv_v, dg_v, (opts & GLA_OPT_ALL_SCALES) ? 1 : 0);
   }
   GLA_CHECK_LAUNCH();
@@ -2230,6 +2269,52 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
     GLA_TRY((launch_sum_blocks<float, 1>(st, dg_v, dg, B * T, H, R)));
     GLA_TRY((launch_sum_blocks<bf16, 0>(st, dv_v, (bf16*)dv, B * T, H, R)));
     GLA_TRY(launch_state_block(st, dhib, dhidden_init, B * H, R, 0));
+  }
+  return GLA_OK;
+}
+
+// ---- tables of a ragged batch ----------------------------------------------------------------------------------------
+// Built on the device from offsets that travel as kernel parameters (no copy from pageable memory, nothing to keep
+// alive): up to 255 sequences per launch, one block each.
+struct RagSlice { int cu[256], cub[256]; };
+__global__ void __launch_bounds__(128) ragged_table_kernel(const __grid_constant__ RagSlice a, int first, int n, int* __restrict__ cu,
+                                                           int* __restrict__ cub, int2* __restrict__ tab) {
+  const int s = blockIdx.x, lo = a.cu[s], hi = a.cu[s + 1], c0 = a.cub[s], c1 = a.cub[s + 1];
+  if (threadIdx.x == 0) {
+    cu[first + s] = lo; cub[first + s] = c0;
+    if (s == n - 1) { cu[first + n] = hi; cub[first + n] = c1; }
+  }
+  for (int c = c0 + threadIdx.x; c < c1; c += 128) {
+    const int t = lo + (c - c0) * TC;
+    tab[c] = make_int2(t, hi - t < TC ? hi - t : TC);
+  }
+}
+int64_t ragged_chunks(int64_t nseq, const int* cu_host) {
+  int64_t n = 0;
+  for (int64_t s = 0; s < nseq; ++s) n += (cu_host[s + 1] - cu_host[s] + TC - 1) / TC;
+  return n;
+}
+size_t ragged_table_bytes(int64_t nseq, int64_t chunks) {
+  return align_up((size_t)chunks * sizeof(int2), 256) + 2 * align_up((size_t)(nseq + 1) * sizeof(int), 256);
+}
+int ragged_tables(cudaStream_t st, int64_t nseq, const int* cu_host, void* mem, Ragged* r) {
+  r->chunks = ragged_chunks(nseq, cu_host);
+  int2* tab = (int2*)mem;
+  int* cu = (int*)((char*)mem + align_up((size_t)r->chunks * sizeof(int2), 256));
+  int* cub = (int*)((char*)cu + align_up((size_t)(nseq + 1) * sizeof(int), 256));
+  r->tab = tab; r->cu = cu; r->cub = cub;
+  int c = 0;
+  for (int64_t s0 = 0; s0 < nseq; s0 += 255) {
+    const int n = nseq - s0 < 255 ? (int)(nseq - s0) : 255;
+    RagSlice a;
+    for (int s = 0; s <= n; ++s) {
+      a.cu[s] = cu_host[s0 + s];
+      a.cub[s] = c;
+      if (s < n) c += (cu_host[s0 + s + 1] - cu_host[s0 + s] + TC - 1) / TC;
+    }
+    ProfScope ps("ragged_table_kernel", st);
+    ragged_table_kernel<<<n, 128, 0, st>>>(a, (int)s0, n, cu, cub, tab);
+    GLA_CHECK_LAUNCH();
   }
   return GLA_OK;
 }

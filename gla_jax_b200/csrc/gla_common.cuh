@@ -121,18 +121,24 @@ unsigned int tc_read_wait_timeouts();
 size_t tc_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C);
 size_t tc_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C);
 size_t tc_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C);
+// Sequences of any length on one time axis (device tables, see gla_chunk_fwd_ragged): sequence s holds tokens
+// [cu[s], cu[s + 1]) and owns chunks [cub[s], cub[s + 1]); chunk n starts at token tab[n].x and has tab[n].y rows.
+struct Ragged { const int *cu, *cub; const int2* tab; int64_t chunks; };
 int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int64_t C,
                  const void* hidden_init, const float* g, const void* v, const void* k, const void* q,
                  void* hidden_final, void* out, void* saved, void* ws, int state_only,
                  float* G_total, float* S_local, int opts = 0, int64_t nseq = 0, const int* cu = nullptr,
-                 int sp_phase = 0, const float* H_in = nullptr);
+                 int sp_phase = 0, const float* H_in = nullptr, const Ragged* rag = nullptr);
 // One-pass chunk states (product and recurrence fused); mode 0 forward states, mode 1 gradient states.
 bool tc_state_fused_preferred(int64_t BH, int64_t N, int opts);
 int tc_state_fused(cudaStream_t st, int mode, int64_t B, int64_t T, int64_t H, int R, const float* g, const void* x,
                    const void* y, const void* init, void* states, void* fin, float* Gc, int64_t nseq = 0,
                    const int* cu = nullptr, unsigned int* done = nullptr, unsigned int* done_target = nullptr,
-                   float* fin32 = nullptr, int nsegs = 1);
+                   float* fin32 = nullptr, int nsegs = 1, const int* cub = nullptr, int64_t Nchunks = 0);
 int tc_state_segments(int64_t BH, int64_t N, int opts);
+int64_t ragged_chunks(int64_t nseq, const int* cu_host);
+size_t ragged_table_bytes(int64_t nseq, int64_t chunks);
+int ragged_tables(cudaStream_t st, int64_t nseq, const int* cu_host, void* mem, Ragged* r);
 unsigned int tc_state_read_wait_timeouts();
 unsigned int scan_read_wait_timeouts();
 unsigned int tc_state_read_bad_offsets();
@@ -140,7 +146,7 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
                  const float* g, const void* v, const void* k, const void* q, const void* saved,
                  const void* dhidden_final, const void* dout, void* dhidden_init, float* dg,
                  void* dv, void* dk, void* dq, void* ws, int opts = 0, int64_t nseq = 0, const int* cu = nullptr,
-                 int sp_phase = 0, float* A_local = nullptr, const float* dH_out = nullptr);
+                 int sp_phase = 0, float* A_local = nullptr, const float* dH_out = nullptr, const Ragged* rag = nullptr);
 
 }  // namespace gla
 

@@ -174,6 +174,89 @@ std::optional<std::tuple<Tensor, Tensor>> recurrent_gla(const Tensor& h, const T
   return std::make_tuple(r[0], r[1]);
 }
 
+// ---- chunk_gla over packed sequences ---------------------------------------------------------------------------------
+// Offsets either in host memory (any rising sequence) or as a CUDA int32 tensor (multiples of the chunk).
+struct PackedFn : torch::autograd::Function<PackedFn> {
+  static variable_list run(const Dims& d, int64_t nseq, const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
+                           const Tensor& offsets, int64_t chunk, bool residuals) {
+    Tensor hf = torch::empty_like(h), out = torch::empty_like(v);
+    void* st = stream_of(v);
+    if (!offsets.is_cuda()) {
+      const int32_t* cu = offsets.data_ptr<int32_t>();
+      const size_t n = gla_chunk_ragged_workspace_bytes(d.H, d.D, d.dt, nseq, cu, 0);
+      if (n == 0) raise("chunk_gla_packed: unsupported configuration " + shape_text(d, chunk, v));
+      Tensor saved = residuals ? bytes(v, gla_chunk_ragged_saved_bytes(d.H, d.D, d.dt, nseq, cu)) : Tensor(), ws = bytes(v, n);
+      check(gla_chunk_fwd_ragged(st, d.T, d.H, d.D, d.dt, nseq, cu, ptr(h), (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(hf), ptr(out),
+                                 ptr(saved), ptr(ws), n), "gla_chunk_fwd_ragged");
+      return {hf, out, saved};
+    }
+    const size_t n = gla_chunk_fwd_workspace_bytes(1, d.T, d.H, d.D, chunk, d.dt, GLA_IMPL_TCGEN05);
+    if (n == 0) raise("chunk_gla_packed: unsupported configuration " + shape_text(d, chunk, v));
+    Tensor saved = residuals ? bytes(v, gla_chunk_saved_bytes(1, d.T, d.H, d.D, chunk, d.dt, GLA_IMPL_TCGEN05)) : Tensor(), ws = bytes(v, n);
+    check(gla_chunk_fwd_packed(st, d.T, d.H, d.D, chunk, d.dt, nseq, offsets.data_ptr<int32_t>(), ptr(h), (const float*)ptr(g), ptr(v), ptr(k),
+                               ptr(q), ptr(hf), ptr(out), ptr(saved), ptr(ws), n), "gla_chunk_fwd_packed");
+    return {hf, out, saved};
+  }
+  static variable_list forward(AutogradContext* ctx, const Tensor& h0, const Tensor& g0, const Tensor& v0, const Tensor& k0,
+                               const Tensor& q0, const Tensor& cu, int64_t chunk, int64_t dt) {
+    const Dims d{1, v0.size(0), v0.size(1), v0.size(2), (int)dt};
+    Tensor h = h0.contiguous(), g = f32(g0), v = v0.contiguous(), k = k0.contiguous(), q = q0.contiguous();
+    variable_list r = run(d, h.size(0), h, g, v, k, q, cu, chunk, true);
+    ctx->save_for_backward({g, v, k, q, r[2], cu});
+    ctx->set_materialize_grads(false);
+    ctx->saved_data["d"] = std::vector<int64_t>{h.size(0), chunk, dt, !cu.is_cuda(), (int64_t)g0.scalar_type()};
+    return {r[0], r[1]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto a = ctx->saved_data["d"].toIntVector();
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &g = s[0], &v = s[1], &k = s[2], &q = s[3];
+    const int64_t nseq = a[0], T = v.size(0), H = v.size(1), D = v.size(2);
+    const int dt = (int)a[2];
+    Tensor dh = torch::empty({nseq, H, D, D}, v.options());
+    Tensor dhf = grad_or_zeros(grads[0], dh), dout = grad_or_zeros(grads[1], v);
+    Tensor dg = torch::empty_like(g), dv = torch::empty_like(v), dk = torch::empty_like(k), dq = torch::empty_like(q);
+    const int32_t* cu = s[5].data_ptr<int32_t>();
+    if (a[3]) {
+      const size_t n = gla_chunk_ragged_workspace_bytes(H, D, dt, nseq, cu, 1);
+      Tensor ws = bytes(v, n);
+      check(gla_chunk_bwd_ragged(stream_of(v), T, H, D, dt, nseq, cu, (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(s[4]), ptr(dhf),
+                                 ptr(dout), ptr(dh), (float*)ptr(dg), ptr(dv), ptr(dk), ptr(dq), ptr(ws), n), "gla_chunk_bwd_ragged");
+    } else {
+      const size_t n = gla_chunk_bwd_workspace_bytes(1, T, H, D, a[1], dt, GLA_IMPL_TCGEN05);
+      Tensor ws = bytes(v, n);
+      check(gla_chunk_bwd_packed(stream_of(v), T, H, D, a[1], dt, nseq, cu, (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(s[4]), ptr(dhf),
+                                 ptr(dout), ptr(dh), (float*)ptr(dg), ptr(dv), ptr(dk), ptr(dq), ptr(ws), n), "gla_chunk_bwd_packed");
+    }
+    const auto gt = (torch::ScalarType)a[4];
+    variable_list r{dh, gt == torch::kFloat32 ? dg : dg.to(gt), dv, dk, dq};
+    r.resize(8);
+    return r;
+  }
+};
+std::optional<std::tuple<Tensor, Tensor>> chunk_gla_packed(const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k,
+                                                           const Tensor& q, const Tensor& cu, int64_t chunk) {
+  if (!v.defined() || !here(v) || v.dim() != 3 || h.dim() != 4 || cu.dim() != 1 || cu.numel() != h.size(0) + 1) return std::nullopt;
+  Dims d{1, v.size(0), v.size(1), v.size(2), dt_of(v)};
+  for (const Tensor* t : {&h, &g, &k, &q}) if (t->device() != v.device()) return std::nullopt;
+  if (g.sizes() != v.sizes() || k.sizes() != v.sizes() || q.sizes() != v.sizes() || !g.is_floating_point()) return std::nullopt;
+  if (h.size(1) != d.H || h.size(2) != d.D || h.size(3) != d.D || d.dt < 0 || cu.scalar_type() != torch::kInt32) return std::nullopt;
+  for (const Tensor* t : {&h, &k, &q}) if (t->scalar_type() != v.scalar_type()) return std::nullopt;
+  if (chunk <= 0 || (chunk & (chunk - 1)) || chunk % 128) return std::nullopt;
+  Tensor c = cu.contiguous();
+  if (!c.is_cuda()) {
+    const int32_t* p = c.data_ptr<int32_t>();
+    if (p[0] != 0 || p[h.size(0)] != d.T) return std::nullopt;
+    for (int64_t s = 0; s < h.size(0); ++s) if (p[s + 1] <= p[s]) return std::nullopt;
+  } else if (c.device() != v.device()) {
+    return std::nullopt;
+  }
+  variable_list r = wants_grad({&h, &g, &v, &k, &q})
+                        ? PackedFn::apply(h, g, v, k, q, c, chunk, (int64_t)d.dt)
+                        : PackedFn::run(d, h.size(0), h.contiguous(), f32(g), v.contiguous(), k.contiguous(), q.contiguous(), c, chunk, false);
+  return std::make_tuple(r[0], r[1]);
+}
+
 // ---- decode step ---------------------------------------------------------------------------------------------------
 std::optional<Tensor> decode_step(Tensor state, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
                                   std::optional<torch::ScalarType> out_dtype) {
@@ -243,6 +326,7 @@ PYBIND11_MODULE(gla_b200_host, m) {
   m.def("set_error_class", [](py::object c) { g_error = c.release().ptr(); });
   m.def("chunk_gla", &chunk_gla, release());
   m.def("recurrent_gla", &recurrent_gla, release());
+  m.def("chunk_gla_packed", &chunk_gla_packed, release());
   m.def("decode_step", &decode_step, release());
   m.def("scan", &scan, release());
   m.def("rnn", &rnn, release());

@@ -75,9 +75,9 @@ __device__ unsigned int g_state_bad_offsets = 0;      // packed sequences whose 
 
 struct StMaps { CUtensorMap g, x, y; };
 
-template <int MODE>
+template <int MODE, bool RAG>
 __global__ void __launch_bounds__(STHREADS, 1)
-tc_state_kernel(const __grid_constant__ StMaps maps, int64_t T, int64_t H, int R, int Nall, const int* __restrict__ cu,
+tc_state_kernel(const __grid_constant__ StMaps maps, int64_t T, int64_t H, int R, int Nall, const int* __restrict__ cu, const int* __restrict__ cub,
                 const bf16* __restrict__ init, bf16* __restrict__ states, bf16* __restrict__ fin, float* __restrict__ fin32,
                 float* __restrict__ Gc, unsigned int* __restrict__ done, int nsegs) {
   extern __shared__ uint8_t smem_raw[];
@@ -113,8 +113,15 @@ tc_state_kernel(const __grid_constant__ StMaps maps, int64_t T, int64_t H, int R
   // Offsets come from device memory nobody has validated: whatever they hold, this block only touches chunks
   // [base, base + N) inside [0, Nall).  Offsets that are not rising multiples of the chunk length inside the
   // array are clamped (the sequence is cut short or skipped) and counted in g_state_bad_offsets.
-  int base = 0, N = Nall;
-  if (cu) {
+  // Sequences of any length (RAG; offsets validated on the host): sequence s holds tokens [cu[s], cu[s + 1]) and owns
+  // chunks [cub[s], cub[s + 1]) of the state arrays; the rows of its last chunk past its end belong to the next
+  // sequence and are masked (no decay, no key or query, a zeroed value row).
+  int base = 0, N = Nall, len = 0;
+  if (RAG) {
+    base = cub[bh / H];
+    N = cub[bh / H + 1] - base;
+    len = cu[bh / H + 1] - cu[bh / H];
+  } else if (cu) {
     const int lo = cu[bh / H], hi = cu[bh / H + 1];
     base = min(max(lo / SC, 0), Nall);
     N = min(max((hi - lo) / SC, 0), Nall - base);
@@ -160,7 +167,7 @@ tc_state_kernel(const __grid_constant__ StMaps maps, int64_t T, int64_t H, int R
 
   if (warp == (NBUILD + NUPD) / 32 + 1) {
     // ================= TMA producer warp =================
-    const int z0 = (int)(b * T) + base * SC, yk = (int)hk, yv = (int)hv;
+    const int z0 = RAG ? cu[bh / H] : (int)(b * T) + base * SC, yk = (int)hk, yv = (int)hv;
     const int zstep = MODE == 0 ? SC : -SC;
     const uint32_t sm_base = smem_u32(sm), fully0 = smem_u32(fully), fullgx0 = smem_u32(fullgx);
     auto load_y = [&](int z, int s) {
@@ -247,6 +254,18 @@ tc_state_kernel(const __grid_constant__ StMaps maps, int64_t T, int64_t H, int R
       for (int j = 0; j < 16; ++j) {
         f[j] = gt[(r0 + j) * SL + lane];
         xr[j] = xt[(r0 + j) * SL + lane];
+      }
+      const int nv = RAG ? len - chunk_of(i) * SC : SC;
+      if (RAG && nv < SC) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (r0 + j >= nv) { f[j] = 0.f; xr[j] = 0u; }
+        if (ok) ok = mbar_wait(smem_u32(fully + (i % NY)), (uint32_t)((i / NY) & 1));
+        uint8_t* yt = sm + StSmem::Y + (i % NY) * 32768;
+        for (int r = nv + w; r < SC; r += 8) {              // a swizzled row is 128 bytes of each half
+          *reinterpret_cast<uint32_t*>(yt + r * 128 + lane * 4) = 0u;
+          *reinterpret_cast<uint32_t*>(yt + 16384 + r * 128 + lane * 4) = 0u;
+        }
       }
       // The product of the 16 gates first (as the exponential of their sum), so that the groups can exchange
       // totals early and the running products below start from the cross-group factor.
@@ -425,18 +444,20 @@ int tc_state_segments(int64_t BH, int64_t N, int opts) {
 // mode 1: states[n] = gradient state after chunk n (from init = dhidden_final), fin = dhidden_init.
 int tc_state_fused(cudaStream_t st, int mode, int64_t B, int64_t T, int64_t H, int R, const float* g, const void* x,
                    const void* y, const void* init, void* states, void* fin, float* Gc, int64_t nseq, const int* cu,
-                   unsigned int* done, unsigned int* done_target, float* fin32, int nsegs) {
+                   unsigned int* done, unsigned int* done_target, float* fin32, int nsegs, const int* cub, int64_t Nchunks) {
   if (nsegs < 1 || (nsegs > 1 && (cu != nullptr || fin32 == nullptr || done != nullptr || nsegs > T / SC))) return GLA_ERR_UNSUPPORTED;
   // packed sequences: B == 1, cu (device, nseq + 1 token offsets) non-null, init / fin are (nseq, H, 128, 128)
-  const int64_t N = T / SC, BH = (cu ? nseq : B) * H;          // H: virtual heads (real heads x R x R)
+  // cub (with cu): sequences of any length, Nchunks chunks in all
+  const int64_t N = cub ? Nchunks : T / SC, BH = (cu ? nseq : B) * H;          // H: virtual heads (real heads x R x R)
   const int64_t HK = H / R;                      // heads of the (B, T, HK, 128) view of the arrays
   StMaps maps;
   GLA_TRY(make_map_bthd(&maps.g, g, 1, B, T, HK, SL, 0));
   GLA_TRY(make_map_bthd(&maps.x, x, 0, B, T, HK, SL, 0));
   GLA_TRY(make_map_bthd(&maps.y, y, 0, B, T, HK, 64, 1));
-  auto kern = mode == 0 ? tc_state_kernel<0> : tc_state_kernel<1>;
-  static SmemAttrOnce attr[2];
-  GLA_TRY(attr[mode != 0].ensure(kern, ST_SMEM));
+  auto kern = cub ? (mode == 0 ? tc_state_kernel<0, true> : tc_state_kernel<1, true>)
+                  : (mode == 0 ? tc_state_kernel<0, false> : tc_state_kernel<1, false>);
+  static SmemAttrOnce attr[4];
+  GLA_TRY(attr[(mode != 0) + 2 * (cub != nullptr)].ensure(kern, ST_SMEM));
   cudaError_t e;
   if (done != nullptr) {
     e = cudaMemsetAsync(done, 0, sizeof(unsigned int), st);
@@ -446,7 +467,7 @@ int tc_state_fused(cudaStream_t st, int mode, int64_t B, int64_t T, int64_t H, i
   {
     ProfScope ps(mode == 0 ? "tc_state_kernel" : "tc_dstate_scan_kernel", st);
     if (BH * 4 * nsegs > 2147483647LL) return GLA_ERR_TOO_LARGE;
-    kern<<<(unsigned)(BH * 4 * nsegs), STHREADS, ST_SMEM, st>>>(maps, T, H, R, (int)N, cu, (const bf16*)init, (bf16*)states,
+    kern<<<(unsigned)(BH * 4 * nsegs), STHREADS, ST_SMEM, st>>>(maps, T, H, R, (int)N, cu, cub, (const bf16*)init, (bf16*)states,
                                                                 (bf16*)fin, fin32, Gc, done, nsegs);
   }
   GLA_CHECK_LAUNCH();

@@ -141,52 +141,6 @@ def recurrent_gla_naive(hidden, log_fgate, value, key, query, reverse: bool = Fa
     return r if r is not None else _refused("recurrent_gla_naive", hidden, log_fgate, value, key, query)
 
 
-class _ChunkGLAPacked(torch.autograd.Function):
-    """chunk_gla over sequences laid end to end on one time axis (gla_chunk_fwd_packed / gla_chunk_bwd_packed)."""
-
-    @staticmethod
-    def forward(ctx, hidden, g, v, k, q, cu, chunk):
-        lib = _lib.load()
-        T, H, D = v.shape
-        nseq = hidden.shape[0]
-        dt = _DT[v.dtype]
-        g32 = g if g.dtype == torch.float32 else g.float()
-        ws_n = lib.gla_chunk_fwd_workspace_bytes(1, T, H, D, chunk, dt, _lib.IMPL_TCGEN05)
-        if ws_n == 0:
-            raise _lib.GlaError(f"chunk_gla_packed: unsupported configuration T={T} H={H} D={D} chunk={chunk} dtype={v.dtype}")
-        need_grad = any(ctx.needs_input_grad[:5])
-        saved = torch.empty(lib.gla_chunk_saved_bytes(1, T, H, D, chunk, dt, _lib.IMPL_TCGEN05), dtype=torch.uint8,
-                            device=v.device) if need_grad else None
-        ws = torch.empty(ws_n, dtype=torch.uint8, device=v.device)
-        hf, out = torch.empty_like(hidden), torch.empty_like(v)
-        st = lib.gla_chunk_fwd_packed(_stream(v.device), T, H, D, chunk, dt, nseq, _ptr(cu), _ptr(hidden), _ptr(g32), _ptr(v),
-                                      _ptr(k), _ptr(q), _ptr(hf), _ptr(out), _ptr(saved), _ptr(ws), ws_n)
-        _lib.check(st, "gla_chunk_fwd_packed")
-        if need_grad:
-            ctx.save_for_backward(g32, v, k, q, cu, saved)
-        ctx.chunk, ctx.g_dtype, ctx.nseq = chunk, g.dtype, nseq
-        return hf, out
-
-    @staticmethod
-    def backward(ctx, dhf, dout):
-        lib = _lib.load()
-        g32, v, k, q, cu, saved = ctx.saved_tensors
-        T, H, D = v.shape
-        dt = _DT[v.dtype]
-        dhf = torch.zeros(ctx.nseq, H, D, D, dtype=v.dtype, device=v.device) if dhf is None else dhf.to(v.dtype).contiguous()
-        dout = torch.zeros_like(v) if dout is None else dout.to(v.dtype).contiguous()
-        ws_n = lib.gla_chunk_bwd_workspace_bytes(1, T, H, D, ctx.chunk, dt, _lib.IMPL_TCGEN05)
-        ws = torch.empty(ws_n, dtype=torch.uint8, device=v.device)
-        dh = torch.empty_like(dhf)
-        dg = torch.empty_like(g32)
-        dv, dk, dq = torch.empty_like(v), torch.empty_like(k), torch.empty_like(q)
-        st = lib.gla_chunk_bwd_packed(_stream(v.device), T, H, D, ctx.chunk, dt, ctx.nseq, _ptr(cu), _ptr(g32), _ptr(v),
-                                      _ptr(k), _ptr(q), _ptr(saved), _ptr(dhf), _ptr(dout), _ptr(dh), _ptr(dg), _ptr(dv),
-                                      _ptr(dk), _ptr(dq), _ptr(ws), ws_n)
-        _lib.check(st, "gla_chunk_bwd_packed")
-        return dh, dg.to(ctx.g_dtype), dv, dk, dq, None, None
-
-
 def chunk_gla_packed(hidden_init, log_fgate, value, key, query, cu_seqlens, chunk_size: int = 128):
     """``chunk_gla`` for variable-length sequences packed end to end on one time axis.
 
@@ -196,17 +150,19 @@ def chunk_gla_packed(hidden_init, log_fgate, value, key, query, cu_seqlens, chun
     differentiable.  The reference has one length per call and asserts T % chunk == 0 (gla.py:499-500, 674); this
     runs on the tensor-core kernels only (bf16, D = 128).
 
-    Offsets given as a list or CPU tensor may be ANY rising sequence: the kernels work on chunks of 128 rows that
-    must not straddle two sequences, so sequences whose lengths are not multiples of 128 are first laid out with
-    their tails padded to the next multiple (padding tokens have log_fgate = 0 and key = value = query = 0: no decay,
-    no update, so states and gradients are those of the unpadded sequence) and the outputs are gathered back; the
-    two copies are differentiable torch index operations.  Offsets given as a CUDA int32 tensor are used as they
-    are, without a host round trip, and must be multiples of 128 (the kernels clamp anything else and count it in
-    ``gla_device_bad_offsets``)."""
+    Offsets given as a list or CPU tensor may be ANY rising sequence: every sequence starts a chunk of its own at its
+    first token and the rows of its last chunk past its end are masked inside the kernels.  Offsets given as a CUDA
+    int32 tensor are used as they are, without a host round trip, and must be multiples of 128 (the kernels clamp
+    anything else and count it in ``gla_device_bad_offsets``)."""
+    cu = cu_seqlens if torch.is_tensor(cu_seqlens) else torch.tensor(cu_seqlens, dtype=torch.int32)
+    if cu.dtype != torch.int32:
+        cu = cu.to(torch.int32)
+    r = _lib.native().chunk_gla_packed(hidden_init, log_fgate, value, key, query, cu, int(chunk_size))
+    if r is not None:
+        return r
     if value.dim() != 3 or hidden_init.dim() != 4:
         raise ValueError("chunk_gla_packed: expected value (T, H, D) and hidden_init (nseq, H, D, D)")
     T, H, D = value.shape
-    cu = torch.as_tensor(cu_seqlens, dtype=torch.int32) if not torch.is_tensor(cu_seqlens) else cu_seqlens.to(torch.int32)
     nseq = cu.numel() - 1
     if nseq < 1 or tuple(hidden_init.shape) != (nseq, H, D, D):
         raise ValueError("chunk_gla_packed: cu_seqlens must have nseq + 1 entries for hidden_init (nseq, H, D, D)")
@@ -214,26 +170,12 @@ def chunk_gla_packed(hidden_init, log_fgate, value, key, query, cu_seqlens, chun
         raise ValueError("chunk_gla_packed: log_fgate, value, key, query must all be (T, H, D)")
     if not value.is_cuda:
         raise TypeError("chunk_gla_packed: CUDA tensors required (there is no CPU path)")
-    idx = None
-    if not cu.is_cuda:
-        # offsets given on the host are checked here; a CUDA tensor is taken as is (checking it would synchronise)
-        if int(cu[0]) != 0 or int(cu[-1]) != T or bool(((cu[1:] - cu[:-1]) <= 0).any()):
-            raise ValueError("chunk_gla_packed: cu_seqlens must rise from 0 to T")
-        if bool((cu % 128 != 0).any()):
-            # ragged lengths: positions of the tokens on a time axis where every sequence starts at a multiple of 128
-            lens = (cu[1:] - cu[:-1]).to(torch.int64)
-            plen = (lens + 127) // 128 * 128
-            pcu = torch.zeros(nseq + 1, dtype=torch.int64)
-            pcu[1:] = torch.cumsum(plen, 0)
-            idx = torch.cat([torch.arange(int(lens[s_]), dtype=torch.int64) + int(pcu[s_]) for s_ in range(nseq)]).to(value.device)
-            Tp = int(pcu[-1])
-            pad = lambda x: x.new_zeros((Tp,) + tuple(x.shape[1:])).index_copy(0, idx, x)
-            log_fgate, value, key, query = pad(log_fgate), pad(value), pad(key), pad(query)
-            cu = pcu.to(torch.int32)
-    cu = cu.to(value.device).contiguous()
-    hf, out = _ChunkGLAPacked.apply(hidden_init.contiguous(), log_fgate.contiguous(), value.contiguous(), key.contiguous(),
-                                    query.contiguous(), cu, int(chunk_size))
-    return (hf, out) if idx is None else (hf, out.index_select(0, idx))
+    if not cu.is_cuda and (int(cu[0]) != 0 or int(cu[-1]) != T or bool(((cu[1:] - cu[:-1]) <= 0).any())):
+        raise ValueError("chunk_gla_packed: cu_seqlens must rise from 0 to T")
+    _stream(value.device)
+    if int(chunk_size) % 128 or int(chunk_size) <= 0 or int(chunk_size) & (int(chunk_size) - 1):
+        raise _lib.GlaError(f"chunk_gla_packed: unsupported configuration T={T} H={H} D={D} chunk={chunk_size} dtype={value.dtype}")
+    raise TypeError("chunk_gla_packed: bfloat16 arrays with a floating-point log_fgate, all on one device, are required")
 
 
 def decode_step(state, log_fgate, value, key, query, out_dtype=None):

@@ -371,6 +371,25 @@ GLA_API int gla_chunk_bwd_packed(void* stream, int64_t T, int64_t H, int64_t D, 
                          void* dhidden_init, float* dlog_fgate, void* dvalue, void* dkey, void* dquery,
                          void* workspace, size_t workspace_bytes);
 
+/* The same for sequences of ANY length (at least one token each), with the offsets in HOST memory: cu_seqlens rises
+ * strictly from 0 to T and is read before the call returns.  Every sequence starts a chunk of its own at its first
+ * token; the rows of its last chunk past its end are masked inside the kernels, so nothing is copied or padded.
+ * saved / workspace sizes from the functions here (0: invalid offsets or unsupported sizes). */
+GLA_API size_t gla_chunk_ragged_saved_bytes(int64_t H, int64_t D, int dtype, int64_t nseq, const int32_t* cu_seqlens_host);
+GLA_API size_t gla_chunk_ragged_workspace_bytes(int64_t H, int64_t D, int dtype, int64_t nseq, const int32_t* cu_seqlens_host,
+                         int backward);
+GLA_API int gla_chunk_fwd_ragged(void* stream, int64_t T, int64_t H, int64_t D, int dtype,
+                         int64_t nseq, const int32_t* cu_seqlens_host,
+                         const void* hidden_init, const float* log_fgate, const void* value,
+                         const void* key, const void* query, void* hidden_final, void* out,
+                         void* saved, void* workspace, size_t workspace_bytes);
+GLA_API int gla_chunk_bwd_ragged(void* stream, int64_t T, int64_t H, int64_t D, int dtype,
+                         int64_t nseq, const int32_t* cu_seqlens_host,
+                         const float* log_fgate, const void* value, const void* key, const void* query,
+                         const void* saved, const void* dhidden_final, const void* dout,
+                         void* dhidden_init, float* dlog_fgate, void* dvalue, void* dkey, void* dquery,
+                         void* workspace, size_t workspace_bytes);
+
 /* ------------------------------------------------------------------------------------
  * Sequence-parallel support (no counterpart in the reference, which is single-device; the
  * algebra is ops.py:286 binary_operator applied across ranks and the exact chaining of
