@@ -53,6 +53,33 @@ struct ProfScope {
   ~ProfScope();
 };
 
+// Launch that may begin while the kernel before it on the stream drains (programmatic stream serialisation): its blocks
+// are placed and its prologue runs, and `grid_dep_wait` in the kernel then waits for everything the stream holds before
+// it.  The kernel calls `grid_dep_launch` to let its own successor do the same.  This takes the launch gap (2 to 3 us)
+// out of sequences of short kernels.
+template <typename... KP, typename... A>
+static inline cudaError_t launch_overlapped(void (*kern)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, KP(args)...);
+}
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#define GLA_LAUNCHED(expr)                                   \
+  do {                                                       \
+    ::gla::count_launch();                                   \
+    int _s = ::gla::record_cuda_error(expr);                 \
+    if (_s != GLA_OK) return _s;                             \
+  } while (0)
+
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 static inline bool is_pow2(int64_t x) { return x > 0 && (x & (x - 1)) == 0; }
 static inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }

@@ -9,53 +9,72 @@
 // would run recurrent_gla with T = 1.
 //
 // The step is pure HBM streaming: 2 * 4 * D * D bytes of state per (request, head) against 5 D bytes of
-// everything else.  A block owns 32 value columns of one head's state: 256 threads = 32 columns x 8 row
-// lanes, each thread walks D / 8 key rows (coalesced 128-byte rows, loads of a whole 8-row group issued
-// before they are used), keeps its partial of o, and the 8 row lanes are summed through shared memory.
+// everything else.  A block owns 32 value columns of one head's state: 8 lanes of four columns x 16 row lanes, every
+// 16-byte load of its rows issued before one is used (16 KB per block at D = 128, sixteen blocks per SM), partial sums
+// of o combined through shared memory.  Steps of one model follow each other back to back, so the launch overlaps the
+// kernel before it.  Measured, 32 requests x 16 heads, D = 128: 14.3 us (scalar loads, plain launch) -> 12.0 us (the bytes at the copy
+// rate: 10.4).
 #include "gla_common.cuh"
 
 namespace gla {
 
 constexpr int DC = 32;       // value columns per block
-constexpr int DR = 8;        // row lanes
+constexpr int DL = DC / 4;   // column lanes
+constexpr int DR = 16;       // row lanes
 
-template <int D>
-__global__ void __launch_bounds__(DC * DR) decode_step_kernel(float* __restrict__ S, const float* __restrict__ g,
+// a state whose base is not 16-byte aligned (a view) takes four scalar accesses instead
+template <bool AL> __device__ __forceinline__ float4 ld_state(const float* p) {
+  if constexpr (AL) return *reinterpret_cast<const float4*>(p);
+  else return make_float4(p[0], p[1], p[2], p[3]);
+}
+template <bool AL> __device__ __forceinline__ void st_state(float* p, float4 x) {
+  if constexpr (AL) *reinterpret_cast<float4*>(p) = x;
+  else { p[0] = x.x; p[1] = x.y; p[2] = x.z; p[3] = x.w; }
+}
+template <int D, bool AL>
+__global__ void __launch_bounds__(DL * DR) decode_step_kernel(float* __restrict__ S, const float* __restrict__ g,
                                                               const void* __restrict__ v, const void* __restrict__ k,
                                                               const void* __restrict__ q, void* __restrict__ out,
                                                               int bf, int out_bf) {
   constexpr int RPT = D / DR;                   // key rows per thread
   __shared__ float red[DR][DC];
   __shared__ float fk[3][D];                    // exp(g), k, q of this (request, head)
-  const int col = threadIdx.x % DC, rl = threadIdx.x / DC;
+  const int cl = threadIdx.x % DL, rl = threadIdx.x / DL;
   const int64_t bh = blockIdx.y;
-  const int c0 = blockIdx.x * DC;
-  for (int i = threadIdx.x; i < D; i += DC * DR) {
+  const int c0 = blockIdx.x * DC + 4 * cl;
+  float* Sp = S + (bh * D + rl) * (int64_t)D + c0;     // rows rl, rl + 16, ...
+  grid_dep_wait();
+  grid_dep_launch();
+  float4 s[RPT];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) s[i] = ld_state<AL>(Sp + (int64_t)i * DR * D);
+  for (int i = threadIdx.x; i < D; i += DL * DR) {
     fk[0][i] = expf(g[bh * D + i]);
     fk[1][i] = ld_any(k, bf, bh * D + i);
     fk[2][i] = ld_any(q, bf, bh * D + i);
   }
-  const float vv = ld_any(v, bf, bh * D + c0 + col);
-  float* Sp = S + (bh * D + rl) * (int64_t)D + c0 + col;     // rows rl, rl + 8, ...
-  float s[RPT];
-#pragma unroll
-  for (int i = 0; i < RPT; ++i) s[i] = Sp[(int64_t)i * DR * D];
+  float4 vv;
+  vv.x = ld_any(v, bf, bh * D + c0); vv.y = ld_any(v, bf, bh * D + c0 + 1);
+  vv.z = ld_any(v, bf, bh * D + c0 + 2); vv.w = ld_any(v, bf, bh * D + c0 + 3);
   __syncthreads();
-  float acc = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < RPT; ++i) {
     const int r = rl + i * DR;
-    const float ns = fmaf(fk[0][r], s[i], fk[1][r] * vv);
-    Sp[(int64_t)i * DR * D] = ns;
-    acc = fmaf(fk[2][r], ns, acc);
+    const float f = fk[0][r], kr = fk[1][r], qr = fk[2][r];
+    float4 n;
+    n.x = fmaf(f, s[i].x, kr * vv.x); n.y = fmaf(f, s[i].y, kr * vv.y);
+    n.z = fmaf(f, s[i].z, kr * vv.z); n.w = fmaf(f, s[i].w, kr * vv.w);
+    st_state<AL>(Sp + (int64_t)i * DR * D, n);
+    acc.x = fmaf(qr, n.x, acc.x); acc.y = fmaf(qr, n.y, acc.y); acc.z = fmaf(qr, n.z, acc.z); acc.w = fmaf(qr, n.w, acc.w);
   }
-  red[rl][col] = acc;
+  *reinterpret_cast<float4*>(&red[rl][4 * cl]) = acc;
   __syncthreads();
-  if (rl == 0) {
+  if (threadIdx.x < DC) {
     float o = 0.f;
 #pragma unroll
-    for (int j = 0; j < DR; ++j) o += red[j][col];
-    st_any(out, out_bf, bh * D + c0 + col, o);
+    for (int j = 0; j < DR; ++j) o += red[j][threadIdx.x];
+    st_any(out, out_bf, bh * D + blockIdx.x * DC + threadIdx.x, o);
   }
 }
 
@@ -64,8 +83,7 @@ static int launch_decode(cudaStream_t st, int64_t BH, float* S, const float* g, 
                          const void* q, void* out, int bf, int out_bf) {
   if (BH > 65535) return GLA_ERR_TOO_LARGE;
   ProfScope ps("decode_step_kernel", st);
-  decode_step_kernel<D><<<dim3(D / DC, (unsigned)BH), DC * DR, 0, st>>>(S, g, v, k, q, out, bf, out_bf);
-  GLA_CHECK_LAUNCH();
+  GLA_LAUNCHED(launch_overlapped(aligned16(S) ? decode_step_kernel<D, true> : decode_step_kernel<D, false>, dim3(D / DC, (unsigned)BH), dim3(DL * DR), 0, st, S, g, v, k, q, out, bf, out_bf));
   return GLA_OK;
 }
 

@@ -88,6 +88,8 @@ __global__ void __launch_bounds__(32 * SK_RL, 4) scan_kernel(const TI* __restric
   float carry[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) carry[v] = OP::id();
+  grid_dep_wait();
+  grid_dep_launch();
   if (init != nullptr && cvalid) sk_load<TI, VEC>(init + n * D + c, carry);
   // scan position p lies at row p (forward) or T - 1 - p (reversed); a thread's rows are `rs` elements apart
   const int64_t rs = reverse ? -D : D, p0 = (int64_t)rank * ROWS + rl * RPT;
@@ -423,11 +425,13 @@ static int launch_scan_rows(cudaStream_t st, int64_t N, int64_t T, int64_t D, co
   cfg.gridDim = dim3((unsigned)(items * cl));
   cfg.blockDim = dim3(32, SK_RL);
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;        // see launch_overlapped
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cl; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cl > 1 ? 1 : 0;
+  cfg.numAttrs = cl > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, scan_kernel<TI, TO, OP, VEC, RPT>, (const TI*)src, (const TI*)sub, (const TI*)init,
                                            (TO*)dst, T, D, (int)gy, cl, reverse);
   if (e != cudaSuccess) return record_cuda_error(e);
@@ -507,6 +511,8 @@ __global__ void __launch_bounds__(128) rnn_scan_vec4_kernel(int64_t T, int64_t K
   if (e4 >= K * V4) return;
   const int64_t kk = e4 / V4, e = e4 * 4;
   const bool writes_log = (e4 % V4) == 0;
+  grid_dep_wait();
+  grid_dep_launch();
   float A = (ig && seg == 0) ? ig[prob * K + kk] : 0.f;
   float4 b = (ikv && seg == 0) ? ld4_f(ikv + prob * KV + e) : make_float4(0.f, 0.f, 0.f, 0.f);
   const float* gp = g + prob * T * K + kk;
@@ -677,19 +683,13 @@ int launch_rnn_scan(cudaStream_t st, int64_t batch, int64_t T, int64_t K, int64_
     }
     if (nblk * batch * nseg > 2147483647LL) return GLA_ERR_TOO_LARGE;
     dim3 grid((unsigned)(nblk * batch * nseg)), block(128);
-    if (kv_bf16 && nseg > 1)
-      rnn_scan_vec4_kernel<bf16, true><<<grid, block, 0, st>>>(T, K, V, nblk, g, (const bf16*)kv, ig, (const bf16*)ikv,
-                                                               out_log, (bf16*)out_state, reverse, last_only, nseg, L);
-    else if (kv_bf16)
-      rnn_scan_vec4_kernel<bf16, false><<<grid, block, 0, st>>>(T, K, V, nblk, g, (const bf16*)kv, ig, (const bf16*)ikv,
-                                                                out_log, (bf16*)out_state, reverse, last_only, 1, T);
-    else if (nseg > 1)
-      rnn_scan_vec4_kernel<float, true><<<grid, block, 0, st>>>(T, K, V, nblk, g, (const float*)kv, ig, (const float*)ikv,
-                                                                out_log, (float*)out_state, reverse, last_only, nseg, L);
-    else
-      rnn_scan_vec4_kernel<float, false><<<grid, block, 0, st>>>(T, K, V, nblk, g, (const float*)kv, ig, (const float*)ikv,
-                                                                 out_log, (float*)out_state, reverse, last_only, 1, T);
-    GLA_CHECK_LAUNCH();
+    auto run = [&](auto kern, auto t) {
+      using TKV = decltype(t);
+      return launch_overlapped(kern, grid, block, 0, st, T, K, V, nblk, g, (const TKV*)kv, ig, (const TKV*)ikv, out_log, (TKV*)out_state,
+                               reverse, last_only, nseg, nseg > 1 ? L : T);
+    };
+    if (kv_bf16) GLA_LAUNCHED(run(nseg > 1 ? rnn_scan_vec4_kernel<bf16, true> : rnn_scan_vec4_kernel<bf16, false>, bf16()));
+    else GLA_LAUNCHED(run(nseg > 1 ? rnn_scan_vec4_kernel<float, true> : rnn_scan_vec4_kernel<float, false>, 0.f));
     if (nseg > 1) {
       float* wsL = ws;
       float* wsS = ws + batch * nseg * K;      // batch * nseg * K floats: a multiple of 16 bytes when K % 4 == 0
