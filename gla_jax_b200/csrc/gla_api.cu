@@ -219,6 +219,22 @@ int gla_layer_gate_bwd(void* stream, int64_t n, int dtype, const void* z, const 
   return layer_gate_bwd((cudaStream_t)stream, n, dtype == GLA_BF16, z, dlog_fgate, inv_tau, dz);
 }
 
+size_t gla_layer_gate_bwd_bias_workspace_bytes(int64_t rows, int64_t cols) {
+  if (rows <= 0 || cols <= 0) return 0;
+  return layer_gate_bwd_bias_ws_bytes(rows, cols);
+}
+
+int gla_layer_gate_bwd_bias(void* stream, int64_t rows, int64_t cols, int dtype, const void* z, const float* dlog_fgate,
+                            float inv_tau, void* dz, void* dbias, void* workspace, size_t workspace_bytes) {
+  if (!z || !dlog_fgate || !dz || !dbias) return GLA_ERR_NULL_POINTER;
+  if (rows <= 0 || cols <= 0) return GLA_ERR_BAD_DIMS;
+  GLA_TRY(check_dtype(dtype));
+  if (cols % 8 != 0 || cols > (1 << 24)) return GLA_ERR_UNSUPPORTED;
+  if (!aligned16(z) || !aligned16(dlog_fgate) || !aligned16(dz)) return GLA_ERR_ALIGNMENT;
+  if (!workspace || workspace_bytes < layer_gate_bwd_bias_ws_bytes(rows, cols)) return GLA_ERR_WORKSPACE;
+  return layer_gate_bwd_bias((cudaStream_t)stream, rows, cols, dtype == GLA_BF16, z, dlog_fgate, inv_tau, dz, dbias, workspace);
+}
+
 static int check_head_dim(int64_t D) { return (D == 32 || D == 64 || D == 128 || D == 256) ? GLA_OK : GLA_ERR_UNSUPPORTED; }
 
 int gla_layer_headnorm_gate_fwd(void* stream, int64_t rows, int64_t D, int dtype, const void* x, const void* gate,

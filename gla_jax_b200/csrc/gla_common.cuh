@@ -106,6 +106,9 @@ int decode_step(cudaStream_t st, int64_t B, int64_t H, int64_t D, int bf, float*
 // Element-wise stages of a GLA layer either side of the op.
 int layer_gate_fwd(cudaStream_t st, int64_t n, int bf, const void* z, float inv_tau, float* g);
 int layer_gate_bwd(cudaStream_t st, int64_t n, int bf, const void* z, const float* dg, float inv_tau, void* dz);
+size_t layer_gate_bwd_bias_ws_bytes(int64_t rows, int64_t cols);
+int layer_gate_bwd_bias(cudaStream_t st, int64_t rows, int64_t cols, int bf, const void* z, const float* dg, float inv_tau, void* dz,
+                        void* dbias, void* ws);
 int layer_headnorm_gate_fwd(cudaStream_t st, int64_t rows, int64_t D, int bf, const void* x, const void* gate,
                             const float* w, float eps, void* y, float* rstd);
 size_t layer_headnorm_gate_bwd_ws_bytes(int64_t rows, int64_t D);

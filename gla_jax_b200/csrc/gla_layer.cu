@@ -245,31 +245,70 @@ __global__ void __launch_bounds__(LY_THREADS) headnorm_gate_bwd_kernel(int64_t r
   }
 }
 
-// out[d] = sum over the rows of partial (nrows, D): a block owns 32 columns, its 8 row lanes walk
-// the rows eight apart (four loads in flight each) and are summed through shared memory.
-__global__ void __launch_bounds__(LY_THREADS) column_sum_kernel(int nrows, int D, const float* __restrict__ partial,
-                                                               float* __restrict__ out) {
-  __shared__ float red[LY_WARPS][33];
+// out[d] = sum over the rows of partial (nrows, D): a block owns 32 columns, its 32 row lanes walk the rows 32 apart and
+// are summed through shared memory in a fixed order.
+constexpr int CS_LANES = 32;
+__global__ void __launch_bounds__(32 * CS_LANES) column_sum_kernel(int nrows, int D, const float* __restrict__ partial,
+                                                                   void* __restrict__ out, int out_bf) {
+  __shared__ float red[CS_LANES][33];
   const int tx = threadIdx.x % 32, rl = threadIdx.x / 32;
   const int d = blockIdx.x * 32 + tx;
   float s = 0.f;
   if (d < D) {
-    int r = rl;
-    for (; r + 3 * LY_WARPS < nrows; r += 4 * LY_WARPS) {
-      const float a = partial[(int64_t)r * D + d], b = partial[(int64_t)(r + LY_WARPS) * D + d];
-      const float c = partial[(int64_t)(r + 2 * LY_WARPS) * D + d], e = partial[(int64_t)(r + 3 * LY_WARPS) * D + d];
-      s += (a + b) + (c + e);
-    }
-    for (; r < nrows; r += LY_WARPS) s += partial[(int64_t)r * D + d];
+#pragma unroll 4
+    for (int r = rl; r < nrows; r += CS_LANES) s += partial[(int64_t)r * D + d];
   }
   red[rl][tx] = s;
   __syncthreads();
   if (rl == 0 && d < D) {
     float t = 0.f;
 #pragma unroll
-    for (int k = 0; k < LY_WARPS; ++k) t += red[k][tx];
-    out[d] = t;
+    for (int k = 0; k < CS_LANES; ++k) t += red[k][tx];
+    st_any(out, out_bf, d, t);
   }
+}
+
+// gate_bwd over a (rows, cols) array with the column sums of dz (the gradient of the gate projection's bias) formed on
+// the way: a block owns 256 columns (32 lanes of eight) and every gridDim.y-th group of eight rows; one row of partial
+// sums per block, added up by column_sum_kernel.  The sums are of the rounded dz, as a reduction over the stored array
+// gives.  What this saves is that array's second trip through HBM (32 us of reduction at 16384 x 768 in bf16).
+template <typename TZ>
+__global__ void __launch_bounds__(LY_THREADS) gate_bwd_bias_kernel(int64_t rows, int64_t cols, const TZ* __restrict__ z,
+                                                                   const float* __restrict__ dg, float inv_tau,
+                                                                   TZ* __restrict__ dz, float* __restrict__ partial) {
+  __shared__ float red[LY_WARPS][256];
+  const int lane = threadIdx.x % 32, rl = threadIdx.x / 32;
+  const int64_t c = (int64_t)blockIdx.x * 256 + lane * 8;
+  float acc[8] = {};
+  if (c < cols) {
+    const int64_t step = (int64_t)gridDim.y * LY_WARPS;
+    for (int64_t r0 = (int64_t)blockIdx.y * LY_WARPS + rl; r0 < rows; r0 += 2 * step) {
+      float v[2][8], d[2][8];              // two rows' loads in flight
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int64_t o = (r0 + u * step < rows ? r0 + u * step : r0) * cols + c;
+        ld_vec<8>(z + o, v[u]);
+        ld_vec<8>(dg + o, d[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (u == 1 && r0 + step >= rows) break;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[u][e] = d[u][e] * inv_tau * sigmoid(-v[u][e]);
+        st_vec<8>(dz + (r0 + u * step) * cols + c, v[u]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += sizeof(TZ) == 2 ? __bfloat162float(__float2bfloat16_rn(v[u][e])) : v[u][e];
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) red[rl][e * 32 + lane] = acc[e];
+  __syncthreads();
+  float s = 0.f;
+#pragma unroll
+  for (int k = 0; k < LY_WARPS; ++k) s += red[k][threadIdx.x];
+  const int64_t cc = (int64_t)blockIdx.x * 256 + (threadIdx.x % 32) * 8 + threadIdx.x / 32;
+  if (cc < cols) partial[(int64_t)blockIdx.y * cols + cc] = s;
 }
 
 int stream_grid(int64_t units_per_block_total) {
@@ -344,6 +383,27 @@ int layer_gate_bwd(cudaStream_t st, int64_t n, int bf, const void* z, const floa
   return GLA_OK;
 }
 
+static int gate_bias_splits(int64_t rows, int64_t cols) {
+  const int64_t gx = (cols + 255) / 256, want = (148 * 4 + gx - 1) / gx, most = (rows + LY_WARPS - 1) / LY_WARPS;
+  return (int)(want < most ? want : most);
+}
+size_t layer_gate_bwd_bias_ws_bytes(int64_t rows, int64_t cols) { return (size_t)gate_bias_splits(rows, cols) * cols * sizeof(float); }
+int layer_gate_bwd_bias(cudaStream_t st, int64_t rows, int64_t cols, int bf, const void* z, const float* dg, float inv_tau, void* dz,
+                        void* dbias, void* ws) {
+  const int ny = gate_bias_splits(rows, cols);
+  const dim3 grid((unsigned)((cols + 255) / 256), (unsigned)ny);
+  {
+    ProfScope ps("gate_bwd_kernel", st);
+    if (bf) gate_bwd_bias_kernel<bf16><<<grid, LY_THREADS, 0, st>>>(rows, cols, (const bf16*)z, dg, inv_tau, (bf16*)dz, (float*)ws);
+    else gate_bwd_bias_kernel<float><<<grid, LY_THREADS, 0, st>>>(rows, cols, (const float*)z, dg, inv_tau, (float*)dz, (float*)ws);
+    GLA_CHECK_LAUNCH();
+  }
+  ProfScope ps("column_sum_kernel", st);
+  column_sum_kernel<<<(unsigned)((cols + 31) / 32), 32 * CS_LANES, 0, st>>>(ny, (int)cols, (const float*)ws, dbias, bf);
+  GLA_CHECK_LAUNCH();
+  return GLA_OK;
+}
+
 int layer_headnorm_gate_fwd(cudaStream_t st, int64_t rows, int64_t D, int bf, const void* x, const void* gate,
                             const float* w, float eps, void* y, float* rstd) {
   ProfScope ps("headnorm_gate_fwd_kernel", st);
@@ -366,8 +426,7 @@ int layer_headnorm_gate_bwd(cudaStream_t st, int64_t rows, int64_t D, int bf, co
   }
   if (dweight) {
     ProfScope ps("column_sum_kernel", st);
-    column_sum_kernel<<<(unsigned)((D + 31) / 32), LY_THREADS, 0, st>>>(headnorm_bwd_blocks(rows), (int)D,
-                                                                                           partial, dweight);
+    column_sum_kernel<<<(unsigned)((D + 31) / 32), 32 * CS_LANES, 0, st>>>(headnorm_bwd_blocks(rows), (int)D, partial, dweight, 0);
     GLA_CHECK_LAUNCH();
   }
   return GLA_OK;

@@ -9,7 +9,7 @@ the smallest real caller of it, built from the published GLA layer recipe:
     o         = rmsnorm_per_head(out) * w_norm * swish(x Wgate)
     y         = o Wo
 
-The projections are library GEMMs (``torch.nn.functional.linear``).  The two element-wise stages
+The projections are library GEMMs.  The two element-wise stages
 run as single CUDA passes through the C ABI (``gla_layer_gate_*``, ``gla_layer_headnorm_gate_*``),
 each with a hand-written backward, so that ``log_fgate`` is produced in float32 directly from the
 projection's dtype and ``out`` is read once for normalisation, weight and output gate together.
@@ -24,6 +24,9 @@ import torch
 
 from . import _lib
 from .gla import _DT, _ptr, _stream, chunk_gla, recurrent_gla
+
+
+_HOOKS = torch.nn.modules.module
 
 
 def _need_cuda(t, what):
@@ -137,7 +140,25 @@ class GLALayer(torch.nn.Module):
         self.o_proj = torch.nn.Linear(inner, d_model, bias=False, **kw)
         self.norm_weight = torch.nn.Parameter(torch.ones(head_dim, device=device, dtype=torch.float32))
 
+    def _plain(self) -> bool:
+        """Whether the submodules are as this class made them: plain linear layers that nothing hooks into, outside
+        autocast.  The whole layer then runs as one native autograd node; anything else goes module by module."""
+        if self.mode != "chunk" or torch.is_autocast_enabled() or _HOOKS._has_any_global_hook():
+            return False
+        for m in (self.q_proj, self.k_proj, self.v_proj, self.gate_down, self.gate_up, self.out_gate, self.o_proj):
+            if type(m) is not torch.nn.Linear or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or \
+                    m._backward_pre_hooks or (m.bias is None) != (m is not self.gate_up):
+                return False
+        return True
+
     def forward(self, x: torch.Tensor, hidden: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
+        if self._plain():
+            r = _lib.native().gla_layer(x, hidden, [
+                self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.gate_down.weight, self.gate_up.weight,
+                self.gate_up.bias, self.out_gate.weight, self.o_proj.weight, self.norm_weight],
+                self.num_heads, self.head_dim, self.chunk_size, 1.0 / self.gate_normalizer, self.eps)
+            if r is not None:
+                return r
         if x.dim() != 3 or x.shape[-1] != self.d_model:
             raise ValueError(f"x must be (B, T, {self.d_model}), got {tuple(x.shape)}")
         B, T, _ = x.shape

@@ -173,6 +173,12 @@ GLA_API int gla_layer_gate_fwd(void* stream, int64_t n, int dtype, const void* z
                        float* log_fgate);
 GLA_API int gla_layer_gate_bwd(void* stream, int64_t n, int dtype, const void* z,
                        const float* dlog_fgate, float inv_tau, void* dz);
+/* The same over a (rows, cols) array, cols a multiple of 8 and z, dlog_fgate, dz 16-byte aligned, with the column sums of
+ * dz (the gradient of the projection's bias, (cols) in dtype) formed in the same pass. */
+GLA_API size_t gla_layer_gate_bwd_bias_workspace_bytes(int64_t rows, int64_t cols);
+GLA_API int gla_layer_gate_bwd_bias(void* stream, int64_t rows, int64_t cols, int dtype, const void* z,
+                       const float* dlog_fgate, float inv_tau, void* dz, void* dbias,
+                       void* workspace, size_t workspace_bytes);
 GLA_API int gla_layer_headnorm_gate_fwd(void* stream, int64_t rows, int64_t D, int dtype,
                                 const void* x, const void* gate, const float* weight, float eps,
                                 void* y, float* rstd);
