@@ -253,7 +253,7 @@ __device__ __forceinline__ bool gate_sums(const float2 (&g)[C::RPT], float* seg,
 // MODE 0: S slot n + 1 = k^^T V, k^ = k exp(G - lam);  MODE 1: dS slot n = q^^T dO, q^ = q exp(lam).  The weights are
 // anchored at the chunk's ends here and never exceed one for log gates <= 0.  Also leaves exp(G).
 template <class C, typename TI, typename TY, int MODE>
-__global__ void __launch_bounds__(C::NT) px_product_kernel(PxParams p) {
+__global__ void __launch_bounds__(C::NT, sizeof(TI) + sizeof(TY) == 4 ? 1024 / C::NT : 512 / C::NT) px_product_kernel(PxParams p) {
   constexpr int NSY = planes_of<TY>();
   extern __shared__ __align__(16) uint8_t sm[];
   uint8_t* sX = sm;
@@ -263,6 +263,8 @@ __global__ void __launch_bounds__(C::NT) px_product_kernel(PxParams p) {
   const ChunkAt<C> at(p, blockIdx.x);
   float2 g[C::RPT];
   Pair<TI> x[C::RPT];
+  grid_dep_wait();
+  grid_dep_launch();
   load_gates<C>(g, p.g, at, r0, cp);
   load_pairs<C, TI>(x, MODE == 0 ? p.k : p.q, at, r0, cp);
   copy_rows<C, TY>(sY, MODE == 0 ? p.v : p.dout, at);
@@ -332,6 +334,8 @@ __global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, 
   const int64_t bh = e4 * 4 / DD, e = e4 * 4 % DD, dk = e / D;
   float* sp = S + bh * (N + 1) * DD + e;
   const float* gp = eG + bh * N * D + dk;
+  grid_dep_wait();
+  grid_dep_launch();
   float4 s;
   s.x = ld_f(init, bh * DD + e); s.y = ld_f(init, bh * DD + e + 1); s.z = ld_f(init, bh * DD + e + 2); s.w = ld_f(init, bh * DD + e + 3);
   *reinterpret_cast<float4*>(sp + (mode ? N : 0) * DD) = s;
@@ -508,15 +512,18 @@ template <class C, typename TI>
 struct FwdLay {
   static constexpr int NSV = planes_of<TI>();
   static constexpr uint32_t most(uint32_t a, uint32_t b) { return a > b ? a : b; }
-  // two pieces of the state: the second takes the region of k~ once the scores are formed; one piece: the scores do
-  static constexpr uint32_t KREG = C::NP > 1 ? most(3 * C::SPLANE, 3 * C::PLANE) : most(3 * C::TPLANE, 3 * C::PLANE);
-  static constexpr uint32_t Q = 0, K = Q + 3 * C::PLANE, V = K + KREG, S = V + NSV * C::PLANE;
-  static constexpr uint32_t T = C::NP > 1 ? S + 3 * C::SPLANE : K, SEG = C::NP > 1 ? T + 3 * C::TPLANE : S + 3 * C::SPLANE;
+  // The region of k~ takes the scores once they are formed and, with one piece of the state (D <= 64), that piece once
+  // the scores are consumed: three blocks per SM at head size 64 in bf16 instead of two (100 -> FWD_US us at 202752
+  // token-heads).  Two pieces: the first has a region of its own, the second follows k~.
+  static constexpr uint32_t KREG = most(C::NP > 1 ? 0 : 3 * C::TPLANE, most(3 * C::SPLANE, 3 * C::PLANE));
+  static constexpr uint32_t Q = 0, K = Q + 3 * C::PLANE, V = K + KREG, S = C::NP > 1 ? V + NSV * C::PLANE : K;
+  static constexpr uint32_t T = C::NP > 1 ? S + 3 * C::SPLANE : K, SEG = C::NP > 1 ? T + 3 * C::TPLANE : V + NSV * C::PLANE;
   static constexpr uint32_t EM = SEG + 2 * C::RG * C::D * 4, END = EM + C::D * 4;
+  static constexpr int BLOCKS = C::NP > 1 ? 1 : sizeof(TI) == 2 ? 3 : 2;
   static_assert(C::L * C::D * 4 <= 3 * C::PLANE, "the pairwise form keeps lam where k~ would be");
 };
 template <class C, typename TI>
-__global__ void __launch_bounds__(C::NT) px_fwd_kernel(PxParams p) {
+__global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(PxParams p) {
   using Lay = FwdLay<C, TI>;
   extern __shared__ __align__(16) uint8_t sm[];
   float* seg = reinterpret_cast<float*>(sm + Lay::SEG);
@@ -529,23 +536,26 @@ __global__ void __launch_bounds__(C::NT) px_fwd_kernel(PxParams p) {
   {
     float2 g[C::RPT];
     Pair<TI> q[C::RPT], k[C::RPT];
+    // the inputs were complete before the state product, which waited for everything before it, could start
     load_gates<C>(g, p.g, at, r0, cp);
     load_pairs<C, TI>(q, p.q, at, r0, cp);
     load_pairs<C, TI>(k, p.k, at, r0, cp);
     copy_rows<C, TI>(sm + Lay::V, p.v, at);
-    fetch_piece<C>(sx, Sn, 0);
     float2 before, own, total;
     sharp = gate_sums<C>(g, seg, seg + C::RG * C::D, rg, cp, before, own, total);
     build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, sharp, before, own, total, rg, cp);
     __syncthreads();
-    if (sharp) store_lam<C>(reinterpret_cast<float*>(sm + Lay::K), p.g, at, before, rg, cp);
+    if (sharp) {
+      store_lam<C>(reinterpret_cast<float*>(sm + Lay::K), p.g, at, before, rg, cp);
+      __syncthreads();
+    }
   }
-  store_piece<C>(sm + Lay::S, sx, em);
-  if (C::NP > 1) fetch_piece<C>(sx, Sn, 1);
-  if (sharp) __syncthreads();
   const int wr = warp % C::WR, wc = warp / C::WR, m0 = 16 * wr;
   const uint32_t aQ = smem_u32(sm + Lay::Q), aK = smem_u32(sm + Lay::K), aV = smem_u32(sm + Lay::V), aS = smem_u32(sm + Lay::S);
   const uint32_t aT = smem_u32(sm + Lay::T);
+  float o[C::NP][C::PC / 8][4];
+#pragma unroll
+  for (int pc = 0; pc < C::NP; ++pc) zero_acc(o[pc]);
   {
     float x[C::NB][2][4];
     if (!sharp) score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);
@@ -553,11 +563,16 @@ __global__ void __launch_bounds__(C::NT) px_fwd_kernel(PxParams p) {
     __syncthreads();                      // the scores are formed: the region of k~ is free
     store_scores<C>(sm + Lay::T, x, wr, wc, lane);
   }
-  if (C::NP > 1) store_piece<C>(sm + Lay::K, sx, em);
+  grid_dep_wait();                        // the states of the scan before this kernel
+  grid_dep_launch();
+  fetch_piece<C>(sx, Sn, 0);
+  if (C::NP > 1) {
+    float4 s1[C::SREG];
+    fetch_piece<C>(s1, Sn, 1);
+    store_piece<C>(sm + Lay::S, sx, em);
+    store_piece<C>(sm + Lay::K, s1, em);
+  }
   __syncthreads();
-  float o[C::NP][C::PC / 8][4];
-#pragma unroll
-  for (int pc = 0; pc < C::NP; ++pc) zero_acc(o[pc]);
 #pragma unroll 1
   for (int kk = 0; kk <= wr; ++kk) {
     uint32_t a[3][4];
@@ -565,6 +580,11 @@ __global__ void __launch_bounds__(C::NT) px_fwd_kernel(PxParams p) {
 #pragma unroll
     for (int pc = 0; pc < C::NP; ++pc)
       mma_step<3, Lay::NSV, C::PC / 16, true>(o[pc], a, aV, C::PLANE, C::LD, pc * C::PW + wc * C::PC, 16 * kk, lane);
+  }
+  if (C::NP == 1) {
+    __syncthreads();                      // the scores are consumed
+    store_piece<C>(sm + Lay::S, sx, em);
+    __syncthreads();
   }
 #pragma unroll 2
   for (int ks = 0; ks < C::D / 16; ++ks) {
@@ -684,6 +704,8 @@ __global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
     sharp = gate_sums<C>(g, seg, seg + C::RG * D, rg, cp, before, own, total);
     build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, sharp, before, own, total, rg, cp);
   }
+  grid_dep_wait();                        // the gradient states of the scan before this kernel
+  grid_dep_launch();
   fetch_piece<C>(sx, Sn, 0);
   __syncthreads();
 
@@ -847,16 +869,15 @@ int launch_product(cudaStream_t st, const PxParams& p, int64_t chunks) {
   static SmemAttrOnce attr;
   GLA_TRY(attr.ensure(px_product_kernel<C, TI, TY, MODE>, smem));
   ProfScope ps(MODE == 0 ? "px_state_product" : "px_dstate_product", st);
-  px_product_kernel<C, TI, TY, MODE><<<(unsigned)chunks, C::NT, smem, st>>>(p);
-  GLA_CHECK_LAUNCH();
+  GLA_LAUNCHED(launch_overlapped(px_product_kernel<C, TI, TY, MODE>, dim3((unsigned)chunks), dim3(C::NT), smem, st, p));
   return GLA_OK;
 }
 template <typename TS>
 int launch_scan(cudaStream_t st, int64_t BH, int64_t D, int64_t N, const float* eG, const void* init, float* S, void* fin, int mode) {
   const int64_t total = BH * D * D;
   ProfScope ps("px_scan_kernel", st);
-  px_scan_kernel<TS><<<(unsigned)((total / 4 + 127) / 128), 128, 0, st>>>(total, D, N, eG, (const TS*)init, S, (TS*)fin, mode);
-  GLA_CHECK_LAUNCH();
+  GLA_LAUNCHED(launch_overlapped(px_scan_kernel<TS>, dim3((unsigned)((total / 4 + 127) / 128)), dim3(128), 0, st, total, D, N, eG,
+                                 (const TS*)init, S, (TS*)fin, mode));
   return GLA_OK;
 }
 template <class C, typename TI>
@@ -867,8 +888,7 @@ int run_fwd(cudaStream_t st, const PxParams& p, const void* init, void* fin) {
   static SmemAttrOnce attr;
   GLA_TRY(attr.ensure(px_fwd_kernel<C, TI>, FwdLay<C, TI>::END));
   ProfScope ps(p.label, st);
-  px_fwd_kernel<C, TI><<<(unsigned)chunks, C::NT, FwdLay<C, TI>::END, st>>>(p);
-  GLA_CHECK_LAUNCH();
+  GLA_LAUNCHED(launch_overlapped(px_fwd_kernel<C, TI>, dim3((unsigned)chunks), dim3(C::NT), FwdLay<C, TI>::END, st, p));
   return GLA_OK;
 }
 // states != 0: the states are in p.S and p.eG already (a forward's residuals); otherwise they are formed here first
@@ -884,8 +904,7 @@ int run_bwd(cudaStream_t st, const PxParams& p, int states, const void* init, co
   static SmemAttrOnce attr;
   GLA_TRY(attr.ensure(px_bwd_kernel<C, TI, TY>, BwdLay<C, TI, TY>::END));
   ProfScope ps("px_bwd_kernel", st);
-  px_bwd_kernel<C, TI, TY><<<(unsigned)chunks, C::NT, BwdLay<C, TI, TY>::END, st>>>(p);
-  GLA_CHECK_LAUNCH();
+  GLA_LAUNCHED(launch_overlapped(px_bwd_kernel<C, TI, TY>, dim3((unsigned)chunks), dim3(C::NT), BwdLay<C, TI, TY>::END, st, p));
   return GLA_OK;
 }
 template <int D, int L>
