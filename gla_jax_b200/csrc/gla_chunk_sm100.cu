@@ -195,9 +195,8 @@ tc_kv_kernel(int64_t T, int64_t H, int64_t N, const float* __restrict__ g, const
   if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
-// Number of thread blocks resident at a time (SMs x blocks per SM) = how far ahead in block index the
-// block that follows on the same SM lies; 0 disables the L2 prefetch.
-static int prefetch_distance(int blocks_per_sm) {
+// SMs of the current device (0: unknown).
+static int sm_count() {
   static int sms[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
@@ -206,7 +205,12 @@ static int prefetch_distance(int blocks_per_sm) {
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 0;
     sms[dev] = n;
   }
-  return sms[dev] * blocks_per_sm;
+  return sms[dev];
+}
+// Grid of a kernel whose blocks walk the chunks with a stride of the grid: one block fills an SM.
+static unsigned walking_blocks(int64_t chunks) {
+  const int n = sm_count();
+  return (unsigned)(n > 0 && n < chunks ? n : chunks);
 }
 
 constexpr size_t KV_SMEM = 1024 + 4 * TILE_BYTES + 2 * 8 * TD * sizeof(float) + 64;
@@ -247,8 +251,12 @@ struct FwdSmem {
   static constexpr uint32_t DIAG = TOT + 8 * TD * 4;       // 2 x 128 float
   static constexpr uint32_t GAB = DIAG + 2 * TC * 4;       // 8 x 128 float: sums of |g| per 16 rows
   static constexpr uint32_t BAR = GAB + 8 * TD * 4;        // 5 mbarriers + tmem slot
-  static constexpr uint32_t END = BAR + 64;
+  static constexpr uint32_t SPOT = BAR + 64;               // 2 x ChunkSpot
+  static constexpr uint32_t END = SPOT + 32;
 };
+// Where the chunk in work lies: first output element, index among the stored states, rows.  Kept in shared memory by the
+// thread that requests the inputs: registers are what the kernel lacks.
+struct ChunkSpot { int64_t out; int chunk, rows; };
 // A chunk whose gates satisfy sum_rows |g| <= ONE_SCALE_LIMIT for every feature needs no secondary chunking: with
 // one anchor for the whole chunk every decay weight stays within exp(+-limit), far inside the range of bf16 and
 // float32, so the dyadic levels (which exist to keep exponents non-positive, gla.py:986-993) collapse into one.
@@ -265,7 +273,7 @@ constexpr float BALANCED_LIMIT = 140.f;
 constexpr uint32_t KC_TILE = 64 * 128;    // one SW128 tile of 64 rows
 
 // TMA descriptors of one launch (built on the host per call, passed by value).
-struct FwdMaps { CUtensorMap g, q, k, v, s; };
+struct FwdMaps { CUtensorMap g, q, k, v, s, p; };
 
 
 // Operands of level slot S (half size 2^S) for the thread's 16 rows x 2 columns, with the decay
@@ -364,9 +372,9 @@ __device__ __forceinline__ void zero_tail_rows(uint8_t* tile, int nv) {
 // own so that the dense one carries nothing extra.
 template <bool RAG>
 __global__ void __launch_bounds__(TTHREADS, 1)
-tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, int R, int64_t N, const int2* __restrict__ tab, bf16* __restrict__ out,
-                    bf16* __restrict__ P_saved, const unsigned int* __restrict__ state_done, unsigned int state_target,
-                    int all_scales, int pf_dist) {
+tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T, int64_t H, int R, int64_t N, const int2* __restrict__ tab,
+                    bf16* __restrict__ out, int save_p, const unsigned int* __restrict__ state_done, unsigned int state_target,
+                    int all_scales, int prefetch) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   float* tot = reinterpret_cast<float*>(sm + FwdSmem::TOT);
@@ -382,29 +390,34 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
   // problems, virtual head (h R + a) R + c, whose results the caller sums over a.  In the (B, T, H_real R, 128) view
   // of the inputs the key-side tensors of a virtual head are head h R + a, the value-side ones head h R + c; the
   // output is written per virtual head, (B, T, H, 128).  R = 1: everything coincides with the real layout.
-  // Block order: chunk-major, LAST chunks first.  The state kernel that runs before this one walks the chunks of all
+  // Chunk order: chunk-major, LAST chunks first.  The state kernel that runs before this one walks the chunks of all
   // heads in step, first to last, so the inputs it read most recently (g, k, v of the late chunks) and the states
   // it wrote last are the ones most likely to be still in L2.
-  const int64_t BHn = (int64_t)gridDim.x / N;
-  const int64_t n = N - 1 - (int64_t)blockIdx.x / BHn, bh = (int64_t)blockIdx.x % BHn, b = bh / H, h_ = bh % H;
-  const int64_t hk_ = (h_ / (R * R)) * R + (h_ % (R * R)) / R, hv_ = (h_ / (R * R)) * R + h_ % R;
-  const int64_t HD = H * TD;
-  const int2 span = RAG ? tab[n] : make_int2((int)(b * T + n * TC), TC);        // first token and rows of the chunk
-  const int nv = RAG ? span.y : TC;
-  const int64_t row0 = ((RAG ? (int64_t)span.x : b * T + n * TC) * H + h_) * TD;
-  const int64_t chunk_id = bh * N + n;
-
-  if (tid == 0) {
-    mbar_init(smem_u32(bars + 0), 1);
-    mbar_init(smem_u32(bars + 1), 1);
-    mbar_init(smem_u32(bars + 2), 1);
-    mbar_init(smem_u32(bars + 3), 1);
-    mbar_init(smem_u32(bars + 4), 1);
-    mbar_fence_init();
-    // ---- all global inputs of the chunk through TMA: 192 KB in flight.  g, q, k (needed at once) come first on
-    // their own barrier; v and S_prev are only needed by the output product and land while the levels run.
+  constexpr bool WALK = !RAG;
+  struct Where { int n, bh, b, h, hk, hv; };
+  auto locate = [&](int item) {
+    const uint32_t heads = (uint32_t)(chunks / (int)N);
+    Where s;
+    s.n = (int)N - 1 - (int)((uint32_t)item / heads);
+    s.bh = (int)((uint32_t)item % heads);
+    s.b = (int)((uint32_t)s.bh / (uint32_t)H);
+    s.h = s.bh - s.b * (int)H;
+    s.hk = (int)((uint32_t)s.h / (uint32_t)(R * R)) * R + (int)((uint32_t)s.h % (uint32_t)(R * R)) / R;
+    s.hv = (int)((uint32_t)s.h / (uint32_t)(R * R)) * R + (int)((uint32_t)s.h % (uint32_t)R);
+    return s;
+  };
+  // ---- all global inputs of a chunk through TMA: 192 KB in flight (one thread).  g, q, k (needed at once) come first on
+  // their own barrier; v and S_prev are only needed by the output product and land while the scores are formed.
+  // Leaves where the chunk lies for all threads (visible with the barrier that g, q, k complete).
+  ChunkSpot* spots = reinterpret_cast<ChunkSpot*>(sm + FwdSmem::SPOT);
+  auto request = [&](int item, uint32_t turn, bool with_state) {
+    const Where s = locate(item);
     const uint32_t lb = smem_u32(bars + 3), lb2 = smem_u32(bars + 4);
-    const int z = span.x, y = (int)hk_, yv = (int)hv_;
+    const int2 span = RAG ? tab[s.n] : make_int2(s.b * (int)T + s.n * TC, TC);       // first token and rows
+    const int z = span.x, y = s.hk, yv = s.hv, chunk = s.bh * (int)N + s.n;
+    spots[turn].out = ((int64_t)z * H + s.h) * TD;
+    spots[turn].chunk = chunk;
+    spots[turn].rows = span.y;
     mbar_arrive_expect_tx(lb, 4 * 2 * TILE_BYTES);
     mbar_arrive_expect_tx(lb2, 2 * 2 * TILE_BYTES);
     tma_load_3d(smem_u32(sm + FwdSmem::Q), &maps.g, 0, y, z, lb);                       // 128 x 128 float, row pitch 512 B
@@ -413,26 +426,17 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
       tma_load_3d(smem_u32(sm + FwdSmem::K + half * TILE_BYTES), &maps.q, 64 * half, y, z, lb);
       tma_load_3d(smem_u32(sm + FwdSmem::P + half * TILE_BYTES), &maps.k, 64 * half, y, z, lb);
     }
-    // state_done (optional): this grid was launched as a programmatic dependent of the state kernel and may be
-    // running beside it, on SMs that kernel leaves idle.  One look at the counter (no waiting on it): if every
-    // state block has finished, the state tile is loaded now; otherwise its load is left to thread 32 at the
-    // point where the tile is needed, behind the grid dependency (everything before that needs no state).
-    const bool s_pending = state_done != nullptr && ld_acquire_u32(state_done) < state_target;
-    *s_pending_sm = s_pending ? 1u : 0u;
-    if (!s_pending && state_done != nullptr) fence_proxy_async_global();
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       tma_load_3d(smem_u32(sm + FwdSmem::V + half * TILE_BYTES), &maps.v, 64 * half, yv, z, lb2);
-      if (!s_pending) tma_load_2d(smem_u32(sm + FwdSmem::S + half * TILE_BYTES), &maps.s, 64 * half, (int)(chunk_id * TD), lb2);
+      if (with_state) tma_load_2d(smem_u32(sm + FwdSmem::S + half * TILE_BYTES), &maps.s, 64 * half, chunk * TD, lb2);
     }
-    // The same boxes of the block that the scheduler starts on this SM when this one retires (pf_dist blocks
-    // ahead), requested into L2 only: seven instructions of this one thread, so that the next block's load phase
-    // is served from L2.
-    const int64_t nb = (int64_t)blockIdx.x + pf_dist;
-    if (!RAG && pf_dist > 0 && nb < (int64_t)gridDim.x) {
-      const int64_t n2 = N - 1 - nb / BHn, bh2 = nb % BHn, h2 = bh2 % H;
-      const int y2 = (int)((h2 / (R * R)) * R + (h2 % (R * R)) / R), yv2 = (int)((h2 / (R * R)) * R + h2 % R);
-      const int z2 = (int)((bh2 / H) * T + n2 * TC);
+    // The same boxes of the chunk that follows, requested into L2 only: seven instructions of this one thread, so that
+    // its load phase is served from L2.
+    const int next = item + (int)gridDim.x;
+    if (WALK && prefetch && next < chunks) {
+      const Where t = locate(next);
+      const int y2 = t.hk, yv2 = t.hv, z2 = t.b * (int)T + t.n * TC;
       tma_prefetch_l2_3d(&maps.g, 0, y2, z2);
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -441,6 +445,20 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
         tma_prefetch_l2_3d(&maps.v, 64 * half, yv2, z2);
       }
     }
+  };
+
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) mbar_init(smem_u32(bars + i), 1);
+    mbar_fence_init();
+    // state_done (optional): this grid was launched as a programmatic dependent of the state kernel and may be
+    // running beside it, on SMs that kernel leaves idle.  One look at the counter (no waiting on it): if every
+    // state block has finished, the state tile is loaded now; otherwise its load is left to thread 32 at the
+    // point where the tile is needed, behind the grid dependency (everything before that needs no state).
+    const bool s_pending = state_done != nullptr && ld_acquire_u32(state_done) < state_target;
+    *s_pending_sm = s_pending ? 1u : 0u;
+    if (!s_pending && state_done != nullptr) fence_proxy_async_global();
+    request((int)blockIdx.x, 0u, !s_pending);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), 512);
@@ -450,7 +468,18 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
   __syncthreads();          // barrier inits and the TMEM address are visible
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  bool ok = mbar_wait(smem_u32(bars + 3), 0);
+  // A block walks the chunks with a stride of the grid (WALK): its TMEM, barriers and launch are paid once, and the next
+  // chunk's inputs come in while the current one's output leaves.  Ragged batches keep one chunk per block: the loop's live
+  // values on top of the masks cost more in spills than it gives (49 -> 53 us for 69 chunks x 8 heads).  (One chunk per block before: 512 -> 436 us per launch for 8192
+  // chunks of head size 128, 540 -> 458 us for 8192 with the middle anchor.)
+  // Parities: barriers 2, 3, 4 complete once per chunk (`turn`); with one anchor barrier 0 completes once and barrier 1
+  // not at all, with all levels four and three times.
+  uint32_t turn = 0, par0 = 0, par1 = 0;
+#pragma unroll 1
+  for (int item = (int)blockIdx.x; item < chunks; item += (int)gridDim.x, turn ^= 1u) {
+  bool ok = mbar_wait(smem_u32(bars + 3), turn);
+  const ChunkSpot* spot = spots + turn;
+  const int nv = RAG ? spot->rows : TC;
   // ---- gates, q, k of the thread's 16 rows x 2 columns from the landed tiles ---------------------
   float2 f[16];
   uint32_t qv[16], kv[16];
@@ -544,7 +573,8 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
         umma_bf16(tmem + 128, kslice_kmajor(a0, TILE_BYTES, ks), kslice_kmajor(b0, TILE_BYTES, ks), idesc, ks > 0);
       umma_commit(smem_u32(bars + 0));
     }
-    ok = mbar_wait(smem_u32(bars + 0), 0) && ok;
+    ok = mbar_wait(smem_u32(bars + 0), par0) && ok;
+    par0 ^= 1u;
     tc_fence_after();
     // scores back into the bf16 P tile: row i = 32 q4 + lane, columns 32 cj + [0, 32); the diagonal entry
     // q_hat_i . k~_i = q_i . k_i comes out of the same product
@@ -616,7 +646,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
   };
   auto wait_buffer_free = [&](int slot) {
     // before rebuilding buffer (slot & 1): the MMA of level slot-2 must have consumed it
-    if (slot >= 2) ok = mbar_wait(smem_u32(bars + (slot & 1)), (uint32_t)(((slot - 2) >> 1) & 1)) && ok;
+    if (slot >= 2) ok = mbar_wait(smem_u32(bars + (slot & 1)), (uint32_t)(((slot - 2) >> 1) & 1) ^ ((slot & 1) ? par1 : par0)) && ok;
   };
 
   fwd_emit<0>(f, qv, kv, sQb[0], sKb[0], rg, cp, tot); level_sync_and_issue(0);
@@ -633,7 +663,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
   fwd_emit<6>(f, qv, kv, sQb[0], sKb[0], rg, cp, tot); level_sync_and_issue(6);
 
   // ---- q_hat into Q buffer 1 (free once the MMA of level slot 5 has completed); overlaps slot 6's MMA
-  ok = mbar_wait(smem_u32(bars + 1), 0) && ok;     // buffer 1, third use (level slot 5)
+  ok = mbar_wait(smem_u32(bars + 1), par1) && ok;     // buffer 1, third use (level slot 5)
   {
     float2 run = make_float2(1.f, 1.f);
     for (int r2 = 0; r2 < rg; ++r2) {
@@ -650,7 +680,8 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
     }
   }
   // all seven level MMAs done when the last commit (buffer 0, fourth use) completes
-  ok = mbar_wait(smem_u32(bars + 0), 1) && ok;
+  ok = mbar_wait(smem_u32(bars + 0), par0 ^ 1u) && ok;
+  par1 ^= 1u;
   tc_fence_after();
 
   // ---- read the scores back into the bf16 P tile -----------------------------------------------------
@@ -738,12 +769,12 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
     // the q_hat operand carries exp(-m_d): row d of the state tile takes exp(m_d) before the product (and a short
     // chunk's value rows past its end are cleared).  Every thread waits for the tiles itself here (a block that started beside the state kernel requests it first).
     if (tid == 32 && *s_pending_sm != 0u) {
-      if (!fwd_load_state_late(state_done, state_target, &maps.s, smem_u32(sm + FwdSmem::S), (int)(chunk_id * TD), smem_u32(bars + 4)))
+      if (!fwd_load_state_late(state_done, state_target, &maps.s, smem_u32(sm + FwdSmem::S), spot->chunk * TD, smem_u32(bars + 4)))
         atomicAdd(&g_tc_wait_timeouts, 1u);
       *s_pending_sm = 0u;
     }
     __syncwarp();
-    ok = mbar_wait(smem_u32(bars + 4), 0) && ok;
+    ok = mbar_wait(smem_u32(bars + 4), turn) && ok;
     if (RAG && nv < TC) zero_tail_rows(sm + FwdSmem::V, nv);
     if (balanced)
 #pragma unroll
@@ -761,7 +792,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
     __syncthreads();
   }
   if (tid == 0) {
-    ok = mbar_wait(smem_u32(bars + 4), 0) && ok;       // v and S_prev have landed (long ago, as a rule)
+    ok = mbar_wait(smem_u32(bars + 4), turn) && ok;       // v and S_prev have landed (long ago, as a rule)
     tc_fence_after();
     constexpr uint32_t idesc = idesc_bf16(128, 128, 0, 1);
     const uint64_t aq = desc_kmajor(sQ0 + 2 * TILE_BYTES, TILE_BYTES, 0), bs = desc_mnmajor(smem_u32(sm + FwdSmem::S), TILE_BYTES, 0);
@@ -773,32 +804,42 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
     for (int ks = 0; ks < 8; ++ks)
       umma_bf16(tmem, kslice_kmajor(ap, TILE_BYTES, ks), kslice_mnmajor(bv, ks), idesc, 1);
     umma_commit(smem_u32(bars + 2));
+    // The saved copy of P leaves from the assembled tile while the output product runs: two tensor stores instead of 2048
+    // 16-byte loads and stores of all threads.
+    if (save_p) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+        tma_store_2d(&maps.p, 64 * half, spot->chunk * TC, smem_u32(sm + FwdSmem::P + half * TILE_BYTES));
+      tma_commit();
+    }
   } else if (tid == 32) {
     // a block that started beside the state kernel: the state tile's load, issued here by another warp than the
     // one that waits for it, so that the common path above carries nothing extra
-    if (*s_pending_sm != 0u && !fwd_load_state_late(state_done, state_target, &maps.s, smem_u32(sm + FwdSmem::S), (int)(chunk_id * TD), smem_u32(bars + 4)))
-      atomicAdd(&g_tc_wait_timeouts, 1u);
-  }
-  // The saved copy of P goes out from the assembled shared-memory tile while the output product runs: rows are
-  // written whole (a warp stores two full 256-byte rows per instruction) instead of in 16-byte pieces of 32
-  // different rows from the read-back above.
-  if (P_saved) {
-    bf16* pg = P_saved + chunk_id * TC * TC;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int id = tid + TTHREADS * j, row = id >> 4, ch = id & 15;
-      const uint4 u = *reinterpret_cast<const uint4*>(sm + FwdSmem::P + (ch >> 3) * TILE_BYTES + sw128_chunk(row, ch & 7));
-      *reinterpret_cast<uint4*>(pg + row * TC + ch * 8) = u;
+    if (*s_pending_sm != 0u) {
+      if (!fwd_load_state_late(state_done, state_target, &maps.s, smem_u32(sm + FwdSmem::S), spot->chunk * TD, smem_u32(bars + 4)))
+        atomicAdd(&g_tc_wait_timeouts, 1u);
+      *s_pending_sm = 0u;
     }
   }
-  ok = mbar_wait(smem_u32(bars + 2), 0) && ok;
+  ok = mbar_wait(smem_u32(bars + 2), turn) && ok;
   tc_fence_after();
+  // The products have consumed their operands: the next chunk's inputs come in while this one's output leaves.  (The state
+  // kernel is complete: this chunk's state tile came through its grid dependency, or after a look at its counter.)
+  const bool failed = __syncthreads_or(!ok) != 0;       // ... and the rest of shared memory has been read by everybody
+  if (WALK && tid == 0 && !failed && item + (int)gridDim.x < chunks) {
+    tma_wait_read();
+    if (state_done != nullptr) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      fence_proxy_async_global();
+    }
+    request(item + (int)gridDim.x, turn ^ 1u, true);
+  }
   if (ok) {
     const int q4 = warp & 3, cg = warp >> 2;
     uint32_t r[32];
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(cg * 32), r);
     tmem_ld_wait();
-    bf16* o = out + row0 + (int64_t)(q4 * 32 + lane) * HD + cg * 32;
+    bf16* o = out + spot->out + (int64_t)(q4 * 32 + lane) * (H * TD) + cg * 32;
     // 64 contiguous bytes of one row per thread, rows of a warp far apart: two 32-byte stores
 #pragma unroll
     for (int c8 = 0; c8 < 2; ++c8) {
@@ -807,10 +848,12 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int64_t T, int64_t H, 
       for (int m = 0; m < 8; ++m) u[m] = pack_bf16x2(__uint_as_float(r[16 * c8 + 2 * m]), __uint_as_float(r[16 * c8 + 2 * m + 1]));
       if (!RAG || q4 * 32 + lane < nv) st_global_v8(o + 16 * c8, u);
     }
-  } else if (tid == 0) {
-    atomicAdd(&g_tc_wait_timeouts, 1u);
   }
-  tc_fence_before();
+  tc_fence_before();        // (the next chunk's first product comes after block barriers)
+  if (failed && tid == 0) atomicAdd(&g_tc_wait_timeouts, 1u);
+  if (!WALK || failed) break;         // (a wait gave up: no more chunks)
+  }   // chunks
+  if (tid == 0) tma_wait_stored();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
@@ -2128,14 +2171,17 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   GLA_TRY(make_map_bthd(&maps.k, k, 0, B, T, HK, 64, 1));
   GLA_TRY(make_map_bthd(&maps.v, v, 0, B, T, HK, 64, 1));
   GLA_TRY(make_map_rows(&maps.s, S_prev, BHV * N * TD, 64, 128));
+  if (P != nullptr) GLA_TRY(make_map_rows(&maps.p, P, BHV * N * TC, 64, 128));
+  else maps.p = maps.s;        // not used
   {
     ProfScope ps("tc_chunk_fwd_kernel", st);
     bf16* out_p = R > 1 ? out_v : (bf16*)out;
-    const int pf_dist = (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : prefetch_distance(1);
+    const int prefetch = (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : 1, chunks = (int)(BHV * N);
+    const unsigned blocks = rag ? (unsigned)chunks : walking_blocks(chunks);
     if (early_flag != nullptr) {
       // programmatic dependent of the state kernel launched just before: may start while that one runs
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(BHV * N));
+      cfg.gridDim = dim3(blocks);
       cfg.blockDim = dim3(TTHREADS);
       cfg.dynamicSmemBytes = FWD_SMEM;
       cfg.stream = st;
@@ -2144,11 +2190,11 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
       attr[0].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, fwd_kernel, maps, T, HV, R, N, tab, out_p, P, (const unsigned int*)early_flag,
-                             early_target, all_scales, pf_dist);
+      e = cudaLaunchKernelEx(&cfg, fwd_kernel, maps, chunks, T, HV, R, N, tab, out_p, P != nullptr ? 1 : 0, (const unsigned int*)early_flag,
+                             early_target, all_scales, prefetch);
       if (e != cudaSuccess) return record_cuda_error(e);
     } else {
-      fwd_kernel<<<(unsigned)(BHV * N), TTHREADS, FWD_SMEM, st>>>(maps, T, HV, R, N, tab, out_p, P, nullptr, 0u, all_scales, pf_dist);
+      fwd_kernel<<<blocks, TTHREADS, FWD_SMEM, st>>>(maps, chunks, T, HV, R, N, tab, out_p, P != nullptr, nullptr, 0u, all_scales, prefetch);
     }
   }
   GLA_CHECK_LAUNCH();
@@ -2259,7 +2305,7 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   {
     ProfScope ps("tc_chunk_bwd_kernel", st);
     bwd_kernel<<<(unsigned)(BHV * N), TTHREADS, BWD_SMEM, st>>>(
-        bmaps, T, HV, R, N, rag ? rag->tab : nullptr, (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : prefetch_distance(1), g, (const bf16*)v, (const bf16*)k,
+        bmaps, T, HV, R, N, rag ? rag->tab : nullptr, (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : sm_count(), g, (const bf16*)v, (const bf16*)k,
         (const bf16*)q, (const bf16*)dout, S_prev, dS_next, P, dq_v, dk_v, dv_v, dg_v, (opts & GLA_OPT_ALL_SCALES) ? 1 : 0);
   }
   GLA_CHECK_LAUNCH();

@@ -138,6 +138,14 @@ __device__ __forceinline__ void tma_prefetch_l2_3d(const void* tmap, int x, int 
                :: "l"((uint64_t)tmap), "r"(x), "r"(y), "r"(z) : "memory");
 }
 // Bulk tensor store shared -> global of one box (bulk-group completion); never start one at a negative coordinate.
+__device__ __forceinline__ void tma_store_2d(const void* tmap, int x, int y, uint32_t smem_src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+               :: "l"((uint64_t)tmap), "r"(x), "r"(y), "r"(smem_src) : "memory");
+}
+__device__ __forceinline__ void tma_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// The thread's bulk stores have read their shared memory / have completed.
+__device__ __forceinline__ void tma_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_wait_stored() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_3d(const void* tmap, int x, int y, int z, uint32_t smem_src) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];"
                :: "l"((uint64_t)tmap), "r"(x), "r"(y), "r"(z), "r"(smem_src) : "memory");
