@@ -990,8 +990,8 @@ __device__ __forceinline__ void st_bf16(uint8_t* p, float v) { *reinterpret_cast
 // rescaling of the dS_next tile.  Row d of the tile takes w = 1 / A (this thread: its columns 32 wq + [0, 32)), so that
 // k_hat dS_next and dS_next V^T come out as with the end anchor, the latter divided by A like the dk~ term that joins
 // it.  Waits (bounded) for the tile to have landed first and leaves it alone if it has not.
-__device__ __noinline__ void bwd_rescale_ds(uint8_t* ds, uint32_t bar, float w, int d, int wq) {
-  if (!mbar_wait(bar, 0)) return;
+__device__ __noinline__ void bwd_rescale_ds(uint8_t* ds, uint32_t bar, uint32_t parity, float w, int d, int wq) {
+  if (!mbar_wait(bar, parity)) return;
   uint8_t* td = ds + (wq >> 1) * TILE_BYTES;
 #pragma unroll
   for (int c4 = 0; c4 < 4; ++c4) {
@@ -1003,7 +1003,24 @@ __device__ __noinline__ void bwd_rescale_ds(uint8_t* ds, uint32_t bar, float w, 
   }
 }
 
-template <bool RAG>
+// sum over the thread's 32 columns of row d of the product of two operand tiles
+__device__ __forceinline__ float dot_tiles(const uint8_t* ts, const uint8_t* td, int d, int wq) {
+  float s = 0.f;
+#pragma unroll
+  for (int c4 = 0; c4 < 4; ++c4) {
+    const uint4 a = *reinterpret_cast<const uint4*>(ts + sw128_chunk(d, (wq & 1) * 4 + c4));
+    const uint4 c = *reinterpret_cast<const uint4*>(td + sw128_chunk(d, (wq & 1) * 4 + c4));
+    s += bf16_lo(a.x) * bf16_lo(c.x) + bf16_hi(a.x) * bf16_hi(c.x) + bf16_lo(a.y) * bf16_lo(c.y) + bf16_hi(a.y) * bf16_hi(c.y) +
+         bf16_lo(a.z) * bf16_lo(c.z) + bf16_hi(a.z) * bf16_hi(c.z) + bf16_lo(a.w) * bf16_lo(c.w) + bf16_hi(a.w) * bf16_hi(c.w);
+  }
+  return s;
+}
+// WIDE (head size 256, R = 2): a block takes one key block of a head with both of its value blocks.  dq, dk and dg are
+// linear in dP, dO S_prev^T and v dS_next^T, so the three products of the second value block accumulate in TMEM onto
+// those of the first, and the gates, k_hat, the closing products and the results are formed once instead of twice (a block
+// per (key block, value block) wrote partial results that passes of their own added: 1035 + 254 -> 853 us at B = 2, T = 16384, H = 8).
+// Only dv is still written per (key block, value block).
+template <bool RAG, bool WIDE>
 __global__ void __launch_bounds__(TTHREADS, 1)
 tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, int R, int64_t N, const int2* __restrict__ tab, int pf_dist, const float* __restrict__ g, const bf16* __restrict__ v,
                     const bf16* __restrict__ k, const bf16* __restrict__ q, const bf16* __restrict__ dO,
@@ -1029,18 +1046,21 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
   const int q4 = warp & 3, wq_ = warp >> 2;        // TMEM lane quadrant, and which quarter of the columns
   const int d = 32 * q4 + lane;                     // column layout: feature index
   // H counts virtual heads (see the forward kernel).  Inputs are addressed in the (B, T, H / R, 128) view: key-side
-  // tensors (g, q, k) at head hk_, value-side tensors (v, dO) at head hv_; the gradients are written per virtual
-  // head, (B, T, H, 128), and the caller sums dq, dk, dg over the value blocks and dv over the key blocks.
+  // tensors (g, q, k) at head hk_, value-side tensors (v, dO) at head hv_; dq, dk, dg are written at head hk_ of that view,
+  // dv per virtual head, (B, T, H, 128), and the caller sums it over the key blocks.
   // Block order: chunk-major, FIRST chunks first: the gradient-state kernel before this one walks the chunks of all
   // heads last to first, so g, q, dO of the early chunks and the gradient states written last are freshest in L2.
   const int64_t BHn = (int64_t)gridDim.x / N;
-  const int64_t n = (int64_t)blockIdx.x / BHn, bh = (int64_t)blockIdx.x % BHn, b = bh / H, h_ = bh % H;
+  const int64_t HB = WIDE ? H / 2 : H;                                // blocks per batch element and chunk = heads of the outputs
+  const int64_t n = (int64_t)blockIdx.x / BHn, bh = (int64_t)blockIdx.x % BHn, b = bh / HB, ho = bh % HB;
+  const int64_t h_ = WIDE ? 2 * ho : ho;                              // virtual head (WIDE: the one of value block 0)
   const int64_t hk_ = (h_ / (R * R)) * R + (h_ % (R * R)) / R, hv_ = (h_ / (R * R)) * R + h_ % R;
-  const int64_t HD = H * TD;                                          // output row pitch (virtual heads)
+  const int64_t HD = HB * TD;                                         // output row pitch
   const int2 span = RAG ? tab[n] : make_int2((int)(b * T + n * TC), TC);        // first token and rows of the chunk
   const int nv = RAG ? span.y : TC;
-  const int64_t row0 = ((RAG ? (int64_t)span.x : b * T + n * TC) * H + h_) * TD;   // outputs
-  const int64_t chunk_id = bh * N + n;
+  const int64_t row0 = ((RAG ? (int64_t)span.x : b * T + n * TC) * HB + ho) * TD;  // outputs
+  const int64_t chunk_id = WIDE ? (b * H + h_) * N + n : bh * N + n;               // (WIDE: value block 1 lies N further)
+  constexpr uint32_t LAST = WIDE ? 1 : 0;                             // parity of the last value block's barriers 0, 5, 7
 
   if (warp == 0) {
     tmem_alloc(smem_u32(tmem_slot), 512);
@@ -1073,6 +1093,15 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     for (int half = 0; half < 2; ++half) {
       tma_load_3d(smem_u32(sm + BwdSmem::DO + half * TILE_BYTES), &maps.dO, 64 * half, yv, z, lb);
       tma_load_3d(smem_u32(sm + BwdSmem::V + half * TILE_BYTES), &maps.v, 64 * half, yv, z, lb);
+    }
+    if (WIDE) {           // the second value block's tiles, into L2
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        tma_prefetch_l2_3d(&maps.dO, 64 * half, yv + 1, z);
+        tma_prefetch_l2_3d(&maps.v, 64 * half, yv + 1, z);
+      }
+      l2_prefetch_bulk(S_prev + (chunk_id + N) * TD * TD, 2 * TD * TD);
+      l2_prefetch_bulk(dS_next + (chunk_id + N) * TD * TD, 2 * TD * TD);
     }
   }
 
@@ -1163,13 +1192,16 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
-  if (balanced) {
-    // (its wait is not folded into `ok`: measured, that dependency alone cost the common path 3.5 us per launch; a
-    // tile that never lands fails the issuing threads' wait on the same barrier below)
-    bwd_rescale_ds(sm + BwdSmem::DS, smem_u32(bars + 7), 1.f / A, d, wq_);
-    fence_async_smem();
-    __syncthreads();
-  }
+  auto rescale = [&](uint32_t parity) {
+    if (balanced) {
+      // (its wait is not folded into `ok`: measured, that dependency alone cost the common path 3.5 us per launch; a
+      // tile that never lands fails the issuing threads' wait on the same barrier below)
+      bwd_rescale_ds(sm + BwdSmem::DS, smem_u32(bars + 7), parity, 1.f / A, d, wq_);
+      fence_async_smem();
+      __syncthreads();
+    }
+  };
+  rescale(0);
 
   if (RAG && nv < TC) {
     ok = mbar_wait(smem_u32(bars + 5), 0) && ok;
@@ -1183,39 +1215,86 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
   // Issued by four threads of four warps on different schedulers (8 to 16 MMAs each instead of 40 from one): the
   // issuing thread's instruction stream is serial, so this shortens the wait of everybody else.  The two halves of
   // dV come from the same thread, in order.
-  if (lane == 0 && (warp == 3 || warp == 6 || warp == 9 || warp == 12)) {
-    ok = mbar_wait(smem_u32(bars + 5), 0) && ok;    // operand tiles landed
+  auto dense_products = [&](uint32_t parity) {
+    if (lane == 0 && (warp == 3 || warp == 6 || warp == 9 || warp == 12)) {
+      ok = mbar_wait(smem_u32(bars + 5), parity) && ok;    // operand tiles landed
+      ok = mbar_wait(smem_u32(bars + 7), parity) && ok;
+      tc_fence_after();
+      constexpr uint32_t iKK = idesc_bf16(128, 128, 0, 0), iMM = idesc_bf16(128, 128, 1, 1);
+      const uint32_t aDO = smem_u32(sm + BwdSmem::DO), aV = smem_u32(sm + BwdSmem::V);
+      if (warp == 3) {
+        const uint64_t kDO = desc_kmajor(aDO, TILE_BYTES, 0), kV = desc_kmajor(aV, TILE_BYTES, 0);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)   // dP[i][j] = sum_dv dO[i][dv] v[j][dv]
+          umma_bf16(tmem + TM_DP, kslice_kmajor(kDO, TILE_BYTES, ks), kslice_kmajor(kV, TILE_BYTES, ks), iKK, (WIDE && parity != 0) || ks > 0);
+      } else if (warp == 6) {
+        const uint64_t kSP = desc_kmajor(smem_u32(sm + BwdSmem::SP), TILE_BYTES, 0), kDO = desc_kmajor(aDO, TILE_BYTES, 0);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)   // dQh^T[dk][i] = sum_dv S_prev[dk][dv] dO[i][dv]
+          umma_bf16(tmem + TM_DQH, kslice_kmajor(kSP, TILE_BYTES, ks), kslice_kmajor(kDO, TILE_BYTES, ks), iKK, (WIDE && parity != 0) || ks > 0);
+      } else if (warp == 9) {
+        const uint64_t kDS = desc_kmajor(smem_u32(sm + BwdSmem::DS), TILE_BYTES, 0), kV = desc_kmajor(aV, TILE_BYTES, 0);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)   // dKh^T[dk][j] = sum_dv dS_next[dk][dv] v[j][dv]
+          umma_bf16(tmem + TM_DKH, kslice_kmajor(kDS, TILE_BYTES, ks), kslice_kmajor(kV, TILE_BYTES, ks), iKK, (WIDE && parity != 0) || ks > 0);
+      } else {
+        const uint64_t mP = desc_mnmajor(smem_u32(sm + BwdSmem::P), TILE_BYTES, 0), mDO = desc_mnmajor(aDO, TILE_BYTES, 0);
+        const uint64_t mKH = desc_mnmajor(smem_u32(sm + BwdSmem::KH), TILE_BYTES, 0), mDS = desc_mnmajor(smem_u32(sm + BwdSmem::DS), TILE_BYTES, 0);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)   // dV[j][dv] = sum_i P[i][j] dO[i][dv]
+          umma_bf16(tmem + TM_DV, kslice_mnmajor(mP, ks), kslice_mnmajor(mDO, ks), iMM, ks > 0);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)   //          + sum_dk k_hat[j][dk] dS_next[dk][dv]
+          umma_bf16(tmem + TM_DV, kslice_mnmajor(mKH, ks), kslice_mnmajor(mDS, ks), iMM, 1);
+      }
+      umma_commit(smem_u32(bars + 0));
+    }
+  };
+  float s2 = 0.f;           // the thread's part of dG2[d] = sum_v S_prev[d][v] dS_next[d][v]
+  if constexpr (WIDE) {
+    dense_products(0);
+    __syncwarp();
+    ok = mbar_wait(smem_u32(bars + 0), 0) && ok;
+    ok = mbar_wait(smem_u32(bars + 5), 0) && ok;
     ok = mbar_wait(smem_u32(bars + 7), 0) && ok;
     tc_fence_after();
-    constexpr uint32_t iKK = idesc_bf16(128, 128, 0, 0), iMM = idesc_bf16(128, 128, 1, 1);
-    const uint32_t aDO = smem_u32(sm + BwdSmem::DO), aV = smem_u32(sm + BwdSmem::V);
-    if (warp == 3) {
-      const uint64_t kDO = desc_kmajor(aDO, TILE_BYTES, 0), kV = desc_kmajor(aV, TILE_BYTES, 0);
+    s2 = dot_tiles(sm + BwdSmem::SP + (wq_ >> 1) * TILE_BYTES, sm + BwdSmem::DS + (wq_ >> 1) * TILE_BYTES, d, wq_);
+    tc_fence_before();
+    __syncthreads();        // the first value block's tiles are consumed: the second's take their place
+    if (tid == 0) {
+      const uint32_t lb = smem_u32(bars + 5), lb7 = smem_u32(bars + 7);
+      const int cr = (int)((chunk_id + N) * TD), yv = (int)hv_ + 1;
+      mbar_arrive_expect_tx(lb, 2 * 2 * TILE_BYTES);
+      mbar_arrive_expect_tx(lb7, 2 * 2 * TILE_BYTES);
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks)   // dP[i][j] = sum_dv dO[i][dv] v[j][dv]
-        umma_bf16(tmem + TM_DP, kslice_kmajor(kDO, TILE_BYTES, ks), kslice_kmajor(kV, TILE_BYTES, ks), iKK, ks > 0);
-    } else if (warp == 6) {
-      const uint64_t kSP = desc_kmajor(smem_u32(sm + BwdSmem::SP), TILE_BYTES, 0), kDO = desc_kmajor(aDO, TILE_BYTES, 0);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)   // dQh^T[dk][i] = sum_dv S_prev[dk][dv] dO[i][dv]
-        umma_bf16(tmem + TM_DQH, kslice_kmajor(kSP, TILE_BYTES, ks), kslice_kmajor(kDO, TILE_BYTES, ks), iKK, ks > 0);
-    } else if (warp == 9) {
-      const uint64_t kDS = desc_kmajor(smem_u32(sm + BwdSmem::DS), TILE_BYTES, 0), kV = desc_kmajor(aV, TILE_BYTES, 0);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)   // dKh^T[dk][j] = sum_dv dS_next[dk][dv] v[j][dv]
-        umma_bf16(tmem + TM_DKH, kslice_kmajor(kDS, TILE_BYTES, ks), kslice_kmajor(kV, TILE_BYTES, ks), iKK, ks > 0);
-    } else {
-      const uint64_t mP = desc_mnmajor(smem_u32(sm + BwdSmem::P), TILE_BYTES, 0), mDO = desc_mnmajor(aDO, TILE_BYTES, 0);
-      const uint64_t mKH = desc_mnmajor(smem_u32(sm + BwdSmem::KH), TILE_BYTES, 0), mDS = desc_mnmajor(smem_u32(sm + BwdSmem::DS), TILE_BYTES, 0);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)   // dV[j][dv] = sum_i P[i][j] dO[i][dv]
-        umma_bf16(tmem + TM_DV, kslice_mnmajor(mP, ks), kslice_mnmajor(mDO, ks), iMM, ks > 0);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks)   //          + sum_dk k_hat[j][dk] dS_next[dk][dv]
-        umma_bf16(tmem + TM_DV, kslice_mnmajor(mKH, ks), kslice_mnmajor(mDS, ks), iMM, 1);
+      for (int half = 0; half < 2; ++half) {
+        tma_load_3d(smem_u32(sm + BwdSmem::DO + half * TILE_BYTES), &maps.dO, 64 * half, yv, span.x, lb);
+        tma_load_3d(smem_u32(sm + BwdSmem::V + half * TILE_BYTES), &maps.v, 64 * half, yv, span.x, lb);
+        tma_load_2d(smem_u32(sm + BwdSmem::SP + half * TILE_BYTES), &maps.sp, 64 * half, cr, lb7);
+        tma_load_2d(smem_u32(sm + BwdSmem::DS + half * TILE_BYTES), &maps.ds, 64 * half, cr, lb7);
+      }
     }
-    umma_commit(smem_u32(bars + 0));
+    {                       // dv of value block 0 leaves meanwhile
+      uint32_t r[32];
+      tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + TM_DV + 32 * wq_, r);
+      tmem_ld_wait();
+      if (ok) {
+        bf16* o = dv_out + ((b * T + n * TC + d) * H + h_) * TD + 32 * wq_;
+#pragma unroll
+        for (int c8 = 0; c8 < 2; ++c8) {
+          uint32_t u[8];
+#pragma unroll
+          for (int m = 0; m < 8; ++m) u[m] = pack_bf16x2(__uint_as_float(r[16 * c8 + 2 * m]), __uint_as_float(r[16 * c8 + 2 * m + 1]));
+          st_global_v8(o + 16 * c8, u);
+        }
+      }
+    }
+    tc_fence_before();
+    __syncthreads();        // the next products overwrite the accumulator of dv
+    tc_fence_after();
+    rescale(1);
   }
+  dense_products(LAST);
   __syncwarp();
   // This chunk's operands have landed: ask L2 for those of the chunk that the block scheduler will
   // start on this SM when this block retires (pf_dist blocks ahead), so that its load phase streams
@@ -1225,10 +1304,10 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
   {
     const int64_t nb = (int64_t)blockIdx.x + pf_dist;
     if (!RAG && pf_dist > 0 && nb < (int64_t)gridDim.x && tid == 0) {
-      const int64_t n2 = nb / BHn, bh2 = nb % BHn, h2 = bh2 % H;
+      const int64_t n2 = nb / BHn, bh2 = nb % BHn, h2 = WIDE ? 2 * (bh2 % HB) : bh2 % H;
       const int y2 = (int)((h2 / (R * R)) * R + (h2 % (R * R)) / R), yv2 = (int)((h2 / (R * R)) * R + h2 % R);
-      const int z2 = (int)((bh2 / H) * T + n2 * TC);
-      const int64_t c2 = (bh2 * N + n2) * TD * TD;
+      const int z2 = (int)((bh2 / HB) * T + n2 * TC);
+      const int64_t c2 = (((bh2 / HB) * H + h2) * N + n2) * TD * TD;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         tma_prefetch_l2_3d(&maps.g, 0, y2, z2 + 64 * half);
@@ -1240,12 +1319,12 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
       // contiguous 32 KB tiles: one bulk request each
       l2_prefetch_bulk(S_prev + c2, 2 * TD * TD);
       l2_prefetch_bulk(dS_next + c2, 2 * TD * TD);
-      l2_prefetch_bulk(P_saved + (bh2 * N + n2) * TC * TC, 2 * TC * TC);
+      l2_prefetch_bulk(P_saved + c2, 2 * TC * TC);
     }
   }
-  ok = mbar_wait(smem_u32(bars + 0), 0) && ok;
-  ok = mbar_wait(smem_u32(bars + 5), 0) && ok;      // every thread observes the tiles' arrival itself before reading them
-  ok = mbar_wait(smem_u32(bars + 7), 0) && ok;
+  ok = mbar_wait(smem_u32(bars + 0), LAST) && ok;
+  ok = mbar_wait(smem_u32(bars + 5), LAST) && ok;      // every thread observes the tiles' arrival itself before reading them
+  ok = mbar_wait(smem_u32(bars + 7), LAST) && ok;
   tc_fence_after();
   // dO, v and P have been consumed by the products: their regions take g, q, k of rows 64..127 and k of rows
   // 0..63 by TMA while phase 1.5 runs, so that the W64 build and the first pass read them from shared memory.
@@ -1279,7 +1358,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
     tmem_ld32(lane_base + TM_DKH + 32 * wq_, r2);     // feature d, rows 32 wq_ + m (column layout)
     tmem_ld_wait();
     if (ok && (!RAG || d < nv)) {
-      bf16* o = dv_out + row0 + (int64_t)d * HD + 32 * wq_;
+      bf16* o = WIDE ? dv_out + ((b * T + n * TC + d) * H + h_ + 1) * TD + 32 * wq_ : dv_out + row0 + (int64_t)d * HD + 32 * wq_;
       // a thread owns 64 contiguous bytes of one row; the rows of a warp are far apart, so what counts is the
       // number of store requests: two 32-byte stores instead of four 16-byte ones
 #pragma unroll
@@ -1342,16 +1421,7 @@ tc_chunk_bwd_kernel(const __grid_constant__ BwdMaps maps, int64_t T, int64_t H, 
       }
     }
     // dG2[d] = sum_v S_prev[d][v] dS_next[d][v]    (this thread: v in 32 wq_ + [0, 32))
-    float s2 = 0.f;
-    const uint8_t* ts = sm + BwdSmem::SP + (wq_ >> 1) * TILE_BYTES;
-    const uint8_t* td = sm + BwdSmem::DS + (wq_ >> 1) * TILE_BYTES;
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-      const uint4 a = *reinterpret_cast<const uint4*>(ts + sw128_chunk(d, (wq_ & 1) * 4 + c4));
-      const uint4 c = *reinterpret_cast<const uint4*>(td + sw128_chunk(d, (wq_ & 1) * 4 + c4));
-      s2 += bf16_lo(a.x) * bf16_lo(c.x) + bf16_hi(a.x) * bf16_hi(c.x) + bf16_lo(a.y) * bf16_lo(c.y) + bf16_hi(a.y) * bf16_hi(c.y) +
-            bf16_lo(a.z) * bf16_lo(c.z) + bf16_hi(a.z) * bf16_hi(c.z) + bf16_lo(a.w) * bf16_lo(c.w) + bf16_hi(a.w) * bf16_hi(c.w);
-    }
+    s2 += dot_tiles(sm + BwdSmem::SP + (wq_ >> 1) * TILE_BYTES, sm + BwdSmem::DS + (wq_ >> 1) * TILE_BYTES, d, wq_);
     dG2[wq_ * TD + d] = s2;
   }
   tc_fence_before();
@@ -1988,8 +2058,7 @@ __global__ void __launch_bounds__(256) state_block_kernel(const bf16* __restrict
   if (to_blocked) *reinterpret_cast<uint4*>(out + blocked) = *reinterpret_cast<const uint4*>(in + real);
   else            *reinterpret_cast<uint4*>(out + real) = *reinterpret_cast<const uint4*>(in + blocked);
 }
-// Per-virtual-head results (rows, H R R, 128) summed into (rows, H, 128 R): key-side arrays (dq, dk, dg) keep the
-// key block a and sum over the value blocks c; value-side arrays (out, dv) keep c and sum over a.  Float32 sums.
+// Per-virtual-head results (rows, H R R, 128) summed over the key blocks a into (rows, H, 128 R): out and dv.  Float32 sums.
 // Eight consecutive features of one array as floats, through 16-byte accesses.
 __device__ __forceinline__ void ld8_f32(const bf16* p, float (&x)[8]) {
   const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
@@ -1997,21 +2066,12 @@ __device__ __forceinline__ void ld8_f32(const bf16* p, float (&x)[8]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) { const float2 f = unpack_bf16x2(w[i]); x[2 * i] = f.x; x[2 * i + 1] = f.y; }
 }
-__device__ __forceinline__ void ld8_f32(const float* p, float (&x)[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-}
 __device__ __forceinline__ void st8_f32(bf16* p, const float (&x)[8]) {
   uint4 u;
   u.x = pack_bf16x2(x[0], x[1]); u.y = pack_bf16x2(x[2], x[3]); u.z = pack_bf16x2(x[4], x[5]); u.w = pack_bf16x2(x[6], x[7]);
   *reinterpret_cast<uint4*>(p) = u;
 }
-__device__ __forceinline__ void st8_f32(float* p, const float (&x)[8]) {
-  reinterpret_cast<float4*>(p)[0] = make_float4(x[0], x[1], x[2], x[3]);
-  reinterpret_cast<float4*>(p)[1] = make_float4(x[4], x[5], x[6], x[7]);
-}
-template <typename T, int KEYSIDE>
-__global__ void __launch_bounds__(256) sum_blocks_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t rows,
+__global__ void __launch_bounds__(256) sum_blocks_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int64_t rows,
                                                          int64_t H, int R) {
   const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;      // eight consecutive features
   if (e >= rows * H * R * (TD / 8)) return;
@@ -2020,9 +2080,8 @@ __global__ void __launch_bounds__(256) sum_blocks_kernel(const T* __restrict__ i
   const int64_t h = (e / (TD / 8) / R) % H, row = e / (TD / 8) / R / H;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int s2 = 0; s2 < R; ++s2) {
-    const int a = KEYSIDE ? keep : s2, c = KEYSIDE ? s2 : keep;
     float x[8];
-    ld8_f32(in + ((row * H * R * R + (h * R + a) * R + c) * (int64_t)TD + j * 8), x);
+    ld8_f32(in + ((row * H * R * R + (h * R + s2) * R + keep) * (int64_t)TD + j * 8), x);
 #pragma unroll
     for (int u = 0; u < 8; ++u) acc[u] += x[u];
   }
@@ -2035,11 +2094,10 @@ static int launch_state_block(cudaStream_t st, const void* in, void* out, int64_
   GLA_CHECK_LAUNCH();
   return GLA_OK;
 }
-template <typename T, int KEYSIDE>
-static int launch_sum_blocks(cudaStream_t st, const T* in, T* out, int64_t rows, int64_t H, int R) {
+static int launch_sum_blocks(cudaStream_t st, const bf16* in, bf16* out, int64_t rows, int64_t H, int R) {
   const int64_t n = rows * H * R * (TD / 8);
   ProfScope ps("sum_blocks_kernel", st);
-  sum_blocks_kernel<T, KEYSIDE><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, out, rows, H, R);
+  sum_blocks_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, out, rows, H, R);
   GLA_CHECK_LAUNCH();
   return GLA_OK;
 }
@@ -2059,11 +2117,11 @@ size_t tc_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
   return n;
 }
 // bwd workspace: dstate f32 (R = 1 only) | dS_next bf16 | R > 1: blocked dhidden_final, dhidden_init |
-//                dq, dk, dv per virtual head bf16 | dg per virtual head f32
+//                dv per virtual head bf16
 size_t tc_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
   const int64_t R = D / TD, N = T / TC, BHV = B * H * R * R;
   size_t n = (R == 1 ? f32b(BHV * N * TD * TD) : 0) + b16b(BHV * N * TD * TD);
-  if (R > 1) n += 2 * b16b(BHV * TD * TD) + 3 * b16b(B * T * H * R * R * TD) + f32b(B * T * H * R * R * TD);
+  if (R > 1) n += 2 * b16b(BHV * TD * TD) + b16b(B * T * H * R * R * TD);
   return n;
 }
 
@@ -2199,7 +2257,7 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   }
   GLA_CHECK_LAUNCH();
   if (R > 1) {
-    GLA_TRY((launch_sum_blocks<bf16, 0>(st, out_v, (bf16*)out, B * T, H, R)));
+    GLA_TRY(launch_sum_blocks(st, out_v, (bf16*)out, B * T, H, R));
     GLA_TRY(launch_state_block(st, hfb, hidden_final, B * H, R, 0));
   }
   return GLA_OK;
@@ -2235,15 +2293,11 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   char* w = (char*)ws;
   float* dstate = (float*)w; w += (R == 1 ? f32b(BHV * N * TD * TD) : 0);
   bf16* dS_next = (bf16*)w; w += b16b(BHV * N * TD * TD);
-  bf16 *dhfb = nullptr, *dhib = nullptr, *dq_v = (bf16*)dq, *dk_v = (bf16*)dk, *dv_v = (bf16*)dv;
-  float* dg_v = dg;
+  bf16 *dhfb = nullptr, *dhib = nullptr, *dv_v = (bf16*)dv;
   if (R > 1) {
     dhfb = (bf16*)w; w += b16b(BHV * TD * TD);
     dhib = (bf16*)w; w += b16b(BHV * TD * TD);
-    dq_v = (bf16*)w; w += b16b(B * T * HV * TD);
-    dk_v = (bf16*)w; w += b16b(B * T * HV * TD);
-    dv_v = (bf16*)w; w += b16b(B * T * HV * TD);
-    dg_v = (float*)w;
+    dv_v = (bf16*)w;
   }
   const char* s = (const char*)saved;
   const bf16* S_prev = (const bf16*)s; s += b16b(BHV * N * TD * TD);
@@ -2290,9 +2344,9 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
     GLA_TRY((launch_tc_kv<1>(st, B, T, H, g, q, dout, dstate, nullptr)));
     GLA_TRY(launch_state_scan(st, BHV, N, TD, Gc, dstate, 0, dhidden_final, 1, dS_next, 1, dhidden_init, 1, 1));
   }
-  static SmemAttrOnce bwd_attr[2];
-  auto bwd_kernel = rag ? tc_chunk_bwd_kernel<true> : tc_chunk_bwd_kernel<false>;
-  GLA_TRY(bwd_attr[rag != nullptr].ensure(bwd_kernel, BWD_SMEM));
+  static SmemAttrOnce bwd_attr[3];
+  auto bwd_kernel = rag ? tc_chunk_bwd_kernel<true, false> : R > 1 ? tc_chunk_bwd_kernel<false, true> : tc_chunk_bwd_kernel<false, false>;
+  GLA_TRY(bwd_attr[rag ? 1 : R > 1 ? 2 : 0].ensure(bwd_kernel, BWD_SMEM));
   BwdMaps bmaps;
   GLA_TRY(make_map_bthd(&bmaps.g, g, 1, B, T, HK, 128, 0, 64));
   GLA_TRY(make_map_bthd(&bmaps.q, q, 0, B, T, HK, 128, 0, 64));
@@ -2304,16 +2358,13 @@ int tc_chunk_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   GLA_TRY(make_map_rows(&bmaps.p, P, BHV * N * TC, 64, 128));
   {
     ProfScope ps("tc_chunk_bwd_kernel", st);
-    bwd_kernel<<<(unsigned)(BHV * N), TTHREADS, BWD_SMEM, st>>>(
+    bwd_kernel<<<(unsigned)(B * HK * N), TTHREADS, BWD_SMEM, st>>>(
         bmaps, T, HV, R, N, rag ? rag->tab : nullptr, (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : sm_count(), g, (const bf16*)v, (const bf16*)k,
-        (const bf16*)q, (const bf16*)dout, S_prev, dS_next, P, dq_v, dk_v, dv_v, dg_v, (opts & GLA_OPT_ALL_SCALES) ? 1 : 0);
+        (const bf16*)q, (const bf16*)dout, S_prev, dS_next, P, (bf16*)dq, (bf16*)dk, dv_v, dg, (opts & GLA_OPT_ALL_SCALES) ? 1 : 0);
   }
   GLA_CHECK_LAUNCH();
   if (R > 1) {
-    GLA_TRY((launch_sum_blocks<bf16, 1>(st, dq_v, (bf16*)dq, B * T, H, R)));
-    GLA_TRY((launch_sum_blocks<bf16, 1>(st, dk_v, (bf16*)dk, B * T, H, R)));
-    GLA_TRY((launch_sum_blocks<float, 1>(st, dg_v, dg, B * T, H, R)));
-    GLA_TRY((launch_sum_blocks<bf16, 0>(st, dv_v, (bf16*)dv, B * T, H, R)));
+    GLA_TRY(launch_sum_blocks(st, dv_v, (bf16*)dv, B * T, H, R));
     GLA_TRY(launch_state_block(st, dhib, dhidden_init, B * H, R, 0));
   }
   return GLA_OK;
