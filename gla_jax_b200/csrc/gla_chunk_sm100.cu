@@ -370,11 +370,24 @@ __device__ __forceinline__ void zero_tail_rows(uint8_t* tile, int nv) {
 }
 // RAG: sequences of any length on one time axis; `tab` gives every chunk its first token and its rows.  A kernel of its
 // own so that the dense one carries nothing extra.
-template <bool RAG>
+//
+// WIDE (head size 256, R = 2): a block takes the two key blocks of a value block one after the other; the second's output
+// product accumulates in TMEM onto the first's and one finished output leaves.  (Both outputs used to go out in bf16 and a
+// pass of their own added them: 458 + 82 -> 451 us at B = 2, T = 16384, H = 8.)  The levels of a sharp second key block need the
+// accumulator's columns: it waits in `stash` (128 x 128 floats per block) meanwhile.
+__device__ __noinline__ void fwd_stash_out(uint32_t taddr, float* p) {
+  uint32_t r[32];
+  tmem_ld32(taddr, r);
+  tmem_ld_wait();
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+    reinterpret_cast<uint4*>(p)[m * TTHREADS] = make_uint4(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3]);
+}
+template <bool RAG, bool WIDE>
 __global__ void __launch_bounds__(TTHREADS, 1)
 tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T, int64_t H, int R, int64_t N, const int2* __restrict__ tab,
                     bf16* __restrict__ out, int save_p, const unsigned int* __restrict__ state_done, unsigned int state_target,
-                    int all_scales, int prefetch) {
+                    int all_scales, int prefetch, float* stash) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   float* tot = reinterpret_cast<float*>(sm + FwdSmem::TOT);
@@ -388,8 +401,8 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
   const int rg = tid >> 6, cp = tid & 63;
   // H counts VIRTUAL heads of size 128: a head of size 128 R is R x R independent (key block a, value block c)
   // problems, virtual head (h R + a) R + c, whose results the caller sums over a.  In the (B, T, H_real R, 128) view
-  // of the inputs the key-side tensors of a virtual head are head h R + a, the value-side ones head h R + c; the
-  // output is written per virtual head, (B, T, H, 128).  R = 1: everything coincides with the real layout.
+  // of the inputs the key-side tensors of a virtual head are head h R + a, the value-side ones and the output head
+  // h R + c.  R = 1: everything coincides with the real layout.
   // Chunk order: chunk-major, LAST chunks first.  The state kernel that runs before this one walks the chunks of all
   // heads in step, first to last, so the inputs it read most recently (g, k, v of the late chunks) and the states
   // it wrote last are the ones most likely to be still in L2.
@@ -400,6 +413,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
     Where s;
     s.n = (int)N - 1 - (int)((uint32_t)item / heads);
     s.bh = (int)((uint32_t)item % heads);
+    if (WIDE) s.bh = (s.bh & ~3) | ((s.bh & 1) << 1) | ((s.bh >> 1) & 1);        // items 2 i, 2 i + 1: key blocks 0, 1
     s.b = (int)((uint32_t)s.bh / (uint32_t)H);
     s.h = s.bh - s.b * (int)H;
     s.hk = (int)((uint32_t)s.h / (uint32_t)(R * R)) * R + (int)((uint32_t)s.h % (uint32_t)(R * R)) / R;
@@ -409,13 +423,14 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
   // ---- all global inputs of a chunk through TMA: 192 KB in flight (one thread).  g, q, k (needed at once) come first on
   // their own barrier; v and S_prev are only needed by the output product and land while the scores are formed.
   // Leaves where the chunk lies for all threads (visible with the barrier that g, q, k complete).
+  auto after = [&](int item) { return !WIDE ? item + (int)gridDim.x : (item & 1) ? item - 1 + 2 * (int)gridDim.x : item + 1; };
   ChunkSpot* spots = reinterpret_cast<ChunkSpot*>(sm + FwdSmem::SPOT);
   auto request = [&](int item, uint32_t turn, bool with_state) {
     const Where s = locate(item);
     const uint32_t lb = smem_u32(bars + 3), lb2 = smem_u32(bars + 4);
     const int2 span = RAG ? tab[s.n] : make_int2(s.b * (int)T + s.n * TC, TC);       // first token and rows
     const int z = span.x, y = s.hk, yv = s.hv, chunk = s.bh * (int)N + s.n;
-    spots[turn].out = ((int64_t)z * H + s.h) * TD;
+    spots[turn].out = WIDE ? ((int64_t)z * (H / 2) + yv) * TD : ((int64_t)z * H + s.h) * TD;
     spots[turn].chunk = chunk;
     spots[turn].rows = span.y;
     mbar_arrive_expect_tx(lb, 4 * 2 * TILE_BYTES);
@@ -433,7 +448,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
     }
     // The same boxes of the chunk that follows, requested into L2 only: seven instructions of this one thread, so that
     // its load phase is served from L2.
-    const int next = item + (int)gridDim.x;
+    const int next = after(item);
     if (WALK && prefetch && next < chunks) {
       const Where t = locate(next);
       const int y2 = t.hk, yv2 = t.hv, z2 = t.b * (int)T + t.n * TC;
@@ -458,7 +473,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
     const bool s_pending = state_done != nullptr && ld_acquire_u32(state_done) < state_target;
     *s_pending_sm = s_pending ? 1u : 0u;
     if (!s_pending && state_done != nullptr) fence_proxy_async_global();
-    request((int)blockIdx.x, 0u, !s_pending);
+    request((WIDE ? 2 : 1) * (int)blockIdx.x, 0u, !s_pending);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), 512);
@@ -476,7 +491,9 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
   // not at all, with all levels four and three times.
   uint32_t turn = 0, par0 = 0, par1 = 0;
 #pragma unroll 1
-  for (int item = (int)blockIdx.x; item < chunks; item += (int)gridDim.x, turn ^= 1u) {
+  for (int item = (WIDE ? 2 : 1) * (int)blockIdx.x; item < chunks; item = after(item), turn ^= 1u) {
+  // WIDE: `add`: the output product goes onto the accumulator; turn is the key block, since items come in pairs
+  bool add = WIDE && turn != 0u, stashed = false;
   bool ok = mbar_wait(smem_u32(bars + 3), turn);
   const ChunkSpot* spot = spots + turn;
   const int nv = RAG ? spot->rows : TC;
@@ -601,6 +618,11 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
       }
     }
   } else {
+  if (WIDE && add) {
+    fwd_stash_out(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 32), stash + (size_t)blockIdx.x * TC * TD + 4 * tid);
+    add = false; stashed = true;
+    tc_fence_before();        // (the first level's product comes after block barriers)
+  }
   // diagonal: sum_d q k, reduced over the 64 column-pair threads of a row group (two warps)
   {
     float part[16];
@@ -799,7 +821,7 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
     const uint64_t ap = desc_kmajor(smem_u32(sm + FwdSmem::P), TILE_BYTES, 0), bv = desc_mnmajor(smem_u32(sm + FwdSmem::V), TILE_BYTES, 0);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks)
-      umma_bf16(tmem, kslice_kmajor(aq, TILE_BYTES, ks), kslice_mnmajor(bs, ks), idesc, ks > 0);
+      umma_bf16(tmem, kslice_kmajor(aq, TILE_BYTES, ks), kslice_mnmajor(bs, ks), idesc, (WIDE && add) || ks > 0);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks)
       umma_bf16(tmem, kslice_kmajor(ap, TILE_BYTES, ks), kslice_mnmajor(bv, ks), idesc, 1);
@@ -826,20 +848,29 @@ tc_chunk_fwd_kernel(const __grid_constant__ FwdMaps maps, int chunks, int64_t T,
   // The products have consumed their operands: the next chunk's inputs come in while this one's output leaves.  (The state
   // kernel is complete: this chunk's state tile came through its grid dependency, or after a look at its counter.)
   const bool failed = __syncthreads_or(!ok) != 0;       // ... and the rest of shared memory has been read by everybody
-  if (WALK && tid == 0 && !failed && item + (int)gridDim.x < chunks) {
+  if (WALK && tid == 0 && !failed && after(item) < chunks) {
     tma_wait_read();
     if (state_done != nullptr) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       fence_proxy_async_global();
     }
-    request(item + (int)gridDim.x, turn ^ 1u, true);
+    request(after(item), turn ^ 1u, true);
   }
-  if (ok) {
+  if (ok && (!WIDE || turn != 0u)) {
     const int q4 = warp & 3, cg = warp >> 2;
     uint32_t r[32];
     tmem_ld32(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(cg * 32), r);
     tmem_ld_wait();
-    bf16* o = out + spot->out + (int64_t)(q4 * 32 + lane) * (H * TD) + cg * 32;
+    if (WIDE && stashed) {
+      const float4* x = reinterpret_cast<const float4*>(stash + (size_t)blockIdx.x * TC * TD + 4 * tid);     // the thread's own values
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const float4 y = x[m * TTHREADS];
+        r[4 * m] = __float_as_uint(__uint_as_float(r[4 * m]) + y.x); r[4 * m + 1] = __float_as_uint(__uint_as_float(r[4 * m + 1]) + y.y);
+        r[4 * m + 2] = __float_as_uint(__uint_as_float(r[4 * m + 2]) + y.z); r[4 * m + 3] = __float_as_uint(__uint_as_float(r[4 * m + 3]) + y.w);
+      }
+    }
+    bf16* o = out + spot->out + (int64_t)(q4 * 32 + lane) * (WIDE ? H / 2 * TD : H * TD) + cg * 32;
     // 64 contiguous bytes of one row per thread, rows of a warp far apart: two 32-byte stores
 #pragma unroll
     for (int c8 = 0; c8 < 2; ++c8) {
@@ -2058,7 +2089,7 @@ __global__ void __launch_bounds__(256) state_block_kernel(const bf16* __restrict
   if (to_blocked) *reinterpret_cast<uint4*>(out + blocked) = *reinterpret_cast<const uint4*>(in + real);
   else            *reinterpret_cast<uint4*>(out + real) = *reinterpret_cast<const uint4*>(in + blocked);
 }
-// Per-virtual-head results (rows, H R R, 128) summed over the key blocks a into (rows, H, 128 R): out and dv.  Float32 sums.
+// dv per virtual head, (rows, H R R, 128), summed over the key blocks a into (rows, H, 128 R).  Float32 sums.
 // Eight consecutive features of one array as floats, through 16-byte accesses.
 __device__ __forceinline__ void ld8_f32(const bf16* p, float (&x)[8]) {
   const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
@@ -2102,6 +2133,8 @@ static int launch_sum_blocks(cudaStream_t st, const bf16* in, bf16* out, int64_t
   return GLA_OK;
 }
 
+// Blocks of the forward chunk kernel at head size 256, at most (the workspace holds a tile for each).
+constexpr int WIDE_BLOCKS = 256;
 // Sizes.  R = D / 128, HV = H R R virtual heads, N = T / 128 chunks whatever chunk size the caller named.
 // saved: S_prev bf16 (B HV, N, 128, 128) | Gc f32 (B HV, N, 128) | P bf16 (B HV, N, 128, 128)
 size_t tc_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
@@ -2109,11 +2142,11 @@ size_t tc_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
   return b16b(BHV * N * TD * TD) + f32b(BHV * N * TD) + b16b(BHV * N * TC * TC);
 }
 // fwd workspace: kv f32 (R = 1 only: the product + scan pair) | Gc f32 | S_prev bf16 (used when nothing is saved)
-//                | R > 1: blocked hidden_init, blocked hidden_final bf16 (B HV, 128, 128) | out per virtual head bf16
+//                | R > 1: blocked hidden_init, blocked hidden_final bf16 (B HV, 128, 128) | one 128 x 128 f32 tile per resident block
 size_t tc_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
   const int64_t R = D / TD, N = T / TC, BHV = B * H * R * R;
   size_t n = (R == 1 ? f32b(BHV * N * TD * TD) : 0) + f32b(BHV * N * TD) + b16b(BHV * N * TD * TD);
-  if (R > 1) n += 2 * b16b(BHV * TD * TD) + b16b(B * T * H * R * R * TD);
+  if (R > 1) n += 2 * b16b(BHV * TD * TD) + f32b((int64_t)WIDE_BLOCKS * TC * TD);
   return n;
 }
 // bwd workspace: dstate f32 (R = 1 only) | dS_next bf16 | R > 1: blocked dhidden_final, dhidden_init |
@@ -2144,11 +2177,12 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   float* kv = (float*)w; w += (R == 1 ? f32b(BHV * N * TD * TD) : 0);
   float* Gc = (float*)w; w += f32b(BHV * N * TD);
   bf16* S_prev = (bf16*)w; w += b16b(BHV * N * TD * TD);
-  bf16 *hib = nullptr, *hfb = nullptr, *out_v = nullptr;
+  bf16 *hib = nullptr, *hfb = nullptr;
+  float* stash = nullptr;
   if (R > 1) {
     hib = (bf16*)w; w += b16b(BHV * TD * TD);
     hfb = (bf16*)w; w += b16b(BHV * TD * TD);
-    out_v = (bf16*)w;
+    stash = (float*)w;
   }
   bf16* P = nullptr;
   if (saved) {
@@ -2217,10 +2251,10 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
     return GLA_OK;
   }
   if (!fused_states && sp_phase == 0) GLA_TRY(launch_state_scan(st, BHV, N, TD, Gc, kv, 0, hidden_init, 1, S_prev, 1, hidden_final, 1, 0));
-  static SmemAttrOnce fwd_attr[2];
-  auto fwd_kernel = rag ? tc_chunk_fwd_kernel<true> : tc_chunk_fwd_kernel<false>;
+  static SmemAttrOnce fwd_attr[3];
+  auto fwd_kernel = rag ? tc_chunk_fwd_kernel<true, false> : R > 1 ? tc_chunk_fwd_kernel<false, true> : tc_chunk_fwd_kernel<false, false>;
   const int2* tab = rag ? rag->tab : nullptr;
-  GLA_TRY(fwd_attr[rag != nullptr].ensure(fwd_kernel, FWD_SMEM));
+  GLA_TRY(fwd_attr[rag ? 1 : R > 1 ? 2 : 0].ensure(fwd_kernel, FWD_SMEM));
   cudaError_t e;
   const int all_scales = (opts & GLA_OPT_ALL_SCALES) ? 1 : 0;
   FwdMaps maps;
@@ -2233,9 +2267,10 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
   else maps.p = maps.s;        // not used
   {
     ProfScope ps("tc_chunk_fwd_kernel", st);
-    bf16* out_p = R > 1 ? out_v : (bf16*)out;
+    bf16* out_p = (bf16*)out;
     const int prefetch = (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : 1, chunks = (int)(BHV * N);
-    const unsigned blocks = rag ? (unsigned)chunks : walking_blocks(chunks);
+    unsigned blocks = rag ? (unsigned)chunks : walking_blocks(R > 1 ? chunks / 2 : chunks);
+    if (R > 1 && blocks > WIDE_BLOCKS) blocks = WIDE_BLOCKS;
     if (early_flag != nullptr) {
       // programmatic dependent of the state kernel launched just before: may start while that one runs
       cudaLaunchConfig_t cfg = {};
@@ -2249,15 +2284,14 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       e = cudaLaunchKernelEx(&cfg, fwd_kernel, maps, chunks, T, HV, R, N, tab, out_p, P != nullptr ? 1 : 0, (const unsigned int*)early_flag,
-                             early_target, all_scales, prefetch);
+                             early_target, all_scales, prefetch, stash);
       if (e != cudaSuccess) return record_cuda_error(e);
     } else {
-      fwd_kernel<<<blocks, TTHREADS, FWD_SMEM, st>>>(maps, chunks, T, HV, R, N, tab, out_p, P != nullptr, nullptr, 0u, all_scales, prefetch);
+      fwd_kernel<<<blocks, TTHREADS, FWD_SMEM, st>>>(maps, chunks, T, HV, R, N, tab, out_p, P != nullptr, nullptr, 0u, all_scales, prefetch, stash);
     }
   }
   GLA_CHECK_LAUNCH();
   if (R > 1) {
-    GLA_TRY(launch_sum_blocks(st, out_v, (bf16*)out, B * T, H, R));
     GLA_TRY(launch_state_block(st, hfb, hidden_final, B * H, R, 0));
   }
   return GLA_OK;
