@@ -2134,7 +2134,7 @@ static int launch_sum_blocks(cudaStream_t st, const bf16* in, bf16* out, int64_t
 }
 
 // Blocks of the forward chunk kernel at head size 256, at most (the workspace holds a tile for each).
-constexpr int WIDE_BLOCKS = 256;
+static int64_t wide_blocks_max(int64_t chunks) { return chunks / 2 < 256 ? chunks / 2 : 256; }
 // Sizes.  R = D / 128, HV = H R R virtual heads, N = T / 128 chunks whatever chunk size the caller named.
 // saved: S_prev bf16 (B HV, N, 128, 128) | Gc f32 (B HV, N, 128) | P bf16 (B HV, N, 128, 128)
 size_t tc_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
@@ -2146,7 +2146,7 @@ size_t tc_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
 size_t tc_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t) {
   const int64_t R = D / TD, N = T / TC, BHV = B * H * R * R;
   size_t n = (R == 1 ? f32b(BHV * N * TD * TD) : 0) + f32b(BHV * N * TD) + b16b(BHV * N * TD * TD);
-  if (R > 1) n += 2 * b16b(BHV * TD * TD) + f32b((int64_t)WIDE_BLOCKS * TC * TD);
+  if (R > 1) n += 2 * b16b(BHV * TD * TD) + f32b(wide_blocks_max(BHV * N) * TC * TD);
   return n;
 }
 // bwd workspace: dstate f32 (R = 1 only) | dS_next bf16 | R > 1: blocked dhidden_final, dhidden_init |
@@ -2270,7 +2270,7 @@ int tc_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, in
     bf16* out_p = (bf16*)out;
     const int prefetch = (opts & GLA_OPT_NO_L2_PREFETCH) ? 0 : 1, chunks = (int)(BHV * N);
     unsigned blocks = rag ? (unsigned)chunks : walking_blocks(R > 1 ? chunks / 2 : chunks);
-    if (R > 1 && blocks > WIDE_BLOCKS) blocks = WIDE_BLOCKS;
+    if (R > 1 && blocks > wide_blocks_max(chunks)) blocks = (unsigned)wide_blocks_max(chunks);
     if (early_flag != nullptr) {
       // programmatic dependent of the state kernel launched just before: may start while that one runs
       cudaLaunchConfig_t cfg = {};
