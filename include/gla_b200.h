@@ -338,6 +338,7 @@ GLA_API int gla_chunk_bwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t
  *   - the array is gla_chunk_fwd_static_max_bytes() = 32 MiB of device memory PER GPU, held
  *     from the first use of the library on that GPU until the process exits;
  *   - a problem whose gla_chunk_fwd_workspace_bytes() exceeds it returns GLA_ERR_TOO_LARGE
+ *     (head size 128 on the split-operand kernels: exceeds it by more than their extra state per head)
  *     and launches nothing (32 MiB covers, e.g., one sequence of T=4096, H=6, D=128);
  *   - the function allocates nothing and frees nothing, on host or device.  The first call
  *     on each device looks up the array's device address (a symbol query, with that device
