@@ -20,9 +20,8 @@
 //   dV = P^T dO + k~ (e^m dS)              dP = tril(dO V^T)
 // (S: the state entering the chunk, dS: the gradient of the state leaving it; the factor e^m rides on the rows of
 // the state while they are split.)  The weights stay within exp(+-LIMIT / 2) as long as sum |g| <= LIMIT over the
-// chunk and no single |g| exceeds ONE_GATE (the weights are running products of exp(g), which must not vanish); chunks beyond that ("sharp") take
-// the weights anchored at the chunk's ends for the state products and form the scores and their gradients pair by
-// pair with the exponent lam_i - lam_j, in float32.
+// chunk and no single |g| exceeds ONE_GATE (the weights are running products of exp(g), which must not vanish); chunks
+// beyond that ("sharp") are walked token by token from the state that enters them, in float32 FMAs.
 //
 // Three launches forward, three backward: per-chunk state products (k^^T V, resp. q^^T dO), a scan over the chunks
 // in place, and the chunk kernel.  States are float32, N + 1 of them per head (slot n enters chunk n; slot N is the
@@ -41,7 +40,6 @@ namespace {
 
 constexpr float PX_LIMIT = 140.f;
 constexpr float PX_ONE_GATE = 60.f;
-constexpr float PX_GATE_FLOOR = -1000.f;      // exp() is zero far above this; a gate of -inf must not make inf - inf
 
 // D features, chunks of L rows.  Element-wise stages: a thread owns a column pair and RPT consecutive rows.  Products:
 // warps in WR row groups of 16 x WC column groups.
@@ -59,6 +57,7 @@ struct Px {
   static constexpr int LDT = 2 * L + 16, TPLANE = L * LDT;                // score tile
   static constexpr int SREG = D * PW / 4 / NT;   // float4 loads per thread and state piece
   static constexpr int AP = D + 8;               // row pitch (floats) of the float32 tiles of the closing pass
+  static constexpr int TP = 4 * NT / D, TE = D / TP;   // walk by token: threads per four rows or columns of the state, elements of each
   static_assert(PC % 16 == 0 && CW % 16 == 0, "a warp's columns come in pairs of 8-wide tiles");
 };
 
@@ -185,14 +184,11 @@ struct ChunkAt {
   }
   __device__ __forceinline__ int64_t row(int r) const { return row0 + (int64_t)r * step; }
 };
-__device__ __forceinline__ float clamp_gate(float g) { return g < PX_GATE_FLOOR ? PX_GATE_FLOOR : g; }      // NaN stays
 template <class C>
 __device__ __forceinline__ void load_gates(float2 (&g)[C::RPT], const float* gp, const ChunkAt<C>& at, int r0, int cp) {
 #pragma unroll
   for (int i = 0; i < C::RPT; ++i)
     g[i] = r0 + i < at.nv ? __ldg(reinterpret_cast<const float2*>(gp + at.row(r0 + i) + 2 * cp)) : make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < C::RPT; ++i) g[i] = make_float2(clamp_gate(g[i].x), clamp_gate(g[i].y));
 }
 template <class C, typename TI>
 __device__ __forceinline__ void load_pairs(Pair<TI> (&x)[C::RPT], const void* xp, const ChunkAt<C>& at, int r0, int cp) {
@@ -222,10 +218,10 @@ __device__ __forceinline__ void copy_rows(uint8_t* dst, const void* src, const C
   }
 }
 // Gate sums of the thread's rows, exchanged between the row groups: sums before the thread's rows, of the whole chunk,
-// and whether the chunk needs the pairwise form.  seg: [RG][D], sab: [RG][D] floats.
+// and whether the chunk is sharp.  seg: [RG][D], sab: [RG][D] floats.
 template <class C>
 __device__ __forceinline__ bool gate_sums(const float2 (&g)[C::RPT], float* seg, float* sab, int rg, int cp,
-                                          float2& before, float2& own, float2& total) {
+                                          float2& before, float2& total) {
   float2 s = make_float2(0.f, 0.f), a = s;
   bool big = false;
 #pragma unroll
@@ -237,7 +233,7 @@ __device__ __forceinline__ bool gate_sums(const float2 (&g)[C::RPT], float* seg,
   *reinterpret_cast<float2*>(seg + rg * C::D + 2 * cp) = s;
   *reinterpret_cast<float2*>(sab + rg * C::D + 2 * cp) = a;
   __syncthreads();
-  own = s; before = total = make_float2(0.f, 0.f); a = before;
+  before = total = make_float2(0.f, 0.f); a = before;
 #pragma unroll
   for (int r = 0; r < C::RG; ++r) {
     const float2 t = *reinterpret_cast<const float2*>(seg + r * C::D + 2 * cp);
@@ -366,14 +362,12 @@ __global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, 
 }
 
 // ---- pieces of the chunk kernels -------------------------------------------------------------------------------------------
-// q~ and k~ (mild chunk), or q^ = q exp(lam) and k^ = k exp(G - lam) (sharp chunk) as split planes; em[d] = the factor
-// that the rows of the states take.
+// q~ and k~ as split planes; em[d] = the factor that the rows of the states take.
 template <class C, typename TI>
 __device__ __forceinline__ void build_qk(uint8_t* sQ, uint8_t* sK, float* em, float2 (&g)[C::RPT], const Pair<TI> (&q)[C::RPT],
-                                         const Pair<TI> (&k)[C::RPT], bool sharp, float2 before, float2 own, float2 total,
-                                         int rg, int cp) {
+                                         const Pair<TI> (&k)[C::RPT], float2 before, float2 total, int rg, int cp) {
   const int r0 = rg * C::RPT;
-  const float2 half = sharp ? make_float2(0.f, 0.f) : make_float2(0.5f * total.x, 0.5f * total.y);
+  const float2 half = make_float2(0.5f * total.x, 0.5f * total.y);
   if (rg == 0) *reinterpret_cast<float2*>(em + 2 * cp) = make_float2(expf(half.x), expf(half.y));
   float2 run = make_float2(expf(before.x - half.x), expf(before.y - half.y));
 #pragma unroll
@@ -383,8 +377,7 @@ __device__ __forceinline__ void build_qk(uint8_t* sQ, uint8_t* sK, float* em, fl
     const float2 x = q[i].get();
     st_split3(sQ + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
   }
-  if (sharp) run = make_float2(expf(total.x - before.x - own.x), expf(total.y - before.y - own.y));
-  else run = make_float2(1.f / run.x, 1.f / run.y);
+  run = make_float2(1.f / run.x, 1.f / run.y);
 #pragma unroll
   for (int i = C::RPT - 1; i >= 0; --i) {
     const float2 x = k[i].get();
@@ -410,40 +403,6 @@ __device__ __forceinline__ void store_piece(uint8_t* dst, const float4 (&x)[C::S
     st_split3(dst + r * C::LDS + c * 8, C::SPLANE, make_float4(x[j].x * w, x[j].y * w, x[j].z * w, x[j].w * w));
   }
 }
-// lam of the chunk, float32, [L][D]
-template <class C>
-__device__ __forceinline__ void store_lam(float* lam, const float* gp, const ChunkAt<C>& at, float2 before, int rg, int cp) {
-  float2 run = before;
-#pragma unroll 1
-  for (int i = 0; i < C::RPT; ++i) {
-    const int r = rg * C::RPT + i;
-    float2 x = make_float2(0.f, 0.f);
-    if (r < at.nv) x = __ldg(reinterpret_cast<const float2*>(gp + at.row(r) + 2 * cp));
-    run.x += clamp_gate(x.x); run.y += clamp_gate(x.y);
-    *reinterpret_cast<float2*>(lam + r * C::D + 2 * cp) = run;
-  }
-}
-// A 16 x 16 block of P = tril(q~ k~^T) of a sharp chunk, pair by pair: rows m0 + lane / 4 (+ 8), columns c0 + 8 j +
-// 2 (lane % 4) (+ 1), the accumulator layout.
-template <class C, typename TI>
-__device__ __noinline__ void block_by_pair(float (*acc)[4], const float* lam, const void* q, const void* k,
-                                           const ChunkAt<C>& at, int m0, int c0, int lane) {
-  const int ra = m0 + (lane >> 2), rb = ra + 8;
-#pragma unroll 1
-  for (int d = 0; d < C::D; ++d) {
-    const float qa = ra < at.nv ? ld_f((const TI*)q, at.row(ra) + d) : 0.f, qb = rb < at.nv ? ld_f((const TI*)q, at.row(rb) + d) : 0.f;
-    const float la = lam[ra * C::D + d], lb = lam[rb * C::D + d];
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int c = c0 + 8 * j + 2 * (lane & 3) + e;
-        const float y = c < at.nv ? ld_f((const TI*)k, at.row(c) + d) : 0.f, lc = lam[c * C::D + d];
-        if (c <= ra) acc[j][e] = fmaf(qa * y, expf(la - lc), acc[j][e]);
-        if (c <= rb) acc[j][2 + e] = fmaf(qb * y, expf(lb - lc), acc[j][2 + e]);
-      }
-  }
-}
 // The warp's score blocks (row block wr, column blocks wc, wc + WC, ... up to the diagonal): A B^T over D.
 template <class C, int NSA, int NSB>
 __device__ __forceinline__ void score_blocks(float (&x)[C::NB][2][4], uint32_t aA, uint32_t aB, int wr, int wc, int lane) {
@@ -462,19 +421,6 @@ __device__ __forceinline__ void score_blocks(float (&x)[C::NB][2][4], uint32_t a
       for (int i = 0; i < C::NB; ++i)
         if (wc + C::WC * i <= wr) mma_step<NSA, NSB, 1, false>(x[i], a, aB, C::PLANE, C::LD, 16 * (wc + C::WC * i), 16 * ks, lane);
     }
-  }
-}
-template <class C, typename TI>
-__device__ __forceinline__ void score_blocks_by_pair(float (&x)[C::NB][2][4], const float* lam, const PxParams& p,
-                                                     const ChunkAt<C>& at, int wr, int wc, int lane) {
-#pragma unroll
-  for (int i = 0; i < C::NB; ++i) {
-    float y[2][4] = {};                                    // (its address is taken; x stays in registers)
-    if (wc + C::WC * i <= wr) block_by_pair<C, TI>(y, lam, p.q, p.k, at, 16 * wr, 16 * (wc + C::WC * i), lane);
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) x[i][j][e] = y[j][e];
   }
 }
 // ... as split planes of the score tile [i][j], entries above the diagonal zero
@@ -507,6 +453,165 @@ __device__ __forceinline__ void zero_acc(float (&c)[N][4]) {
     for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
 }
 
+// ---- a sharp chunk, token by token ---------------------------------------------------------------------------------------
+// The recurrence itself, from the state that enters the chunk: every weight is a product of exp(g), so that a gate that
+// resets the state costs the later tokens nothing.  (Weights exp(lam_i - lam_j) from running sums, which stood here
+// before, lost what the sums had grown to: 4e-5 of out after one gate of -1e4, 1.1e-4 after eight, against 2e-7.)
+// A thread holds TE elements of each of four rows (COL = false) or columns (COL = true) of the state, so that a value it
+// reads from shared memory, which bounds the walk, serves four sums; TP consecutive threads share the four.  What a
+// token adds is w[element] scalar(token)[row or column], and out(token, row or column, sum_e z[e] state[e]) leaves
+// through lanes 0 to 3 of the TP.  f, w, z: float32 [L][D].
+//   REV = false: state = f state + w scalar, then the sum;   REV = true: state += w scalar, then the sum, then state *= f
+// Measured, bf16 4 x 2048 tokens, 6 heads, every chunk sharp, forward and with the backward: head size 128 1288, 3322 us
+// (pair by pair) -> 333, 1063; head size 64 579, 1567 -> 110, 375 (mild chunks: 126, 389 and 44, 150).
+template <int VW> __device__ __forceinline__ void ld_vec(float (&x)[VW], const float* p) {
+  if constexpr (VW == 2) { const float2 v = *reinterpret_cast<const float2*>(p); x[0] = v.x; x[1] = v.y; }
+  else { const float4 v = *reinterpret_cast<const float4*>(p); x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
+}
+// The four sums over TP lanes: lane lp of the TP is left with x[quarter(lp)].
+__device__ __forceinline__ int quarter(int lp) { return 2 * (lp & 1) + ((lp >> 1) & 1); }
+template <int TP>
+__device__ __forceinline__ float sum_quarters(const float (&x)[4], int lp) {
+  const bool o1 = (lp & 1) != 0, o2 = (lp & 2) != 0;
+  const float a = (o1 ? x[2] : x[0]) + __shfl_xor_sync(0xffffffffu, o1 ? x[0] : x[2], 1);
+  const float b = (o1 ? x[3] : x[1]) + __shfl_xor_sync(0xffffffffu, o1 ? x[1] : x[3], 1);
+  float c = (o2 ? b : a) + __shfl_xor_sync(0xffffffffu, o2 ? a : b, 2);
+#pragma unroll
+  for (int d = 4; d < TP; d <<= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
+  return c;
+}
+template <class C, bool COL, bool REV, class Scalar, class Out>
+__device__ __forceinline__ void walk(float (&m)[4][C::TE], const float* f, const float* w, const float* z, int nv, int own, int part,
+                                     Scalar scalar, Out out) {
+  constexpr int VW = C::TE < 4 ? C::TE : 4;
+  float s[4], next[4];
+  scalar(REV ? nv - 1 : 0, s);
+#pragma unroll 1
+  for (int i = 0; i < nv; ++i) {
+    const int t = REV ? nv - 1 - i : i;
+    if (i + 1 < nv) scalar(REV ? t - 1 : t + 1, next);
+    float o[4] = {0.f, 0.f, 0.f, 0.f}, fr[4];
+    if (!COL) ld_vec<4>(fr, f + t * C::D + own);
+#pragma unroll
+    for (int j = 0; j < C::TE / VW; ++j) {
+      const int e = t * C::D + VW * (part + C::TP * j);
+      float we[VW], ze[VW], fe[VW];
+      ld_vec<VW>(we, w + e);
+      ld_vec<VW>(ze, z + e);
+      if (COL) ld_vec<VW>(fe, f + e);
+#pragma unroll
+      for (int u = 0; u < VW; ++u)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          float& x = m[r][VW * j + u];
+          const float ft = COL ? fe[u] : fr[r];
+          x = REV ? fmaf(we[u], s[r], x) : fmaf(ft, x, we[u] * s[r]);
+          o[r] = fmaf(ze[u], x, o[r]);
+          if (REV) x *= ft;
+        }
+    }
+    const float c = sum_quarters<C::TP>(o, part);
+    if (part < 4) out(t, own + quarter(part), c);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r] = next[r];
+  }
+}
+template <class C, bool COL>
+__device__ __forceinline__ void load_state(float (&m)[4][C::TE], const float* st, int own, int part) {
+  constexpr int VW = C::TE < 4 ? C::TE : 4;
+#pragma unroll
+  for (int j = 0; j < C::TE / VW; ++j) {
+    const int e = VW * (part + C::TP * j);
+    float x[4];
+    if (COL) {
+#pragma unroll
+      for (int u = 0; u < VW; ++u) {
+        ld_vec<4>(x, st + (e + u) * C::D + own);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) m[r][VW * j + u] = x[r];
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float y[VW];
+        ld_vec<VW>(y, st + (own + r) * C::D + e);
+#pragma unroll
+        for (int u = 0; u < VW; ++u) m[r][VW * j + u] = y[u];
+      }
+    }
+  }
+}
+// a chunk of an array, or exp of it, as float32 [L][D]
+template <class C, typename TI, bool EXP = false>
+__device__ __forceinline__ void stage(float* dst, const void* src, const ChunkAt<C>& at) {
+#pragma unroll 4
+  for (int id = threadIdx.x; id < at.nv * C::CP; id += C::NT) {
+    const int r = id / C::CP, c = id % C::CP;
+    Pair<TI> x;
+    x.load(src, at.row(r) + 2 * c);
+    const float2 y = x.get();
+    *reinterpret_cast<float2*>(dst + r * C::D + 2 * c) = EXP ? make_float2(expf(y.x), expf(y.y)) : y;
+  }
+}
+template <class C, typename TI>
+__device__ __noinline__ void fwd_by_token(float* f, const float* Sn, const PxParams& p) {
+  const ChunkAt<C> at(p, blockIdx.x);
+  float *k = f + C::L * C::D, *q = k + C::L * C::D;
+  stage<C, float, true>(f, p.g, at);
+  stage<C, TI>(k, p.k, at);
+  stage<C, TI>(q, p.q, at);
+  __syncthreads();
+  const int own = threadIdx.x / C::TP * 4, part = threadIdx.x % C::TP;
+  float m[4][C::TE];
+  load_state<C, true>(m, Sn, own, part);
+  walk<C, true, false>(m, f, k, q, at.nv, own, part, [&](int t, float (&s)[4]) {
+    Pair<TI> a, b;
+    a.load(p.v, at.row(t) + own);
+    b.load(p.v, at.row(t) + own + 2);
+    s[0] = a.get().x; s[1] = a.get().y; s[2] = b.get().x; s[3] = b.get().y;
+  }, [&](int t, int c, float o) { st_any(p.out, p.out_bf, at.row(t) + c, o); });
+}
+// dq forwards and dk backwards by rows of the states, dv backwards by columns; dg collects q dq, then the sums
+template <class C, typename TI, typename TY>
+__device__ __noinline__ void bwd_by_token(float* f, const float* Sn, const float* dSn, const PxParams& p) {
+  const ChunkAt<C> at(p, blockIdx.x);
+  float *k = f + C::L * C::D, *q = k + C::L * C::D, *v = q + C::L * C::D, *dout = v + C::L * C::D;
+  stage<C, float, true>(f, p.g, at);
+  stage<C, TI>(k, p.k, at);
+  stage<C, TI>(q, p.q, at);
+  stage<C, TI>(v, p.v, at);
+  stage<C, TY>(dout, p.dout, at);
+  __syncthreads();
+  const int own = threadIdx.x / C::TP * 4, part = threadIdx.x % C::TP;
+  auto from = [&](const float* x) { return [=](int t, float (&s)[4]) { ld_vec<4>(s, x + t * C::D + own); }; };
+  float m[4][C::TE];
+  load_state<C, false>(m, Sn, own, part);
+  walk<C, false, false>(m, f, v, dout, at.nv, own, part, from(k), [&](int t, int d, float o) {
+    st_f((TI*)p.dq, at.row(t) + d, o);
+    p.dg[at.row(t) + d] = q[t * C::D + d] * o;
+  });
+  float dots[4] = {0.f, 0.f, 0.f, 0.f};
+  load_state<C, false>(m, dSn, own, part);
+  constexpr int VW = C::TE < 4 ? C::TE : 4;
+#pragma unroll
+  for (int j = 0; j < C::TE / VW; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float y[VW];                              // of the state that leaves the chunk
+      ld_vec<VW>(y, Sn + (C::D + own + r) * C::D + VW * (part + C::TP * j));
+#pragma unroll
+      for (int u = 0; u < VW; ++u) dots[r] = fmaf(y[u], m[r][VW * j + u], dots[r]);
+    }
+  float sum = sum_quarters<C::TP>(dots, part);
+  walk<C, false, true>(m, f, dout, v, at.nv, own, part, from(q), [&](int t, int d, float o) {
+    st_f((TI*)p.dk, at.row(t) + d, o);
+    sum += p.dg[at.row(t) + d] - k[t * C::D + d] * o;
+    p.dg[at.row(t) + d] = sum;
+  });
+  load_state<C, true>(m, dSn, own, part);
+  walk<C, true, true>(m, f, q, k, at.nv, own, part, from(dout), [&](int t, int c, float o) { st_f((TI*)p.dv, at.row(t) + c, o); });
+}
+
 // ---- forward chunk kernel ---------------------------------------------------------------------------------------------
 template <class C, typename TI>
 struct FwdLay {
@@ -520,10 +625,10 @@ struct FwdLay {
   static constexpr uint32_t T = C::NP > 1 ? S + 3 * C::SPLANE : K, SEG = C::NP > 1 ? T + 3 * C::TPLANE : V + NSV * C::PLANE;
   static constexpr uint32_t EM = SEG + 2 * C::RG * C::D * 4, END = EM + C::D * 4;
   static constexpr int BLOCKS = C::NP > 1 ? 1 : sizeof(TI) == 2 ? 3 : 2;
-  static_assert(C::L * C::D * 4 <= 3 * C::PLANE, "the pairwise form keeps lam where k~ would be");
+  static_assert(3 * C::L * C::D * 4 <= V, "the walk by token keeps exp(g), k and q over q~ and k~");
 };
 template <class C, typename TI>
-__global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(PxParams p) {
+__global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(const __grid_constant__ PxParams p) {
   using Lay = FwdLay<C, TI>;
   extern __shared__ __align__(16) uint8_t sm[];
   float* seg = reinterpret_cast<float*>(sm + Lay::SEG);
@@ -532,7 +637,6 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(Px
   const ChunkAt<C> at(p, blockIdx.x);
   const float* Sn = p.S + (at.bh * (p.N + 1) + at.n) * C::D * C::D;
   float4 sx[C::SREG];
-  bool sharp;
   {
     float2 g[C::RPT];
     Pair<TI> q[C::RPT], k[C::RPT];
@@ -541,14 +645,15 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(Px
     load_pairs<C, TI>(q, p.q, at, r0, cp);
     load_pairs<C, TI>(k, p.k, at, r0, cp);
     copy_rows<C, TI>(sm + Lay::V, p.v, at);
-    float2 before, own, total;
-    sharp = gate_sums<C>(g, seg, seg + C::RG * C::D, rg, cp, before, own, total);
-    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, sharp, before, own, total, rg, cp);
-    __syncthreads();
-    if (sharp) {
-      store_lam<C>(reinterpret_cast<float*>(sm + Lay::K), p.g, at, before, rg, cp);
-      __syncthreads();
+    float2 before, total;
+    if (gate_sums<C>(g, seg, seg + C::RG * C::D, rg, cp, before, total)) {
+      grid_dep_wait();
+      grid_dep_launch();
+      fwd_by_token<C, TI>(reinterpret_cast<float*>(sm), Sn, p);
+      return;
     }
+    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, before, total, rg, cp);
+    __syncthreads();
   }
   const int wr = warp % C::WR, wc = warp / C::WR, m0 = 16 * wr;
   const uint32_t aQ = smem_u32(sm + Lay::Q), aK = smem_u32(sm + Lay::K), aV = smem_u32(sm + Lay::V), aS = smem_u32(sm + Lay::S);
@@ -558,8 +663,7 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(Px
   for (int pc = 0; pc < C::NP; ++pc) zero_acc(o[pc]);
   {
     float x[C::NB][2][4];
-    if (!sharp) score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);
-    else score_blocks_by_pair<C, TI>(x, reinterpret_cast<const float*>(sm + Lay::K), p, at, wr, wc, lane);
+    score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);
     __syncthreads();                      // the scores are formed: the region of k~ is free
     store_scores<C>(sm + Lay::T, x, wr, wc, lane);
   }
@@ -619,12 +723,12 @@ template <class C, typename TI, typename TY>
 struct BwdLay {
   static constexpr int NSV = planes_of<TI>(), NSD = planes_of<TY>();
   static constexpr uint32_t most(uint32_t a, uint32_t b) { return a > b ? a : b; }
-  // score tile, state pieces; the pairwise form also keeps lam there for a while
-  static constexpr uint32_t SREGION = most(3 * C::SPLANE, most(3 * C::TPLANE, C::L * C::D * 4));
+  static constexpr uint32_t SREGION = most(3 * C::SPLANE, 3 * C::TPLANE);      // score tile, state pieces
   static constexpr uint32_t Q = 0, K = Q + 3 * C::PLANE, V = K + 3 * C::PLANE, DO = V + NSV * C::PLANE, S = DO + NSD * C::PLANE;
   static constexpr uint32_t SEG = S + SREGION, EM = SEG + 2 * C::RG * C::D * 4, DG = EM + C::D * 4, END = DG + C::D * 4;
+  static constexpr int BLOCKS = 232448 / (END + 1024);      // per SM, what shared memory holds (registers must not hold fewer)
   static_assert(C::L * C::AP * 4 <= 3 * C::PLANE, "dq and dk are staged in float32 over q~ and k~");
-  static_assert(C::L * C::D * 4 <= (NSV + NSD) * C::PLANE, "pairwise form: lam over V and dO at the end");
+  static_assert(5 * C::L * C::D * 4 <= SEG, "the walk by token keeps exp(g), k, q, v and dO over the operands");
 };
 // dG[d] += <S_{n+1}[d, piece], dS_n[d, piece]>: PW / 4 consecutive threads hold a row of the piece
 template <class C>
@@ -640,46 +744,8 @@ __device__ __forceinline__ void dot_piece(float* dG, const float4 (&x)[C::SREG],
     if (id % (C::PW / 4) == 0) dG[r] = pc == 0 ? s : dG[r] + s;
   }
 }
-// Sharp chunk: the accumulators of dq and dk hold the inter-chunk terms only; applies their weights exp(lam) and
-// exp(G - lam) and adds the pairs inside the chunk, dP (three planes) times exp(lam_i - lam_j).
-template <class C, typename TI>
-__device__ __noinline__ void close_by_pair(float* tq, float* tk, const uint8_t* dP, const float* lam, const PxParams& p,
-                                           const ChunkAt<C>& at, float2 total, int r0, int cp) {
-  auto dp_at = [&](int i, int j) {
-    const bf16* t = reinterpret_cast<const bf16*>(dP + i * C::LDT + j * 2);
-    return (__bfloat162float(t[C::TPLANE]) + __bfloat162float(t[C::TPLANE / 2])) + __bfloat162float(t[0]);
-  };
-  auto at2 = [&](const float* t, int r, int pitch) { return *reinterpret_cast<const float2*>(t + r * pitch + 2 * cp); };
-#pragma unroll 1
-  for (int r = r0; r < r0 + C::RPT; ++r) {
-    const float2 lr = at2(lam, r, C::D);
-    float2 x = at2(tq, r, C::AP), y = at2(tk, r, C::AP);
-    x.x *= expf(lr.x); x.y *= expf(lr.y);
-    y.x *= expf(total.x - lr.x); y.y *= expf(total.y - lr.y);
-#pragma unroll 1
-    for (int j = 0; j <= r && j < at.nv; ++j) {
-      Pair<TI> kj;
-      kj.load(p.k, at.row(j) + 2 * cp);
-      const float2 kf = kj.get(), lj = at2(lam, j, C::D);
-      const float w = dp_at(r, j);
-      x.x = fmaf(w * kf.x, expf(lr.x - lj.x), x.x);
-      x.y = fmaf(w * kf.y, expf(lr.y - lj.y), x.y);
-    }
-#pragma unroll 1
-    for (int i = r; i < at.nv; ++i) {
-      Pair<TI> qi;
-      qi.load(p.q, at.row(i) + 2 * cp);
-      const float2 qf = qi.get(), li = at2(lam, i, C::D);
-      const float w = dp_at(i, r);
-      y.x = fmaf(w * qf.x, expf(li.x - lr.x), y.x);
-      y.y = fmaf(w * qf.y, expf(li.y - lr.y), y.y);
-    }
-    *reinterpret_cast<float2*>(tq + r * C::AP + 2 * cp) = x;
-    *reinterpret_cast<float2*>(tk + r * C::AP + 2 * cp) = y;
-  }
-}
 template <class C, typename TI, typename TY>
-__global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
+__global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kernel(const __grid_constant__ PxParams p) {
   using Lay = BwdLay<C, TI, TY>;
   constexpr int NSV = Lay::NSV, NSD = Lay::NSD, L = C::L, D = C::D;
   extern __shared__ __align__(16) uint8_t sm[];
@@ -691,8 +757,7 @@ __global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
   const float* Sn = p.S + (at.bh * (p.N + 1) + at.n) * D * D;
   const float* dSn = p.dS + (at.bh * (p.N + 1) + at.n + 1) * D * D;
   float4 sx[C::SREG];
-  float2 before, own, total;
-  bool sharp;
+  float2 before, total;
   {
     float2 g[C::RPT];
     Pair<TI> q[C::RPT], k[C::RPT];
@@ -701,8 +766,13 @@ __global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
     load_pairs<C, TI>(k, p.k, at, r0, cp);
     copy_rows<C, TI>(sm + Lay::V, p.v, at);
     copy_rows<C, TY>(sm + Lay::DO, p.dout, at);
-    sharp = gate_sums<C>(g, seg, seg + C::RG * D, rg, cp, before, own, total);
-    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, sharp, before, own, total, rg, cp);
+    if (gate_sums<C>(g, seg, seg + C::RG * D, rg, cp, before, total)) {
+      grid_dep_wait();
+      grid_dep_launch();
+      bwd_by_token<C, TI, TY>(reinterpret_cast<float*>(sm), Sn, dSn, p);
+      return;
+    }
+    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, before, total, rg, cp);
   }
   grid_dep_wait();                        // the gradient states of the scan before this kernel
   grid_dep_launch();
@@ -719,29 +789,22 @@ __global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
 #pragma unroll
   for (int pc = 0; pc < C::NP; ++pc) zero_acc(dv[pc]);
   float x[C::NB][2][4];
-  if (!sharp) {
-    score_blocks<C, NSD, NSV>(x, aD, aV, wr, wc, lane);               // dP = tril(dO V^T)
-    store_scores<C>(sm + Lay::S, x, wr, wc, lane);
-    __syncthreads();
+  score_blocks<C, NSD, NSV>(x, aD, aV, wr, wc, lane);               // dP = tril(dO V^T)
+  store_scores<C>(sm + Lay::S, x, wr, wc, lane);
+  __syncthreads();
 #pragma unroll 1
-    for (int kk = 0; kk <= wr; ++kk) {                                // dq += dP k~
-      uint32_t a[3][4];
-      ld_a<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
-      mma_step<3, 3, C::CW / 16, true>(dq, a, aK, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
-    }
-#pragma unroll 1
-    for (int kk = wr; kk < L / 16; ++kk) {                            // dk += dP^T q~
-      uint32_t a[3][4];
-      ld_a_t<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
-      mma_step<3, 3, C::CW / 16, true>(dk, a, aQ, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
-    }
-    score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);                   // P = tril(q~ k~^T)
-  } else {
-    float* lam = reinterpret_cast<float*>(sm + Lay::S);
-    store_lam<C>(lam, p.g, at, before, rg, cp);
-    __syncthreads();
-    score_blocks_by_pair<C, TI>(x, lam, p, at, wr, wc, lane);
+  for (int kk = 0; kk <= wr; ++kk) {                                // dq += dP k~
+    uint32_t a[3][4];
+    ld_a<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
+    mma_step<3, 3, C::CW / 16, true>(dq, a, aK, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
   }
+#pragma unroll 1
+  for (int kk = wr; kk < L / 16; ++kk) {                            // dk += dP^T q~
+    uint32_t a[3][4];
+    ld_a_t<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
+    mma_step<3, 3, C::CW / 16, true>(dk, a, aQ, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
+  }
+  score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);                   // P = tril(q~ k~^T)
   __syncthreads();
   store_scores<C>(sm + Lay::S, x, wr, wc, lane);
   __syncthreads();
@@ -805,15 +868,6 @@ __global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
       *reinterpret_cast<float2*>(tq + e) = make_float2(dq[j][2 * h], dq[j][2 * h + 1]);
       *reinterpret_cast<float2*>(tk + e) = make_float2(dk[j][2 * h], dk[j][2 * h + 1]);
     }
-  if (sharp) {
-    score_blocks<C, NSD, NSV>(x, aD, aV, wr, wc, lane);
-    store_scores<C>(sm + Lay::S, x, wr, wc, lane);
-    __syncthreads();
-    float* lam = reinterpret_cast<float*>(sm + Lay::V);
-    store_lam<C>(lam, p.g, at, before, rg, cp);
-    __syncthreads();
-    close_by_pair<C, TI>(tq, tk, sm + Lay::S, lam, p, at, total, r0, cp);     // a thread's own entries of tq and tk
-  }
   __syncthreads();
 
   // ---- closing pass: a thread finishes RPT rows of two features ------------------------------------------------------
@@ -822,12 +876,12 @@ __global__ void __launch_bounds__(C::NT) px_bwd_kernel(PxParams p) {
   load_gates<C>(g, p.g, at, r0, cp);
   load_pairs<C, TI>(q, p.q, at, r0, cp);
   load_pairs<C, TI>(k, p.k, at, r0, cp);
-  float2 run = sharp ? make_float2(1.f, 1.f) : make_float2(expf(before.x - 0.5f * total.x), expf(before.y - 0.5f * total.y));
+  float2 run = make_float2(expf(before.x - 0.5f * total.x), expf(before.y - 0.5f * total.y));
   float2 dl[C::RPT];
 #pragma unroll
   for (int i = 0; i < C::RPT; ++i) {
     const int r = r0 + i;
-    g[i] = sharp ? make_float2(1.f, 1.f) : make_float2(expf(g[i].x), expf(g[i].y));
+    g[i] = make_float2(expf(g[i].x), expf(g[i].y));
     run.x *= g[i].x; run.y *= g[i].y;
     float2 y = *reinterpret_cast<const float2*>(tq + r * C::AP + 2 * cp);
     y.x *= run.x; y.y *= run.y;

@@ -64,6 +64,17 @@ def test_chunks_on_both_sides_of_the_gate_limits(cuda_device, D):
     assert O.rel_l2(hf0, hf[0].cpu()) < 5e-6 and O.rel_l2(out0, out[0].cpu()) < 5e-6
 
 
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("gate,at", [(-1e4, (70,)), (-1e4, (5, 64, 100, 127)), (-float("inf"), (3, 40, 41, 90)),
+                                     (-100.0, (20, 63, 80)), (-float("inf"), tuple(range(2, 130, 9)))])
+def test_resets_in_every_feature(cuda_device, D, gate, at):
+    """Tokens whose gate resets the whole state, mild gates in between: what follows a reset keeps its precision."""
+    from gla_jax_b200 import recurrent_gla
+    case = _case(1, 130, 2, D, torch.float32, 15, 5.0)
+    case[1][:, list(at)] = gate
+    _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"resets {D, gate, at}")
+
+
 def test_naive_with_bf16_inputs_and_float32_cotangent(cuda_device):
     """bf16 operands with a float32 output and output gradient (recurrent_gla_naive), head size 128: shorter chunks."""
     from gla_jax_b200 import recurrent_gla_naive
