@@ -127,7 +127,11 @@ __device__ __forceinline__ void ld_a_t(uint32_t (&a)[NS][4], uint32_t base, uint
 }
 // c[2 NQ tiles of 8 columns] += A B over 16 of K.  B is stored [n][k] (BT = false) or [k][n] (BT = true).  Products of
 // planes sa and sb with sa + sb > 2 lie below 2^-24 of the result and are left out; the small ones come first.
-template <int NSA, int NSB, int NQ, bool BT>
+// EX (what leaves in float32, or makes what does): the tensor cores cut off what an addition shifts out, which over the
+// length of a product adds up to 0.7e-6 (head size 32) to 1.7e-6 (128) of a float32 result; so 16 of K are summed from
+// zero and added in float32: 1.8e-7, and 2.5e-7 for the recurrence in FMAs.  It costs 4 % of a float32 call (587 -> 608 us
+// for 4 x 2048 tokens of 6 heads of 128, forward and backward) and 1 to 3 % of a bf16 one, whose dlog_fgate is float32.
+template <int NSA, int NSB, int NQ, bool BT, bool EX>
 __device__ __forceinline__ void mma_step(float (*c)[4], const uint32_t (&a)[NSA][4], uint32_t base, uint32_t plane,
                                          uint32_t ld, int n0, int k0, int lane) {
   const int r8 = lane & 7, h3 = (lane >> 3) & 1, h4 = (lane >> 4) & 1;
@@ -141,16 +145,21 @@ __device__ __forceinline__ void mma_step(float (*c)[4], const uint32_t (&a)[NSA]
     for (int s = 0; s < NSB; ++s) {
       if (BT) ldsm4t(b[s], addr + s * plane); else ldsm4(b[s], addr + s * plane);
     }
+    float y[2][4] = {};
+    float (&c0)[4] = EX ? y[0] : c[2 * j], (&c1)[4] = EX ? y[1] : c[2 * j + 1];
 #pragma unroll
     for (int t = 2; t >= 0; --t)
 #pragma unroll
       for (int sa = 0; sa < NSA; ++sa) {
         const int sb = t - sa;
         if (sb >= 0 && sb < NSB) {
-          hmma(c[2 * j], a[sa], b[sb][0], b[sb][1]);
-          hmma(c[2 * j + 1], a[sa], b[sb][2], b[sb][3]);
+          hmma(c0, a[sa], b[sb][0], b[sb][1]);
+          hmma(c1, a[sa], b[sb][2], b[sb][3]);
         }
       }
+    if (EX)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { c[2 * j][e] += y[0][e]; c[2 * j + 1][e] += y[1][e]; }
   }
 }
 template <typename TI> struct Pair;
@@ -307,7 +316,7 @@ __global__ void __launch_bounds__(C::NT, sizeof(TI) + sizeof(TY) == 4 ? 1024 / C
   for (int ks = 0; ks < C::L / 16; ++ks) {
     uint32_t a[3][4];
     ld_a_t<3>(a, aX, C::PLANE, C::LD, m0, 16 * ks, lane);
-    mma_step<3, NSY, NW / 16, true>(acc, a, aY, C::PLANE, C::LD, c0, 16 * ks, lane);
+    mma_step<3, NSY, NW / 16, true, (sizeof(TI) + sizeof(TY) > 4)>(acc, a, aY, C::PLANE, C::LD, c0, 16 * ks, lane);
   }
   float* o = (MODE == 0 ? p.S : p.dS) + (at.bh * (p.N + 1) + at.n + (MODE == 0 ? 1 : 0)) * C::D * C::D;
 #pragma unroll
@@ -404,7 +413,7 @@ __device__ __forceinline__ void store_piece(uint8_t* dst, const float4 (&x)[C::S
   }
 }
 // The warp's score blocks (row block wr, column blocks wc, wc + WC, ... up to the diagonal): A B^T over D.
-template <class C, int NSA, int NSB>
+template <class C, int NSA, int NSB, bool EX>
 __device__ __forceinline__ void score_blocks(float (&x)[C::NB][2][4], uint32_t aA, uint32_t aB, int wr, int wc, int lane) {
 #pragma unroll
   for (int i = 0; i < C::NB; ++i)
@@ -419,7 +428,7 @@ __device__ __forceinline__ void score_blocks(float (&x)[C::NB][2][4], uint32_t a
       ld_a<NSA>(a, aA, C::PLANE, C::LD, 16 * wr, 16 * ks, lane);
 #pragma unroll
       for (int i = 0; i < C::NB; ++i)
-        if (wc + C::WC * i <= wr) mma_step<NSA, NSB, 1, false>(x[i], a, aB, C::PLANE, C::LD, 16 * (wc + C::WC * i), 16 * ks, lane);
+        if (wc + C::WC * i <= wr) mma_step<NSA, NSB, 1, false, EX>(x[i], a, aB, C::PLANE, C::LD, 16 * (wc + C::WC * i), 16 * ks, lane);
     }
   }
 }
@@ -627,7 +636,7 @@ struct FwdLay {
   static constexpr int BLOCKS = C::NP > 1 ? 1 : sizeof(TI) == 2 ? 3 : 2;
   static_assert(3 * C::L * C::D * 4 <= V, "the walk by token keeps exp(g), k and q over q~ and k~");
 };
-template <class C, typename TI>
+template <class C, typename TI, bool EX>
 __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(const __grid_constant__ PxParams p) {
   using Lay = FwdLay<C, TI>;
   extern __shared__ __align__(16) uint8_t sm[];
@@ -663,7 +672,7 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(co
   for (int pc = 0; pc < C::NP; ++pc) zero_acc(o[pc]);
   {
     float x[C::NB][2][4];
-    score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);
+    score_blocks<C, 3, 3, EX>(x, aQ, aK, wr, wc, lane);
     __syncthreads();                      // the scores are formed: the region of k~ is free
     store_scores<C>(sm + Lay::T, x, wr, wc, lane);
   }
@@ -683,7 +692,7 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(co
     ld_a<3>(a, aT, C::TPLANE, C::LDT, m0, 16 * kk, lane);
 #pragma unroll
     for (int pc = 0; pc < C::NP; ++pc)
-      mma_step<3, Lay::NSV, C::PC / 16, true>(o[pc], a, aV, C::PLANE, C::LD, pc * C::PW + wc * C::PC, 16 * kk, lane);
+      mma_step<3, Lay::NSV, C::PC / 16, true, EX>(o[pc], a, aV, C::PLANE, C::LD, pc * C::PW + wc * C::PC, 16 * kk, lane);
   }
   if (C::NP == 1) {
     __syncthreads();                      // the scores are consumed
@@ -696,7 +705,7 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(co
     ld_a<3>(a, aQ, C::PLANE, C::LD, m0, 16 * ks, lane);
 #pragma unroll
     for (int pc = 0; pc < C::NP; ++pc)
-      mma_step<3, 3, C::PC / 16, true>(o[pc], a, pc == 0 ? aS : aK, C::SPLANE, C::LDS, wc * C::PC, 16 * ks, lane);
+      mma_step<3, 3, C::PC / 16, true, EX>(o[pc], a, pc == 0 ? aS : aK, C::SPLANE, C::LDS, wc * C::PC, 16 * ks, lane);
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -748,6 +757,7 @@ template <class C, typename TI, typename TY>
 __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kernel(const __grid_constant__ PxParams p) {
   using Lay = BwdLay<C, TI, TY>;
   constexpr int NSV = Lay::NSV, NSD = Lay::NSD, L = C::L, D = C::D;
+  constexpr bool EX = sizeof(TI) == 4;    // dv; dq and dk make dg, which is float32 always
   extern __shared__ __align__(16) uint8_t sm[];
   float* seg = reinterpret_cast<float*>(sm + Lay::SEG);
   float* em = reinterpret_cast<float*>(sm + Lay::EM);
@@ -789,22 +799,22 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
 #pragma unroll
   for (int pc = 0; pc < C::NP; ++pc) zero_acc(dv[pc]);
   float x[C::NB][2][4];
-  score_blocks<C, NSD, NSV>(x, aD, aV, wr, wc, lane);               // dP = tril(dO V^T)
+  score_blocks<C, NSD, NSV, true>(x, aD, aV, wr, wc, lane);               // dP = tril(dO V^T)
   store_scores<C>(sm + Lay::S, x, wr, wc, lane);
   __syncthreads();
 #pragma unroll 1
   for (int kk = 0; kk <= wr; ++kk) {                                // dq += dP k~
     uint32_t a[3][4];
     ld_a<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
-    mma_step<3, 3, C::CW / 16, true>(dq, a, aK, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
+    mma_step<3, 3, C::CW / 16, true, true>(dq, a, aK, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
   }
 #pragma unroll 1
   for (int kk = wr; kk < L / 16; ++kk) {                            // dk += dP^T q~
     uint32_t a[3][4];
     ld_a_t<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
-    mma_step<3, 3, C::CW / 16, true>(dk, a, aQ, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
+    mma_step<3, 3, C::CW / 16, true, true>(dk, a, aQ, C::PLANE, C::LD, wc * C::CW, 16 * kk, lane);
   }
-  score_blocks<C, 3, 3>(x, aQ, aK, wr, wc, lane);                   // P = tril(q~ k~^T)
+  score_blocks<C, 3, 3, EX>(x, aQ, aK, wr, wc, lane);                   // P = tril(q~ k~^T)
   __syncthreads();
   store_scores<C>(sm + Lay::S, x, wr, wc, lane);
   __syncthreads();
@@ -814,7 +824,7 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
     ld_a_t<3>(a, aS, C::TPLANE, C::LDT, m0, 16 * kk, lane);
 #pragma unroll
     for (int pc = 0; pc < C::NP; ++pc)
-      mma_step<3, NSD, C::PC / 16, true>(dv[pc], a, aD, C::PLANE, C::LD, pc * C::PW + wc * C::PC, 16 * kk, lane);
+      mma_step<3, NSD, C::PC / 16, true, EX>(dv[pc], a, aD, C::PLANE, C::LD, pc * C::PW + wc * C::PC, 16 * kk, lane);
   }
 #pragma unroll
   for (int i = 0; i < 2 * C::NP; ++i) {       // the pieces of S_n (dq += dO S^T), then those of dS_n (dk += V dS^T, dV += k~ dS)
@@ -829,20 +839,20 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
       for (int ks = 0; ks < C::PW / 16; ++ks) {
         uint32_t a[NSD][4];
         ld_a<NSD>(a, aD, C::PLANE, C::LD, m0, pc * C::PW + 16 * ks, lane);
-        mma_step<NSD, 3, C::CW / 16, false>(dq, a, aS, C::SPLANE, C::LDS, wc * C::CW, 16 * ks, lane);
+        mma_step<NSD, 3, C::CW / 16, false, true>(dq, a, aS, C::SPLANE, C::LDS, wc * C::CW, 16 * ks, lane);
       }
     } else {
 #pragma unroll 1
       for (int ks = 0; ks < C::PW / 16; ++ks) {
         uint32_t a[NSV][4];
         ld_a<NSV>(a, aV, C::PLANE, C::LD, m0, pc * C::PW + 16 * ks, lane);
-        mma_step<NSV, 3, C::CW / 16, false>(dk, a, aS, C::SPLANE, C::LDS, wc * C::CW, 16 * ks, lane);
+        mma_step<NSV, 3, C::CW / 16, false, true>(dk, a, aS, C::SPLANE, C::LDS, wc * C::CW, 16 * ks, lane);
       }
 #pragma unroll 1
       for (int ks = 0; ks < D / 16; ++ks) {
         uint32_t a[3][4];
         ld_a<3>(a, aK, C::PLANE, C::LD, m0, 16 * ks, lane);
-        mma_step<3, 3, C::PC / 16, true>(dv[pc], a, aS, C::SPLANE, C::LDS, wc * C::PC, 16 * ks, lane);
+        mma_step<3, 3, C::PC / 16, true, EX>(dv[pc], a, aS, C::SPLANE, C::LDS, wc * C::PC, 16 * ks, lane);
       }
     }
   }
@@ -934,16 +944,22 @@ int launch_scan(cudaStream_t st, int64_t BH, int64_t D, int64_t N, const float* 
                                  (const TS*)init, S, (TS*)fin, mode));
   return GLA_OK;
 }
+template <class C, typename TI, bool EX>
+int launch_fwd(cudaStream_t st, const PxParams& p, int64_t chunks) {
+  static SmemAttrOnce attr;
+  GLA_TRY(attr.ensure(px_fwd_kernel<C, TI, EX>, FwdLay<C, TI>::END));
+  ProfScope ps(p.label, st);
+  GLA_LAUNCHED(launch_overlapped(px_fwd_kernel<C, TI, EX>, dim3((unsigned)chunks), dim3(C::NT), FwdLay<C, TI>::END, st, p));
+  return GLA_OK;
+}
 template <class C, typename TI>
 int run_fwd(cudaStream_t st, const PxParams& p, const void* init, void* fin) {
   const int64_t BH = p.B * p.H, chunks = BH * p.N;
   GLA_TRY((launch_product<C, TI, TI, 0>(st, p, chunks)));
   GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.eG, init, p.S, fin, 0));
-  static SmemAttrOnce attr;
-  GLA_TRY(attr.ensure(px_fwd_kernel<C, TI>, FwdLay<C, TI>::END));
-  ProfScope ps(p.label, st);
-  GLA_LAUNCHED(launch_overlapped(px_fwd_kernel<C, TI>, dim3((unsigned)chunks), dim3(C::NT), FwdLay<C, TI>::END, st, p));
-  return GLA_OK;
+  if constexpr (sizeof(TI) == 2)
+    if (p.out_bf) return launch_fwd<C, TI, false>(st, p, chunks);
+  return launch_fwd<C, TI, true>(st, p, chunks);
 }
 // states != 0: the states are in p.S and p.eG already (a forward's residuals); otherwise they are formed here first
 template <class C, typename TI, typename TY>

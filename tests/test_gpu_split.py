@@ -75,6 +75,25 @@ def test_resets_in_every_feature(cuda_device, D, gate, at):
     _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"resets {D, gate, at}")
 
 
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("shift,gate", [(5.0, None)])
+def test_float32_rounding_and_no_more(cuda_device, D, shift, gate):
+    """A weight is a product of up to 64 rounded factors, a sum has up to 12 float32 additions of 16 products each; with a
+    mean square of 2^-24 / sqrt(3) per rounding that is (8 + 3.5) 3.4e-8 = 4e-7.  The gate gradient (float32 for bf16
+    callers too) is a sum of terms that cancel: three times that."""
+    from gla_jax_b200 import recurrent_gla
+    case = _case(1, 192, 2, D, torch.float32, 17, shift)
+    if gate is not None:
+        case[1][:, [5, 90, 180]] = gate
+    ref, got = _oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case)
+    errs = [O.rel_l2(a, b) for a, b in zip((ref[0], ref[1], *ref[2]), (got[0], got[1], *got[2]))]
+    bound = [4e-7, 4e-7, *(1.2e-6 if n == "dlog_fgate" else 4e-7 for n in NAMES)]
+    assert all(e < b for e, b in zip(errs, bound)), errs
+    half = [x if i == 1 else x.to(torch.bfloat16) for i, x in enumerate(case)]
+    i = NAMES.index("dlog_fgate")
+    assert O.rel_l2(_oracle(*half)[2][i], _run_gpu(recurrent_gla, cuda_device, *half)[2][i]) < 1.2e-6
+
+
 def test_naive_with_bf16_inputs_and_float32_cotangent(cuda_device):
     """bf16 operands with a float32 output and output gradient (recurrent_gla_naive), head size 128: shorter chunks."""
     from gla_jax_b200 import recurrent_gla_naive
