@@ -16,12 +16,13 @@
 // One anchor per chunk.  lam = running sum of the log gates inside the chunk, G = its total.  With m = G / 2 per
 // feature, q~ = q exp(lam - m) and k~ = k exp(m - lam) give every product of the chunk:
 //   P = tril(q~ k~^T)                      O  = P V + q~ (e^m S)
-//   dq = exp(lam - m) (dP k~ + dO (e^m S)^T)   dk = exp(m - lam) (dP^T q~ + V (e^m dS)^T)
-//   dV = P^T dO + k~ (e^m dS)              dP = tril(dO V^T)
-// (S: the state entering the chunk, dS: the gradient of the state leaving it; the factor e^m rides on the rows of
-// the state while they are split.)  The weights stay within exp(+-LIMIT / 2) as long as sum |g| <= LIMIT over the
-// chunk and no single |g| exceeds ONE_GATE (the weights are running products of exp(g), which must not vanish); chunks
-// beyond that ("sharp") are walked token by token from the state that enters them, in float32 FMAs.
+//   dq = exp(lam - m) (dP k~ + dO (e^m S)^T)   dk = exp(m - lam) (dP^T q~ + V (e^(G - m) dS)^T)
+//   dV = P^T dO + k~ (e^(G - m) dS)        dP = tril(dO V^T)
+// (S: the state entering the chunk, dS: the gradient of the state leaving it; the factors e^m ride on the rows of
+// the states while they are split.)  The weights stay within exp(+-LIMIT / 2) as long as sum |g| <= LIMIT over the
+// chunk, no single |g| exceeds ONE_GATE and no thread's rows exceed GROUP together (the weights are products of exp(g),
+// which must not vanish); chunks beyond that ("sharp") are walked token by token from the state that enters them, in
+// float32 FMAs.
 //
 // Three launches forward, three backward: per-chunk state products (k^^T V, resp. q^^T dO), a scan over the chunks
 // in place, and the chunk kernel.  States are float32, N + 1 of them per head (slot n enters chunk n; slot N is the
@@ -39,7 +40,7 @@ using namespace tc;
 namespace {
 
 constexpr float PX_LIMIT = 140.f;
-constexpr float PX_ONE_GATE = 60.f;
+constexpr float PX_ONE_GATE = 60.f, PX_GROUP = 80.f;      // of a thread's rows together
 
 // D features, chunks of L rows.  Element-wise stages: a thread owns a column pair and RPT consecutive rows.  Products:
 // warps in WR row groups of 16 x WC column groups.
@@ -226,31 +227,45 @@ __device__ __forceinline__ void copy_rows(uint8_t* dst, const void* src, const C
     }
   }
 }
-// Gate sums of the thread's rows, exchanged between the row groups: sums before the thread's rows, of the whole chunk,
-// and whether the chunk is sharp.  seg: [RG][D], sab: [RG][D] floats.
+// From the log gates of the thread's rows (exp of them on return), exchanged between the row groups: half of the chunk's
+// total, exp(lam - half) before the thread's rows, and whether the chunk is sharp.  The weight is a product from the
+// anchor on, not the exponential of a sum: with gates of -30 to -55 a sum of that size left 0.5e-6 to 1.1e-6 in a float32
+// result, the products 2e-7.  seg: [3][RG][D] floats.
 template <class C>
-__device__ __forceinline__ bool gate_sums(const float2 (&g)[C::RPT], float* seg, float* sab, int rg, int cp,
-                                          float2& before, float2& total) {
-  float2 s = make_float2(0.f, 0.f), a = s;
+__device__ __forceinline__ bool gate_weights(float2 (&g)[C::RPT], float* seg, int rg, int cp, float2& half, float2& start) {
+  float* sab = seg + C::RG * C::D;
+  float* prod = sab + C::RG * C::D;
+  float2 s = make_float2(0.f, 0.f), a = s, f = make_float2(1.f, 1.f);
   bool big = false;
 #pragma unroll
   for (int i = 0; i < C::RPT; ++i) {
     s.x += g[i].x; s.y += g[i].y;
     a.x += fabsf(g[i].x); a.y += fabsf(g[i].y);
     big = big || !(fabsf(g[i].x) <= PX_ONE_GATE) || !(fabsf(g[i].y) <= PX_ONE_GATE);
+    g[i] = make_float2(expf(g[i].x), expf(g[i].y));
+    f.x *= g[i].x; f.y *= g[i].y;
   }
+  big = big || a.x > PX_GROUP || a.y > PX_GROUP;
   *reinterpret_cast<float2*>(seg + rg * C::D + 2 * cp) = s;
   *reinterpret_cast<float2*>(sab + rg * C::D + 2 * cp) = a;
+  *reinterpret_cast<float2*>(prod + rg * C::D + 2 * cp) = f;
   __syncthreads();
-  before = total = make_float2(0.f, 0.f); a = before;
+  s = make_float2(0.f, 0.f); a = s;
 #pragma unroll
   for (int r = 0; r < C::RG; ++r) {
     const float2 t = *reinterpret_cast<const float2*>(seg + r * C::D + 2 * cp);
     const float2 u = *reinterpret_cast<const float2*>(sab + r * C::D + 2 * cp);
-    if (r < rg) { before.x += t.x; before.y += t.y; }
-    total.x += t.x; total.y += t.y;
+    s.x += t.x; s.y += t.y;
     a.x += u.x; a.y += u.y;
   }
+  half = make_float2(0.5f * s.x, 0.5f * s.y);
+  start = make_float2(expf(-half.x), expf(-half.y));
+#pragma unroll
+  for (int r = 0; r < C::RG - 1; ++r)
+    if (r < rg) {
+      const float2 t = *reinterpret_cast<const float2*>(prod + r * C::D + 2 * cp);
+      start.x *= t.x; start.y *= t.y;
+    }
   return __syncthreads_or(big || !(a.x <= PX_LIMIT) || !(a.y <= PX_LIMIT)) != 0;
 }
 
@@ -371,27 +386,27 @@ __global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, 
 }
 
 // ---- pieces of the chunk kernels -------------------------------------------------------------------------------------------
-// q~ and k~ as split planes; em[d] = the factor that the rows of the states take.
+// q~ and k~ as split planes; em[d] = e^m, which the rows of S take, and ed[d] = exp(G - m), from the same products as the
+// weights, which those of dS take.
 template <class C, typename TI>
-__device__ __forceinline__ void build_qk(uint8_t* sQ, uint8_t* sK, float* em, float2 (&g)[C::RPT], const Pair<TI> (&q)[C::RPT],
-                                         const Pair<TI> (&k)[C::RPT], float2 before, float2 total, int rg, int cp) {
+__device__ __forceinline__ void build_qk(uint8_t* sQ, uint8_t* sK, float* em, float* ed, const float2 (&f)[C::RPT], const Pair<TI> (&q)[C::RPT],
+                                         const Pair<TI> (&k)[C::RPT], float2 half, float2 start, int rg, int cp) {
   const int r0 = rg * C::RPT;
-  const float2 half = make_float2(0.5f * total.x, 0.5f * total.y);
   if (rg == 0) *reinterpret_cast<float2*>(em + 2 * cp) = make_float2(expf(half.x), expf(half.y));
-  float2 run = make_float2(expf(before.x - half.x), expf(before.y - half.y));
+  float2 run = start;
 #pragma unroll
   for (int i = 0; i < C::RPT; ++i) {
-    g[i] = make_float2(expf(g[i].x), expf(g[i].y));
-    run.x *= g[i].x; run.y *= g[i].y;
+    run.x *= f[i].x; run.y *= f[i].y;
     const float2 x = q[i].get();
     st_split3(sQ + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
   }
+  if (ed != nullptr && rg == C::RG - 1) *reinterpret_cast<float2*>(ed + 2 * cp) = run;
   run = make_float2(1.f / run.x, 1.f / run.y);
 #pragma unroll
   for (int i = C::RPT - 1; i >= 0; --i) {
     const float2 x = k[i].get();
     st_split3(sK + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
-    run.x *= g[i].x; run.y *= g[i].y;
+    run.x *= f[i].x; run.y *= f[i].y;
   }
 }
 // Value columns [PW pc, PW pc + PW) of a state (float32, D x D), rows scaled by em, as split planes.
@@ -632,7 +647,7 @@ struct FwdLay {
   static constexpr uint32_t KREG = most(C::NP > 1 ? 0 : 3 * C::TPLANE, most(3 * C::SPLANE, 3 * C::PLANE));
   static constexpr uint32_t Q = 0, K = Q + 3 * C::PLANE, V = K + KREG, S = C::NP > 1 ? V + NSV * C::PLANE : K;
   static constexpr uint32_t T = C::NP > 1 ? S + 3 * C::SPLANE : K, SEG = C::NP > 1 ? T + 3 * C::TPLANE : V + NSV * C::PLANE;
-  static constexpr uint32_t EM = SEG + 2 * C::RG * C::D * 4, END = EM + C::D * 4;
+  static constexpr uint32_t EM = SEG + 3 * C::RG * C::D * 4, END = EM + C::D * 4;
   static constexpr int BLOCKS = C::NP > 1 ? 1 : sizeof(TI) == 2 ? 3 : 2;
   static_assert(3 * C::L * C::D * 4 <= V, "the walk by token keeps exp(g), k and q over q~ and k~");
 };
@@ -654,14 +669,14 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(co
     load_pairs<C, TI>(q, p.q, at, r0, cp);
     load_pairs<C, TI>(k, p.k, at, r0, cp);
     copy_rows<C, TI>(sm + Lay::V, p.v, at);
-    float2 before, total;
-    if (gate_sums<C>(g, seg, seg + C::RG * C::D, rg, cp, before, total)) {
+    float2 half, start;
+    if (gate_weights<C>(g, seg, rg, cp, half, start)) {
       grid_dep_wait();
       grid_dep_launch();
       fwd_by_token<C, TI>(reinterpret_cast<float*>(sm), Sn, p);
       return;
     }
-    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, before, total, rg, cp);
+    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, nullptr, g, q, k, half, start, rg, cp);
     __syncthreads();
   }
   const int wr = warp % C::WR, wc = warp / C::WR, m0 = 16 * wr;
@@ -734,7 +749,7 @@ struct BwdLay {
   static constexpr uint32_t most(uint32_t a, uint32_t b) { return a > b ? a : b; }
   static constexpr uint32_t SREGION = most(3 * C::SPLANE, 3 * C::TPLANE);      // score tile, state pieces
   static constexpr uint32_t Q = 0, K = Q + 3 * C::PLANE, V = K + 3 * C::PLANE, DO = V + NSV * C::PLANE, S = DO + NSD * C::PLANE;
-  static constexpr uint32_t SEG = S + SREGION, EM = SEG + 2 * C::RG * C::D * 4, DG = EM + C::D * 4, END = DG + C::D * 4;
+  static constexpr uint32_t SEG = S + SREGION, EM = SEG + 3 * C::RG * C::D * 4, ED = EM + C::D * 4, DG = ED + C::D * 4, END = DG + C::D * 4;
   static constexpr int BLOCKS = 232448 / (END + 1024);      // per SM, what shared memory holds (registers must not hold fewer)
   static_assert(C::L * C::AP * 4 <= 3 * C::PLANE, "dq and dk are staged in float32 over q~ and k~");
   static_assert(5 * C::L * C::D * 4 <= SEG, "the walk by token keeps exp(g), k, q, v and dO over the operands");
@@ -761,13 +776,14 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
   extern __shared__ __align__(16) uint8_t sm[];
   float* seg = reinterpret_cast<float*>(sm + Lay::SEG);
   float* em = reinterpret_cast<float*>(sm + Lay::EM);
+  float* ed = reinterpret_cast<float*>(sm + Lay::ED);
   float* dG = reinterpret_cast<float*>(sm + Lay::DG);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
   const ChunkAt<C> at(p, blockIdx.x);
   const float* Sn = p.S + (at.bh * (p.N + 1) + at.n) * D * D;
   const float* dSn = p.dS + (at.bh * (p.N + 1) + at.n + 1) * D * D;
   float4 sx[C::SREG];
-  float2 before, total;
+  float2 start;
   {
     float2 g[C::RPT];
     Pair<TI> q[C::RPT], k[C::RPT];
@@ -776,13 +792,14 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
     load_pairs<C, TI>(k, p.k, at, r0, cp);
     copy_rows<C, TI>(sm + Lay::V, p.v, at);
     copy_rows<C, TY>(sm + Lay::DO, p.dout, at);
-    if (gate_sums<C>(g, seg, seg + C::RG * D, rg, cp, before, total)) {
+    float2 half;
+    if (gate_weights<C>(g, seg, rg, cp, half, start)) {
       grid_dep_wait();
       grid_dep_launch();
       bwd_by_token<C, TI, TY>(reinterpret_cast<float*>(sm), Sn, dSn, p);
       return;
     }
-    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, g, q, k, before, total, rg, cp);
+    build_qk<C, TI>(sm + Lay::Q, sm + Lay::K, em, ed, g, q, k, half, start, rg, cp);
   }
   grid_dep_wait();                        // the gradient states of the scan before this kernel
   grid_dep_launch();
@@ -831,7 +848,7 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
     const int pc = i % C::NP;
     __syncthreads();                          // what the buffer held is consumed
     if (i >= C::NP) dot_piece<C>(dG, sx, Snext, pc);
-    store_piece<C>(sm + Lay::S, sx, em);
+    store_piece<C>(sm + Lay::S, sx, i < C::NP ? em : ed);
     if (i + 1 < 2 * C::NP) fetch_piece<C>(sx, i + 1 < C::NP ? Sn : dSn, (i + 1) % C::NP);
     __syncthreads();
     if (i < C::NP) {
@@ -886,7 +903,7 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
   load_gates<C>(g, p.g, at, r0, cp);
   load_pairs<C, TI>(q, p.q, at, r0, cp);
   load_pairs<C, TI>(k, p.k, at, r0, cp);
-  float2 run = make_float2(expf(before.x - 0.5f * total.x), expf(before.y - 0.5f * total.y));
+  float2 run = start;
   float2 dl[C::RPT];
 #pragma unroll
   for (int i = 0; i < C::RPT; ++i) {

@@ -49,6 +49,16 @@ def test_recurrent_gla_in_chunks_vs_oracle(cuda_device, B, T, H, D, shift, rever
 
 
 @pytest.mark.parametrize("D", [32, 64, 128])
+def test_gates_that_one_thread_holds(cuda_device, D):
+    """Eight consecutive gates just inside and just beyond what the weights of one thread's rows may fall by together."""
+    from gla_jax_b200 import recurrent_gla
+    for total in (79.0, 81.0):
+        case = _case(1, 128, 1, D, torch.float32, 19, 5.0)
+        case[1][0, 16:24, 0] = -total / 8
+        _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"group {D, total}")
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
 def test_chunks_on_both_sides_of_the_gate_limits(cuda_device, D):
     """Three chunks: mild, one feature past the sum limit, one single gate whose exponential vanishes (and an infinite one)."""
     from gla_jax_b200 import chunk_gla, recurrent_gla
@@ -76,7 +86,7 @@ def test_resets_in_every_feature(cuda_device, D, gate, at):
 
 
 @pytest.mark.parametrize("D", [32, 64, 128])
-@pytest.mark.parametrize("shift,gate", [(5.0, None)])
+@pytest.mark.parametrize("shift,gate", [(5.0, None), (0.0, None), (5.0, -30.0), (5.0, -55.0)])
 def test_float32_rounding_and_no_more(cuda_device, D, shift, gate):
     """A weight is a product of up to 64 rounded factors, a sum has up to 12 float32 additions of 16 products each; with a
     mean square of 2^-24 / sqrt(3) per rounding that is (8 + 3.5) 3.4e-8 = 4e-7.  The gate gradient (float32 for bf16
