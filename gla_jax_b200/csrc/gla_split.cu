@@ -269,215 +269,7 @@ __device__ __forceinline__ bool gate_weights(float2 (&g)[C::RPT], float* seg, in
   return __syncthreads_or(big || !(a.x <= PX_LIMIT) || !(a.y <= PX_LIMIT)) != 0;
 }
 
-// ---- per-chunk state products ----------------------------------------------------------------------------------------
-// MODE 0: S slot n + 1 = k^^T V, k^ = k exp(G - lam);  MODE 1: dS slot n = q^^T dO, q^ = q exp(lam).  The weights are
-// anchored at the chunk's ends here and never exceed one for log gates <= 0.  Also leaves exp(G).
-template <class C, typename TI, typename TY, int MODE>
-__global__ void __launch_bounds__(C::NT, sizeof(TI) + sizeof(TY) == 4 ? 1024 / C::NT : 512 / C::NT) px_product_kernel(PxParams p) {
-  constexpr int NSY = planes_of<TY>();
-  extern __shared__ __align__(16) uint8_t sm[];
-  uint8_t* sX = sm;
-  uint8_t* sY = sm + 3 * C::PLANE;
-  float* seg = reinterpret_cast<float*>(sY + NSY * C::PLANE);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
-  const ChunkAt<C> at(p, blockIdx.x);
-  float2 g[C::RPT];
-  Pair<TI> x[C::RPT];
-  grid_dep_wait();
-  grid_dep_launch();
-  load_gates<C>(g, p.g, at, r0, cp);
-  load_pairs<C, TI>(x, MODE == 0 ? p.k : p.q, at, r0, cp);
-  copy_rows<C, TY>(sY, MODE == 0 ? p.v : p.dout, at);
-  float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < C::RPT; ++i) { s.x += g[i].x; s.y += g[i].y; }
-  *reinterpret_cast<float2*>(seg + rg * C::D + 2 * cp) = s;
-  __syncthreads();
-  float2 side = make_float2(0.f, 0.f), total = side;        // gates after (MODE 0) or before (MODE 1) the thread's rows
-#pragma unroll
-  for (int r = 0; r < C::RG; ++r) {
-    const float2 t = *reinterpret_cast<const float2*>(seg + r * C::D + 2 * cp);
-    if (MODE == 0 ? r > rg : r < rg) { side.x += t.x; side.y += t.y; }
-    total.x += t.x; total.y += t.y;
-  }
-  float2 run = make_float2(expf(side.x), expf(side.y));
-  if (rg == 0) *reinterpret_cast<float2*>(p.eG + (at.bh * p.N + at.n) * C::D + 2 * cp) = make_float2(expf(total.x), expf(total.y));
-  if (MODE == 0) {
-#pragma unroll
-    for (int i = C::RPT - 1; i >= 0; --i) {
-      const float2 v = x[i].get();
-      st_split3(sX + (r0 + i) * C::LD + cp * 4, C::PLANE, v.x * run.x, v.y * run.y);
-      run.x *= expf(g[i].x); run.y *= expf(g[i].y);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < C::RPT; ++i) {
-      const float2 v = x[i].get();
-      run.x *= expf(g[i].x); run.y *= expf(g[i].y);
-      st_split3(sX + (r0 + i) * C::LD + cp * 4, C::PLANE, v.x * run.x, v.y * run.y);
-    }
-  }
-  __syncthreads();
-  constexpr int WM = C::D / 16, WN = (C::NT / 32) / WM, NW = C::D / WN;       // warps over key rows, value columns per warp
-  static_assert(WM * WN == C::NT / 32, "warps must tile the state");
-  const int m0 = 16 * (warp % WM), c0 = NW * (warp / WM);
-  float acc[NW / 8][4];
-#pragma unroll
-  for (int j = 0; j < NW / 8; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
-  const uint32_t aX = smem_u32(sX), aY = smem_u32(sY);
-#pragma unroll 2
-  for (int ks = 0; ks < C::L / 16; ++ks) {
-    uint32_t a[3][4];
-    ld_a_t<3>(a, aX, C::PLANE, C::LD, m0, 16 * ks, lane);
-    mma_step<3, NSY, NW / 16, true, (sizeof(TI) + sizeof(TY) > 4)>(acc, a, aY, C::PLANE, C::LD, c0, 16 * ks, lane);
-  }
-  float* o = (MODE == 0 ? p.S : p.dS) + (at.bh * (p.N + 1) + at.n + (MODE == 0 ? 1 : 0)) * C::D * C::D;
-#pragma unroll
-  for (int j = 0; j < NW / 8; ++j)
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      *reinterpret_cast<float2*>(o + (m0 + (lane >> 2) + 8 * h) * C::D + c0 + 8 * j + 2 * (lane & 3)) =
-          make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
-}
-
-// ---- scan over the chunks, in place --------------------------------------------------------------------------------------
-// mode 0: slot 0 = init, slot n + 1 = eG_n slot n + slot n + 1;  mode 1: slot N = init, slot n = eG_n slot n + 1 + slot n.
-// One thread per four value columns; eight chunks' loads in flight (the chain itself is one FMA per chunk).
-template <typename TS>
-__global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, int64_t N, const float* __restrict__ eG,
-                                                      const TS* __restrict__ init, float* S, TS* __restrict__ fin, int mode) {
-  constexpr int AHEAD = 8;
-  const int64_t e4 = (int64_t)blockIdx.x * 128 + threadIdx.x, DD = D * D;
-  if (e4 * 4 >= total) return;
-  const int64_t bh = e4 * 4 / DD, e = e4 * 4 % DD, dk = e / D;
-  float* sp = S + bh * (N + 1) * DD + e;
-  const float* gp = eG + bh * N * D + dk;
-  grid_dep_wait();
-  grid_dep_launch();
-  float4 s;
-  s.x = ld_f(init, bh * DD + e); s.y = ld_f(init, bh * DD + e + 1); s.z = ld_f(init, bh * DD + e + 2); s.w = ld_f(init, bh * DD + e + 3);
-  *reinterpret_cast<float4*>(sp + (mode ? N : 0) * DD) = s;
-  float4 x[AHEAD];
-  float f[AHEAD];
-  auto fetch = [&](int64_t i, int u) {
-    const int64_t n = mode ? N - 1 - i : i;
-    x[u] = *reinterpret_cast<const float4*>(sp + (mode ? n : n + 1) * DD);
-    f[u] = __ldg(gp + n * D);
-  };
-#pragma unroll
-  for (int u = 0; u < AHEAD; ++u) if (u < N) fetch(u, u);
-  for (int64_t i0 = 0; i0 < N; i0 += AHEAD) {
-#pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      const int64_t i = i0 + u;
-      if (i < N) {
-        const int64_t n = mode ? N - 1 - i : i;
-        s = make_float4(fmaf(f[u], s.x, x[u].x), fmaf(f[u], s.y, x[u].y), fmaf(f[u], s.z, x[u].z), fmaf(f[u], s.w, x[u].w));
-        *reinterpret_cast<float4*>(sp + (mode ? n : n + 1) * DD) = s;
-        if (i + AHEAD < N) fetch(i + AHEAD, u);
-      }
-    }
-  }
-  if (fin != nullptr) {
-    st_f(fin, bh * DD + e, s.x); st_f(fin, bh * DD + e + 1, s.y); st_f(fin, bh * DD + e + 2, s.z); st_f(fin, bh * DD + e + 3, s.w);
-  }
-}
-
-// ---- pieces of the chunk kernels -------------------------------------------------------------------------------------------
-// q~ and k~ as split planes; em[d] = e^m, which the rows of S take, and ed[d] = exp(G - m), from the same products as the
-// weights, which those of dS take.
-template <class C, typename TI>
-__device__ __forceinline__ void build_qk(uint8_t* sQ, uint8_t* sK, float* em, float* ed, const float2 (&f)[C::RPT], const Pair<TI> (&q)[C::RPT],
-                                         const Pair<TI> (&k)[C::RPT], float2 half, float2 start, int rg, int cp) {
-  const int r0 = rg * C::RPT;
-  if (rg == 0) *reinterpret_cast<float2*>(em + 2 * cp) = make_float2(expf(half.x), expf(half.y));
-  float2 run = start;
-#pragma unroll
-  for (int i = 0; i < C::RPT; ++i) {
-    run.x *= f[i].x; run.y *= f[i].y;
-    const float2 x = q[i].get();
-    st_split3(sQ + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
-  }
-  if (ed != nullptr && rg == C::RG - 1) *reinterpret_cast<float2*>(ed + 2 * cp) = run;
-  run = make_float2(1.f / run.x, 1.f / run.y);
-#pragma unroll
-  for (int i = C::RPT - 1; i >= 0; --i) {
-    const float2 x = k[i].get();
-    st_split3(sK + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
-    run.x *= f[i].x; run.y *= f[i].y;
-  }
-}
-// Value columns [PW pc, PW pc + PW) of a state (float32, D x D), rows scaled by em, as split planes.
-template <class C>
-__device__ __forceinline__ void fetch_piece(float4 (&x)[C::SREG], const float* st, int pc) {
-#pragma unroll
-  for (int j = 0; j < C::SREG; ++j) {
-    const int id = threadIdx.x + C::NT * j, r = id / (C::PW / 4), c = id % (C::PW / 4);
-    x[j] = *reinterpret_cast<const float4*>(st + r * C::D + pc * C::PW + c * 4);
-  }
-}
-template <class C>
-__device__ __forceinline__ void store_piece(uint8_t* dst, const float4 (&x)[C::SREG], const float* em) {
-#pragma unroll
-  for (int j = 0; j < C::SREG; ++j) {
-    const int id = threadIdx.x + C::NT * j, r = id / (C::PW / 4), c = id % (C::PW / 4);
-    const float w = em[r];
-    st_split3(dst + r * C::LDS + c * 8, C::SPLANE, make_float4(x[j].x * w, x[j].y * w, x[j].z * w, x[j].w * w));
-  }
-}
-// The warp's score blocks (row block wr, column blocks wc, wc + WC, ... up to the diagonal): A B^T over D.
-template <class C, int NSA, int NSB, bool EX>
-__device__ __forceinline__ void score_blocks(float (&x)[C::NB][2][4], uint32_t aA, uint32_t aB, int wr, int wc, int lane) {
-#pragma unroll
-  for (int i = 0; i < C::NB; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) x[i][j][e] = 0.f;
-  if (wc <= wr) {
-#pragma unroll 2
-    for (int ks = 0; ks < C::D / 16; ++ks) {
-      uint32_t a[NSA][4];
-      ld_a<NSA>(a, aA, C::PLANE, C::LD, 16 * wr, 16 * ks, lane);
-#pragma unroll
-      for (int i = 0; i < C::NB; ++i)
-        if (wc + C::WC * i <= wr) mma_step<NSA, NSB, 1, false, EX>(x[i], a, aB, C::PLANE, C::LD, 16 * (wc + C::WC * i), 16 * ks, lane);
-    }
-  }
-}
-// ... as split planes of the score tile [i][j], entries above the diagonal zero
-template <class C>
-__device__ __forceinline__ void store_scores(uint8_t* t, const float (&x)[C::NB][2][4], int wr, int wc, int lane) {
-#pragma unroll
-  for (int i = 0; i < C::NB; ++i) {
-    const int cb = wc + C::WC * i;
-    if (cb <= wr) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = 16 * wr + (lane >> 2) + 8 * h, c = 16 * cb + 8 * j + 2 * (lane & 3);
-          st_split3(t + r * C::LDT + c * 2, C::TPLANE, c <= r ? x[i][j][2 * h] : 0.f, c + 1 <= r ? x[i][j][2 * h + 1] : 0.f);
-        }
-    }
-  }
-}
-template <typename TI>
-__device__ __forceinline__ void st_pair(void* p, int64_t e, float x, float y) {
-  if constexpr (sizeof(TI) == 2) *reinterpret_cast<uint32_t*>((bf16*)p + e) = pack_bf16x2(x, y);
-  else *reinterpret_cast<float2*>((float*)p + e) = make_float2(x, y);
-}
-template <int N>
-__device__ __forceinline__ void zero_acc(float (&c)[N][4]) {
-#pragma unroll
-  for (int j = 0; j < N; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
-}
-
-// ---- a sharp chunk, token by token ---------------------------------------------------------------------------------------
+// ---- a chunk token by token -----------------------------------------------------------------------------------------------
 // The recurrence itself, from the state that enters the chunk: every weight is a product of exp(g), so that a gate that
 // resets the state costs the later tokens nothing.  (Weights exp(lam_i - lam_j) from running sums, which stood here
 // before, lost what the sums had grown to: 4e-5 of out after one gate of -1e4, 1.1e-4 after eight, against 2e-7.)
@@ -488,6 +280,18 @@ __device__ __forceinline__ void zero_acc(float (&c)[N][4]) {
 //   REV = false: state = f state + w scalar, then the sum;   REV = true: state += w scalar, then the sum, then state *= f
 // Measured, bf16 4 x 2048 tokens, 6 heads, every chunk sharp, forward and with the backward: head size 128 1288, 3322 us
 // (pair by pair) -> 333, 1063; head size 64 579, 1567 -> 110, 375 (mild chunks: 126, 389 and 44, 150).
+// It also serves a chunk in which the tensor cores leave something that is not finite.  Their products meet the zeros
+// above the diagonal, so a not-a-number or an infinity reached up to 15 earlier tokens, an infinity became
+// not-a-number in the split, and a weighted q or k beyond 1e38 overflowed: the recurrence does none of that.
+// What they leave shows every case (0 x inf and inf - inf included), so nothing but the sums needs looking at.
+template <int N>
+__device__ __forceinline__ float not_finite(const float (&c)[N][4], float z) {       // 0 as long as everything is finite
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) z = fmaf(c[j][e], 0.f, z);
+  return z;
+}
 template <int VW> __device__ __forceinline__ void ld_vec(float (&x)[VW], const float* p) {
   if constexpr (VW == 2) { const float2 v = *reinterpret_cast<const float2*>(p); x[0] = v.x; x[1] = v.y; }
   else { const float4 v = *reinterpret_cast<const float4*>(p); x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
@@ -636,6 +440,258 @@ __device__ __noinline__ void bwd_by_token(float* f, const float* Sn, const float
   walk<C, true, true>(m, f, q, k, at.nv, own, part, from(dout), [&](int t, int c, float o) { st_f((TI*)p.dv, at.row(t) + c, o); });
 }
 
+// MODE 0: S = f S + k v;  MODE 1, backwards: dS = f (dS + q dO); both from zero
+template <class C, typename TI, typename TY, int MODE>
+__device__ __noinline__ void product_by_token(float* f, float* st, const PxParams& p) {
+  constexpr int VW = C::TE < 4 ? C::TE : 4;
+  const ChunkAt<C> at(p, blockIdx.x);
+  float* x = f + C::L * C::D;
+  stage<C, float, true>(f, p.g, at);
+  stage<C, TI>(x, MODE == 0 ? p.k : p.q, at);
+  __syncthreads();
+  const int own = threadIdx.x / C::TP * 4, part = threadIdx.x % C::TP;
+  float m[4][C::TE] = {};
+#pragma unroll 1
+  for (int i = 0; i < at.nv; ++i) {
+    const int t = MODE == 0 ? i : at.nv - 1 - i;
+    Pair<TY> a, b;
+    a.load(MODE == 0 ? p.v : p.dout, at.row(t) + own);
+    b.load(MODE == 0 ? p.v : p.dout, at.row(t) + own + 2);
+    const float s[4] = {a.get().x, a.get().y, b.get().x, b.get().y};
+#pragma unroll
+    for (int j = 0; j < C::TE / VW; ++j) {
+      float fe[VW], xe[VW];
+      ld_vec<VW>(fe, f + t * C::D + VW * (part + C::TP * j));
+      ld_vec<VW>(xe, x + t * C::D + VW * (part + C::TP * j));
+#pragma unroll
+      for (int u = 0; u < VW; ++u)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          float& y = m[r][VW * j + u];
+          y = MODE == 0 ? fmaf(fe[u], y, xe[u] * s[r]) : fe[u] * fmaf(xe[u], s[r], y);
+        }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < C::TE / VW; ++j)
+#pragma unroll
+    for (int u = 0; u < VW; ++u)
+      *reinterpret_cast<float4*>(st + (VW * (part + C::TP * j) + u) * C::D + own) =
+          make_float4(m[0][VW * j + u], m[1][VW * j + u], m[2][VW * j + u], m[3][VW * j + u]);
+}
+
+// ---- per-chunk state products ----------------------------------------------------------------------------------------
+// MODE 0: S slot n + 1 = k^^T V, k^ = k exp(G - lam);  MODE 1: dS slot n = q^^T dO, q^ = q exp(lam).  The weights are
+// anchored at the chunk's ends here and never exceed one for log gates <= 0.  Also leaves exp(G).
+template <class C, typename TI, typename TY, int MODE>
+__global__ void __launch_bounds__(C::NT, sizeof(TI) + sizeof(TY) == 4 && C::L == 64 ? 1024 / C::NT : 512 / C::NT) px_product_kernel(const __grid_constant__ PxParams p) {
+  constexpr int NSY = planes_of<TY>();
+  extern __shared__ __align__(16) uint8_t sm[];
+  uint8_t* sX = sm;
+  uint8_t* sY = sm + 3 * C::PLANE;
+  float* seg = reinterpret_cast<float*>(sY + NSY * C::PLANE);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
+  const ChunkAt<C> at(p, blockIdx.x);
+  float2 g[C::RPT];
+  Pair<TI> x[C::RPT];
+  grid_dep_wait();
+  grid_dep_launch();
+  load_gates<C>(g, p.g, at, r0, cp);
+  load_pairs<C, TI>(x, MODE == 0 ? p.k : p.q, at, r0, cp);
+  copy_rows<C, TY>(sY, MODE == 0 ? p.v : p.dout, at);
+  float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i) { s.x += g[i].x; s.y += g[i].y; }
+  *reinterpret_cast<float2*>(seg + rg * C::D + 2 * cp) = s;
+  __syncthreads();
+  float2 side = make_float2(0.f, 0.f), total = side;        // gates after (MODE 0) or before (MODE 1) the thread's rows
+#pragma unroll
+  for (int r = 0; r < C::RG; ++r) {
+    const float2 t = *reinterpret_cast<const float2*>(seg + r * C::D + 2 * cp);
+    if (MODE == 0 ? r > rg : r < rg) { side.x += t.x; side.y += t.y; }
+    total.x += t.x; total.y += t.y;
+  }
+  float2 run = make_float2(expf(side.x), expf(side.y));
+  if (rg == 0) *reinterpret_cast<float2*>(p.eG + (at.bh * p.N + at.n) * C::D + 2 * cp) = make_float2(expf(total.x), expf(total.y));
+  if (MODE == 0) {
+#pragma unroll
+    for (int i = C::RPT - 1; i >= 0; --i) {
+      const float2 v = x[i].get();
+      st_split3(sX + (r0 + i) * C::LD + cp * 4, C::PLANE, v.x * run.x, v.y * run.y);
+      run.x *= expf(g[i].x); run.y *= expf(g[i].y);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < C::RPT; ++i) {
+      const float2 v = x[i].get();
+      run.x *= expf(g[i].x); run.y *= expf(g[i].y);
+      st_split3(sX + (r0 + i) * C::LD + cp * 4, C::PLANE, v.x * run.x, v.y * run.y);
+    }
+  }
+  __syncthreads();
+  constexpr int WM = C::D / 16, WN = (C::NT / 32) / WM, NW = C::D / WN;       // warps over key rows, value columns per warp
+  static_assert(WM * WN == C::NT / 32, "warps must tile the state");
+  const int m0 = 16 * (warp % WM), c0 = NW * (warp / WM);
+  float acc[NW / 8][4];
+#pragma unroll
+  for (int j = 0; j < NW / 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+  const uint32_t aX = smem_u32(sX), aY = smem_u32(sY);
+#pragma unroll 2
+  for (int ks = 0; ks < C::L / 16; ++ks) {
+    uint32_t a[3][4];
+    ld_a_t<3>(a, aX, C::PLANE, C::LD, m0, 16 * ks, lane);
+    mma_step<3, NSY, NW / 16, true, (sizeof(TI) + sizeof(TY) > 4)>(acc, a, aY, C::PLANE, C::LD, c0, 16 * ks, lane);
+  }
+  float* o = (MODE == 0 ? p.S : p.dS) + (at.bh * (p.N + 1) + at.n + (MODE == 0 ? 1 : 0)) * C::D * C::D;
+#pragma unroll
+  for (int j = 0; j < NW / 8; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      *reinterpret_cast<float2*>(o + (m0 + (lane >> 2) + 8 * h) * C::D + c0 + 8 * j + 2 * (lane & 3)) =
+          make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
+  if (__syncthreads_or(!(not_finite(acc, 0.f) == 0.f))) {
+    static_assert(2 * C::L * C::D * 4 <= (3 + NSY) * C::PLANE, "the walk by token keeps exp(g) and k or q over the operands");
+    product_by_token<C, TI, TY, MODE>(reinterpret_cast<float*>(sm), o, p);
+  }
+}
+
+// ---- scan over the chunks, in place --------------------------------------------------------------------------------------
+// mode 0: slot 0 = init, slot n + 1 = eG_n slot n + slot n + 1;  mode 1: slot N = init, slot n = eG_n slot n + 1 + slot n.
+// One thread per four value columns; eight chunks' loads in flight (the chain itself is one FMA per chunk).
+template <typename TS>
+__global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, int64_t N, const float* __restrict__ eG,
+                                                      const TS* __restrict__ init, float* S, TS* __restrict__ fin, int mode) {
+  constexpr int AHEAD = 8;
+  const int64_t e4 = (int64_t)blockIdx.x * 128 + threadIdx.x, DD = D * D;
+  if (e4 * 4 >= total) return;
+  const int64_t bh = e4 * 4 / DD, e = e4 * 4 % DD, dk = e / D;
+  float* sp = S + bh * (N + 1) * DD + e;
+  const float* gp = eG + bh * N * D + dk;
+  grid_dep_wait();
+  grid_dep_launch();
+  float4 s;
+  s.x = ld_f(init, bh * DD + e); s.y = ld_f(init, bh * DD + e + 1); s.z = ld_f(init, bh * DD + e + 2); s.w = ld_f(init, bh * DD + e + 3);
+  *reinterpret_cast<float4*>(sp + (mode ? N : 0) * DD) = s;
+  float4 x[AHEAD];
+  float f[AHEAD];
+  auto fetch = [&](int64_t i, int u) {
+    const int64_t n = mode ? N - 1 - i : i;
+    x[u] = *reinterpret_cast<const float4*>(sp + (mode ? n : n + 1) * DD);
+    f[u] = __ldg(gp + n * D);
+  };
+#pragma unroll
+  for (int u = 0; u < AHEAD; ++u) if (u < N) fetch(u, u);
+  for (int64_t i0 = 0; i0 < N; i0 += AHEAD) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int64_t i = i0 + u;
+      if (i < N) {
+        const int64_t n = mode ? N - 1 - i : i;
+        s = make_float4(fmaf(f[u], s.x, x[u].x), fmaf(f[u], s.y, x[u].y), fmaf(f[u], s.z, x[u].z), fmaf(f[u], s.w, x[u].w));
+        *reinterpret_cast<float4*>(sp + (mode ? n : n + 1) * DD) = s;
+        if (i + AHEAD < N) fetch(i + AHEAD, u);
+      }
+    }
+  }
+  if (fin != nullptr) {
+    st_f(fin, bh * DD + e, s.x); st_f(fin, bh * DD + e + 1, s.y); st_f(fin, bh * DD + e + 2, s.z); st_f(fin, bh * DD + e + 3, s.w);
+  }
+}
+
+// ---- pieces of the chunk kernels -------------------------------------------------------------------------------------------
+// q~ and k~ as split planes; em[d] = e^m, which the rows of S take, and ed[d] = exp(G - m), from the same products as the
+// weights, which those of dS take.
+template <class C, typename TI>
+__device__ __forceinline__ void build_qk(uint8_t* sQ, uint8_t* sK, float* em, float* ed, const float2 (&f)[C::RPT], const Pair<TI> (&q)[C::RPT],
+                                         const Pair<TI> (&k)[C::RPT], float2 half, float2 start, int rg, int cp) {
+  const int r0 = rg * C::RPT;
+  if (rg == 0) *reinterpret_cast<float2*>(em + 2 * cp) = make_float2(expf(half.x), expf(half.y));
+  float2 run = start;
+#pragma unroll
+  for (int i = 0; i < C::RPT; ++i) {
+    run.x *= f[i].x; run.y *= f[i].y;
+    const float2 x = q[i].get();
+    st_split3(sQ + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
+  }
+  if (ed != nullptr && rg == C::RG - 1) *reinterpret_cast<float2*>(ed + 2 * cp) = run;
+  run = make_float2(1.f / run.x, 1.f / run.y);
+#pragma unroll
+  for (int i = C::RPT - 1; i >= 0; --i) {
+    const float2 x = k[i].get();
+    st_split3(sK + (r0 + i) * C::LD + cp * 4, C::PLANE, x.x * run.x, x.y * run.y);
+    run.x *= f[i].x; run.y *= f[i].y;
+  }
+}
+// Value columns [PW pc, PW pc + PW) of a state (float32, D x D), rows scaled by em, as split planes.
+template <class C>
+__device__ __forceinline__ void fetch_piece(float4 (&x)[C::SREG], const float* st, int pc) {
+#pragma unroll
+  for (int j = 0; j < C::SREG; ++j) {
+    const int id = threadIdx.x + C::NT * j, r = id / (C::PW / 4), c = id % (C::PW / 4);
+    x[j] = *reinterpret_cast<const float4*>(st + r * C::D + pc * C::PW + c * 4);
+  }
+}
+template <class C>
+__device__ __forceinline__ void store_piece(uint8_t* dst, const float4 (&x)[C::SREG], const float* em) {
+#pragma unroll
+  for (int j = 0; j < C::SREG; ++j) {
+    const int id = threadIdx.x + C::NT * j, r = id / (C::PW / 4), c = id % (C::PW / 4);
+    const float w = em[r];
+    st_split3(dst + r * C::LDS + c * 8, C::SPLANE, make_float4(x[j].x * w, x[j].y * w, x[j].z * w, x[j].w * w));
+  }
+}
+// The warp's score blocks (row block wr, column blocks wc, wc + WC, ... up to the diagonal): A B^T over D.
+template <class C, int NSA, int NSB, bool EX>
+__device__ __forceinline__ void score_blocks(float (&x)[C::NB][2][4], uint32_t aA, uint32_t aB, int wr, int wc, int lane) {
+#pragma unroll
+  for (int i = 0; i < C::NB; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][j][e] = 0.f;
+  if (wc <= wr) {
+#pragma unroll 2
+    for (int ks = 0; ks < C::D / 16; ++ks) {
+      uint32_t a[NSA][4];
+      ld_a<NSA>(a, aA, C::PLANE, C::LD, 16 * wr, 16 * ks, lane);
+#pragma unroll
+      for (int i = 0; i < C::NB; ++i)
+        if (wc + C::WC * i <= wr) mma_step<NSA, NSB, 1, false, EX>(x[i], a, aB, C::PLANE, C::LD, 16 * (wc + C::WC * i), 16 * ks, lane);
+    }
+  }
+}
+// ... as split planes of the score tile [i][j], entries above the diagonal zero
+template <class C>
+__device__ __forceinline__ void store_scores(uint8_t* t, const float (&x)[C::NB][2][4], int wr, int wc, int lane) {
+#pragma unroll
+  for (int i = 0; i < C::NB; ++i) {
+    const int cb = wc + C::WC * i;
+    if (cb <= wr) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 16 * wr + (lane >> 2) + 8 * h, c = 16 * cb + 8 * j + 2 * (lane & 3);
+          st_split3(t + r * C::LDT + c * 2, C::TPLANE, c <= r ? x[i][j][2 * h] : 0.f, c + 1 <= r ? x[i][j][2 * h + 1] : 0.f);
+        }
+    }
+  }
+}
+template <typename TI>
+__device__ __forceinline__ void st_pair(void* p, int64_t e, float x, float y) {
+  if constexpr (sizeof(TI) == 2) *reinterpret_cast<uint32_t*>((bf16*)p + e) = pack_bf16x2(x, y);
+  else *reinterpret_cast<float2*>((float*)p + e) = make_float2(x, y);
+}
+template <int N>
+__device__ __forceinline__ void zero_acc(float (&c)[N][4]) {
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
+}
+
 // ---- forward chunk kernel ---------------------------------------------------------------------------------------------
 template <class C, typename TI>
 struct FwdLay {
@@ -737,6 +793,10 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(co
         }
     }
   }
+  float z = 0.f;
+#pragma unroll
+  for (int pc = 0; pc < C::NP; ++pc) z = not_finite(o[pc], z);
+  if (__syncthreads_or(!(z == 0.f))) fwd_by_token<C, TI>(reinterpret_cast<float*>(sm), Sn, p);      // writes all of it again
 }
 
 // ---- backward chunk kernel --------------------------------------------------------------------------------------------
@@ -884,7 +944,13 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
         for (int j = 0; j < C::PC / 8; ++j) st_pair<TI>(p.dv, e + pc * C::PW + 8 * j, dv[pc][j][2 * h], dv[pc][j][2 * h + 1]);
     }
   }
-  __syncthreads();                                        // every operand but V and dO is dead
+  float z = not_finite(dk, not_finite(dq, 0.f));
+#pragma unroll
+  for (int pc = 0; pc < C::NP; ++pc) z = not_finite(dv[pc], z);
+  if (__syncthreads_or(!(z == 0.f))) {                    // (every operand is dead)
+    bwd_by_token<C, TI, TY>(reinterpret_cast<float*>(sm), Sn, dSn, p);
+    return;
+  }
   float* tq = reinterpret_cast<float*>(sm + Lay::Q);
   float* tk = reinterpret_cast<float*>(sm + Lay::K);
 #pragma unroll

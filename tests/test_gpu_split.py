@@ -104,6 +104,43 @@ def test_float32_rounding_and_no_more(cuda_device, D, shift, gate):
     assert O.rel_l2(_oracle(*half)[2][i], _run_gpu(recurrent_gla, cuda_device, *half)[2][i]) < 1.2e-6
 
 
+def _same_where_finite(ref, got, tol, what):
+    """Not finite in the same places as the recurrence, and equal elsewhere (an infinity may be either kind)."""
+    ok = torch.isfinite(ref)
+    assert torch.equal(ok, torch.isfinite(got)), what
+    zero = torch.zeros((), dtype=torch.float64)
+    assert O.rel_l2(torch.where(ok, ref.double(), zero), torch.where(ok, got.double(), zero)) < tol, what
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("which,bad,t", [("v", float("nan"), 27), ("v", float("inf"), 75), ("k", float("nan"), 90),
+                                         ("k", -float("inf"), 5), ("q", float("nan"), 70), ("do", float("inf"), 45)])
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_what_is_not_finite_stays_where_the_recurrence_has_it(cuda_device, D, which, bad, t, dtype):
+    """One bad value in a token: earlier tokens (later ones for gradients that run backwards) do not see it."""
+    from gla_jax_b200 import recurrent_gla
+    case = list(_case(1, 150, 2, D, dtype, 21, 5.0))
+    case[{"v": 2, "k": 3, "q": 4, "do": 6}[which]][0, t, 1, 7] = bad
+    leaves = [x.to(cuda_device).requires_grad_(True) for x in case[:5]]
+    hf, out = recurrent_gla(*leaves)
+    grads = torch.autograd.grad([hf, out], leaves, [x.to(cuda_device) for x in case[5:]])
+    ref = _oracle(*case)
+    tol = 5e-6 if dtype == torch.float32 else 1e-2
+    for name, a, b in zip(("hidden_final", "out", *NAMES), (ref[0], ref[1], *ref[2]), (hf, out, *grads)):
+        if name != "dlog_fgate":        # (a sum over later tokens here, a product per token in the oracle)
+            _same_where_finite(a, b.detach().cpu(), tol, name)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_large_values_under_strong_decay(cuda_device, D):
+    """Keys whose weighted values exceed float32 although no state or output does."""
+    from gla_jax_b200 import recurrent_gla
+    case = list(_case(1, 128, 1, D, torch.float32, 23, 5.0))
+    case[1][:] = -2.1
+    case[3] = case[3] * 1e12
+    _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"large keys {D}", shift=-2.0)
+
+
 def test_naive_with_bf16_inputs_and_float32_cotangent(cuda_device):
     """bf16 operands with a float32 output and output gradient (recurrent_gla_naive), head size 128: shorter chunks."""
     from gla_jax_b200 import recurrent_gla_naive
