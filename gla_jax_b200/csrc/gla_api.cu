@@ -178,9 +178,8 @@ int gla_recurrent_fwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, 
 }
 
 size_t gla_recurrent_fwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int dtype) {
-  (void)dtype;
   if (B <= 0 || T <= 0 || H <= 0 || D <= 0) return 0;
-  return recurrent_fwd_ws_bytes(B, T, H, D);
+  return recurrent_fwd_ws_bytes(B, T, H, D, dtype == GLA_BF16);
 }
 
 int gla_recurrent_fwd_ws(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int dtype, const void* hidden_init,
@@ -293,19 +292,19 @@ size_t gla_chunk_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t
   if (check_chunk_dims(B, T, H, D, chunk, dtype) != GLA_OK) return 0;
   int r = resolve_impl(impl, D, chunk, dtype);
   if (r < 0) return 0;
-  return r == GLA_IMPL_TCGEN05 ? tc_saved_bytes(B, T, H, D, chunk) : simt_saved_bytes(B, T, H, D, chunk);
+  return r == GLA_IMPL_TCGEN05 ? tc_saved_bytes(B, T, H, D, chunk) : simt_saved_bytes(B, T, H, D, chunk, dtype);
 }
 size_t gla_chunk_fwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int impl) {
   if (check_chunk_dims(B, T, H, D, chunk, dtype) != GLA_OK) return 0;
   int r = resolve_impl(impl, D, chunk, dtype);
   if (r < 0) return 0;
-  return r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk);
+  return r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk, dtype);
 }
 size_t gla_chunk_bwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int impl) {
   if (check_chunk_dims(B, T, H, D, chunk, dtype) != GLA_OK) return 0;
   int r = resolve_impl(impl, D, chunk, dtype);
   if (r < 0) return 0;
-  return r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk);
+  return r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk, dtype);
 }
 
 int gla_chunk_fwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int impl,
@@ -316,7 +315,7 @@ int gla_chunk_fwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int6
   GLA_TRY(check_chunk_dims(B, T, H, D, chunk, dtype));
   int r = resolve_impl(impl, D, chunk, dtype);
   if (r < 0) return -r;
-  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk);
+  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk, dtype);
   if (!workspace || workspace_bytes < need) return GLA_ERR_WORKSPACE;
   const void* ptrs[] = {hidden_init, log_fgate, value, key, query, hidden_final, out, saved, workspace};
   for (const void* p : ptrs)
@@ -340,7 +339,7 @@ int gla_chunk_bwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int6
   GLA_TRY(check_chunk_dims(B, T, H, D, chunk, dtype));
   int r = resolve_impl(impl, D, chunk, dtype);
   if (r < 0) return -r;
-  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk);
+  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk, dtype);
   if (!workspace || workspace_bytes < need) return GLA_ERR_WORKSPACE;
   const void* ptrs[] = {log_fgate, value, key, query, saved, dhidden_final, dout, dhidden_init, dlog_fgate,
                         dvalue, dkey, dquery, workspace};
@@ -470,7 +469,7 @@ int gla_chunk_local_state(void* stream, int64_t B, int64_t T, int64_t H, int64_t
     if (impl == GLA_IMPL_TCGEN05) return GLA_ERR_UNSUPPORTED;
     r = GLA_IMPL_FP32_SIMT;
   }
-  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk);
+  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk, dtype);
   if (!workspace || workspace_bytes < need) return GLA_ERR_WORKSPACE;
   if (r == GLA_IMPL_TCGEN05)
     return tc_chunk_fwd((cudaStream_t)stream, B, T, H, D, chunk, nullptr, log_fgate, value, key, nullptr, nullptr,
@@ -490,7 +489,7 @@ int gla_chunk_local_dstate(void* stream, int64_t B, int64_t T, int64_t H, int64_
     if (impl == GLA_IMPL_TCGEN05) return GLA_ERR_UNSUPPORTED;
     r = GLA_IMPL_FP32_SIMT;
   }
-  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk);
+  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk, dtype);
   if (!workspace || workspace_bytes < need) return GLA_ERR_WORKSPACE;
   if (r == GLA_IMPL_TCGEN05)
     return tc_local_dstate((cudaStream_t)stream, B, T, H, log_fgate, query, dout, dS_local, workspace);

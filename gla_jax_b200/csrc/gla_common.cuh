@@ -117,9 +117,9 @@ int layer_headnorm_gate_bwd(cudaStream_t st, int64_t rows, int64_t D, int bf, co
                             void* ws);
 
 // fp32 CUDA-core chunk path.
-size_t simt_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C);
-size_t simt_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C);
-size_t simt_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C);
+size_t simt_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int dtype);
+size_t simt_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int dtype);
+size_t simt_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int dtype);
 int simt_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int bf,
                    const void* hidden_init, const float* g, const void* v, const void* k, const void* q,
                    void* hidden_final, void* out, void* saved, void* ws, int state_only,
@@ -134,9 +134,9 @@ int simt_chunk_dstate_only(cudaStream_t st, int64_t B, int64_t T, int64_t H, int
 
 // float32-precision chunk path on the tensor cores (head sizes 32, 64, 128; any number of tokens), gla_split.cu.
 bool px_supported(int64_t D);
-size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D);
+size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf, int final_state);
 int px_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
-           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int reverse, const char* label = "px_fwd_kernel");
+           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int final_state, int reverse, const char* label = "px_fwd_kernel");
 int px_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
            const void* v, const void* k, const void* q, const void* dhidden_final, const void* dout, int do_bf,
            void* dhidden_init, float* dg, void* dv, void* dk, void* dq, void* states, int have_states, void* ws, int reverse);
@@ -191,7 +191,7 @@ int launch_sp_combine(cudaStream_t st, int64_t R, int64_t rank, int64_t BH, int6
 int launch_sp_combine2(cudaStream_t st, int64_t R, int64_t rank, int64_t BH, int64_t D, const float* all_G, int64_t gstride,
                        const float* all_S, int64_t sstride, const void* init, int init_bf16, float* entering, void* total,
                        int total_bf16, int reverse);
-size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D);
+size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf);
 int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, void* hidden_final, void* out,
                   int out_bf, int reverse, void* ws = nullptr, size_t ws_bytes = 0);

@@ -455,15 +455,15 @@ static bool rec_aligned(std::initializer_list<const void*> ps) {
   for (const void* p : ps) if (!aligned16(p)) return false;
   return true;
 }
-size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
-  return rec_chunked(T, D) ? px_state_bytes(B, T, H, D) : 0;
+size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf) {
+  return rec_chunked(T, D) ? px_state_bytes(B, T, H, D, bf, 0) : 0;
 }
 
 int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, void* hidden_final, void* out,
                   int out_bf, int reverse, void* ws, size_t ws_bytes) {
-  if (ws != nullptr && rec_chunked(T, D) && ws_bytes >= px_state_bytes(B, T, H, D) && rec_aligned({hidden_init, g, v, k, q, hidden_final, out, ws}))
-    return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, out_bf, ws, reverse);
+  if (ws != nullptr && rec_chunked(T, D) && ws_bytes >= px_state_bytes(B, T, H, D, bf, 0) && rec_aligned({hidden_init, g, v, k, q, hidden_final, out, ws}))
+    return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, out_bf, ws, 0, reverse);
   RecParams p{};
   p.B = B; p.T = T; p.H = H; p.bf = bf; p.out_bf = out_bf;
   p.hidden_init = hidden_init; p.g = g; p.v = v; p.k = k; p.q = q;
@@ -473,7 +473,7 @@ int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, i
 
 size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
   const size_t n = 2 * align_up((size_t)B * T * H * D * 4, 256) + align_up((size_t)B * H * D * 4, 256);
-  const size_t px = rec_chunked(T, D) ? 2 * px_state_bytes(B, T, H, D) : 0;      // states and gradient states
+  const size_t px = rec_chunked(T, D) ? px_state_bytes(B, T, H, D, 0, 1) + px_state_bytes(B, T, H, D, 0, 0) : 0;      // states and gradient states
   return px > n ? px : n;
 }
 
@@ -483,7 +483,7 @@ int recurrent_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, i
                   int reverse, void* ws) {
   if (rec_chunked(T, D) && rec_aligned({hidden_init, g, v, k, q, dhidden_final, dout, dhidden_init, dg, dv, dk, dq, ws}))
     return px_bwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, dhidden_final, dout, do_bf, dhidden_init, dg, dv, dk, dq, ws, 0,
-                  (char*)ws + px_state_bytes(B, T, H, D), reverse);
+                  (char*)ws + px_state_bytes(B, T, H, D, bf && do_bf, 1), reverse);
   RecParams p{};
   p.B = B; p.T = T; p.H = H; p.bf = bf; p.do_bf = do_bf;
   p.hidden_init = hidden_init; p.g = g; p.v = v; p.k = k; p.q = q;

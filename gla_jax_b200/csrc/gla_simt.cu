@@ -279,24 +279,25 @@ __global__ void __launch_bounds__(256) gsum_kernel(int64_t BH, int64_t N, int64_
 // ---------------------------------------------------------------------------------------
 static size_t f32b(int64_t n) { return align_up((size_t)n * 4, 256); }
 
-size_t simt_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C) {
-  if (px_supported(D)) return px_state_bytes(B, T, H, D);
+size_t simt_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int dtype) {
+  if (px_supported(D)) return px_state_bytes(B, T, H, D, dtype == GLA_BF16, 1);
   int64_t N = T / C, BH = B * H;
   return f32b(BH * N * D * D) + f32b(BH * N * D) + f32b(BH * N * C * C);
 }
 // The k_hat region doubles as the score buffer of a forward without residuals: (BH, N, C, C) floats, which is
 // larger than (B, T, H, D) when chunk > D, so the region is sized for the larger of the two.
 static int64_t khat_region_elems(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C) { return B * T * H * (D > C ? D : C); }
-size_t simt_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C) {
+// (gla_chunk_local_state and gla_chunk_local_dstate run the kernels here at every head size)
+size_t simt_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int dtype) {
   int64_t N = T / C, BH = B * H, E = B * T * H * D;
   const size_t n = 2 * f32b(E) + f32b(khat_region_elems(B, T, H, D, C)) + f32b(BH * N * D * D) + f32b(BH * N * D);
-  const size_t px = px_supported(D) ? px_state_bytes(B, T, H, D) : 0;
+  const size_t px = px_supported(D) ? px_state_bytes(B, T, H, D, dtype == GLA_BF16, 0) : 0;
   return px > n ? px : n;
 }
-size_t simt_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C) {
+size_t simt_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t C, int dtype) {
   int64_t N = T / C, BH = B * H, E = B * T * H * D;
   const size_t n = 5 * f32b(E) + f32b(BH * N * D * D) + f32b(BH * N * C * C) + f32b(BH * N * D);
-  const size_t px = px_supported(D) ? px_state_bytes(B, T, H, D) : 0;
+  const size_t px = px_supported(D) ? px_state_bytes(B, T, H, D, dtype == GLA_BF16, 0) : 0;
   return px > n ? px : n;
 }
 
@@ -308,7 +309,7 @@ int simt_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, 
   const int64_t N = d.N, BH = B * H, E = B * T * H * D;
   if (px_supported(D) && !state_only)
     // (launch profiles know the kernel of this family that forms the scores by one name)
-    return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, bf, saved ? saved : ws, 0, "simt_score_kernel");
+    return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, bf, saved ? saved : ws, saved != nullptr, 0, "simt_score_kernel");
   // every size limit of the launches below, before the first of them
   if (N > 65535 || BH > 65535 || BH * N > 65535) return GLA_ERR_TOO_LARGE;
   char* w = (char*)ws;

@@ -25,8 +25,8 @@
 // float32 FMAs.
 //
 // Three launches forward, three backward: per-chunk state products (k^^T V, resp. q^^T dO), a scan over the chunks
-// in place, and the chunk kernel.  States are float32, N + 1 of them per head (slot n enters chunk n; slot N is the
-// final state; gradient states: slot n + 1 leaves chunk n, slot 0 is the gradient of the initial state), so that
+// in place, and the chunk kernel.  States are float32, N of them per head (slot n: the state that enters chunk n, resp.
+// the gradient of the one that leaves it); for a backward the final state follows as slot N, so that
 //   dG_n[d] = <S_{n+1}[d,:], dS_n[d,:]>
 // is a dot product of two stored rows and dlam = q dq - k dk needs no other inter-chunk term.
 #include "gla_common.cuh"
@@ -68,7 +68,8 @@ struct PxParams {
   int out_bf, in_bf;
   const float* g;
   const void *v, *k, *q, *dout;
-  float *S, *dS;                // (B H, N + 1, D, D)
+  int64_t NS;                   // slots of S per head: N, or N + 1 with the final state
+  float *S, *dS;                // (B H, NS, D, D), (B H, N, D, D)
   float* eG;                    // (B H, N, D): exp of every chunk's total log decay
   void *out, *dq, *dk, *dv;
   float* dg;
@@ -481,7 +482,7 @@ __device__ __noinline__ void product_by_token(float* f, float* st, const PxParam
 }
 
 // ---- per-chunk state products ----------------------------------------------------------------------------------------
-// MODE 0: S slot n + 1 = k^^T V, k^ = k exp(G - lam);  MODE 1: dS slot n = q^^T dO, q^ = q exp(lam).  The weights are
+// MODE 0: S slot n = k^^T V, k^ = k exp(G - lam);  MODE 1: dS slot n = q^^T dO, q^ = q exp(lam).  The weights are
 // anchored at the chunk's ends here and never exceed one for log gates <= 0.  Also leaves exp(G).
 template <class C, typename TI, typename TY, int MODE>
 __global__ void __launch_bounds__(C::NT, sizeof(TI) + sizeof(TY) == 4 && C::L == 64 ? 1024 / C::NT : 512 / C::NT) px_product_kernel(const __grid_constant__ PxParams p) {
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(C::NT, sizeof(TI) + sizeof(TY) == 4 && C::L ==
     ld_a_t<3>(a, aX, C::PLANE, C::LD, m0, 16 * ks, lane);
     mma_step<3, NSY, NW / 16, true, (sizeof(TI) + sizeof(TY) > 4)>(acc, a, aY, C::PLANE, C::LD, c0, 16 * ks, lane);
   }
-  float* o = (MODE == 0 ? p.S : p.dS) + (at.bh * (p.N + 1) + at.n + (MODE == 0 ? 1 : 0)) * C::D * C::D;
+  float* o = (MODE == 0 ? p.S + (at.bh * p.NS + at.n) * C::D * C::D : p.dS + (at.bh * p.N + at.n) * C::D * C::D);
 #pragma unroll
   for (int j = 0; j < NW / 8; ++j)
 #pragma unroll
@@ -558,27 +559,27 @@ __global__ void __launch_bounds__(C::NT, sizeof(TI) + sizeof(TY) == 4 && C::L ==
 }
 
 // ---- scan over the chunks, in place --------------------------------------------------------------------------------------
-// mode 0: slot 0 = init, slot n + 1 = eG_n slot n + slot n + 1;  mode 1: slot N = init, slot n = eG_n slot n + 1 + slot n.
+// s = init; over the chunks (mode 1: backwards): x = slot n, slot n = s, s = eG_n s + x; s goes to `fin` and to slot N if
+// there is one.
 // One thread per four value columns; eight chunks' loads in flight (the chain itself is one FMA per chunk).
 template <typename TS>
-__global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, int64_t N, const float* __restrict__ eG,
+__global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, int64_t N, int64_t NS, const float* __restrict__ eG,
                                                       const TS* __restrict__ init, float* S, TS* __restrict__ fin, int mode) {
   constexpr int AHEAD = 8;
   const int64_t e4 = (int64_t)blockIdx.x * 128 + threadIdx.x, DD = D * D;
   if (e4 * 4 >= total) return;
   const int64_t bh = e4 * 4 / DD, e = e4 * 4 % DD, dk = e / D;
-  float* sp = S + bh * (N + 1) * DD + e;
+  float* sp = S + bh * NS * DD + e;
   const float* gp = eG + bh * N * D + dk;
   grid_dep_wait();
   grid_dep_launch();
   float4 s;
   s.x = ld_f(init, bh * DD + e); s.y = ld_f(init, bh * DD + e + 1); s.z = ld_f(init, bh * DD + e + 2); s.w = ld_f(init, bh * DD + e + 3);
-  *reinterpret_cast<float4*>(sp + (mode ? N : 0) * DD) = s;
   float4 x[AHEAD];
   float f[AHEAD];
   auto fetch = [&](int64_t i, int u) {
     const int64_t n = mode ? N - 1 - i : i;
-    x[u] = *reinterpret_cast<const float4*>(sp + (mode ? n : n + 1) * DD);
+    x[u] = *reinterpret_cast<const float4*>(sp + n * DD);
     f[u] = __ldg(gp + n * D);
   };
 #pragma unroll
@@ -589,12 +590,13 @@ __global__ void __launch_bounds__(128) px_scan_kernel(int64_t total, int64_t D, 
       const int64_t i = i0 + u;
       if (i < N) {
         const int64_t n = mode ? N - 1 - i : i;
+        *reinterpret_cast<float4*>(sp + n * DD) = s;
         s = make_float4(fmaf(f[u], s.x, x[u].x), fmaf(f[u], s.y, x[u].y), fmaf(f[u], s.z, x[u].z), fmaf(f[u], s.w, x[u].w));
-        *reinterpret_cast<float4*>(sp + (mode ? n : n + 1) * DD) = s;
         if (i + AHEAD < N) fetch(i + AHEAD, u);
       }
     }
   }
+  if (NS > N) *reinterpret_cast<float4*>(sp + N * DD) = s;
   if (fin != nullptr) {
     st_f(fin, bh * DD + e, s.x); st_f(fin, bh * DD + e + 1, s.y); st_f(fin, bh * DD + e + 2, s.z); st_f(fin, bh * DD + e + 3, s.w);
   }
@@ -715,7 +717,7 @@ __global__ void __launch_bounds__(C::NT, FwdLay<C, TI>::BLOCKS) px_fwd_kernel(co
   float* em = reinterpret_cast<float*>(sm + Lay::EM);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
   const ChunkAt<C> at(p, blockIdx.x);
-  const float* Sn = p.S + (at.bh * (p.N + 1) + at.n) * C::D * C::D;
+  const float* Sn = p.S + (at.bh * p.NS + at.n) * C::D * C::D;
   float4 sx[C::SREG];
   {
     float2 g[C::RPT];
@@ -840,8 +842,8 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
   float* dG = reinterpret_cast<float*>(sm + Lay::DG);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % C::CP, rg = tid / C::CP, r0 = rg * C::RPT;
   const ChunkAt<C> at(p, blockIdx.x);
-  const float* Sn = p.S + (at.bh * (p.N + 1) + at.n) * D * D;
-  const float* dSn = p.dS + (at.bh * (p.N + 1) + at.n + 1) * D * D;
+  const float* Sn = p.S + (at.bh * p.NS + at.n) * D * D;
+  const float* dSn = p.dS + (at.bh * p.N + at.n) * D * D;
   float4 sx[C::SREG];
   float2 start;
   {
@@ -869,7 +871,7 @@ __global__ void __launch_bounds__(C::NT, BwdLay<C, TI, TY>::BLOCKS) px_bwd_kerne
   const int wr = warp % C::WR, wc = warp / C::WR, m0 = 16 * wr;
   const uint32_t aQ = smem_u32(sm + Lay::Q), aK = smem_u32(sm + Lay::K), aV = smem_u32(sm + Lay::V);
   const uint32_t aD = smem_u32(sm + Lay::DO), aS = smem_u32(sm + Lay::S);
-  const float* Snext = p.S + (at.bh * (p.N + 1) + at.n + 1) * D * D;
+  const float* Snext = Sn + D * D;
   float dq[C::CW / 8][4], dk[C::CW / 8][4], dv[C::NP][C::PC / 8][4];
   zero_acc(dq);
   zero_acc(dk);
@@ -1020,10 +1022,10 @@ int launch_product(cudaStream_t st, const PxParams& p, int64_t chunks) {
   return GLA_OK;
 }
 template <typename TS>
-int launch_scan(cudaStream_t st, int64_t BH, int64_t D, int64_t N, const float* eG, const void* init, float* S, void* fin, int mode) {
+int launch_scan(cudaStream_t st, int64_t BH, int64_t D, int64_t N, int64_t NS, const float* eG, const void* init, float* S, void* fin, int mode) {
   const int64_t total = BH * D * D;
   ProfScope ps("px_scan_kernel", st);
-  GLA_LAUNCHED(launch_overlapped(px_scan_kernel<TS>, dim3((unsigned)((total / 4 + 127) / 128)), dim3(128), 0, st, total, D, N, eG,
+  GLA_LAUNCHED(launch_overlapped(px_scan_kernel<TS>, dim3((unsigned)((total / 4 + 127) / 128)), dim3(128), 0, st, total, D, N, NS, eG,
                                  (const TS*)init, S, (TS*)fin, mode));
   return GLA_OK;
 }
@@ -1039,7 +1041,7 @@ template <class C, typename TI>
 int run_fwd(cudaStream_t st, const PxParams& p, const void* init, void* fin) {
   const int64_t BH = p.B * p.H, chunks = BH * p.N;
   GLA_TRY((launch_product<C, TI, TI, 0>(st, p, chunks)));
-  GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.eG, init, p.S, fin, 0));
+  GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.NS, p.eG, init, p.S, fin, 0));
   if constexpr (sizeof(TI) == 2)
     if (p.out_bf) return launch_fwd<C, TI, false>(st, p, chunks);
   return launch_fwd<C, TI, true>(st, p, chunks);
@@ -1050,10 +1052,10 @@ int run_bwd(cudaStream_t st, const PxParams& p, int states, const void* init, co
   const int64_t BH = p.B * p.H, chunks = BH * p.N;
   if (!states) {
     GLA_TRY((launch_product<C, TI, TI, 0>(st, p, chunks)));
-    GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.eG, init, p.S, nullptr, 0));
+    GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.NS, p.eG, init, p.S, nullptr, 0));
   }
   GLA_TRY((launch_product<C, TI, TY, 1>(st, p, chunks)));
-  GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.eG, dfin, p.dS, dinit, 1));
+  GLA_TRY(launch_scan<TI>(st, BH, C::D, p.N, p.N, p.eG, dfin, p.dS, dinit, 1));
   static SmemAttrOnce attr;
   GLA_TRY(attr.ensure(px_bwd_kernel<C, TI, TY>, BwdLay<C, TI, TY>::END));
   ProfScope ps("px_bwd_kernel", st);
@@ -1071,21 +1073,20 @@ size_t f32b(int64_t n) { return align_up((size_t)n * 4, 256); }
 // Rows of a chunk: 64, or 32 where three planes of every operand at head size 128 leave no room for more.
 static int64_t px_rows(int64_t D, int narrow) { return D >= 128 && narrow ? 32 : 64; }
 bool px_supported(int64_t D) { return D == 32 || D == 64 || D == 128; }
-// states: (B H, N + 1, D, D) float32 | exp(G): (B H, N, D) float32
-size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
-  const int64_t N = (T + 31) / 32;                      // the shorter chunk bounds both
-  const int64_t n = D >= 128 ? N : (T + 63) / 64;
-  return f32b(B * H * (n + 1) * D * D) + f32b(B * H * n * D);
+// states: (B H, N, D, D) float32, N + 1 of them with the final one | exp(G): (B H, N, D) float32.  bf: every array in bf16
+size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf, int final_state) {
+  const int64_t n = (T + px_rows(D, !bf) - 1) / px_rows(D, !bf);
+  return f32b(B * H * (n + (final_state ? 1 : 0)) * D * D) + f32b(B * H * n * D);
 }
 int px_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
-           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int reverse, const char* label) {
+           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int final_state, int reverse, const char* label) {
   const int64_t N = (T + px_rows(D, !bf) - 1) / px_rows(D, !bf);
   if (B * H * N > 2147483647LL || B * H * D * D / 512 > 2147483647LL) return GLA_ERR_TOO_LARGE;
   PxParams p{};
-  p.B = B; p.T = T; p.H = H; p.N = N; p.trev = reverse; p.in_bf = bf; p.out_bf = out_bf;
+  p.B = B; p.T = T; p.H = H; p.N = N; p.NS = N + (final_state ? 1 : 0); p.trev = reverse; p.in_bf = bf; p.out_bf = out_bf;
   p.g = g; p.v = v; p.k = k; p.q = q; p.out = out; p.label = label;
   p.S = (float*)states;
-  p.eG = (float*)((char*)states + f32b(B * H * (N + 1) * D * D));
+  p.eG = (float*)((char*)states + f32b(B * H * p.NS * D * D));
   switch (D) {
     case 32: return dispatch_fwd<32, 64>(st, p, hidden_init, hidden_final);
     case 64: return dispatch_fwd<64, 64>(st, p, hidden_init, hidden_final);
@@ -1101,7 +1102,8 @@ static int dispatch_bwd(cudaStream_t st, const PxParams& p, int do_bf, int state
   return do_bf ? run_bwd<Px<D, LN>, float, bf16>(st, p, states, init, dfin, dinit)
                : run_bwd<Px<D, LN>, float, float>(st, p, states, init, dfin, dinit);
 }
-// states: a forward's (px_fwd) when have_states, else scratch of px_state_bytes; ws: px_state_bytes more
+// states: a forward's (px_fwd) with the final one when have_states, else scratch for as much; ws: scratch for the gradient
+// states, px_state_bytes without a final one
 int px_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
            const void* v, const void* k, const void* q, const void* dhidden_final, const void* dout, int do_bf,
            void* dhidden_init, float* dg, void* dv, void* dk, void* dq, void* states, int have_states, void* ws, int reverse) {
@@ -1109,11 +1111,11 @@ int px_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, 
   if (have_states && L != px_rows(D, !bf)) return GLA_ERR_UNSUPPORTED;
   if (B * H * N > 2147483647LL || B * H * D * D / 512 > 2147483647LL) return GLA_ERR_TOO_LARGE;
   PxParams p{};
-  p.B = B; p.T = T; p.H = H; p.N = N; p.trev = reverse; p.in_bf = bf;
+  p.B = B; p.T = T; p.H = H; p.N = N; p.NS = N + 1; p.trev = reverse; p.in_bf = bf;
   p.g = g; p.v = v; p.k = k; p.q = q; p.dout = dout;
   p.dq = dq; p.dk = dk; p.dv = dv; p.dg = dg;
   p.S = (float*)states;
-  p.eG = (float*)((char*)states + f32b(B * H * (N + 1) * D * D));
+  p.eG = (float*)((char*)states + f32b(B * H * p.NS * D * D));
   p.dS = (float*)ws;
   if (have_states == 0) {
     switch (D) {

@@ -12,14 +12,12 @@
 namespace gla {
 
 constexpr size_t kStaticScratchBytes = 32u << 20;    // 32 MiB per device
-// The split-operand kernels keep one state more per head than the chunk kernels that the limit was set for: head size 128
-// needs up to 64 KB + 12 bytes a token beyond it per (batch, head), below 9 MB in all.  Sizes up to the limit of those
-// kernels stay accepted.
-constexpr size_t kSplitExtraBytes = (size_t)9 << 20;
-static size_t split_extra(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int impl) {
-  if (D != 128 || ((impl & 0xff) != GLA_IMPL_FP32_SIMT && tc_supported(D, chunk, dtype))) return 0;
-  const size_t n = (size_t)(B * H) * (65536 + 12 * (size_t)T);
-  return n < kSplitExtraBytes ? n : kSplitExtraBytes;
+// The limit was set for the kernels that keep lam, k^, q^ and a state per chunk.  The split-operand kernels need no more
+// than those anywhere but for float32 of head size 128 in chunks of 128, which they run in chunks of 32: 2064 bytes a
+// token and head against 2052.  Sizes up to the limit of the former stay accepted.
+constexpr size_t kSplitExtraBytes = 256u << 10;      // 12 / 2052 of 32 MiB
+static size_t split_extra(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype) {
+  return D == 128 && chunk == 128 && dtype == GLA_F32 ? (size_t)(B * H) * 12 * T : 0;
 }
 
 // File-scope device array.  In HOST code this name is only a handle for the runtime's symbol
@@ -65,7 +63,7 @@ GLA_API int gla_chunk_fwd_static(void* stream, int64_t B, int64_t T, int64_t H, 
   if (need == 0)   // invalid or unsupported sizes: the ordinary entry point reports which, before any launch
     return gla_chunk_fwd(stream, B, T, H, D, chunk, dtype, impl, hidden_init, log_fgate, value, key, query,
                          hidden_final, out, nullptr, nullptr, 0);
-  if (need > kStaticScratchBytes + split_extra(B, T, H, D, chunk, dtype, impl)) return GLA_ERR_TOO_LARGE;
+  if (need > kStaticScratchBytes + split_extra(B, T, H, D, chunk, dtype)) return GLA_ERR_TOO_LARGE;
   void* scratch = nullptr;
   GLA_TRY(static_scratch(&scratch));
   return gla_chunk_fwd(stream, B, T, H, D, chunk, dtype, impl, hidden_init, log_fgate, value, key, query, hidden_final,

@@ -335,11 +335,11 @@ GLA_API int gla_chunk_bwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t
  * plugin in a serving process whose memory pool is closed, a callback in a region where
  * cudaMalloc would fail or stall the device.  Such a caller still passes inputs and outputs,
  * but the scratch comes from a fixed array inside the library image:
- *   - the array is gla_chunk_fwd_static_max_bytes() = 32 MiB of device memory PER GPU, held
- *     from the first use of the library on that GPU until the process exits;
- *   - a problem whose gla_chunk_fwd_workspace_bytes() exceeds it returns GLA_ERR_TOO_LARGE
- *     (head size 128 on the split-operand kernels: exceeds it by more than their extra state per head)
- *     and launches nothing (32 MiB covers, e.g., one sequence of T=4096, H=6, D=128);
+ *   - the array is a little more than gla_chunk_fwd_static_max_bytes() = 32 MiB of device memory PER GPU (256 KiB
+ *     more), held from the first use of the library on that GPU until the process exits;
+ *   - a problem whose gla_chunk_fwd_workspace_bytes() exceeds 32 MiB returns GLA_ERR_TOO_LARGE and launches nothing
+ *     (float32 at head size 128 in chunks of 128 may exceed it by the 12 bytes per token and head that its shorter
+ *     chunks take; 32 MiB covers, e.g., one sequence of T=4096, H=6, D=128);
  *   - the function allocates nothing and frees nothing, on host or device.  The first call
  *     on each device looks up the array's device address (a symbol query, with that device
  *     current); make that first call outside any stream capture;
