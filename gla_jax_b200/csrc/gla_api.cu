@@ -264,10 +264,12 @@ int gla_layer_headnorm_gate_bwd(void* stream, int64_t rows, int64_t D, int dtype
                                  dweight, workspace);
 }
 
-size_t gla_recurrent_bwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int dtype) {
-  (void)dtype;
+size_t gla_recurrent_bwd_workspace_bytes_dout(int64_t B, int64_t T, int64_t H, int64_t D, int dtype, int dout_dtype, int least) {
   if (B <= 0 || T <= 0 || H <= 0 || D <= 0) return 0;
-  return recurrent_bwd_ws_bytes(B, T, H, D);
+  return recurrent_bwd_ws_bytes(B, T, H, D, dtype == GLA_BF16, dout_dtype == GLA_BF16, least);
+}
+size_t gla_recurrent_bwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int dtype) {
+  return gla_recurrent_bwd_workspace_bytes_dout(B, T, H, D, dtype, dtype, 0);
 }
 
 int gla_recurrent_bwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int dtype, const void* hidden_init,
@@ -281,11 +283,11 @@ int gla_recurrent_bwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, 
   if (B <= 0 || T <= 0 || H <= 0 || D <= 0) return GLA_ERR_BAD_DIMS;
   GLA_TRY(check_dtype(dtype));
   GLA_TRY(check_dtype(dout_dtype));
-  if (!workspace || workspace_bytes < recurrent_bwd_ws_bytes(B, T, H, D)) return GLA_ERR_WORKSPACE;
+  if (!workspace || workspace_bytes < recurrent_bwd_ws_bytes(B, T, H, D, dtype == GLA_BF16, dout_dtype == GLA_BF16, 1)) return GLA_ERR_WORKSPACE;
   if (!aligned16(workspace)) return GLA_ERR_ALIGNMENT;
   return recurrent_bwd((cudaStream_t)stream, B, T, H, D, dtype == GLA_BF16, hidden_init, log_fgate, value, key,
                        query, dhidden_final, dout, dout_dtype == GLA_BF16, dhidden_init, dlog_fgate, dvalue, dkey,
-                       dquery, reverse, workspace);
+                       dquery, reverse, workspace, workspace_bytes);
 }
 
 size_t gla_chunk_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int impl) {
@@ -307,6 +309,17 @@ size_t gla_chunk_bwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D,
   return r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk, dtype);
 }
 
+static size_t training_ws_bytes(int r, int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int backward) {
+  if (r == GLA_IMPL_TCGEN05) return backward ? tc_bwd_ws_bytes(B, T, H, D, chunk) : tc_fwd_ws_bytes(B, T, H, D, chunk);
+  if (px_supported(D)) return backward ? px_state_bytes(B, T, H, D, dtype == GLA_BF16, 0) : 0;      // the forward's states are saved
+  return backward ? simt_bwd_ws_bytes(B, T, H, D, chunk, dtype) : simt_fwd_ws_bytes(B, T, H, D, chunk, dtype);
+}
+size_t gla_chunk_training_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int impl, int backward) {
+  if (check_chunk_dims(B, T, H, D, chunk, dtype) != GLA_OK) return 0;
+  int r = resolve_impl(impl, D, chunk, dtype);
+  return r < 0 ? 0 : training_ws_bytes(r, B, T, H, D, chunk, dtype, backward);
+}
+
 int gla_chunk_fwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk, int dtype, int impl,
                   const void* hidden_init, const float* log_fgate, const void* value, const void* key,
                   const void* query, void* hidden_final, void* out, void* saved, void* workspace,
@@ -315,8 +328,9 @@ int gla_chunk_fwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int6
   GLA_TRY(check_chunk_dims(B, T, H, D, chunk, dtype));
   int r = resolve_impl(impl, D, chunk, dtype);
   if (r < 0) return -r;
-  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk, dtype);
-  if (!workspace || workspace_bytes < need) return GLA_ERR_WORKSPACE;
+  const size_t need = saved ? training_ws_bytes(r, B, T, H, D, chunk, dtype, 0)
+                            : r == GLA_IMPL_TCGEN05 ? tc_fwd_ws_bytes(B, T, H, D, chunk) : simt_fwd_ws_bytes(B, T, H, D, chunk, dtype);
+  if (need && (!workspace || workspace_bytes < need)) return GLA_ERR_WORKSPACE;
   const void* ptrs[] = {hidden_init, log_fgate, value, key, query, hidden_final, out, saved, workspace};
   for (const void* p : ptrs)
     if (p && !aligned16(p)) return GLA_ERR_ALIGNMENT;
@@ -339,7 +353,7 @@ int gla_chunk_bwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int6
   GLA_TRY(check_chunk_dims(B, T, H, D, chunk, dtype));
   int r = resolve_impl(impl, D, chunk, dtype);
   if (r < 0) return -r;
-  const size_t need = r == GLA_IMPL_TCGEN05 ? tc_bwd_ws_bytes(B, T, H, D, chunk) : simt_bwd_ws_bytes(B, T, H, D, chunk, dtype);
+  const size_t need = training_ws_bytes(r, B, T, H, D, chunk, dtype, 1);
   if (!workspace || workspace_bytes < need) return GLA_ERR_WORKSPACE;
   const void* ptrs[] = {log_fgate, value, key, query, saved, dhidden_final, dout, dhidden_init, dlog_fgate,
                         dvalue, dkey, dquery, workspace};

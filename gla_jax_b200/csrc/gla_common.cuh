@@ -195,9 +195,9 @@ size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf
 int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, void* hidden_final, void* out,
                   int out_bf, int reverse, void* ws = nullptr, size_t ws_bytes = 0);
-size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D);
+size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf, int do_bf, int least);
 int recurrent_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, const void* dhidden_final,
                   const void* dout, int do_bf, void* dhidden_init, float* dg, void* dv, void* dk, void* dq,
-                  int reverse, void* ws);
+                  int reverse, void* ws, size_t ws_bytes);
 }  // namespace gla

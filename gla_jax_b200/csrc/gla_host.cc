@@ -42,6 +42,16 @@ bool here(const Tensor& t) { return t.is_cuda() && t.device().index() == c10::cu
 Tensor bytes(const Tensor& like, size_t n) {
   return n ? torch::empty({(int64_t)n}, like.options().dtype(torch::kUInt8)) : Tensor();
 }
+// as much as the faster form of a call takes, or `least` where that does not fit the device (0 bytes: undefined)
+Tensor bytes_or(const Tensor& like, size_t n, size_t least) {
+  try {
+    return bytes(like, n);
+  } catch (const c10::OutOfMemoryError&) {
+    if (n <= least) throw;
+    return bytes(like, least);
+  }
+}
+size_t size_of(const Tensor& t) { return t.defined() ? (size_t)t.numel() : 0; }
 Tensor f32(const Tensor& g) { return (g.scalar_type() == torch::kFloat32 ? g : g.to(torch::kFloat32)).contiguous(); }
 bool wants_grad(std::initializer_list<const Tensor*> ts) {
   if (!torch::GradMode::is_enabled()) return false;
@@ -74,8 +84,9 @@ std::string shape_text(const Dims& d, int64_t chunk, const Tensor& v) {
 // ---- chunk_gla ---------------------------------------------------------------------------------------------------
 variable_list chunk_forward(const Dims& d, const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
                             int64_t chunk, int64_t impl, bool residuals) {
-  const size_t n = gla_chunk_fwd_workspace_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl);
+  size_t n = gla_chunk_fwd_workspace_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl);
   if (n == 0) raise("chunk_gla: unsupported configuration " + shape_text(d, chunk, v));
+  if (residuals) n = gla_chunk_training_workspace_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl, 0);
   Tensor saved = residuals ? bytes(v, gla_chunk_saved_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl)) : Tensor();
   Tensor ws = bytes(v, n), hf = torch::empty_like(h), out = torch::empty_like(v);
   check(gla_chunk_fwd(stream_of(v), d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl, ptr(h), (const float*)ptr(g), ptr(v), ptr(k), ptr(q),
@@ -89,7 +100,7 @@ variable_list chunk_backward(const Dims& d, const Tensor& g, const Tensor& v, co
   Tensor dh = torch::empty(hs, v.options());
   Tensor dhf = grad_or_zeros(dhf0, dh), dout = grad_or_zeros(dout0, v);
   Tensor dg = torch::empty_like(g), dv = torch::empty_like(v), dk = torch::empty_like(k), dq = torch::empty_like(q);
-  const size_t n = gla_chunk_bwd_workspace_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl);
+  const size_t n = gla_chunk_training_workspace_bytes(d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl, 1);
   Tensor ws = bytes(v, n);
   check(gla_chunk_bwd(stream_of(v), d.B, d.T, d.H, d.D, chunk, d.dt, (int)impl, (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(saved),
                       ptr(dhf), ptr(dout), ptr(dh), (float*)ptr(dg), ptr(dv), ptr(dk), ptr(dq), ptr(ws), n), "gla_chunk_bwd");
@@ -134,10 +145,9 @@ std::optional<std::tuple<Tensor, Tensor>> chunk_gla(const Tensor& h, const Tenso
 variable_list recurrent_forward(const Dims& d, const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q,
                                 bool reverse, bool out_f32) {
   Tensor hf = torch::empty_like(h), out = torch::empty(v.sizes(), v.options().dtype(out_f32 ? torch::kFloat32 : v.scalar_type()));
-  const size_t n = gla_recurrent_fwd_workspace_bytes(d.B, d.T, d.H, d.D, d.dt);
-  Tensor ws = bytes(v, n);
+  Tensor ws = bytes_or(v, gla_recurrent_fwd_workspace_bytes(d.B, d.T, d.H, d.D, d.dt), 0);
   check(gla_recurrent_fwd_ws(stream_of(v), d.B, d.T, d.H, d.D, d.dt, ptr(h), (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(hf),
-                             ptr(out), dt_of(out), reverse, ptr(ws), n), "gla_recurrent_fwd_ws");
+                             ptr(out), dt_of(out), reverse, ptr(ws), size_of(ws)), "gla_recurrent_fwd_ws");
   return {hf, out};
 }
 struct RecurrentFn : torch::autograd::Function<RecurrentFn> {
@@ -159,10 +169,10 @@ struct RecurrentFn : torch::autograd::Function<RecurrentFn> {
     Tensor dout = grads[1].defined() ? grads[1].contiguous() : torch::zeros(v.sizes(), v.options().dtype((torch::ScalarType)a[7]));
     if (dt_of(dout) < 0) dout = dout.to(torch::kFloat32);
     Tensor dh = torch::empty_like(h), dg = torch::empty_like(g), dv = torch::empty_like(v), dk = torch::empty_like(k), dq = torch::empty_like(q);
-    const size_t n = gla_recurrent_bwd_workspace_bytes(a[0], a[1], a[2], a[3], (int)a[4]);
-    Tensor ws = bytes(v, n);
+    const auto n = [&](int least) { return gla_recurrent_bwd_workspace_bytes_dout(a[0], a[1], a[2], a[3], (int)a[4], dt_of(dout), least); };
+    Tensor ws = bytes_or(v, n(0), n(1));
     check(gla_recurrent_bwd(stream_of(v), a[0], a[1], a[2], a[3], (int)a[4], ptr(h), (const float*)ptr(g), ptr(v), ptr(k), ptr(q), ptr(dhf),
-                            ptr(dout), dt_of(dout), ptr(dh), (float*)ptr(dg), ptr(dv), ptr(dk), ptr(dq), (int)a[5], ptr(ws), n),
+                            ptr(dout), dt_of(dout), ptr(dh), (float*)ptr(dg), ptr(dv), ptr(dk), ptr(dq), (int)a[5], ptr(ws), size_of(ws)),
           "gla_recurrent_bwd");
     const auto gt = (torch::ScalarType)a[6];
     variable_list r{dh, gt == torch::kFloat32 ? dg : dg.to(gt), dv, dk, dq};

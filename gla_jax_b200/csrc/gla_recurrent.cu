@@ -1,5 +1,6 @@
 // recurrent_gla forward and backward: the exact step recurrence with the state tile held in
-// registers and never written to memory.
+// registers and never written to memory.  It serves short sequences, head sizes that gla_split.cu does not, arrays that are
+// not 16-byte aligned, and callers without room for the states that the chunked form there stores.
 //
 // Reference: gla.py:50-96 (forward kernel), gla.py:271-360 (backward kernel), gla.py:99-170,
 // 172-269 (wrappers).  The reference tiles the state over (head, key block, value block)
@@ -471,17 +472,21 @@ int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, i
   return launch_rec_fwd_d(st, (int)D, p);
 }
 
-size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D) {
+static size_t rec_chunked_bwd_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf) {      // states and gradient states
+  return px_state_bytes(B, T, H, D, bf, 1) + px_state_bytes(B, T, H, D, bf, 0);
+}
+size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf, int do_bf, int least) {
   const size_t n = 2 * align_up((size_t)B * T * H * D * 4, 256) + align_up((size_t)B * H * D * 4, 256);
-  const size_t px = rec_chunked(T, D) ? px_state_bytes(B, T, H, D, 0, 1) + px_state_bytes(B, T, H, D, 0, 0) : 0;      // states and gradient states
+  const size_t px = rec_chunked(T, D) && !least ? rec_chunked_bwd_bytes(B, T, H, D, bf && do_bf) : 0;
   return px > n ? px : n;
 }
 
 int recurrent_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, const void* dhidden_final,
                   const void* dout, int do_bf, void* dhidden_init, float* dg, void* dv, void* dk, void* dq,
-                  int reverse, void* ws) {
-  if (rec_chunked(T, D) && rec_aligned({hidden_init, g, v, k, q, dhidden_final, dout, dhidden_init, dg, dv, dk, dq, ws}))
+                  int reverse, void* ws, size_t ws_bytes) {
+  if (rec_chunked(T, D) && ws_bytes >= rec_chunked_bwd_bytes(B, T, H, D, bf && do_bf) &&
+      rec_aligned({hidden_init, g, v, k, q, dhidden_final, dout, dhidden_init, dg, dv, dk, dq, ws}))
     return px_bwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, dhidden_final, dout, do_bf, dhidden_init, dg, dv, dk, dq, ws, 0,
                   (char*)ws + px_state_bytes(B, T, H, D, bf && do_bf, 1), reverse);
   RecParams p{};

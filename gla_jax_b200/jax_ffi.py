@@ -142,11 +142,11 @@ def _recurrent_bwd(reverse, out_f32, res, g):
     dhf, dout = g
     B, T, H, D = value.shape
     sds = lambda x, d=None: jax.ShapeDtypeStruct(x.shape, d or x.dtype)
-    call = jax.ffi.ffi_call("GlaRecurrentBwd", (sds(hidden_init), sds(value, jnp.float32), sds(value), sds(key),
-                                                sds(query), _u8(lib.gla_recurrent_bwd_workspace_bytes(B, T, H, D, _dt(value)))),
-                            vmap_method=_VMAP)
     if dout.dtype not in (jnp.float32, jnp.bfloat16):
         dout = dout.astype(jnp.float32)
+    ws = _u8(lib.gla_recurrent_bwd_workspace_bytes_dout(B, T, H, D, _dt(value), _dt(dout), 0))
+    call = jax.ffi.ffi_call("GlaRecurrentBwd", (sds(hidden_init), sds(value, jnp.float32), sds(value), sds(key), sds(query), ws),
+                            vmap_method=_VMAP)
     dh, dg, dv, dk, dq, _ = call(hidden_init, log_fgate.astype(jnp.float32), value, key, query,
                                  dhf.astype(value.dtype), dout, reverse=np.int64(reverse))
     return dh, dg.astype(log_fgate.dtype), dv, dk, dq

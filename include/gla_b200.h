@@ -254,7 +254,8 @@ GLA_API int gla_rnn_scan_ws(void* stream, int64_t batch, int64_t T, int64_t K, i
  * recurrent_gla — replaces gla.py:405 recurrent_gla (forward: gla.py:99, kernel gla.py:50)
  * and, with out_dtype = GLA_F32, gla.py:26 recurrent_gla_naive.
  * Exact step recurrence S_t = exp(g_t) * S_{t-1} + k_t (x) v_t, o_t = q_t S_t with the
- * state held on chip in float32 and never written to memory.  reverse != 0 runs the
+ * state held on chip in float32 and never written to memory (unless a workspace is given,
+ * see gla_recurrent_fwd_ws).  reverse != 0 runs the
  * recurrence from the last token to the first (gla.py:421-423,437-438).
  * `out` has dtype out_dtype (the reference's recurrent_gla returns value's dtype,
  * recurrent_gla_naive returns float32).
@@ -265,15 +266,21 @@ GLA_API int gla_recurrent_fwd(void* stream, int64_t B, int64_t T, int64_t H, int
                       void* hidden_final, void* out, int out_dtype, int reverse);
 
 /* The same with a workspace of gla_recurrent_fwd_workspace_bytes (0 bytes: none is of use for these sizes): chunks of
- * the sequence then run side by side, from states kept in the workspace for the duration of the call.  Without one (or
+ * the sequence then run side by side, from states kept in the workspace for the duration of the call (one float32 state
+ * per head and chunk of 64 tokens; 32 tokens for float32 at head size 128).  Without one (or
  * with arrays that are not 16-byte aligned) this is gla_recurrent_fwd, which walks the tokens in order. */
 GLA_API size_t gla_recurrent_fwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int dtype);
 GLA_API int gla_recurrent_fwd_ws(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int dtype,
                       const void* hidden_init, const float* log_fgate, const void* value, const void* key,
                       const void* query, void* hidden_final, void* out, int out_dtype, int reverse,
                       void* workspace, size_t workspace_bytes);
-/* Bytes of workspace gla_recurrent_bwd needs for these sizes. */
+/* Bytes of workspace for gla_recurrent_bwd at these sizes, with `dout` in `dtype`; with `dout` in dout_dtype; and with
+ * least != 0 the fewest it takes: 8 bytes per element of value, and it then walks the tokens instead of running chunks side
+ * by side from stored states (head sizes 32, 64 and 128: two float32 states per head and chunk of 64 tokens, or of 32 at head
+ * size 128 with any array in float32: D * D / 8 or D * D / 4 bytes per token and head). */
 GLA_API size_t gla_recurrent_bwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int dtype);
+GLA_API size_t gla_recurrent_bwd_workspace_bytes_dout(int64_t B, int64_t T, int64_t H, int64_t D, int dtype, int dout_dtype,
+                      int least);
 
 /* Backward of recurrent_gla — replaces gla.py:172 recurrent_gla_backward (kernel
  * gla.py:271): a recompute pass for dquery, a reverse pass for dvalue, dkey and
@@ -308,6 +315,11 @@ GLA_API size_t gla_chunk_fwd_workspace_bytes(int64_t B, int64_t T, int64_t H, in
                                      int dtype, int impl);
 GLA_API size_t gla_chunk_bwd_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk,
                                      int dtype, int impl);
+/* What gla_chunk_fwd with `saved` (backward = 0; 0 bytes: the workspace may be NULL) or gla_chunk_bwd (backward = 1) itself
+ * needs.  The two functions above never return less; their sizes also serve gla_chunk_local_state and
+ * gla_chunk_local_dstate. */
+GLA_API size_t gla_chunk_training_workspace_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk,
+                                     int dtype, int impl, int backward);
 
 GLA_API int gla_chunk_fwd(void* stream, int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk,
                   int dtype, int impl,

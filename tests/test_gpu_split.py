@@ -155,6 +155,37 @@ def test_naive_with_bf16_inputs_and_float32_cotangent(cuda_device):
     _check((ref[0], ref[0], ref[2]), (hf.detach().cpu(), hf.detach().cpu(), [x.cpu() for x in grads]), torch.bfloat16, "naive")
 
 
+def test_without_room_for_the_states_the_tokens_are_walked(cuda_device):
+    """recurrent_gla where the device has no room for the chunks' states: it runs as it does without a workspace."""
+    from gla_jax_b200 import recurrent_gla, _lib
+    case = _case(1, 4096, 4, 128, torch.float32, 25, 5.0)
+    x = [t.to(cuda_device).requires_grad_(True) for t in case[:5]]
+    co = [t.to(cuda_device) for t in case[5:]]
+    with torch.no_grad():
+        full = [t.cpu() for t in recurrent_gla(*x)]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    lib = _lib.load()
+    need, least = (lib.gla_recurrent_bwd_workspace_bytes_dout(1, 4096, 4, 128, 0, 0, n) for n in (0, 1))
+    assert lib.gla_recurrent_fwd_workspace_bytes(1, 4096, 4, 128, 0) > 16 << 20 and need > 64 << 20 > 3 * least
+    # outputs and gradients take about 7 arrays of 8 MiB, the walk's scratch 16 MiB; the states 33 and 67 MB
+    total = torch.cuda.get_device_properties(cuda_device).total_memory
+    try:
+        with torch.no_grad():
+            torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)
+            hf, out = recurrent_gla(*x)
+        assert O.rel_l2(full[0], hf.cpu()) < 5e-6 and O.rel_l2(full[1], out.cpu()) < 5e-6
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        hf, out = recurrent_gla(*x)
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (72 << 20)) / total)
+        walked = torch.autograd.grad([hf, out], x, co, retain_graph=True)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for n, a, b in zip(NAMES, torch.autograd.grad([hf, out], x, co), walked):
+        assert O.rel_l2(a.cpu(), b.cpu()) < 1e-5, n
+
+
 def test_wait_for_workspace_is_not_needed(cuda_device):
     """The entry point without a workspace walks the tokens; with one it runs chunks: same results to float32 rounding."""
     from gla_jax_b200 import _lib

@@ -55,6 +55,29 @@ def test_size_functions_without_a_gpu(lib):
     assert lib.gla_chunk_fwd_static_max_bytes() == 32 << 20
 
 
+@pytest.mark.parametrize("D,dt,per_token", [(32, 0, 64), (64, 0, 256), (64, 1, 256), (128, 0, 2048), (128, 1, 1024)])
+def test_memory_of_the_split_operand_kernels(lib, D, dt, per_token):
+    """One float32 state per head and chunk of the rows that the types run with, and nothing that no kernel touches."""
+    B, T, H, C = 2, 4096, 3, 64
+    th, eg, spare = B * T * H, per_token / D, 2 * B * H * D * D * 4 + 1024       # exp of the totals; a final state per head
+    one = th * (per_token + eg)
+    assert one <= lib.gla_recurrent_fwd_workspace_bytes(B, T, H, D, dt) <= one + 512
+    walk = 8 * th * D + 4 * B * H * D + 1024               # (arrays that are not aligned are walked)
+    assert 2 * one <= lib.gla_recurrent_bwd_workspace_bytes(B, T, H, D, dt) <= max(2 * one + spare, walk)
+    assert lib.gla_recurrent_bwd_workspace_bytes_dout(B, T, H, D, dt, 0, 1) <= walk
+    fp32 = 1
+    assert one <= lib.gla_chunk_saved_bytes(B, T, H, D, C, dt, fp32) <= one + spare
+    assert lib.gla_chunk_training_workspace_bytes(B, T, H, D, C, dt, fp32, 0) == 0
+    assert one <= lib.gla_chunk_training_workspace_bytes(B, T, H, D, C, dt, fp32, 1) <= one + 512
+
+
+def test_training_workspace_of_the_other_kernels(lib):
+    for D, C, dt, impl in ((128, 128, 1, 2), (256, 256, 1, 2), (48, 64, 0, 1), (256, 64, 0, 1)):
+        for backward, size in ((0, lib.gla_chunk_fwd_workspace_bytes), (1, lib.gla_chunk_bwd_workspace_bytes)):
+            assert lib.gla_chunk_training_workspace_bytes(1, 1024, 2, D, C, dt, impl, backward) == size(1, 1024, 2, D, C, dt, impl) > 0
+    assert lib.gla_chunk_training_workspace_bytes(1, 100, 2, 64, 64, 0, 0, 1) == 0      # not a multiple of the chunk
+
+
 def test_bench_reads_the_traffic_table():
     spec = importlib.util.spec_from_file_location("bench_under_test", ROOT / "bench.py")
     bench = importlib.util.module_from_spec(spec)
