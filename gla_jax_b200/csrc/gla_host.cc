@@ -58,6 +58,13 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
   for (const Tensor* t : ts) if (t->requires_grad()) return true;
   return false;
 }
+// There is no forward-mode formula: refuse a dual tensor (which need not require a gradient) instead of returning outputs
+// without a tangent.
+void no_forward_mode(const char* what, std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (t->defined() && t->_fw_grad(/*level=*/0).defined())
+      TORCH_CHECK_NOT_IMPLEMENTED(false, what, ": forward-mode differentiation (jvp) is not implemented");
+}
 // a gradient that may be absent, in the dtype and layout the library takes
 Tensor grad_or_zeros(const Tensor& g, const Tensor& like) {
   return g.defined() ? g.to(like.scalar_type()).contiguous() : torch::zeros(like.sizes(), like.options().requires_grad(false));
@@ -133,6 +140,7 @@ std::optional<std::tuple<Tensor, Tensor>> chunk_gla(const Tensor& h, const Tenso
                                                     int64_t chunk, int64_t impl) {
   Dims d;
   if (!dims_of(h, g, v, k, q, d) || chunk <= 0 || (chunk & (chunk - 1)) || d.T % chunk) return std::nullopt;
+  no_forward_mode("chunk_gla", {&h, &g, &v, &k, &q});
   if (wants_grad({&h, &g, &v, &k, &q})) {
     variable_list r = ChunkFn::apply(h, g, v, k, q, d.B, d.T, d.H, d.D, d.dt, chunk, impl);
     return std::make_tuple(r[0], r[1]);
@@ -184,6 +192,7 @@ std::optional<std::tuple<Tensor, Tensor>> recurrent_gla(const Tensor& h, const T
                                                         const Tensor& q, bool reverse, bool out_f32) {
   Dims d;
   if (!dims_of(h, g, v, k, q, d)) return std::nullopt;
+  no_forward_mode("recurrent_gla", {&h, &g, &v, &k, &q});
   variable_list r = wants_grad({&h, &g, &v, &k, &q})
                         ? RecurrentFn::apply(h, g, v, k, q, d.B, d.T, d.H, d.D, d.dt, reverse, out_f32)
                         : recurrent_forward(d, h.contiguous(), f32(g), v.contiguous(), k.contiguous(), q.contiguous(), reverse, out_f32);
@@ -267,6 +276,7 @@ std::optional<std::tuple<Tensor, Tensor>> chunk_gla_packed(const Tensor& h, cons
   } else if (c.device() != v.device()) {
     return std::nullopt;
   }
+  no_forward_mode("chunk_gla_packed", {&h, &g, &v, &k, &q});
   variable_list r = wants_grad({&h, &g, &v, &k, &q})
                         ? PackedFn::apply(h, g, v, k, q, c, chunk, (int64_t)d.dt)
                         : PackedFn::run(d, h.size(0), h.contiguous(), f32(g), v.contiguous(), k.contiguous(), q.contiguous(), c, chunk, false);
@@ -404,6 +414,7 @@ std::optional<std::tuple<Tensor, Tensor>> gla_layer(const Tensor& x, const std::
   if (hidden.dim() != 4 || hidden.size(0) != d.B || hidden.size(1) != H || hidden.size(2) != D || hidden.size(3) != D ||
       hidden.scalar_type() != x.scalar_type() || hidden.device() != x.device())
     return std::nullopt;
+  no_forward_mode("GLALayer", {&x, &hidden, &w[0], &w[1], &w[2], &w[3], &w[4], &w[5], &w[6], &w[7], &w[8]});
   if (wants_grad({&x, &hidden, &w[0], &w[1], &w[2], &w[3], &w[4], &w[5], &w[6], &w[7], &w[8]})) {
     variable_list r = LayerFn::apply(x, hidden, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], H, D, (int64_t)d.dt, chunk, tau_inv, eps);
     return std::make_tuple(r[0], r[1]);
