@@ -1033,9 +1033,37 @@ def _alg_tc_state(B, T, H, D, C):
             "what": "chunk states: log_fgate (f32) + two bf16 operands in, one bf16 (D,D) state per chunk out: 8*D + 2*D*D/C B per token-head"}
 
 
+def _alg_px_fwd(B, T, H, D, C):
+    th = B * T * H
+    return {"bound": "hbm", "bytes": th * (12 * D + D * D // 16),
+            "what": "forward: q,k,v (bf16) + log_fgate (f32) in, out (bf16), one f32 state per 64 tokens in: 12*D + D*D/16 B per token-head"}
+
+
+def _alg_px_bwd(B, T, H, D, C):
+    th = B * T * H
+    return {"bound": "hbm", "bytes": th * (22 * D + D * D // 8),
+            "what": "backward: q,k,v,dout (bf16) + log_fgate (f32) in, dq,dk,dv (bf16) + dlog_fgate (f32) out, two f32 states per 64 "
+                    "tokens in: 22*D + D*D/8 B per token-head"}
+
+
+def _alg_px_product(B, T, H, D, C):
+    th = B * T * H
+    return {"bound": "hbm", "bytes": th * (8 * D + D * D // 16),
+            "what": "chunk states: log_fgate (f32) + two bf16 operands in, one f32 state per 64 tokens out: 8*D + D*D/16 B per token-head"}
+
+
+def _alg_px_scan(B, T, H, D, C):
+    return {"bound": "hbm", "bytes": B * T * H * D * D // 8, "what": "one f32 state per 64 tokens in and out: D*D/8 B per token-head"}
+
+
 KERNEL_ALGORITHMIC = {
     "simt_intra_bwd_kernel": _alg_simt_intra_bwd,
     "simt_score_kernel": _alg_simt_score,
+    "px_fwd_kernel": _alg_px_fwd,
+    "px_bwd_kernel": _alg_px_bwd,
+    "px_state_product": _alg_px_product,
+    "px_dstate_product": _alg_px_product,
+    "px_scan_kernel": _alg_px_scan,
     "tc_chunk_fwd_kernel": _alg_tc_fwd,
     "tc_chunk_bwd_kernel": _alg_tc_bwd,
     "tc_state_kernel": _alg_tc_state,

@@ -136,7 +136,7 @@ int simt_chunk_dstate_only(cudaStream_t st, int64_t B, int64_t T, int64_t H, int
 bool px_supported(int64_t D);
 size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf, int final_state);
 int px_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
-           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int final_state, int reverse, const char* label = "px_fwd_kernel");
+           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int final_state, int reverse);
 int px_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
            const void* v, const void* k, const void* q, const void* dhidden_final, const void* dout, int do_bf,
            void* dhidden_init, float* dg, void* dv, void* dk, void* dq, void* states, int have_states, void* ws, int reverse);

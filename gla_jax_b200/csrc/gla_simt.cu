@@ -308,8 +308,7 @@ int simt_chunk_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, 
   Dims d{B, T, H, D, C, T / C};
   const int64_t N = d.N, BH = B * H, E = B * T * H * D;
   if (px_supported(D) && !state_only)
-    // (launch profiles know the kernel of this family that forms the scores by one name)
-    return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, bf, saved ? saved : ws, saved != nullptr, 0, "simt_score_kernel");
+    return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, bf, saved ? saved : ws, saved != nullptr, 0);
   // every size limit of the launches below, before the first of them
   if (N > 65535 || BH > 65535 || BH * N > 65535) return GLA_ERR_TOO_LARGE;
   char* w = (char*)ws;

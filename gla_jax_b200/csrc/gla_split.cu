@@ -73,7 +73,6 @@ struct PxParams {
   float* eG;                    // (B H, N, D): exp of every chunk's total log decay
   void *out, *dq, *dk, *dv;
   float* dg;
-  const char* label;            // name of the forward chunk kernel in launch profiles
 };
 
 // ---- operands --------------------------------------------------------------------------------------------------
@@ -1033,7 +1032,7 @@ template <class C, typename TI, bool EX>
 int launch_fwd(cudaStream_t st, const PxParams& p, int64_t chunks) {
   static SmemAttrOnce attr;
   GLA_TRY(attr.ensure(px_fwd_kernel<C, TI, EX>, FwdLay<C, TI>::END));
-  ProfScope ps(p.label, st);
+  ProfScope ps("px_fwd_kernel", st);
   GLA_LAUNCHED(launch_overlapped(px_fwd_kernel<C, TI, EX>, dim3((unsigned)chunks), dim3(C::NT), FwdLay<C, TI>::END, st, p));
   return GLA_OK;
 }
@@ -1079,12 +1078,12 @@ size_t px_state_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf, int fi
   return f32b(B * H * (n + (final_state ? 1 : 0)) * D * D) + f32b(B * H * n * D);
 }
 int px_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init, const float* g,
-           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int final_state, int reverse, const char* label) {
+           const void* v, const void* k, const void* q, void* hidden_final, void* out, int out_bf, void* states, int final_state, int reverse) {
   const int64_t N = (T + px_rows(D, !bf) - 1) / px_rows(D, !bf);
   if (B * H * N > 2147483647LL || B * H * D * D / 512 > 2147483647LL) return GLA_ERR_TOO_LARGE;
   PxParams p{};
   p.B = B; p.T = T; p.H = H; p.N = N; p.NS = N + (final_state ? 1 : 0); p.trev = reverse; p.in_bf = bf; p.out_bf = out_bf;
-  p.g = g; p.v = v; p.k = k; p.q = q; p.out = out; p.label = label;
+  p.g = g; p.v = v; p.k = k; p.q = q; p.out = out;
   p.S = (float*)states;
   p.eG = (float*)((char*)states + f32b(B * H * p.NS * D * D));
   switch (D) {

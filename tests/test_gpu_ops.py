@@ -211,7 +211,7 @@ def test_auto_picks_tcgen05_for_readme_shape(cuda_device):
     import ctypes
     from gla_jax_b200 import chunk_gla, _lib
     lib = _lib.load()
-    for dtype, D, C, want in ((torch.bfloat16, 128, 128, b"tc_chunk_fwd_kernel"), (torch.float32, 64, 64, b"simt_score_kernel")):
+    for dtype, D, C, want in ((torch.bfloat16, 128, 128, b"tc_chunk_fwd_kernel"), (torch.float32, 64, 64, b"px_fwd_kernel")):
         h, g, v, k, q = (x.to(cuda_device) for x in O.make_inputs(1, 2 * C, 2, D, dtype, seed=3))
         lib.gla_profile_enable(1)
         chunk_gla(h, g, v, k, q, chunk_size=C)
