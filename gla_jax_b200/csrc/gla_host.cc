@@ -53,11 +53,11 @@ Tensor bytes_or(const Tensor& like, size_t n, size_t least) {
 }
 size_t size_of(const Tensor& t) { return t.defined() ? (size_t)t.numel() : 0; }
 Tensor f32(const Tensor& g) { return (g.scalar_type() == torch::kFloat32 ? g : g.to(torch::kFloat32)).contiguous(); }
-bool wants_grad(std::initializer_list<const Tensor*> ts) {
-  if (!torch::GradMode::is_enabled()) return false;
+bool wants_any(std::initializer_list<const Tensor*> ts) {
   for (const Tensor* t : ts) if (t->requires_grad()) return true;
   return false;
 }
+bool wants_grad(std::initializer_list<const Tensor*> ts) { return torch::GradMode::is_enabled() && wants_any(ts); }
 // There is no forward-mode formula: refuse a dual tensor (which need not require a gradient) instead of returning outputs
 // without a tangent.
 void no_forward_mode(const char* what, std::initializer_list<const Tensor*> ts) {
@@ -341,6 +341,7 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     ctx->set_materialize_grads(false);
     ctx->saved_data["i"] = std::vector<int64_t>{d.B, d.T, H, D, dt, chunk};
     ctx->saved_data["t"] = tau_inv;
+    if (!wants_any({&x0, &hidden0, &wq, &wk, &wv, &wgd, &wgu, &bgu})) ctx->mark_non_differentiable({r[1]});
     return {r[0], r[1]};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -355,42 +356,57 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     const auto heads = [&](const Tensor& t) { return t.view({d.B, d.T, d.H, d.D}); };
     const auto flat = [&](const Tensor& t) { return t.view({rows, inner}); };
     Tensor x2 = x.view({rows, x.size(2)});
+    const auto need = [&](size_t i) { return ctx->needs_input_grad(i); };
+    const bool need_gate = need(WGD) || need(WGU) || need(BGU) || need(X);      // of the gate projection's output
+    const bool need_core = need_gate || need(HID) || need(WQ) || need(WK) || need(WV);
     Tensor dout, dog, dnw, dwo;
     if (grads[0].defined()) {
       Tensor dy = grads[0].to(x.scalar_type()).contiguous().view({rows, wo.size(0)});
-      Tensor dy0 = at::mm(dy, wo);
-      dwo = at::mm(dy.t(), y0);
-      dout = torch::empty_like(out);
-      dog = torch::empty_like(og);
-      dnw = torch::empty_like(nw);
-      const size_t n = gla_layer_headnorm_gate_bwd_workspace_bytes(rows * d.H, d.D);
-      Tensor ws = bytes(x, n);
-      check(gla_layer_headnorm_gate_bwd(st, rows * d.H, d.D, d.dt, ptr(out), ptr(og), (const float*)ptr(nw), (const float*)ptr(rstd), ptr(dy0),
-                                        ptr(dout), ptr(dog), (float*)ptr(dnw), ptr(ws), n), "gla_layer_headnorm_gate_bwd");
+      if (need(WO)) dwo = at::mm(dy.t(), y0);
+      if (need_core || need(WOG) || need(NW)) {
+        Tensor dy0 = at::mm(dy, wo);
+        dout = torch::empty_like(out);
+        dog = torch::empty_like(og);
+        if (need(NW)) dnw = torch::empty_like(nw);
+        const size_t n = need(NW) ? gla_layer_headnorm_gate_bwd_workspace_bytes(rows * d.H, d.D) : 0;
+        Tensor ws = bytes(x, n);
+        check(gla_layer_headnorm_gate_bwd(st, rows * d.H, d.D, d.dt, ptr(out), ptr(og), (const float*)ptr(nw), (const float*)ptr(rstd), ptr(dy0),
+                                          ptr(dout), ptr(dog), (float*)ptr(dnw), ptr(ws), n), "gla_layer_headnorm_gate_bwd");
+      }
     }
-    variable_list c = chunk_backward(d, g, heads(v), heads(k), heads(q), s[19], grads[1], dout, a[5], GLA_IMPL_AUTO);
-    Tensor dz = torch::empty_like(z), dbgu = torch::empty({inner}, x.options());
-    {
-      const size_t n = gla_layer_gate_bwd_bias_workspace_bytes(rows, inner);
-      Tensor ws = bytes(x, n);
-      check(gla_layer_gate_bwd_bias(st, rows, inner, d.dt, ptr(z), (const float*)ptr(c[1]), (float)tau_inv, ptr(dz), ptr(dbgu), ptr(ws), n),
-            "gla_layer_gate_bwd_bias");
+    variable_list r(NIN + 6);
+    if (need_core) {
+      variable_list c = chunk_backward(d, g, heads(v), heads(k), heads(q), s[19], grads[1], dout, a[5], GLA_IMPL_AUTO);
+      const double ks = 1.0 / std::sqrt((double)d.D);
+      Tensor dv = flat(c[2]), dk = flat(c[3]), dq = flat(c[4]), dz1;
+      r[HID] = c[0];
+      if (need_gate) {
+        Tensor dz = torch::empty_like(z), dbgu = torch::empty({inner}, x.options());
+        const size_t n = gla_layer_gate_bwd_bias_workspace_bytes(rows, inner);
+        Tensor ws = bytes(x, n);
+        check(gla_layer_gate_bwd_bias(st, rows, inner, d.dt, ptr(z), (const float*)ptr(c[1]), (float)tau_inv, ptr(dz), ptr(dbgu), ptr(ws), n),
+              "gla_layer_gate_bwd_bias");
+        r[BGU] = dbgu;
+        if (need(WGU)) r[WGU] = at::mm(dz.t(), z1);
+        if (need(WGD) || need(X)) dz1 = at::mm(dz, wgu);
+        if (need(WGD)) r[WGD] = at::mm(dz1.t(), x2);
+      }
+      if (need(WQ)) r[WQ] = at::mm(dq.t(), x2);
+      if (need(WV)) r[WV] = at::mm(dv.t(), x2);
+      if (need(WK)) {
+        r[WK] = torch::empty(wk.sizes(), x.options());
+        at::addmm_out(r[WK], r[WK], dk.t(), x2, 0, ks);
+      }
+      if (need(X)) {
+        Tensor dx = at::mm(dq, wq);
+        dx.addmm_(dk, wk, 1, ks).addmm_(dv, wv).addmm_(dz1, wgd);
+        if (dog.defined()) dx.addmm_(dog, wog);
+        r[X] = dx.view(x.sizes());
+      }
     }
-    const double ks = 1.0 / std::sqrt((double)d.D);
-    Tensor dv = flat(c[2]), dk = flat(c[3]), dq = flat(c[4]);
-    Tensor dz1 = at::mm(dz, wgu), dwgu = at::mm(dz.t(), z1), dwgd = at::mm(dz1.t(), x2);
-    Tensor dwq = at::mm(dq.t(), x2), dwv = at::mm(dv.t(), x2), dwk = torch::empty_like(wk), dwog;
-    at::addmm_out(dwk, dwk, dk.t(), x2, 0, ks);
-    Tensor dx;
-    if (ctx->needs_input_grad(X)) {
-      dx = at::mm(dq, wq);
-      dx.addmm_(dk, wk, 1, ks).addmm_(dv, wv).addmm_(dz1, wgd);
-      if (dog.defined()) dx.addmm_(dog, wog);
-      dx = dx.view(x.sizes());
-    }
-    if (dog.defined()) dwog = at::mm(dog.t(), x2);
-    variable_list r{dx, c[0], dwq, dwk, dwv, dwgd, dwgu, dbgu, dwog, dwo, dnw};
-    r.resize(NIN + 6);
+    if (dog.defined() && need(WOG)) r[WOG] = at::mm(dog.t(), x2);
+    r[WO] = dwo;
+    r[NW] = dnw;
     return r;
   }
 };

@@ -56,3 +56,38 @@ def test_gate_backward_with_bias_gradient(cuda_device, rows, cols):
                                            dz.data_ptr(), db.data_ptr(), ws.data_ptr(), n), "gla_layer_gate_bwd_bias")
     ref = dg.double() * 0.0625 * torch.sigmoid(-z.double())
     assert O.rel_l2(ref.cpu(), dz.cpu().double()) < 1e-6 and O.rel_l2(ref.sum(0).cpu(), db.cpu().double()) < 1e-5
+
+
+@pytest.mark.parametrize("trained", [(), ("o_proj",), ("norm_weight",), ("out_gate",), ("gate_up",), ("gate_down",), ("q_proj", "k_proj"), ("v_proj",)])
+@pytest.mark.parametrize("inputs", [(), ("x",), ("hidden",)])
+def test_frozen_weights(cuda_device, trained, inputs):
+    """Whatever asks for a gradient gets what it gets when everything does; what does not costs no product."""
+    from gla_jax_b200 import GLALayer
+    from torch.profiler import profile, ProfilerActivity
+    if not trained and not inputs:
+        pytest.skip("nothing to differentiate")
+    torch.manual_seed(7)
+    layer = GLALayer(256, 2, chunk_size=128, device=cuda_device)
+    x, h = torch.randn(2, 128, 256, device=cuda_device).bfloat16(), torch.randn(2, 2, 128, 128, device=cuda_device).bfloat16()
+    dy, dh = torch.randn_like(x), torch.randn_like(h)
+
+    def run():
+        x_, h_ = x.clone().requires_grad_("x" in inputs or full), h.clone().requires_grad_("hidden" in inputs or full)
+        for n, p in layer.named_parameters():
+            p.requires_grad_(full or n.split(".")[0] in trained)
+        leaves = {n: p for n, p in [("x", x_), ("hidden", h_), *layer.named_parameters()] if p.requires_grad}
+        y, hf = layer(x_, h_)
+        assert hf.requires_grad == (full or bool(inputs) or trained[0] not in ("o_proj", "norm_weight", "out_gate"))
+        with profile(activities=[ProfilerActivity.CPU]) as prof:
+            g = torch.autograd.grad([y, hf] if hf.requires_grad else [y], list(leaves.values()), [dy, dh] if hf.requires_grad else [dy],
+                                    allow_unused=True)
+        products = sum(e.count for e in prof.key_averages() if e.key in ("aten::mm", "aten::addmm", "aten::addmm_"))
+        return dict(zip(leaves, g)), products
+
+    full = True
+    every, most = run()
+    full = False
+    some, fewer = run()
+    assert most == 14 and fewer <= most - 5
+    for n, g in some.items():
+        assert torch.equal(g, every[n]), n
