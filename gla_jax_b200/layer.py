@@ -141,12 +141,13 @@ class GLALayer(torch.nn.Module):
         self.norm_weight = torch.nn.Parameter(torch.ones(head_dim, device=device, dtype=torch.float32))
 
     def _plain(self) -> bool:
-        """Whether the submodules are as this class made them: plain linear layers that nothing hooks into, outside
-        autocast.  The whole layer then runs as one native autograd node; anything else goes module by module."""
+        """Whether the submodules are as this class made them: plain linear layers that nothing hooks into and that no
+        forward of their own was set on, outside autocast.  The whole layer then runs as one native autograd node; anything
+        else goes module by module."""
         if self.mode != "chunk" or torch.is_autocast_enabled() or _HOOKS._has_any_global_hook():
             return False
         for m in (self.q_proj, self.k_proj, self.v_proj, self.gate_down, self.gate_up, self.out_gate, self.o_proj):
-            if type(m) is not torch.nn.Linear or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or \
+            if type(m) is not torch.nn.Linear or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or \
                     m._backward_pre_hooks or (m.bias is None) != (m is not self.gate_up):
                 return False
         return True

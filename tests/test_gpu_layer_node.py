@@ -91,3 +91,14 @@ def test_frozen_weights(cuda_device, trained, inputs):
     assert most == 14 and fewer <= most - 5
     for n, g in some.items():
         assert torch.equal(g, every[n]), n
+
+
+def test_a_forward_set_on_a_submodule_is_called(cuda_device):
+    from gla_jax_b200 import GLALayer
+    layer = GLALayer(128, 1, chunk_size=128, device=cuda_device)
+    x = torch.randn(1, 128, 128, device=cuda_device).bfloat16()
+    plain = layer.o_proj.forward
+    layer.o_proj.forward = lambda t: 2 * plain(t)
+    y = layer(x)[0]
+    del layer.o_proj.forward
+    assert O.rel_l2((2 * layer(x)[0]).cpu(), y.cpu()) < 1e-2
