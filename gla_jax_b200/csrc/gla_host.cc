@@ -347,6 +347,7 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto a = ctx->saved_data["i"].toIntVector();
     const double tau_inv = ctx->saved_data["t"].toDouble();
+    torch::NoGradGuard no_grad;       // (under create_graph: no second derivative of parts of the layer)
     const variable_list s = ctx->get_saved_variables();
     const Tensor &x = s[0], &wq = s[1], &wk = s[2], &wv = s[3], &wgd = s[4], &wgu = s[5], &wog = s[6], &wo = s[7], &nw = s[8];
     const Tensor &q = s[9], &k = s[10], &v = s[11], &g = s[12], &og = s[13], &z1 = s[14], &z = s[15], &out = s[16], &rstd = s[17], &y0 = s[18];

@@ -102,3 +102,14 @@ def test_a_forward_set_on_a_submodule_is_called(cuda_device):
     y = layer(x)[0]
     del layer.o_proj.forward
     assert O.rel_l2((2 * layer(x)[0]).cpu(), y.cpu()) < 1e-2
+
+
+def test_gradients_under_create_graph(cuda_device):
+    """A gradient taken with create_graph=True is the same one (a second differentiation of the node is not offered)."""
+    from gla_jax_b200 import GLALayer
+    layer = GLALayer(128, 1, chunk_size=128, device=cuda_device)
+    x = torch.randn(1, 128, 128, device=cuda_device).bfloat16().requires_grad_(True)
+    leaves = [x, *layer.parameters()]
+    one = torch.autograd.grad(layer(x)[0].float().sum(), leaves)
+    two = torch.autograd.grad(layer(x)[0].float().sum(), leaves, create_graph=True)
+    assert all(torch.equal(a, b) and not b.requires_grad for a, b in zip(one, two))
