@@ -75,7 +75,7 @@ struct Dims { int64_t B, T, H, D; int dt; };
 bool dims_of(const Tensor& h, const Tensor& g, const Tensor& v, const Tensor& k, const Tensor& q, Dims& d) {
   if (!v.defined() || !here(v) || (v.dim() != 3 && v.dim() != 4)) return false;
   for (const Tensor* t : {&h, &g, &k, &q}) if (!t->defined() || t->device() != v.device()) return false;
-  if (g.sizes() != v.sizes() || k.sizes() != v.sizes() || q.sizes() != v.sizes() || !g.is_floating_point()) return false;
+  if (g.sizes() != v.sizes() || k.sizes() != v.sizes() || q.sizes() != v.sizes()) return false;
   d.dt = dt_of(v);
   if (d.dt < 0 || k.scalar_type() != v.scalar_type() || q.scalar_type() != v.scalar_type() || h.scalar_type() != v.scalar_type()) return false;
   const int b = v.dim() == 4;
@@ -264,7 +264,7 @@ std::optional<std::tuple<Tensor, Tensor>> chunk_gla_packed(const Tensor& h, cons
   if (!v.defined() || !here(v) || v.dim() != 3 || h.dim() != 4 || cu.dim() != 1 || cu.numel() != h.size(0) + 1) return std::nullopt;
   Dims d{1, v.size(0), v.size(1), v.size(2), dt_of(v)};
   for (const Tensor* t : {&h, &g, &k, &q}) if (t->device() != v.device()) return std::nullopt;
-  if (g.sizes() != v.sizes() || k.sizes() != v.sizes() || q.sizes() != v.sizes() || !g.is_floating_point()) return std::nullopt;
+  if (g.sizes() != v.sizes() || k.sizes() != v.sizes() || q.sizes() != v.sizes()) return std::nullopt;
   if (h.size(1) != d.H || h.size(2) != d.D || h.size(3) != d.D || d.dt < 0 || cu.scalar_type() != torch::kInt32) return std::nullopt;
   for (const Tensor* t : {&h, &k, &q}) if (t->scalar_type() != v.scalar_type()) return std::nullopt;
   if (chunk <= 0 || (chunk & (chunk - 1)) || chunk % 128) return std::nullopt;

@@ -53,7 +53,7 @@ def _refused(what, hidden, log_fgate, value, key, query):
     if not (key.dtype == query.dtype == hidden.dtype == value.dtype):
         raise TypeError("value, key, query and hidden must share one dtype")
     _stream(value.device)
-    raise ValueError(f"{what}: log_fgate must be a floating-point tensor and all arrays must be on {value.device}")
+    raise ValueError(f"{what}: all arrays must be on {value.device}")
 
 
 def _chunk_fwd_raw(hidden, g32, v, k, q, chunk, impl, need_grad):
@@ -178,7 +178,7 @@ def chunk_gla_packed(hidden_init, log_fgate, value, key, query, cu_seqlens, chun
     _stream(value.device)
     if int(chunk_size) % 128 or int(chunk_size) <= 0 or int(chunk_size) & (int(chunk_size) - 1):
         raise _lib.GlaError(f"chunk_gla_packed: unsupported configuration T={T} H={H} D={D} chunk={chunk_size} dtype={value.dtype}")
-    raise TypeError("chunk_gla_packed: bfloat16 arrays with a floating-point log_fgate, all on one device, are required")
+    raise TypeError("chunk_gla_packed: bfloat16 arrays, all on one device, are required")
 
 
 def decode_step(state, log_fgate, value, key, query, out_dtype=None):

@@ -35,3 +35,17 @@ def test_forward_mode_is_refused(cuda_device, name, grad):
             with pytest.raises(NotImplementedError), torch.no_grad():
                 fn(*x)
     fn(*args)
+
+
+@pytest.mark.parametrize("name", ["chunk", "recurrent", "packed"])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.bool, torch.float16, torch.float64])
+def test_gates_of_any_type(cuda_device, name, dtype):
+    """log_fgate is converted to float32, whatever it is."""
+    fn, args = _call(name, cuda_device)
+    g = -(torch.arange(args[1].numel(), device=cuda_device).view(args[1].shape) % 2)
+    args[1] = torch.zeros_like(g, dtype=dtype) if dtype == torch.bool else g.to(dtype)      # (a gate of +1 per token overflows)
+    want = fn(args[0], args[1].float(), *args[2:])
+    got = fn(*[a.requires_grad_(a.is_floating_point()) for a in args])
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    (got[1].float().sum() + got[0].float().sum()).backward()
+    assert all(a.grad is not None and a.grad.dtype == a.dtype for a in args if a.is_floating_point())
