@@ -160,6 +160,8 @@ def chunk_gla_packed(hidden_init, log_fgate, value, key, query, cu_seqlens, chun
     cu = cu_seqlens if torch.is_tensor(cu_seqlens) else torch.tensor(cu_seqlens, dtype=torch.int32)
     if cu.dtype != torch.int32:
         cu = cu.to(torch.int32)
+    if cu.is_cuda and (cu.dim() != 1 or cu.device != value.device):
+        cu = cu.to(value.device).reshape(-1)
     r = _lib.native().chunk_gla_packed(hidden_init, log_fgate, value, key, query, cu, int(chunk_size))
     if r is not None:
         return r

@@ -49,3 +49,12 @@ def test_gates_of_any_type(cuda_device, name, dtype):
     assert all(torch.equal(a, b) for a, b in zip(want, got))
     (got[1].float().sum() + got[0].float().sum()).backward()
     assert all(a.grad is not None and a.grad.dtype == a.dtype for a in args if a.is_floating_point())
+
+
+def test_packed_offsets_on_the_device_in_any_shape(cuda_device):
+    import gla_jax_b200 as gla
+    _, (h, *x) = _call("packed", cuda_device)
+    want = gla.chunk_gla_packed(h, *x, [0, 128, 256])
+    for cu in (torch.tensor([[0, 128, 256]], dtype=torch.int32), torch.tensor([[0], [128], [256]])):
+        got = gla.chunk_gla_packed(h, *x, cu.to(cuda_device))
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
