@@ -272,7 +272,13 @@ std::optional<std::tuple<Tensor, Tensor>> chunk_gla_packed(const Tensor& h, cons
   if (!c.is_cuda()) {
     const int32_t* p = c.data_ptr<int32_t>();
     if (p[0] != 0 || p[h.size(0)] != d.T) return std::nullopt;
-    for (int64_t s = 0; s < h.size(0); ++s) if (p[s + 1] <= p[s]) return std::nullopt;
+    int64_t padded = 0;          // sequences in whole chunks of 128, which `chunk` has to divide
+    for (int64_t s = 0; s < h.size(0); ++s) {
+      if (p[s + 1] <= p[s]) return std::nullopt;
+      padded += (p[s + 1] - p[s] + 127) / 128 * 128;
+    }
+    if (chunk > 256 || padded % chunk)
+      raise("chunk_gla_packed: unsupported configuration " + shape_text({1, padded, d.H, d.D, d.dt}, chunk, v));
   } else if (c.device() != v.device()) {
     return std::nullopt;
   }

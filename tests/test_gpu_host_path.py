@@ -58,3 +58,14 @@ def test_packed_offsets_on_the_device_in_any_shape(cuda_device):
     for cu in (torch.tensor([[0, 128, 256]], dtype=torch.int32), torch.tensor([[0], [128], [256]])):
         got = gla.chunk_gla_packed(h, *x, cu.to(cuda_device))
         assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+@pytest.mark.parametrize("cu,chunk", [([0, 100, 256], 256), ([0, 128, 256], 512), ([0, 1, 256], 1024)])
+def test_packed_chunk_sizes_that_do_not_divide_the_sequences(cuda_device, cu, chunk):
+    """Whole chunks of 128 per sequence that `chunk` does not divide, or a chunk beyond the largest, are refused."""
+    import gla_jax_b200 as gla
+    from gla_jax_b200 import _lib
+    _, x = _call("packed", cuda_device)
+    with pytest.raises(_lib.GlaError, match="unsupported configuration"):
+        gla.chunk_gla_packed(*x, cu, chunk)
+    assert torch.equal(gla.chunk_gla_packed(*x, [0, 130, 256], 128)[1], gla.chunk_gla_packed(*x, torch.tensor([0, 130, 256]))[1])
