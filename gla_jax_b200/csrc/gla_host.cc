@@ -227,7 +227,8 @@ struct PackedFn : torch::autograd::Function<PackedFn> {
     const Dims d{1, v0.size(0), v0.size(1), v0.size(2), (int)dt};
     Tensor h = h0.contiguous(), g = f32(g0), v = v0.contiguous(), k = k0.contiguous(), q = q0.contiguous();
     variable_list r = run(d, h.size(0), h, g, v, k, q, cu, chunk, true);
-    ctx->save_for_backward({g, v, k, q, r[2], cu});
+    // (a copy of offsets in host memory: the caller may fill its array with the next batch's before the backward)
+    ctx->save_for_backward({g, v, k, q, r[2], cu.is_cuda() ? cu : cu.clone()});
     ctx->set_materialize_grads(false);
     ctx->saved_data["d"] = std::vector<int64_t>{h.size(0), chunk, dt, !cu.is_cuda(), (int64_t)g0.scalar_type()};
     return {r[0], r[1]};

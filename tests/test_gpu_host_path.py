@@ -69,3 +69,18 @@ def test_packed_chunk_sizes_that_do_not_divide_the_sequences(cuda_device, cu, ch
     with pytest.raises(_lib.GlaError, match="unsupported configuration"):
         gla.chunk_gla_packed(*x, cu, chunk)
     assert torch.equal(gla.chunk_gla_packed(*x, [0, 130, 256], 128)[1], gla.chunk_gla_packed(*x, torch.tensor([0, 130, 256]))[1])
+
+
+def test_packed_offsets_may_change_before_the_backward(cuda_device):
+    import gla_jax_b200 as gla
+    _, x = _call("packed", cuda_device)
+    cu = torch.tensor([0, 100, 256], dtype=torch.int32)
+
+    def grads(change):
+        leaves = [a.detach().requires_grad_(True) for a in x]
+        out = gla.chunk_gla_packed(*leaves, cu)[1]
+        if change:
+            cu[1] = 7
+        return torch.autograd.grad(out.float().sum(), leaves)
+
+    assert all(torch.equal(a, b) for a, b in zip(grads(False), grads(True)))
