@@ -449,21 +449,34 @@ static int launch_rec_fwd_d(cudaStream_t st, int D, const RecParams& p) { REC_DI
 static int launch_rec_bwd_d(cudaStream_t st, int D, const RecParams& p) { REC_DISPATCH_D(launch_rec_bwd, st, D, p) }
 
 // The chunked form (gla_split.cu) serves sequences of more than a chunk or so; below that the walk over the tokens here
-// is one launch instead of three.  Its vector accesses need aligned arrays; the walk's need less.
-constexpr int64_t REC_CHUNKED_MIN_T = 48;
-static bool rec_chunked(int64_t T, int64_t D) { return px_supported(D) && T >= REC_CHUNKED_MIN_T; }
+// is fewer launches, and with few heads, which leave either form the device to itself, it is the faster one for longer.
+// Its vector accesses need aligned arrays; the walk's need less.  Measured, us on the device, walk | chunks:
+//   forward, 4 heads                       T = 32     48     64     96    128
+//     bf16, head size 64                   8 |  9  14|10  14|10  20| 9  25| 9
+//     bf16, head size 128                  10|18  16|18  15|19  20|18  25|18
+//     64 heads of 64, of 128               9|13, 27|21  15|13, 40|21  15|14, 39|21  21|17, 50|26  27|17, 62|26
+//   backward                               T = 48     64     96    128    160    192    224
+//     8 heads of 64 bf16, f32              21|21, 21|26  20|21, 20|26  25|21, 25|26  30|22, 31|26
+//     8 heads of 128 bf16, f32             22|41, 21|33  22|41, 20|34  27|41, 26|34  33|42, 32|34  40|41, 40|34  47|42, 45|34
+//     16 heads of 64, of 128 (bf16)        22|22, 38|41  22|22, 36|42  29|22, 49|44  37|22, 61|44
+constexpr int64_t REC_CHUNKED_MIN_T = 48, REC_MANY_HEADS = 16;
+static bool rec_chunked(int64_t BH, int64_t T, int64_t D, bool backward) {
+  if (!px_supported(D) || T < REC_CHUNKED_MIN_T) return false;
+  if (BH >= REC_MANY_HEADS) return true;
+  return backward ? T >= (D >= 128 ? 192 : 96) : D < 128 || T >= 96;
+}
 static bool rec_aligned(std::initializer_list<const void*> ps) {
   for (const void* p : ps) if (!aligned16(p)) return false;
   return true;
 }
 size_t recurrent_fwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf) {
-  return rec_chunked(T, D) ? px_state_bytes(B, T, H, D, bf, 0) : 0;
+  return rec_chunked(B * H, T, D, false) ? px_state_bytes(B, T, H, D, bf, 0) : 0;
 }
 
 int recurrent_fwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, int bf, const void* hidden_init,
                   const float* g, const void* v, const void* k, const void* q, void* hidden_final, void* out,
                   int out_bf, int reverse, void* ws, size_t ws_bytes) {
-  if (ws != nullptr && rec_chunked(T, D) && ws_bytes >= px_state_bytes(B, T, H, D, bf, 0) && rec_aligned({hidden_init, g, v, k, q, hidden_final, out, ws}))
+  if (ws != nullptr && rec_chunked(B * H, T, D, false) && ws_bytes >= px_state_bytes(B, T, H, D, bf, 0) && rec_aligned({hidden_init, g, v, k, q, hidden_final, out, ws}))
     return px_fwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, hidden_final, out, out_bf, ws, 0, reverse);
   RecParams p{};
   p.B = B; p.T = T; p.H = H; p.bf = bf; p.out_bf = out_bf;
@@ -477,7 +490,7 @@ static size_t rec_chunked_bwd_bytes(int64_t B, int64_t T, int64_t H, int64_t D, 
 }
 size_t recurrent_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int bf, int do_bf, int least) {
   const size_t n = 2 * align_up((size_t)B * T * H * D * 4, 256) + align_up((size_t)B * H * D * 4, 256);
-  const size_t px = rec_chunked(T, D) && !least ? rec_chunked_bwd_bytes(B, T, H, D, bf && do_bf) : 0;
+  const size_t px = rec_chunked(B * H, T, D, true) && !least ? rec_chunked_bwd_bytes(B, T, H, D, bf && do_bf) : 0;
   return px > n ? px : n;
 }
 
@@ -485,7 +498,7 @@ int recurrent_bwd(cudaStream_t st, int64_t B, int64_t T, int64_t H, int64_t D, i
                   const float* g, const void* v, const void* k, const void* q, const void* dhidden_final,
                   const void* dout, int do_bf, void* dhidden_init, float* dg, void* dv, void* dk, void* dq,
                   int reverse, void* ws, size_t ws_bytes) {
-  if (rec_chunked(T, D) && ws_bytes >= rec_chunked_bwd_bytes(B, T, H, D, bf && do_bf) &&
+  if (rec_chunked(B * H, T, D, true) && ws_bytes >= rec_chunked_bwd_bytes(B, T, H, D, bf && do_bf) &&
       rec_aligned({hidden_init, g, v, k, q, dhidden_final, dout, dhidden_init, dg, dv, dk, dq, ws}))
     return px_bwd(st, B, T, H, D, bf, hidden_init, g, v, k, q, dhidden_final, dout, do_bf, dhidden_init, dg, dv, dk, dq, ws, 0,
                   (char*)ws + px_state_bytes(B, T, H, D, bf && do_bf, 1), reverse);

@@ -122,10 +122,10 @@ def chunk_gla(hidden_init, log_fgate, value, key, query, chunk_size: int,
 def recurrent_gla(hidden_init, log_fgate, value, key, query, reverse: bool = False,
                   max_block_size: int = 64, num_warps: int = 1, num_stages: int = 1,
                   interpret: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
-    """Exact recurrence in float32 (reference: gla.py:405-439).  From 48 tokens on, at head sizes 32, 64 and 128, chunks run
-    side by side, with a float32 state per head and 64 tokens (32 where an array at head size 128 is float32) in memory
-    during the call: D * D / 16 (D * D / 8) bytes per token and head in the forward, twice that in the backward.  Where that
-    does not fit, and elsewhere, it walks the tokens and writes no states.
+    """Exact recurrence in float32 (reference: gla.py:405-439).  At head sizes 32, 64 and 128, from 48 tokens on (up to 192
+    where the batch has fewer than 16 heads), chunks run side by side, with a float32 state per head and 64 tokens (32 where
+    an array at head size 128 is float32) in memory during the call: D * D / 16 (D * D / 8) bytes per token and head in the
+    forward, twice that in the backward.  Where that does not fit, and elsewhere, it walks the tokens and writes no states.
     ``max_block_size``, ``num_warps``, ``num_stages``, ``interpret`` are accepted and ignored."""
     del max_block_size, num_warps, num_stages, interpret
     r = _lib.native().recurrent_gla(hidden_init, log_fgate, value, key, query, bool(reverse), False)

@@ -53,9 +53,23 @@ def test_gates_that_one_thread_holds(cuda_device, D):
     """Eight consecutive gates just inside and just beyond what the weights of one thread's rows may fall by together."""
     from gla_jax_b200 import recurrent_gla
     for total in (79.0, 81.0):
-        case = _case(1, 128, 1, D, torch.float32, 19, 5.0)
+        case = _case(1, 200, 1, D, torch.float32, 19, 5.0)
         case[1][0, 16:24, 0] = -total / 8
         _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"group {D, total}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,T,H,D,shift,reverse", [
+    (8, 48, 2, 64, 5.0, False), (4, 65, 4, 64, 5.0, True), (16, 49, 1, 32, 0.0, False), (4, 97, 4, 32, 5.0, True),
+    (8, 64, 2, 128, 5.0, False), (4, 65, 4, 128, 0.0, True), (8, 127, 2, 128, -4.0, False),     # enough heads for chunks
+    (1, 95, 2, 64, 5.0, False), (1, 96, 2, 64, 5.0, True), (1, 191, 2, 128, 5.0, True), (1, 192, 2, 128, 5.0, False),
+    (3, 64, 5, 128, 5.0, False), (4, 64, 4, 128, 5.0, True),                                    # both sides of the rules
+])
+def test_either_side_of_the_dispatch_by_heads(cuda_device, B, T, H, D, shift, reverse, dtype):
+    from gla_jax_b200 import recurrent_gla
+    case = _case(B, T, H, D, dtype, 27, shift)
+    _check(_oracle(*case, reverse=reverse), _run_gpu(recurrent_gla, cuda_device, *case, reverse=reverse), dtype,
+           f"recurrent {B, T, H, D, shift, reverse, dtype}", shift)
 
 
 @pytest.mark.parametrize("D", [32, 64, 128])
@@ -80,7 +94,7 @@ def test_chunks_on_both_sides_of_the_gate_limits(cuda_device, D):
 def test_resets_in_every_feature(cuda_device, D, gate, at):
     """Tokens whose gate resets the whole state, mild gates in between: what follows a reset keeps its precision."""
     from gla_jax_b200 import recurrent_gla
-    case = _case(1, 130, 2, D, torch.float32, 15, 5.0)
+    case = _case(1, 200, 2, D, torch.float32, 15, 5.0)
     case[1][:, list(at)] = gate
     _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"resets {D, gate, at}")
 
@@ -119,7 +133,7 @@ def _same_where_finite(ref, got, tol, what):
 def test_what_is_not_finite_stays_where_the_recurrence_has_it(cuda_device, D, which, bad, t, dtype):
     """One bad value in a token: earlier tokens (later ones for gradients that run backwards) do not see it."""
     from gla_jax_b200 import recurrent_gla
-    case = list(_case(1, 150, 2, D, dtype, 21, 5.0))
+    case = list(_case(1, 200, 2, D, dtype, 21, 5.0))
     case[{"v": 2, "k": 3, "q": 4, "do": 6}[which]][0, t, 1, 7] = bad
     leaves = [x.to(cuda_device).requires_grad_(True) for x in case[:5]]
     hf, out = recurrent_gla(*leaves)
@@ -135,7 +149,7 @@ def test_what_is_not_finite_stays_where_the_recurrence_has_it(cuda_device, D, wh
 def test_large_values_under_strong_decay(cuda_device, D):
     """Keys whose weighted values exceed float32 although no state or output does."""
     from gla_jax_b200 import recurrent_gla
-    case = list(_case(1, 128, 1, D, torch.float32, 23, 5.0))
+    case = list(_case(1, 192, 1, D, torch.float32, 23, 5.0))
     case[1][:] = -2.1
     case[3] = case[3] * 1e12
     _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"large keys {D}", shift=-2.0)
