@@ -815,14 +815,14 @@ def main():
     prob = AbiProblem(lib, dev, ins, C, impl)
     stream = prob.stream
 
-    rws_n = lib.gla_recurrent_bwd_workspace_bytes(B, T, H, D, dt)
-    rws = torch.empty(rws_n if args.op == "recurrent_gla" else 16, dtype=torch.uint8, device=dev)
+    fws_n, rws_n = lib.gla_recurrent_fwd_workspace_bytes(B, T, H, D, dt), lib.gla_recurrent_bwd_workspace_bytes(B, T, H, D, dt)
+    rws = torch.empty(max(fws_n, rws_n) if args.op == "recurrent_gla" else 16, dtype=torch.uint8, device=dev)
 
     def step_recurrent(i):
         (h, g, v, k, q), o = prob.sets[i % NSETS]
-        st = lib.gla_recurrent_fwd(prob.stream, B, T, H, D, dt, h.data_ptr(), g.data_ptr(), v.data_ptr(), k.data_ptr(),
-                                   q.data_ptr(), o["hf"].data_ptr(), o["out"].data_ptr(), dt, 0)
-        _lib.check(st, "gla_recurrent_fwd")
+        st = lib.gla_recurrent_fwd_ws(prob.stream, B, T, H, D, dt, h.data_ptr(), g.data_ptr(), v.data_ptr(), k.data_ptr(),
+                                      q.data_ptr(), o["hf"].data_ptr(), o["out"].data_ptr(), dt, 0, rws.data_ptr(), fws_n)
+        _lib.check(st, "gla_recurrent_fwd_ws")
         st = lib.gla_recurrent_bwd(prob.stream, B, T, H, D, dt, h.data_ptr(), g.data_ptr(), v.data_ptr(), k.data_ptr(),
                                    q.data_ptr(), o["dhf"].data_ptr(), o["dout"].data_ptr(), dt, o["dh"].data_ptr(),
                                    o["dg"].data_ptr(), o["dv"].data_ptr(), o["dk"].data_ptr(), o["dq"].data_ptr(), 0,

@@ -2133,7 +2133,8 @@ static int launch_sum_blocks(cudaStream_t st, const bf16* in, bf16* out, int64_t
   return GLA_OK;
 }
 
-// Blocks of the forward chunk kernel at head size 256, at most (the workspace holds a tile for each).
+// Blocks of the forward chunk kernel at head size 256, at most: one per SM of any device and one per pair of chunks.  The
+// workspace holds a tile for each, and the sizes must not depend on the device that is current.
 static int64_t wide_blocks_max(int64_t chunks) { return chunks / 2 < 256 ? chunks / 2 : 256; }
 // Sizes.  R = D / 128, HV = H R R virtual heads, N = T / 128 chunks whatever chunk size the caller named.
 // saved: S_prev bf16 (B HV, N, 128, 128) | Gc f32 (B HV, N, 128) | P bf16 (B HV, N, 128, 128)

@@ -45,8 +45,8 @@ struct OpLogAddExp {      // log(exp(a) + exp(b)), evaluated around the larger a
 // there; other blocks' loads cover a block's combine phase (prefetching the next tile in registers instead halves
 // the blocks: measured slower).  Longer axes are walked in steps of a cluster's rows with the carry in registers.
 // Measured, float32 (N, T, D) unless marked, us before (a ring of TMA tiles, one block per 128 columns) -> now, and the
-// time of the bytes at the copy rate: (24, 4096, 136) 70 -> 27, 16; (96, 4096, 128) 72 -> 72, 62; (512, 128, 768)
-// 75 -> 63, 62; (1, 16384, 96) 385 -> 12, 2; (2, 16384, 1024) 263 -> 64, 41; bf16 (9, 1342, 808) 37 -> 17, 6.
+// time of the bytes at the copy rate: (24, 4096, 136) 70 -> 27, 16; (96, 4096, 128) 72 -> 74, 62; (512, 128, 768)
+// 75 -> 66, 62; (1, 16384, 96) 385 -> 12, 2; (2, 16384, 1024) 263 -> 56, 41; bf16 (9, 1342, 808) 37 -> 16, 6.
 constexpr int SK_RL = 8;      // row lanes
 constexpr int SK_MAXCL = 16;  // blocks of a cluster, at most (above 8: opt-in)
 template <typename T, int VEC> __device__ __forceinline__ void sk_load(const T* p, float (&y)[VEC]) {
@@ -391,6 +391,7 @@ static int launch_cumsum_tma_op(cudaStream_t st, int64_t N, int64_t T, int64_t D
 // Blocks per cluster: the time of a grid is its waves over the SMs (four blocks each) times a block's steps; a step costs
 // the larger of its latency (about 2.5 us, 2 us more with the exchange) and of its SM's share of HBM.  The count that
 // minimises that by a clear margin is taken: 1 where rows and columns alone fill the device, up to 16 for a few rows with a long axis.
+// (148 SMs: latency and share were measured there, and the model holds for that number.)
 static int scan_cluster(int64_t items, int64_t T, int rows, double tile_bytes, double* us = nullptr) {
   constexpr int SMS = 148, PER_SM = 4;
   int best = 1;

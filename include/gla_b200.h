@@ -67,10 +67,11 @@ typedef enum gla_dtype {
 } gla_dtype;
 
 /* Which implementation gla_chunk_fwd/bwd use. AUTO picks the tcgen05 tensor-core kernels
- * when the shape has one (bf16, D = 128 or 256, chunk a multiple of 128) and the fp32 CUDA-core kernels otherwise. */
+ * when the shape has one (bf16, D = 128 or 256, chunk a multiple of 128) and the kernels of float32 precision otherwise. */
 typedef enum gla_chunk_impl {
   GLA_IMPL_AUTO = 0,
-  GLA_IMPL_FP32_SIMT = 1,     /* fp32 math on CUDA cores: every dtype, D <= 256, chunk 16..256 */
+  GLA_IMPL_FP32_SIMT = 1,     /* float32 precision: every dtype, D <= 256, chunk 16..256 (D = 32, 64, 128: operands split
+                                 into bf16 planes on the tensor cores; other sizes: CUDA cores) */
   GLA_IMPL_TCGEN05 = 2        /* bf16 operands, fp32 TMEM accumulators (sm_100a tensor cores) */
 } gla_chunk_impl;
 
@@ -307,7 +308,8 @@ GLA_API int gla_recurrent_bwd(void* stream, int64_t B, int64_t T, int64_t H, int
  * The forward writes the residuals the backward needs into `saved` (size
  * gla_chunk_saved_bytes): the state entering every chunk, the per-chunk total log decay
  * and the intra-chunk score matrices (the reference keeps `state` and `score_list`,
- * gla.py:542-549).  Pass saved = NULL for a forward that will not be differentiated.
+ * gla.py:542-549); float32 precision at D = 32, 64, 128 keeps states and decays only, of
+ * chunks of 64 tokens (32 for float32 at D = 128) whatever `chunk` is.  Pass saved = NULL for a forward that will not be differentiated.
  * ---------------------------------------------------------------------------------- */
 GLA_API size_t gla_chunk_saved_bytes(int64_t B, int64_t T, int64_t H, int64_t D, int64_t chunk,
                              int dtype, int impl);
