@@ -150,9 +150,9 @@ def test_large_values_under_strong_decay(cuda_device, D):
     """Keys whose weighted values exceed float32 although no state or output does."""
     from gla_jax_b200 import recurrent_gla
     case = list(_case(1, 192, 1, D, torch.float32, 23, 5.0))
-    case[1][:] = -2.1
-    case[3] = case[3] * 1e12
-    _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"large keys {D}", shift=-2.0)
+    case[1][:] = -1.5
+    case[3] = case[3] * 1e18
+    _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"large keys {D}", shift=-1.5)
 
 
 def test_naive_with_bf16_inputs_and_float32_cotangent(cuda_device):
@@ -215,3 +215,15 @@ def test_wait_for_workspace_is_not_needed(cuda_device):
                                             ws.data_ptr() if ws_n else None, ws_n), "gla_recurrent_fwd_ws")
         res.append((hf.cpu(), out.cpu()))
     assert O.rel_l2(res[0][0], res[1][0]) < 5e-6 and O.rel_l2(res[0][1], res[1][1]) < 5e-6
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("gate", [-1.4, -1.5, -2.1])
+def test_small_values_under_strong_decay(cuda_device, D, gate):
+    """Keys and output gradients far below one: the third plane of what the weights shrink must not vanish.  (At the limit of
+    100 a weight is exp(-50) = 2e-22, and 2^-126 2^16 / 2e-22 = 4e-12.)"""
+    from gla_jax_b200 import recurrent_gla
+    case = list(_case(1, 192, 2, D, torch.float32, 29, 5.0))
+    case[1][:] = gate * (1.0 + 0.02 * torch.rand(case[1].shape, generator=torch.Generator().manual_seed(3)))
+    case[3], case[5], case[6] = case[3] * 1e-6, case[5] * 1e-8, case[6] * 1e-8
+    _check(_oracle(*case), _run_gpu(recurrent_gla, cuda_device, *case), torch.float32, f"small values {D, gate}", shift=gate)
